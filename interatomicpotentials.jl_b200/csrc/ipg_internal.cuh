@@ -235,6 +235,8 @@ struct CellList {
   int32_t* d_cell_atoms = nullptr; // [n] atom ids in cell order (ascending inside a cell)
   int32_t* d_slot_of = nullptr;    // [n] slot of each atom
   double4* d_spos = nullptr;       // [n] positions in slot order (w = species as double)
+  bool want_rel = false;           // in: also build d_srel
+  float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell
 };
 
 // Builds the cell list for `radius` (prefix selects the scratch buffers used).
@@ -328,11 +330,16 @@ __device__ __forceinline__ void stencil_ranges(const ConfGrid& g, const int* c, 
     }
 }
 
+// The position along axis a as the cell grid sees it: wrapped into [0, L], or from the origin
+// of an open axis.
+__device__ __forceinline__ double cell_wrap(const ConfGrid& g, int a, double p) {
+  return isinf(g.L[a]) ? p - g.lo[a] : p - g.L[a] * floor(p / g.L[a]);
+}
 __device__ __forceinline__ void cell_coords(const ConfGrid& g, double x, double y, double z, int* c) {
   double p[3] = {x, y, z};
 #pragma unroll
   for (int a = 0; a < 3; a++) {
-    double w = isinf(g.L[a]) ? p[a] - g.lo[a] : p[a] - g.L[a] * floor(p[a] / g.L[a]);
+    const double w = cell_wrap(g, a, p[a]);
     int k = (int)floor(w / g.cs[a]);
     k = k < 0 ? 0 : k;
     k = k > g.nc[a] - 1 ? g.nc[a] - 1 : k;

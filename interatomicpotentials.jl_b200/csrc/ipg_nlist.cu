@@ -3,10 +3,12 @@
 //
 // Pipeline (all on the context's stream):
 //   k_extent       per-configuration min/max of open axes (only when an axis is open)
-//   k_cell_count   cell id per atom + histogram
+//   k_cell_count   cell id per atom + histogram; the histogram's old value is the atom's arrival
 //   scan           cell_start
-//   k_cell_fill    scatter atom ids into their cells
-//   k_cell_sort    sort each cell ascending (deterministic slot order), slot_of, spos
+//   k_cell_fill    atom ids into their cells, in arrival order
+//   k_cell_place   each atom's rank among its cell's ids (deterministic slot order): cell_atoms,
+//                  slot_of, spos
+//   k_cells_small  all of these in one block, for few atoms and cells
 // and, for a materialised list:
 //   k_pair_count / scan / k_pair_emit / k_pair_sort, optionally the transpose.
 // Membership is decided per candidate with the reference's own arithmetic
@@ -56,11 +58,12 @@ __global__ void k_extent(const double* __restrict__ pos, const ConfGrid* __restr
   }
 }
 
-__global__ void k_cell_count(int64_t n, const double* __restrict__ pos, const int32_t* __restrict__ species, int nsp,
-                             const ConfGrid* __restrict__ grid, int nconf, int32_t* __restrict__ conf,
-                             int32_t* __restrict__ cell_of, int64_t* __restrict__ count, int* status) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// The configuration and cell of atom i (out of range or non-finite inputs are reported and
+// placed in some cell).
+__device__ __forceinline__ int64_t cell_of_atom(int64_t i, const double* __restrict__ pos,
+                                                const int32_t* __restrict__ species, int nsp,
+                                                const ConfGrid* __restrict__ grid, int nconf, int* conf,
+                                                int* status) {
   // configuration by binary search over atom offsets
   int lo = 0, hi = nconf - 1;
   while (lo < hi) {
@@ -77,46 +80,159 @@ __global__ void k_cell_count(int64_t n, const double* __restrict__ pos, const in
   if (species && (species[i] < 0 || species[i] >= nsp)) dev_raise(status, IPG_ERR_SPECIES);
   int c[3];
   cell_coords(g, x, y, z, c);
-  int64_t cell = g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
-  conf[i] = lo;
-  cell_of[i] = (int32_t)cell;
-  atomicAdd((unsigned long long*)&count[cell], 1ull);
+  *conf = lo;
+  return g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
 }
 
-__global__ void k_cell_fill(int64_t n, const int32_t* __restrict__ cell_of, const int64_t* __restrict__ cell_start,
-                            int64_t* __restrict__ fill, int32_t* __restrict__ cell_atoms) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int64_t c = cell_of[i];
-  unsigned long long q = atomicAdd((unsigned long long*)&fill[c], 1ull);
-  cell_atoms[cell_start[c] + (int64_t)q] = (int32_t)i;
-}
-
-__global__ void k_cell_sort(int64_t ncells, const int64_t* __restrict__ cell_start, int32_t* __restrict__ cell_atoms) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  int64_t s = cell_start[c], e = cell_start[c + 1];
-  for (int64_t a = s + 1; a < e; a++) {
-    int32_t v = cell_atoms[a];
-    int64_t b = a - 1;
-    while (b >= s && cell_atoms[b] > v) {
-      cell_atoms[b + 1] = cell_atoms[b];
-      b--;
-    }
-    cell_atoms[b + 1] = v;
+// Atom i of cell c (of grid g) into slot s of the cell order; srel (optional) receives its
+// position relative to the cell's lower corner.
+__device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid& g, int64_t c,
+                                           const double* __restrict__ pos, const int32_t* __restrict__ species,
+                                           int nsp, int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
+                                           double4* __restrict__ spos, float4* __restrict__ srel) {
+  cell_atoms[s] = i;
+  slot_of[i] = (int32_t)s;
+  int sp = species ? species[i] : 0;
+  sp = sp < 0 ? 0 : (sp > nsp - 1 ? nsp - 1 : sp);  // bad ids were reported with the cell
+  const double x = pos[3 * (int64_t)i], y = pos[3 * (int64_t)i + 1], z = pos[3 * (int64_t)i + 2];
+  spos[s] = make_double4(x, y, z, (double)sp);
+  if (srel) {
+    const int k = (int)(c - g.cell_off), nxy = g.nc[0] * g.nc[1];
+    const int cz = k / nxy, cy = (k - cz * nxy) / g.nc[0], cx = k - cz * nxy - cy * g.nc[0];
+    srel[s] = make_float4((float)(cell_wrap(g, 0, x) - cx * g.cs[0]), (float)(cell_wrap(g, 1, y) - cy * g.cs[1]),
+                          (float)(cell_wrap(g, 2, z) - cz * g.cs[2]), 0.0f);
   }
 }
 
-__global__ void k_cell_gather(int64_t n, const int32_t* __restrict__ cell_atoms, const double* __restrict__ pos,
-                              const int32_t* __restrict__ species, int nsp, int32_t* __restrict__ slot_of,
-                              double4* __restrict__ spos) {
-  int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  int32_t i = cell_atoms[s];
-  slot_of[i] = (int32_t)s;
-  int sp = species ? species[i] : 0;
-  sp = sp < 0 ? 0 : (sp > nsp - 1 ? nsp - 1 : sp);  // bad ids were reported by k_cell_count
-  spos[s] = make_double4(pos[3 * (int64_t)i], pos[3 * (int64_t)i + 1], pos[3 * (int64_t)i + 2], (double)sp);
+__global__ void k_cell_count(int64_t n, const double* __restrict__ pos, const int32_t* __restrict__ species, int nsp,
+                             const ConfGrid* __restrict__ grid, int nconf, int32_t* __restrict__ conf,
+                             int32_t* __restrict__ cell_of, int32_t* __restrict__ arrival,
+                             int64_t* __restrict__ count, int* status) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int c;
+  const int64_t cell = cell_of_atom(i, pos, species, nsp, grid, nconf, &c, status);
+  conf[i] = c;
+  cell_of[i] = (int32_t)cell;
+  arrival[i] = (int32_t)atomicAdd((unsigned long long*)&count[cell], 1ull);
+}
+
+__global__ void k_cell_fill(int64_t n, const int32_t* __restrict__ cell_of, const int32_t* __restrict__ arrival,
+                            const int64_t* __restrict__ cell_start, int32_t* __restrict__ unsorted) {
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  unsorted[cell_start[cell_of[i]] + arrival[i]] = (int32_t)i;
+}
+
+// One thread per atom: its slot is its cell's start plus its rank among the cell's ids, so the
+// slots are ascending inside a cell whatever the arrival order.  A sort by one thread per cell
+// was a serial chain of loads: 58 us at 32,000 atoms (about 25 per cell), 13 us at 8,192 in cells of
+// 14; this kernel, which also writes what a separate gather wrote, takes 5.4 and 5.0 us.
+__global__ void __launch_bounds__(128) k_cell_place(int64_t n, const int32_t* __restrict__ unsorted,
+                                                    const int32_t* __restrict__ cell_of,
+                                                    const int64_t* __restrict__ cell_start,
+                                                    const ConfGrid* __restrict__ grid,
+                                                    const int32_t* __restrict__ conf,
+                                                    const double* __restrict__ pos,
+                                                    const int32_t* __restrict__ species, int nsp,
+                                                    int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
+                                                    double4* __restrict__ spos, float4* __restrict__ srel) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int32_t i = unsorted[t];
+  const int64_t c = cell_of[i], s0 = cell_start[c], s1 = cell_start[c + 1];
+  int64_t rank = 0;
+#pragma unroll 8
+  for (int64_t q = s0; q < s1; q++) rank += unsorted[q] < i;
+  place_atom(i, s0 + rank, grid[conf[i]], c, pos, species, nsp, cell_atoms, slot_of, spos, srel);
+}
+
+// The whole cell list in one block (count, scan, fill, rank, place through shared memory), for
+// at most SMALL_ATOMS atoms and SMALL_CELLS cells: there the five launches it replaces cost more
+// than one SM's work: 6.3 us against 39 us of kernels and two clears at 1,000 atoms.
+constexpr int SMALL_T = 1024;
+constexpr int SMALL_ATOMS = 4 * SMALL_T, SMALL_CELLS = 4 * SMALL_T;
+__global__ void __launch_bounds__(SMALL_T) k_cells_small(int n, int ncells, const double* __restrict__ pos,
+                                                         const int32_t* __restrict__ species, int nsp,
+                                                         const ConfGrid* __restrict__ grid, int nconf,
+                                                         int32_t* conf, int64_t* __restrict__ cell_start,
+                                                         int32_t* __restrict__ cell_atoms,
+                                                         int32_t* __restrict__ slot_of, double4* __restrict__ spos,
+                                                         float4* __restrict__ srel, int* status) {
+  __shared__ int start[SMALL_CELLS + 1];
+  __shared__ int32_t unsorted[SMALL_ATOMS];
+  __shared__ int wsum[SMALL_T / 32];
+  constexpr int PER = SMALL_ATOMS / SMALL_T, CPER = SMALL_CELLS / SMALL_T;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  for (int c = t; c <= ncells; c += SMALL_T) start[c] = 0;
+  __syncthreads();
+  int cell[PER], arr[PER];
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    const int i = q * SMALL_T + t;
+    cell[q] = 0;
+    arr[q] = 0;
+    if (i < n) {
+      int cf;
+      cell[q] = (int)cell_of_atom(i, pos, species, nsp, grid, nconf, &cf, status);
+      conf[i] = cf;
+      arr[q] = atomicAdd(&start[cell[q]], 1);
+    }
+  }
+  __syncthreads();
+  // exclusive scan of the counts, CPER consecutive cells per thread
+  int v[CPER], run = 0;
+#pragma unroll
+  for (int q = 0; q < CPER; q++) {
+    const int c = CPER * t + q;
+    v[q] = run;
+    run += c < ncells ? start[c] : 0;
+  }
+  int incl = run;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) wsum[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    int u = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, u, o);
+      if (lane >= o) u += x;
+    }
+    wsum[lane] = u;
+  }
+  __syncthreads();
+  const int excl = incl - run + (w > 0 ? wsum[w - 1] : 0);
+#pragma unroll
+  for (int q = 0; q < CPER; q++) {
+    const int c = CPER * t + q;
+    if (c < ncells) {
+      start[c] = excl + v[q];
+      cell_start[c] = excl + v[q];
+    }
+  }
+  if (t == 0) {
+    start[ncells] = n;
+    cell_start[ncells] = n;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER; q++)
+    if (q * SMALL_T + t < n) unsorted[start[cell[q]] + arr[q]] = q * SMALL_T + t;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    const int i = q * SMALL_T + t;
+    if (i >= n) continue;
+    const int s0 = start[cell[q]], s1 = start[cell[q] + 1];
+    int rank = 0;
+    for (int k = s0; k < s1; k++) rank += unsorted[k] < i;
+    place_atom(i, s0 + rank, grid[conf[i]], cell[q], pos, species, nsp, cell_atoms, slot_of, spos, srel);
+  }
 }
 
 // ---------------------------------------------------------------------------------
@@ -611,26 +727,33 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
   if (!ctx->capturing)  // a captured graph's grid table is uploaded before each replay
     CUDA_RET(ctx, cudaMemcpyAsync(cl.d_grid, cl.h_grid.data(), sizeof(ConfGrid) * nconf, cudaMemcpyHostToDevice,
                                   ctx->stream));
-  int64_t *count, *fill;
-  int32_t* cell_of;
+  int64_t* count;
+  int32_t *cell_of, *arrival, *unsorted;
   IPG_RET(scratch(ctx, (pre + "conf").c_str(), n, &cl.d_conf));
   IPG_RET(scratch(ctx, (pre + "cell_of").c_str(), n, &cell_of));
   IPG_RET(scratch(ctx, (pre + "cell_start").c_str(), cell_total + 1, &cl.d_cell_start));
-  IPG_RET(scratch(ctx, (pre + "cell_fill").c_str(), cell_total + 1, &fill));
+  IPG_RET(scratch(ctx, (pre + "cell_arrival").c_str(), n, &arrival));
+  IPG_RET(scratch(ctx, (pre + "cell_unsorted").c_str(), n, &unsorted));
   IPG_RET(scratch(ctx, (pre + "cell_atoms").c_str(), n, &cl.d_cell_atoms));
   IPG_RET(scratch(ctx, (pre + "slot_of").c_str(), n, &cl.d_slot_of));
   IPG_RET(scratch(ctx, (pre + "spos").c_str(), n, &cl.d_spos));
+  cl.d_srel = nullptr;
+  if (cl.want_rel) IPG_RET(scratch(ctx, (pre + "srel").c_str(), n, &cl.d_srel));
   count = cl.d_cell_start;
+  if (n > 0 && n <= SMALL_ATOMS && cell_total <= SMALL_CELLS) {
+    IPG_LAUNCH(ctx, k_cells_small, 1, SMALL_T, 0, (int)n, (int)cell_total, d_pos, d_species, nsp, cl.d_grid, nconf,
+               cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_slot_of, cl.d_spos, cl.d_srel,
+               ctx->d_status);
+    return IPG_OK;
+  }
   CUDA_RET(ctx, cudaMemsetAsync(count, 0, sizeof(int64_t) * (cell_total + 1), ctx->stream));
-  CUDA_RET(ctx, cudaMemsetAsync(fill, 0, sizeof(int64_t) * (cell_total + 1), ctx->stream));
   if (n == 0) return IPG_OK;
   IPG_LAUNCH(ctx, k_cell_count, nblk(n, 256), 256, 0, n, d_pos, d_species, nsp, cl.d_grid, nconf, cl.d_conf, cell_of,
-             count, ctx->d_status);
+             arrival, count, ctx->d_status);
   IPG_RET(ipg_scan_i64(ctx, count, cl.d_cell_start, cell_total + 1));
-  IPG_LAUNCH(ctx, k_cell_fill, nblk(n, 256), 256, 0, n, cell_of, cl.d_cell_start, fill, cl.d_cell_atoms);
-  IPG_LAUNCH(ctx, k_cell_sort, nblk(cell_total, 128), 128, 0, cell_total, cl.d_cell_start, cl.d_cell_atoms);
-  IPG_LAUNCH(ctx, k_cell_gather, nblk(n, 256), 256, 0, n, cl.d_cell_atoms, d_pos, d_species, nsp, cl.d_slot_of,
-             cl.d_spos);
+  IPG_LAUNCH(ctx, k_cell_fill, nblk(n, 256), 256, 0, n, cell_of, arrival, cl.d_cell_start, unsorted);
+  IPG_LAUNCH(ctx, k_cell_place, nblk(n, 128), 128, 0, n, unsorted, cell_of, cl.d_cell_start, cl.d_grid,
+             cl.d_conf, d_pos, d_species, nsp, cl.d_cell_atoms, cl.d_slot_of, cl.d_spos, cl.d_srel);
   return IPG_OK;
 }
 
