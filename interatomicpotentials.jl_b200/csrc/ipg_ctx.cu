@@ -419,7 +419,6 @@ int ipg_create(int device, ipg_ctx** out) {
   ctx->num_sms = prop.multiProcessorCount;
   if (const char* e = getenv("IPG_WALK_BY_ATOM")) ctx->walk_by_cell = e[0] != '1';
   if (const char* e = getenv("IPG_PAIR_FULL")) ctx->pair_full_stencil = e[0] == '1';
-  if (const char* e = getenv("IPG_PAIR_MINB")) ctx->pair_minb = std::max(3, std::min(5, atoi(e)));
   if (const char* e = getenv("IPG_WALK_SINGLE")) ctx->walk_single = e[0] != '0';
   if (const char* e = getenv("IPG_SIDE_STREAM")) ctx->side_enabled = e[0] != '0';
   if (const char* e = getenv("IPG_COPY_THREADS")) ctx->copy_threads = std::max(1, std::min(64, atoi(e)));

@@ -9,16 +9,21 @@
 // Half-stencil tiles (k_pair_half).  Like the reference's half list (nnlist.jl:39-40, m > n),
 // every unordered pair is evaluated once.  A work item is a (home cell A, offset k) pair,
 // one warp each: k = 0 is A itself (pairs of slots s < s'), k = 1..13 the 13 neighbor cells
-// of the forward half of the 27-cell stencil.  Lanes own the atoms of the target cell
-// (positions in registers), the warp walks the home cell's atoms one row at a time (a
-// broadcast load), the pairs within the largest cutoff are compacted into a per-warp hit
-// buffer in (row, lane) order, and every 32 hits are evaluated by the whole warp.  The force
-// of each hit goes to its two atoms' owner lanes by a broadcast loop in hit order, so every
-// sum runs in a fixed order (no atomics).  A warp writes its row sums and column sums to its
-// own slots of a partial-force buffer, [14 home offsets + 13 target offsets][slot][3], which
-// k_pair_gather sums per atom in a fixed order.  Each pair's force term is the reference's:
+// of the forward half of the 27-cell stencil.  Lanes own the atoms of the target cell, the warp
+// walks the home cell's atoms one row at a time, the pairs that can be within the largest cutoff
+// are queued in (row, lane) order, and every 32 of them are evaluated by the whole warp.  The
+// force of each pair goes to its two atoms' owner lanes, which add the pairs of a batch in queue
+// order, so every sum runs in a fixed order (no atomics).  A warp writes its row sums and column
+// sums to its own slots of a partial-force buffer, [14 home offsets + 13 target offsets][slot][3],
+// which k_pair_finish sums per atom in a fixed order.  Each pair's force term is the reference's:
 // with lo < hi the atom ids, r = get_displacement(x_lo, x_hi) (nnlist.jl:18-21), f = g(R) r,
 // F_lo += f, F_hi -= f; only the order of summation differs.
+//
+// Only one candidate in eight is within the cutoff, so the row walk tests them in 32 bits on
+// cell-relative positions: with at least 3 cells on every periodic axis a pair within the cutoff
+// is at the image that its two cells define, so no minimum image is needed, and the test's
+// threshold covers the rounding of the 32-bit coordinates (pair_prefilter_threshold).  It only
+// proposes; the reference's own test and all arithmetic of the pairs it proposes are 64-bit.
 //
 // The half stencil visits each pair of neighboring cells once only when every periodic axis
 // has at least 3 cells; otherwise the full-stencil walk (ipg_pair.cuh) runs instead.
@@ -84,97 +89,91 @@ __device__ __forceinline__ int shift_axis(int c, int d, int nc, bool periodic) {
   return (t < 0 || t >= nc) ? -1 : t;
 }
 
-struct HalfHit {
-  double r0, r1, r2, dist;
-  int at;  // row (bits 0-7) and lane (bits 8-15) within the tile
-  int sp;  // species of the row atom (bits 0-7) and of the lane atom (bits 8-15)
+struct PairBox {
+  double L[3];  // box lengths, by value: the constant bank instead of registers
 };
 
-// Per-warp staging of half_eval: a force per row and per column of the tile.
-struct HalfStage {
-  double row[32][3];
-  double col[32][3];
+// Per-warp shared memory of the half-stencil walk.
+struct HalfWarp {
+  double f[3][32];     // the forces of a batch
+  float4 home[32];     // the rows' cell-relative positions
+  unsigned rows[32];   // per row: the pairs of the batch that belong to it
+  unsigned cols[32];   // per column, likewise
+  uint16_t q[96];      // queued pairs, row | column << 8
 };
 
-// Evaluates the first nh hits (one per lane) and hands each hit's force to its row owner
-// (fa += f) and its column owner (ft -= f).  Rows: the hits of a row are contiguous (they are
-// appended in row order), so a segmented scan over the lanes (a fixed tree) leaves each row's
-// total at its last hit, which stages it for the row's owner lane.  Columns: a row's hits have
-// distinct columns, so the rows of the batch are handed over one after another (row order),
-// each hit staging its force for its column's owner lane.  E and W accumulate lane-wise.
-__device__ __forceinline__ void half_eval(const PairTerms& TT, const HalfHit* __restrict__ hb, int nh, int lane,
-                                          HalfStage& st, double* acc, double* fa, double* ft) {
+// Evaluates the first nh queued pairs (one per lane) and hands each pair's force to its row
+// owner (fa += f) and its column owner (ft -= f).  E and W accumulate lane-wise.
+//
+// The hand-off: forces go to shared memory, each owner gets the bit mask of its pairs (a row's
+// pairs are contiguous in the queue; a column's come from a match over the lanes) and adds them
+// in queue order: about three steps for the columns and seven for the rows of a batch, where
+// handing the columns over one row at a time took ten, each between two warp barriers.
+__device__ __forceinline__ void half_eval(const PairTerms& TT, const PairBox& B, int nh, int lane,
+                                          int row0, int col0, const int32_t* __restrict__ cell_atoms,
+                                          const double4* __restrict__ spos, HalfWarp& st, double* acc, double* fa,
+                                          double* ft) {
   constexpr unsigned FULL = 0xffffffffu;
   double fx = 0.0, fy = 0.0, fz = 0.0;
-  int row = 64 + lane, col = 0;  // idle lanes: rows that match no hit
+  int row = 64, col = 32 + lane;  // idle lanes: no row, a column of their own
   const bool act = lane < nh;
   if (act) {
-    const HalfHit h = hb[lane];
-    const double R = sqrt(h.r0 * h.r0 + h.r1 * h.r1 + h.r2 * h.r2);
+    const int e = st.q[lane];
+    row = e & 0xff;
+    col = e >> 8;
+    const double4 xa = spos[row0 + row], xt = spos[col0 + col];
+    const int32_t ia = cell_atoms[row0 + row], it = cell_atoms[col0 + col];
+    const double d2 = sumsq3_dev(pe_axis_dev(B.L[0], xa.x, xt.x), pe_axis_dev(B.L[1], xa.y, xt.y),
+                                 pe_axis_dev(B.L[2], xa.z, xt.z));
+    // r = get_displacement(x_lo, x_hi) seen from the row atom
+    const bool lo = ia < it;
+    const double sg = lo ? 1.0 : -1.0;
+    const double r0 = sg * disp_axis_dev(B.L[0], lo ? xa.x : xt.x, lo ? xt.x : xa.x);
+    const double r1 = sg * disp_axis_dev(B.L[1], lo ? xa.y : xt.y, lo ? xt.y : xa.y);
+    const double r2 = sg * disp_axis_dev(B.L[2], lo ? xa.z : xt.z, lo ? xt.z : xa.z);
     double V, g;
-    pair_terms_sum(TT, R, h.dist, h.sp & 0xff, (h.sp >> 8) & 0xff, V, g);
-    fx = g * h.r0;
-    fy = g * h.r1;
-    fz = g * h.r2;
+    pair_terms_sum(TT, r0 * r0 + r1 * r1 + r2 * r2, d2, (int)xa.w, (int)xt.w, V, g);
+    fx = g * r0;
+    fy = g * r1;
+    fz = g * r2;
     acc[0] += V;
     // empirical_potential.jl:63-64: r * f' -> [xx, yy, zz, zy, zx, yx]
-    acc[1] += h.r0 * fx;
-    acc[2] += h.r1 * fy;
-    acc[3] += h.r2 * fz;
-    acc[4] += h.r2 * fy;
-    acc[5] += h.r2 * fx;
-    acc[6] += h.r1 * fx;
-    row = h.at & 0xff;
-    col = (h.at >> 8) & 0xff;
+    acc[1] += r0 * fx;
+    acc[2] += r1 * fy;
+    acc[3] += r2 * fz;
+    acc[4] += r2 * fy;
+    acc[5] += r2 * fx;
+    acc[6] += r1 * fx;
   }
-  // rows: segmented inclusive scan over the lanes
-  double sx = fx, sy = fy, sz = fz;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const double ox = __shfl_up_sync(FULL, sx, off), oy = __shfl_up_sync(FULL, sy, off),
-                 oz = __shfl_up_sync(FULL, sz, off);
-    const int orow = __shfl_up_sync(FULL, row, off);
-    if (lane >= off && orow == row) {
-      sx += ox;
-      sy += oy;
-      sz += oz;
-    }
-  }
-  const int nrow = __shfl_down_sync(FULL, row, 1);
-  const bool last = act && (lane == nh - 1 || nrow != row);
-  if (last) {
-    st.row[row][0] = sx;
-    st.row[row][1] = sy;
-    st.row[row][2] = sz;
-  }
-  const unsigned rows = __reduce_or_sync(FULL, last ? 1u << row : 0u);
+  st.f[0][lane] = fx;
+  st.f[1][lane] = fy;
+  st.f[2][lane] = fz;
+  st.rows[lane] = 0u;
+  st.cols[lane] = 0u;
+  const int prev = __shfl_up_sync(FULL, row, 1);
+  const unsigned heads = __ballot_sync(FULL, lane == 0 || row != prev);  // first pair of each row, first idle lane
+  const unsigned same = __match_any_sync(FULL, col);
   __syncwarp();
-  if ((rows >> lane) & 1u) {
-    fa[0] += st.row[lane][0];
-    fa[1] += st.row[lane][1];
-    fa[2] += st.row[lane][2];
+  if (act && ((heads >> lane) & 1u)) {
+    const unsigned above = heads & (0xfffffffeu << lane);  // later heads
+    const int end = above ? __ffs(above) - 1 : 32;         // idle lanes start a run of their own
+    st.rows[row] = (end == 32 ? FULL : (1u << end) - 1u) & (FULL << lane);
   }
-  // columns: one row of the batch at a time
-  unsigned pend = __ballot_sync(FULL, act);
-  while (pend) {
-    const int r = __shfl_sync(FULL, row, __ffs(pend) - 1);
-    const bool in = act && row == r;
-    const unsigned seg = __ballot_sync(FULL, in);
-    if (in) {
-      st.col[col][0] = fx;
-      st.col[col][1] = fy;
-      st.col[col][2] = fz;
-    }
-    const unsigned cols = __reduce_or_sync(FULL, in ? 1u << col : 0u);
-    __syncwarp();
-    if ((cols >> lane) & 1u) {
-      ft[0] -= st.col[lane][0];
-      ft[1] -= st.col[lane][1];
-      ft[2] -= st.col[lane][2];
-    }
-    __syncwarp();
-    pend &= ~seg;
+  if (act && (same & ((1u << lane) - 1u)) == 0u) st.cols[col] = same;
+  __syncwarp();
+  for (unsigned m = st.rows[lane]; m; m &= m - 1u) {
+    const int b = __ffs(m) - 1;
+    fa[0] += st.f[0][b];
+    fa[1] += st.f[1][b];
+    fa[2] += st.f[2][b];
   }
+  for (unsigned m = st.cols[lane]; m; m &= m - 1u) {
+    const int b = __ffs(m) - 1;
+    ft[0] -= st.f[0][b];
+    ft[1] -= st.f[1][b];
+    ft[2] -= st.f[2][b];
+  }
+  __syncwarp();
 }
 
 __device__ __forceinline__ void pbuf_put(double* __restrict__ P, int64_t n, int slot_kind, int64_t s, const double* f,
@@ -191,28 +190,34 @@ __device__ __forceinline__ void pbuf_put(double* __restrict__ P, int64_t n, int 
   }
 }
 
-// MINB: resident blocks per SM the register allocation is bounded for (3: 168 registers, the
-// default; 4: 128; 5: 96, with spills; 36.0 / 36.6 / 66 ms at 4.1 M atoms, five terms).
-template <int MINB>
-__global__ void __launch_bounds__(PAIR_T, MINB) k_pair_half(const __grid_constant__ PairTerms TT, int64_t n,
-                                                         const ConfGrid* __restrict__ grid, int64_t ncells,
-                                                         const int64_t* __restrict__ cell_start,
-                                                         const int32_t* __restrict__ cell_atoms,
-                                                         const double4* __restrict__ spos, double* __restrict__ P,
-                                                         double* __restrict__ partial) {
-  __shared__ HalfHit hits[PAIR_WARPS][64];
-  __shared__ HalfStage stage[PAIR_WARPS];
+// Bound by FP64 issue and latency of the term code.  Against full 64-bit tests of every candidate,
+// rows loaded one by one and the old hand-off: 4.1 M atoms, five terms 35.8 -> 17.7 ms a call;
+// 32,000 atoms 540 -> 309 us; 1,000 atoms, one term 92 -> 70 us.
+// PAIR_MINB: resident blocks per SM the register allocation is bounded for; 3, 4, 5, 6 (164, 128,
+// 96, 80 registers) took 21.2, 17.7, 17.9, 17.5 ms at 4.1 M atoms and 364, 309, 314, 322 us at
+// 32,000.
+constexpr int PAIR_MINB = 4;
+__global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_constant__ PairTerms TT,
+                                                                 const __grid_constant__ PairBox B, int64_t n,
+                                                                 const ConfGrid* __restrict__ grid, int64_t ncells,
+                                                                 const int64_t* __restrict__ cell_start,
+                                                                 const int32_t* __restrict__ cell_atoms,
+                                                                 const double4* __restrict__ spos,
+                                                                 const float4* __restrict__ srel, float thr,
+                                                                 double* __restrict__ P,
+                                                                 double* __restrict__ partial) {
+  __shared__ HalfWarp stage[PAIR_WARPS];
   __shared__ double red[PAIR_WARPS][7];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  HalfWarp& st = stage[w];
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};  // E, W[6] of every item this warp takes
-  const double L0 = grid[0].L[0], L1 = grid[0].L[1], L2 = grid[0].L[2];
   // grid-stride over the items (a fixed assignment, so E and W sum in a fixed order); the
   // block's warps meet at a barrier only once, at the end
   const int64_t nitems = ncells * HALF_OFFSETS;
   const int64_t wstride = (int64_t)gridDim.x * PAIR_WARPS;
   for (int64_t item = (int64_t)blockIdx.x * PAIR_WARPS + w; item < nitems; item += wstride) {  // warp-uniform
     const ConfGrid& g = grid[0];
-    // cells number below 2^31 (ipg_build_cells): 32-bit index arithmetic
+    // cells and atoms number below 2^31: 32-bit index arithmetic
     const int A = (int)(item / HALF_OFFSETS);
     const int k = (int)(item - (int64_t)A * HALF_OFFSETS);
     const int nxy = g.nc[0] * g.nc[1];
@@ -220,12 +225,15 @@ __global__ void __launch_bounds__(PAIR_T, MINB) k_pair_half(const __grid_constan
     const int cy = rem / g.nc[0], cx = rem - cy * g.nc[0];
     int dx, dy, dz;
     half_offset(k, dx, dy, dz);
-    const int tx = shift_axis(cx, dx, g.nc[0], !isinf(L0));
-    const int ty = shift_axis(cy, dy, g.nc[1], !isinf(L1));
-    const int tz = shift_axis(cz, dz, g.nc[2], !isinf(L2));
+    const int tx = shift_axis(cx, dx, g.nc[0], !isinf(B.L[0]));
+    const int ty = shift_axis(cy, dy, g.nc[1], !isinf(B.L[1]));
+    const int tz = shift_axis(cz, dz, g.nc[2], !isinf(B.L[2]));
     if (tx < 0 || ty < 0 || tz < 0) continue;
-    const int64_t T = ((int64_t)tz * g.nc[1] + ty) * g.nc[0] + tx;
-    const int64_t a0 = cell_start[A], a1 = cell_start[A + 1], t0 = cell_start[T], t1 = cell_start[T + 1];
+    const int T = (tz * g.nc[1] + ty) * g.nc[0] + tx;
+    const int a0 = (int)cell_start[A], a1 = (int)cell_start[A + 1], t0 = (int)cell_start[T],
+              t1 = (int)cell_start[T + 1];
+    // the target cell's corner relative to the home cell's, at the image these two cells define
+    const float sx = (float)(dx * g.cs[0]), sy = (float)(dy * g.cs[1]), sz = (float)(dz * g.cs[2]);
     const int home_kind = k, tgt_kind = k == 0 ? 0 : HALF_OFFSETS - 1 + k;
     // cells of at most 32 atoms are one tile and its sums are stored; larger cells take
     // several tiles, whose sums accumulate into zeroed slots, as do the row and column sums
@@ -234,69 +242,55 @@ __global__ void __launch_bounds__(PAIR_T, MINB) k_pair_half(const __grid_constan
     const bool multi = (a1 - a0 > 32) || (t1 - t0 > 32) || k == 0;
     if (multi) {
       const double z[3] = {0.0, 0.0, 0.0};
-      for (int64_t s = a0 + lane; s < a1; s += 32) pbuf_put(P, n, home_kind, s, z, false);
+      for (int s = a0 + lane; s < a1; s += 32) pbuf_put(P, n, home_kind, s, z, false);
       if (k != 0)
-        for (int64_t s = t0 + lane; s < t1; s += 32) pbuf_put(P, n, tgt_kind, s, z, false);
+        for (int s = t0 + lane; s < t1; s += 32) pbuf_put(P, n, tgt_kind, s, z, false);
       __syncwarp();
     }
     if (a0 == a1 && k != 0)  // no home atoms: the target atoms still get their (zero) slot
-      for (int64_t s = t0 + lane; s < t1; s += 32) {
+      for (int s = t0 + lane; s < t1; s += 32) {
         const double z[3] = {0.0, 0.0, 0.0};
         pbuf_put(P, n, tgt_kind, s, z, false);
       }
-    HalfHit* hb = hits[w];
     const unsigned lt = (1u << lane) - 1u;
-    const double rmax = TT.rcut_max;
-    for (int64_t rc = a0; rc < a1; rc += 32) {
-      const int ra = (int)(a1 - rc < 32 ? a1 - rc : 32);
+    for (int rc = a0; rc < a1; rc += 32) {
+      const int ra = a1 - rc < 32 ? a1 - rc : 32;
       double fa[3] = {0.0, 0.0, 0.0};  // row sums of row rc + lane
-      for (int64_t cc = t0; cc < t1; cc += 32) {
-        const int64_t ts = cc + lane;
+      __syncwarp();
+      if (lane < ra) st.home[lane] = srel[rc + lane];
+      for (int cc = t0; cc < t1; cc += 32) {
+        const int ts = cc + lane;
         const bool tv = ts < t1;
-        const double4 xt = tv ? spos[ts] : make_double4(0.0, 0.0, 0.0, 0.0);
-        const int32_t it = tv ? cell_atoms[ts] : -1;
+        const float4 b = tv ? srel[ts] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float bx = b.x + sx, by = b.y + sy, bz = b.z + sz;
+        // a cell with itself: the rows before the lane's own slot; another cell: every row
+        const int lim = !tv ? 0 : (k == 0 && ts - rc < ra ? ts - rc : ra);
         double ft[3] = {0.0, 0.0, 0.0};  // column sums of lane atom ts
         int nh = 0;
-        for (int q = 0; q <= ra; q++) {  // q == ra: evaluate what is left
+        __syncwarp();
+        for (int q = 0; q < ra + 2; q += 2) {  // the last step evaluates what is left
           if (q < ra) {
-            const int64_t as = rc + q;
-            const double4 xa = spos[as];
-            const int32_t ia = cell_atoms[as];
-            bool ok = false;
-            HalfHit h;
-            if (tv && (k != 0 || ts > as)) {
-              const double d2 = sumsq3_dev(pe_axis_dev(L0, xa.x, xt.x), pe_axis_dev(L1, xa.y, xt.y),
-                                           pe_axis_dev(L2, xa.z, xt.z));
-              if (d2 <= TT.rmax2_hi) {
-                const double dist = sqrt(d2);
-                if (dist <= rmax) {
-                  ok = true;
-                  h.dist = dist;
-                  h.at = q | (lane << 8);
-                  h.sp = (int)xa.w | ((int)xt.w << 8);
-                  if (ia < it) {  // r = get_displacement(x_lo, x_hi) with the row atom lo
-                    h.r0 = disp_axis_dev(L0, xa.x, xt.x);
-                    h.r1 = disp_axis_dev(L1, xa.y, xt.y);
-                    h.r2 = disp_axis_dev(L2, xa.z, xt.z);
-                  } else {  // the lane atom is lo: r = -get_displacement(x_lane, x_row)
-                    h.r0 = -disp_axis_dev(L0, xt.x, xa.x);
-                    h.r1 = -disp_axis_dev(L1, xt.y, xa.y);
-                    h.r2 = -disp_axis_dev(L2, xt.z, xa.z);
-                  }
-                }
-              }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+              const float4 a = st.home[(q + u) & 31];  // past the last row: any value, lim excludes it
+              const float x = a.x - bx, y = a.y - by, z = a.z - bz;
+              const bool ok = fmaf(x, x, fmaf(y, y, z * z)) <= thr && q + u < lim;
+              const unsigned bal = __ballot_sync(0xffffffffu, ok);
+              if (ok) st.q[nh + __popc(bal & lt)] = (uint16_t)((q + u) | (lane << 8));
+              nh += __popc(bal);
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, ok);
-            if (ok) hb[nh + __popc(bal & lt)] = h;
-            nh += __popc(bal);
             __syncwarp();
           }
           // one call site of the term code: full batches, then the rest after the last row
-          while (nh >= 32 || (q == ra && nh > 0)) {
+          while (nh >= 32 || (q >= ra && nh > 0)) {
             const int m = nh < 32 ? nh : 32;
-            half_eval(TT, hb, m, lane, stage[w], acc, fa, ft);
+            half_eval(TT, B, m, lane, rc, cc, cell_atoms, spos, st, acc, fa, ft);
+            uint16_t e0 = 0, e1 = 0;  // the rest of the queue (fewer than 64 pairs) moves up
+            if (lane < nh - m) e0 = st.q[m + lane];
+            if (lane + 32 < nh - m) e1 = st.q[m + lane + 32];
             __syncwarp();
-            if (lane < nh - m) hb[lane] = hb[m + lane];
+            if (lane < nh - m) st.q[lane] = e0;
+            if (lane + 32 < nh - m) st.q[lane + 32] = e1;
             nh -= m;
             __syncwarp();
           }
@@ -321,59 +315,91 @@ __global__ void __launch_bounds__(PAIR_T, MINB) k_pair_half(const __grid_constan
   }
 }
 
+// Squared threshold of the 32-bit test: no pair within rcut fails it.  Each coordinate of each
+// atom is at most about one cell edge (cs) and rounded to 32 bits, as are the shift between the
+// cells (at most cs) and the difference (at most 2 cs): at most 6 * 2^-24 cs per axis, less than
+// 7e-7 cs in distance; the squares and their sum add a relative 3 * 2^-24.
+float pair_prefilter_threshold(const ConfGrid& g, double rcut) {
+  const double cs = std::max(g.cs[0], std::max(g.cs[1], g.cs[2]));
+  const double r = rcut + 2e-6 * cs;
+  const double t = r * r * (1.0 + 1e-6);
+  return t < 1e30 ? (float)t : 1e30f;
+}
+
+// E and W6 from the per-block partials of nblocks blocks in a fixed order (one block of
+// FINISH_T threads); component 0 goes to E, 1..6 to W6 (either may be null).
+constexpr int FINISH_T = 256;
+__device__ __forceinline__ void reduce_partials(int64_t nblocks, const double* __restrict__ partial,
+                                                double* __restrict__ E, double* __restrict__ W6) {
+  __shared__ double sm[FINISH_T / 32][7];
+  double v[7] = {0, 0, 0, 0, 0, 0, 0};
+  for (int64_t b = threadIdx.x; b < nblocks; b += FINISH_T)
+#pragma unroll
+    for (int k = 0; k < 7; k++) v[k] += partial[b * 7 + k];
+#pragma unroll
+  for (int k = 0; k < 7; k++) {
+    v[k] = warp_sum(v[k]);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5][k] = v[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    double s = 0.0;
+    for (int q = 0; q < FINISH_T / 32; q++) s += sm[q][threadIdx.x];
+    if (threadIdx.x == 0 && E) *E = s;
+    if (threadIdx.x > 0 && W6) W6[threadIdx.x - 1] = s;
+  }
+}
+
+__global__ void __launch_bounds__(FINISH_T) k_reduce_partials(int64_t nblocks, const double* __restrict__ partial,
+                                                              double* __restrict__ E, double* __restrict__ W6) {
+  reduce_partials(nblocks, partial, E, W6);
+}
+
 // F of every atom: its 14 partial sums as a home atom (offsets k whose target cell exists)
 // and its 13 as a target (offsets k whose home cell, its own cell - offset k, exists), in
-// that fixed order.
-__global__ void k_pair_gather(int64_t n, const ConfGrid* __restrict__ grid, const int32_t* __restrict__ cell_atoms,
-                              const double4* __restrict__ spos, const double* __restrict__ P,
-                              double* __restrict__ F) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// that fixed order; the loads are independent of one another, so they are in flight together.
+// The last block reduces E and W6 instead, beside the gather.
+__global__ void __launch_bounds__(FINISH_T) k_pair_finish(int64_t n, const ConfGrid* __restrict__ grid,
+                                                          const int32_t* __restrict__ cell_atoms,
+                                                          const double4* __restrict__ spos,
+                                                          const double* __restrict__ P, double* __restrict__ F,
+                                                          int64_t nblocks, const double* __restrict__ partial,
+                                                          double* __restrict__ E, double* __restrict__ W6) {
+  if (blockIdx.x == gridDim.x - 1) {
+    reduce_partials(nblocks, partial, E, W6);
+    return;
+  }
+  const int64_t s = (int64_t)blockIdx.x * FINISH_T + threadIdx.x;
   if (s >= n) return;
   const ConfGrid& g = grid[0];
   const double4 x = spos[s];
   int c[3];
   cell_coords(g, x.x, x.y, x.z, c);
-  const bool per[3] = {!isinf(g.L[0]), !isinf(g.L[1]), !isinf(g.L[2])};
+  unsigned in[3];  // bit d + 1: the cell at offset d along the axis exists
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const bool per = !isinf(g.L[a]);
+    in[a] = 2u | (per || c[a] > 0 ? 1u : 0u) | (per || c[a] + 1 < g.nc[a] ? 4u : 0u);
+  }
   double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+#pragma unroll
   for (int kind = 0; kind < PBUF_SLOTS; kind++) {
     const int k = kind < HALF_OFFSETS ? kind : kind - (HALF_OFFSETS - 1);
     const int sg = kind < HALF_OFFSETS ? 1 : -1;
     int d[3];
     half_offset(k, d[0], d[1], d[2]);
-    bool ok = true;
-    for (int a = 0; a < 3; a++) ok &= shift_axis(c[a], sg * d[a], g.nc[a], per[a]) >= 0;
-    if (!ok) continue;
+    const bool ok = (in[0] >> (1 + sg * d[0])) & (in[1] >> (1 + sg * d[1])) & (in[2] >> (1 + sg * d[2])) & 1u;
     const double* q = P + 3 * ((int64_t)kind * n + s);
-    f0 += q[0];
-    f1 += q[1];
-    f2 += q[2];
+    if (ok) {
+      f0 += q[0];
+      f1 += q[1];
+      f2 += q[2];
+    }
   }
   const int64_t i = cell_atoms[s];
   F[3 * i] = f0;
   F[3 * i + 1] = f1;
   F[3 * i + 2] = f2;
-}
-
-// Deterministic final reduction of per-block partials (E and W6): one block, fixed order;
-// component 0 goes to E, 1..6 to W6 (either may be null).
-__global__ void k_reduce_partials(int64_t nblocks, int width, const double* __restrict__ partial,
-                                  double* __restrict__ E, double* __restrict__ W6) {
-  __shared__ double sm[256];
-  for (int k = 0; k < width; k++) {
-    double v = 0.0;
-    for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x) v += partial[b * width + k];
-    sm[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      if (k == 0 && E) *E = sm[0];
-      if (k > 0 && W6) W6[k - 1] = sm[0];
-    }
-    __syncthreads();
-  }
 }
 
 int prepare_terms(ipg_ctx* ctx, const ipg_pair_term* terms, int nterms, PairTerms& pt) {
@@ -390,6 +416,7 @@ int pair_eval_device(ipg_ctx* ctx, int64_t n, const double* d_pos, const int32_t
   IPG_RET(ipg_status_reset(ctx));
   int64_t aoff[2] = {0, n};
   CellList cl;
+  cl.want_rel = true;
   IPG_RET(ipg_build_cells(ctx, "pair_", n, d_pos, d_species, 64, 1, aoff, L, pt.rcut_max, cl));
   if (grid_out) *grid_out = cl.h_grid;
   const ConfGrid& g = cl.h_grid[0];
@@ -397,37 +424,32 @@ int pair_eval_device(ipg_ctx* ctx, int64_t n, const double* d_pos, const int32_t
   for (int a = 0; a < 3; a++) half &= std::isinf(g.L[a]) || g.nc[a] >= 3;
   double* partial;
   int64_t nb;
+  double* Eo = (flags & IPG_WANT_E) ? d_E : nullptr;
+  double* Wo = (flags & IPG_WANT_W) ? d_W6 : nullptr;
+  const bool want_f = (flags & IPG_WANT_F) && d_F;
   IPG_RET(ipg_timing_mark(ctx, "pair_eval", true));
   if (half) {
     const int64_t items = cl.ncells * HALF_OFFSETS;
-    // grid-stride: a fixed grid of a few waves of resident blocks (the kernel's register bound
-    // allows pair_minb blocks of four warps per SM)
+    // grid-stride: a fixed grid of a few waves of resident blocks
     nb = std::max<int64_t>(1, std::min<int64_t>((items + PAIR_WARPS - 1) / PAIR_WARPS,
-                                                (int64_t)ctx->num_sms * ctx->pair_minb * 4));
+                                                (int64_t)ctx->num_sms * PAIR_MINB * 4));
+    const PairBox box = {{g.L[0], g.L[1], g.L[2]}};
     double* P;
     IPG_RET(scratch(ctx, "pair_partial", (size_t)nb * 7, &partial));
     IPG_RET(scratch(ctx, "pair_pbuf", (size_t)PBUF_SLOTS * 3 * n, &P));
-    if (ctx->pair_minb == 4)
-      IPG_LAUNCH(ctx, k_pair_half<4>, (unsigned)nb, PAIR_T, 0, pt, n, cl.d_grid, cl.ncells, cl.d_cell_start,
-                 cl.d_cell_atoms, cl.d_spos, P, partial);
-    else if (ctx->pair_minb == 5)
-      IPG_LAUNCH(ctx, k_pair_half<5>, (unsigned)nb, PAIR_T, 0, pt, n, cl.d_grid, cl.ncells, cl.d_cell_start,
-                 cl.d_cell_atoms, cl.d_spos, P, partial);
-    else
-      IPG_LAUNCH(ctx, k_pair_half<3>, (unsigned)nb, PAIR_T, 0, pt, n, cl.d_grid, cl.ncells, cl.d_cell_start,
-                 cl.d_cell_atoms, cl.d_spos, P, partial);
-    if ((flags & IPG_WANT_F) && d_F)
-      IPG_LAUNCH(ctx, k_pair_gather, (unsigned)((n + 255) / 256), 256, 0, n, cl.d_grid, cl.d_cell_atoms, cl.d_spos,
-                 P, d_F);
+    IPG_LAUNCH(ctx, k_pair_half, (unsigned)nb, PAIR_T, 0, pt, box, n, cl.d_grid, cl.ncells, cl.d_cell_start,
+               cl.d_cell_atoms, cl.d_spos, cl.d_srel, pair_prefilter_threshold(g, pt.rcut_max), P, partial);
+    if (want_f)
+      IPG_LAUNCH(ctx, k_pair_finish, (unsigned)((n + FINISH_T - 1) / FINISH_T + 1), FINISH_T, 0, n, cl.d_grid,
+                 cl.d_cell_atoms, cl.d_spos, P, d_F, nb, partial, Eo, Wo);
   } else {
     nb = std::max<int64_t>(1, (n + PAIR_WARPS - 1) / PAIR_WARPS);
     IPG_RET(scratch(ctx, "pair_partial", (size_t)nb * 7, &partial));
     IPG_LAUNCH(ctx, k_pair_eval, (unsigned)nb, PAIR_T, 0, pt, n, cl.d_grid, cl.d_cell_start, cl.d_cell_atoms,
-               cl.d_spos, (flags & IPG_WANT_F) ? d_F : nullptr, partial);
+               cl.d_spos, want_f ? d_F : nullptr, partial);
   }
   IPG_RET(ipg_timing_mark(ctx, "pair_eval", false));
-  IPG_LAUNCH(ctx, k_reduce_partials, 1, 256, 0, nb, 7, partial, (flags & IPG_WANT_E) ? d_E : nullptr,
-             (flags & IPG_WANT_W) ? d_W6 : nullptr);
+  if (!half || !want_f) IPG_LAUNCH(ctx, k_reduce_partials, 1, FINISH_T, 0, nb, partial, Eo, Wo);
   return IPG_OK;
 }
 
@@ -439,8 +461,7 @@ ipg_ctx::PairGraph* pair_graph_find(ipg_ctx* ctx, int64_t n, const double* d_pos
   for (auto& g : ctx->pair_graphs)
     if (g.n == n && g.L[0] == L[0] && g.L[1] == L[1] && g.L[2] == L[2] && g.pos == d_pos && g.sp == d_species &&
         g.E == d_E && g.F == d_F && g.W6 == d_W6 && g.flags == flags && g.terms.size() == tb &&
-        memcmp(g.terms.data(), terms, tb) == 0 && g.full_stencil == (int)ctx->pair_full_stencil &&
-        g.minb == ctx->pair_minb)
+        memcmp(g.terms.data(), terms, tb) == 0 && g.full_stencil == (int)ctx->pair_full_stencil)
       return &g;
   return nullptr;
 }
@@ -486,7 +507,6 @@ void pair_graph_capture(ipg_ctx* ctx, int64_t n, const double* d_pos, const int3
   g.flags = flags;
   g.terms.assign(reinterpret_cast<const char*>(terms), reinterpret_cast<const char*>(terms) + sizeof(ipg_pair_term) * nterms);
   g.full_stencil = ctx->pair_full_stencil;
-  g.minb = ctx->pair_minb;
   const uint64_t gen0 = ctx->scratch_gen;
   std::vector<ConfGrid> grid;
   const bool timing = ctx->timing;

@@ -15,8 +15,9 @@ struct PairTermDev {
   int kind;
   int pad;
   double coeff, rcut;
+  double rc2_lo, rc2_hi;  // rcut^2 (1 -/+ 1e-12): the squared distance settles all but the boundary cases
   unsigned long long mask;
-  double p[8];  // kind-specific precomputed constants (see pair_prepare_terms)
+  double p[12];  // kind-specific precomputed constants (see pair_prepare_terms)
 };
 
 struct PairTerms {
@@ -27,6 +28,14 @@ struct PairTerms {
 };
 
 static_assert(sizeof(PairTerms) <= 4096, "the terms travel as a kernel parameter");
+
+// ZBL screening: weights and decay constants (zbl.jl:27-36).
+__host__ __device__ constexpr double zbl_c(int k) {
+  return k == 0 ? 0.18175 : (k == 1 ? 0.50986 : (k == 2 ? 0.28022 : 0.02817));
+}
+__host__ __device__ constexpr double zbl_a(int k) {
+  return k == 0 ? 3.19980 : (k == 1 ? 0.94229 : (k == 2 ? 0.40290 : 0.20162));
+}
 
 // Host: the kernel-side terms of an ipg_pair_term list.  Returns IPG_OK or IPG_ERR_ARG with a
 // message in err.
@@ -43,6 +52,8 @@ inline int pair_prepare_terms(const ipg_pair_term* terms, int nterms, PairTerms&
     d.kind = s.kind;
     d.coeff = s.coeff;
     d.rcut = s.rcut;
+    d.rc2_lo = s.rcut * s.rcut * (1.0 - 1e-12);
+    d.rc2_hi = s.rcut * s.rcut * (1.0 + 1e-12);
     d.mask = s.species_mask;
     if (!(s.rcut >= 0.0) || std::isinf(s.rcut)) {
       snprintf(err, errlen, "term %d: rcut must be finite and >= 0", k);
@@ -64,7 +75,7 @@ inline int pair_prepare_terms(const ipg_pair_term* terms, int nterms, PairTerms&
       case IPG_PAIR_COUL:  // p = q1, q2, k_e q1 q2 with k_e = 1 (src/constants.jl:7)
         d.p[2] = 1.0 * s.params[0] * s.params[1];
         break;
-      case IPG_PAIR_ZBL: {  // p = Z1, Z2, e, Z1 Z2 e^2, the screening length, ln(e), 1/length
+      case IPG_PAIR_ZBL: {  // p = Z1, Z2, e, Z1 Z2 e^2, the screening length, ln(e), 1/length, -, -a_k ln(e)/length
         const double Z1 = s.params[0], Z2 = s.params[1], e = s.params[2];
         if (!(e > 0.0)) {
           snprintf(err, errlen, "term %d: ZBL e must be > 0", k);
@@ -74,6 +85,7 @@ inline int pair_prepare_terms(const ipg_pair_term* terms, int nterms, PairTerms&
         d.p[4] = 0.8854 * 0.529 / (std::pow(Z1, 0.23) + std::pow(Z2, 0.23));
         d.p[5] = std::log(e);
         d.p[6] = 1.0 / d.p[4];
+        for (int q = 0; q < 4; q++) d.p[8 + q] = -zbl_a(q) * d.p[5] * d.p[6];
         break;
       }
       default:
@@ -121,17 +133,14 @@ __device__ __forceinline__ void pair_term_eval(const PairTermDev& t, double R, d
       break;
     }
     case IPG_PAIR_ZBL: {  // zbl.jl:27-36: e^(-a_k d) with base e = p[2]
-      const double zc[4] = {0.18175, 0.50986, 0.28022, 0.02817};
-      const double za[4] = {3.19980, 0.94229, 0.40290, 0.20162};
       const double d = R * t.p[6];
       double phi = 0.0, dphi = 0.0;
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const double ek = exp(-za[k] * d * t.p[5]);
-        phi += zc[k] * ek;
-        dphi += za[k] * zc[k] * ek;
+        const double ek = exp(R * t.p[8 + k]);
+        phi = fma(zbl_c(k), ek, phi);
+        dphi = fma(-zbl_a(k) * zbl_c(k), ek, dphi);
       }
-      dphi = -dphi;
       V = t.p[3] * phi * ir;
       g = t.p[3] * (phi + d * dphi) * ir * ir2;
       break;
@@ -146,17 +155,20 @@ __device__ __forceinline__ void pair_term_eval(const PairTermDev& t, double R, d
   }
 }
 
-// Sum of c_t V_t and c_t g_t over the terms that apply to a pair (distance `dist` for the
-// cutoffs, R = |r| for the formulas, species si and sj for the filters:
-// src/types/empirical_potential.jl:26-43, both species in the term's set).
-__device__ __forceinline__ void pair_terms_sum(const PairTerms& TT, double R, double dist, int si, int sj, double& V,
+// Sum of c_t V_t and c_t g_t over the terms that apply to a pair: d2 the squared distance of
+// the cutoffs (a term counts when sqrt(d2) <= rcut, decided as by the square root), r2 = |r|^2
+// of the formulas, species si and sj for the filters (src/types/empirical_potential.jl:26-43,
+// both species in the term's set).  One reciprocal square root gives R and every power of 1/R.
+__device__ __forceinline__ void pair_terms_sum(const PairTerms& TT, double r2, double d2, int si, int sj, double& V,
                                                double& g) {
   V = 0.0;
   g = 0.0;
-  const double ir = 1.0 / R, ir2 = ir * ir;
+  const double ir = rsqrt(r2), ir2 = ir * ir;
+  const double R = r2 > 0.0 ? r2 * ir : sqrt(r2);
   for (int t = 0; t < TT.nterms; t++) {
     const PairTermDev& T = TT.t[t];
-    if (dist > T.rcut) continue;
+    if (d2 > T.rc2_hi) continue;
+    if (d2 >= T.rc2_lo && sqrt(d2) > T.rcut) continue;
     if (!((T.mask >> si) & 1ull) || !((T.mask >> sj) & 1ull)) continue;
     double v, gg;
     pair_term_eval(T, R, ir, ir2, v, gg);
@@ -174,7 +186,7 @@ __device__ __forceinline__ void pair_terms_sum(const PairTerms& TT, double R, do
 // is the negated reference displacement of the stored half pair, -get_displacement(x_j, x_i),
 // so every force term equals the reference's term; only the order of summation differs.
 struct PairHit {
-  double r0, r1, r2, dist;
+  double r0, r1, r2, d2;
   int sj, pad;
 };
 
@@ -182,9 +194,8 @@ __device__ __forceinline__ void pair_eval_hits(const PairTerms& TT, const PairHi
                                                int si, double* acc, double& f0, double& f1, double& f2) {
   if (lane >= nh) return;
   const PairHit h = hb[lane];
-  const double R = sqrt(h.r0 * h.r0 + h.r1 * h.r1 + h.r2 * h.r2);
   double V, gsum;
-  pair_terms_sum(TT, R, h.dist, si, h.sj, V, gsum);
+  pair_terms_sum(TT, h.r0 * h.r0 + h.r1 * h.r1 + h.r2 * h.r2, h.d2, si, h.sj, V, gsum);
   const double fx = gsum * h.r0, fy = gsum * h.r1, fz = gsum * h.r2;
   f0 += fx;
   f1 += fy;
@@ -229,10 +240,9 @@ __device__ __forceinline__ void pair_walk_atom(const PairTerms& TT, const ConfGr
           const double d2 = sumsq3_dev(pe_axis_dev(g.L[0], xi.x, xj.x), pe_axis_dev(g.L[1], xi.y, xj.y),
                                        pe_axis_dev(g.L[2], xi.z, xj.z));
           if (d2 <= TT.rmax2_hi) {
-            const double dist = sqrt(d2);
-            if (dist <= rmax) {
+            if (sqrt(d2) <= rmax) {
               ok = true;
-              h.dist = dist;
+              h.d2 = d2;
               h.sj = (int)xj.w;
               if (j > i) {
                 h.r0 = disp_axis_dev(g.L[0], xi.x, xj.x);
