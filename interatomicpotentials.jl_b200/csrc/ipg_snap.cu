@@ -1562,408 +1562,6 @@ __global__ void __launch_bounds__(YS_WARPS * 32, 2) k_snap_yatoms(const __grid_c
   }
 }
 
-// ---------------------------------------------------------------------------------
-// Row-blocked Y kernel.  Same block shape as k_snap_yatoms (32 atoms in the lanes, the
-// half plane of their Utot in shared memory as [h][atom]), but a warp owns whole target
-// rows (j, mb) of Y and, for each triple (j1, j2, j) feeding the row and each of its nb
-// row pairs (mb1, mb2), evaluates the Z entries of every ma of the row at once:
-//   Y(j, mb, ma) += c cg[mb1][mb2] sum_ma2 ca[ma][ma2] U(j1, mb1, ma + d - ma2) U(j2, mb2, ma2),
-// d = (j1 + j2 - j)/2, c = the triple's Y coefficient (compute_yi.jl:86-118).  The j2 row
-// is walked two columns at a time; each element of the j1 row met by those two columns is
-// loaded once and used for both, so a Utot element is read from shared memory about
-// (NMA + 3) / (2 NMA) times per product instead of twice.  Only the target level j is a
-// template parameter: the code of one instantiation stays small enough for the
-// instruction cache although the warps of a block work on different rows.
-
-// Guard entries (zeros) before and after the half plane in shared memory: the column
-// walks below read up to YR_GUARD entries past either end of a row.  Those reads meet a
-// CG factor of exactly zero (the factor tables are zero wherever ma1 or ma2 is out of
-// range), so they only have to stay inside the array and be finite.
-__host__ __device__ constexpr int yr_guard(int J) { return J + 2; }
-
-// Shared memory of k_snap_yrows, in bytes:
-//   front: the triple coefficients [nsp][ntp] (beta-dependent, filled per launch) and the CG
-//          factors of every triple (yca), at least yr_guard entries of Utot long;
-//   Utot:  the half plane of 32 atoms, [u_half][32] double2;
-//   back:  the energy slot of every target row, [rows][32] doubles, at least yr_guard long.
-// The out-of-range window reads fall into front or back: finite values (the free parts are
-// zeroed) that meet CG factors of exactly zero.
-struct YrSmem {
-  int ntp, front, u, back;
-  __host__ __device__ int total() const { return front + u + back; }
-};
-__host__ __device__ inline YrSmem yr_smem(int J, int nsp, int ntrip, int nyca, int uh, int nrows) {
-  YrSmem m;
-  m.ntp = ntrip + (ntrip & 1);
-  const int guard = yr_guard(J) * YS_ATOMS * 16;
-  const int f = (8 * (nsp * m.ntp + nyca) + 15) & ~15;
-  m.front = f > guard ? f : guard;
-  m.u = uh * YS_ATOMS * 16;
-  const int e = nrows * YS_ATOMS * 8;
-  m.back = e > guard ? e : guard;
-  return m;
-}
-
-// One row pair (mb1, mb2) of a triple for the target-row tile ma = ma0 .. ma0+NT-1.  The
-// j1 row is walked as a window: element t of column pair m0 is ma1 = d - m0 - 1 + ma0 + t,
-// met by (ma = ma0 + t - 1, ma2 = m0) and (ma = ma0 + t, ma2 = m0 + 1).  cp: the triple's
-// factors as [m0/2][ma = 0..j][2], rs = j + 1.
-//
-// Mirrored rows cost no extra instructions.  M1 (the j1 row lies beyond the half plane):
-// U(j1, mb1, ma1) = (-1)^(ma1+mb1) conj(v), and with m0 even the sign splits into
-// (-1)^(ma0+d+mb1), folded into cb, times (-1)^(i+q) with i = ma - ma0, a compile-time
-// constant folded into the FMAs along with the conjugate.  A mirrored j2 row gives
-// (-1)^mb2 (into cb) times (-1)^q and a conjugate, folded into the two per-column scales.
-template <int NT, bool M1>
-__device__ __forceinline__ void yr_pair(const double2* __restrict__ usl, const int* __restrict__ hblk,
-                                        const double2* __restrict__ cp, int rs, int ma0, int j1, int j2, int d,
-                                        int mb1, int mb2, double cb, double2 (&acc)[NT]) {
-  const double2* p1 = usl + (size_t)(hblk[j1] + (M1 ? j1 - mb1 : mb1) * (j1 + 1) + (M1 ? j1 : 0)) * YS_ATOMS;
-  const bool m2 = 2 * mb2 > j2;
-  const double2* p2 = usl + (size_t)(hblk[j2] + (m2 ? j2 - mb2 : mb2) * (j2 + 1) + (m2 ? j2 : 0)) * YS_ATOMS;
-  const int st2 = m2 ? -YS_ATOMS : YS_ATOMS;
-  if (M1 && ((ma0 + d + mb1) & 1)) cb = -cb;
-  if (m2 && (mb2 & 1)) cb = -cb;
-  const double sx0 = cb, sy0 = m2 ? -cb : cb, sx1 = m2 ? -cb : cb, sy1 = cb;
-  cp += ma0;
-  int m0 = 0;
-  for (; m0 < j2; m0 += 2, cp += rs) {  // column pairs (m0, m0 + 1) both in range
-    const double2 v0 = p2[0], v1 = p2[st2];
-    p2 += 2 * st2;
-    double2 r[2];
-    r[0] = make_double2(sx0 * v0.x, sy0 * v0.y);
-    r[1] = make_double2(sx1 * v1.x, sy1 * v1.y);
-    double2 a[NT];
-#pragma unroll
-    for (int i = 0; i < NT; i++) a[i] = cp[i];
-    const int base = d - m0 - 1 + ma0;
-    const double2* pb = p1 + (M1 ? -base : base) * YS_ATOMS;
-    double2 u[NT + 1];
-#pragma unroll
-    for (int t = 0; t <= NT; t++) u[t] = pb[(M1 ? -t : t) * YS_ATOMS];
-    // one sweep per column (q = 1: element i, q = 0: element i + 1), so the two updates of an
-    // accumulator are NT terms apart; each term forms the complex product first and adds it
-    // with one FMA per component
-#pragma unroll
-    for (int q = 1; q >= 0; q--) {
-#pragma unroll
-      for (int i = 0; i < NT; i++) {
-        const double2 v = u[i + 1 - q];
-        const double2 w = r[q];
-        double px, py;
-        if (M1) {  // conj(v) w
-          px = fma(v.x, w.x, v.y * w.y);
-          py = fma(v.x, w.y, -(v.y * w.x));
-        } else {
-          px = fma(v.x, w.x, -(v.y * w.y));
-          py = fma(v.x, w.y, v.y * w.x);
-        }
-        const double c0 = q ? a[i].y : a[i].x;
-        const double c = (M1 && ((i + q) & 1)) ? -c0 : c0;
-        acc[i].x = fma(c, px, acc[i].x);
-        acc[i].y = fma(c, py, acc[i].y);
-      }
-    }
-  }
-  if (!(j2 & 1)) {  // even j2: the last column (m0 = j2) alone; its partner j2 + 1 is out of range
-    const double2 v0 = p2[0];
-    const double2 w = make_double2(sx0 * v0.x, sy0 * v0.y);
-    const int base = d - m0 - 1 + ma0;
-    const double2* pb = p1 + (M1 ? -base : base) * YS_ATOMS;
-#pragma unroll
-    for (int i = 0; i < NT; i++) {
-      const double2 v = pb[(M1 ? -(i + 1) : (i + 1)) * YS_ATOMS];
-      double px, py;
-      if (M1) {
-        px = fma(v.x, w.x, v.y * w.y);
-        py = fma(v.x, w.y, -(v.y * w.x));
-      } else {
-        px = fma(v.x, w.x, -(v.y * w.y));
-        py = fma(v.x, w.y, v.y * w.x);
-      }
-      const double c0 = cp[i].x;
-      const double c = (M1 && (i & 1)) ? -c0 : c0;
-      acc[i].x = fma(c, px, acc[i].x);
-      acc[i].y = fma(c, py, acc[i].y);
-    }
-  }
-}
-
-// Tile ma0 .. ma0+NT-1 of target row (j, mb): every triple and row pair of the row.
-// Writes Y' = w Y of the tile's entries below nma and returns their Re(conj(U) Y').
-template <int NT>
-__device__ __forceinline__ double yr_tile(const SnapDev& S, const YConst& T, const YRowDev& row, int ma0, int nma,
-                                          const double2* __restrict__ usl, const double* __restrict__ yc,
-                                          const double2* __restrict__ cas, int64_t n, int64_t atom, bool valid,
-                                          double2* __restrict__ yout) {
-  double2 acc[NT];
-#pragma unroll
-  for (int i = 0; i < NT; i++) acc[i] = make_double2(0.0, 0.0);
-  const int j = row.j, rs = j + 1;
-  const double bn = S.bnorm_flag ? 1.0 / (j + 1) : 1.0;
-  for (int t = row.t0; t < row.t1; t++) {
-    const YItemDev it = T.items[t];
-    const double c = yc[it.trip] * bn;
-    const double2* __restrict__ cp = cas + it.ca / 2;
-    const int j1 = it.j1, j2 = it.j2, d = it.d;
-    for (int ib = 0; ib < it.nb; ib++) {
-      const int mb1 = it.mb1min + ib, mb2 = it.mb2max - ib;
-      const double cb = c * T.cb[it.cg + ib];  // cg[mb1][mb2] of this row pair
-      if (2 * mb1 > j1)
-        yr_pair<NT, true>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, acc);
-      else
-        yr_pair<NT, false>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, acc);
-    }
-  }
-  double e = 0.0;
-#pragma unroll
-  for (int i = 0; i < NT; i++) {
-    const int ma = ma0 + i;
-    if (ma >= nma) break;
-    const double w = (row.mid && ma == nma - 1) ? 0.5 : 1.0;
-    const double2 y = make_double2(w * acc[i].x, w * acc[i].y);
-    const int h = row.h0 + ma;
-    if (valid) yout[(size_t)h * n + atom] = y;
-    const double2 u = usl[(size_t)h * YS_ATOMS];
-    e += u.x * y.x + u.y * y.y;
-  }
-  return e;
-}
-
-// Tiles of a row of nma entries: at most YR_TILE wide, as even as possible.
-#ifndef IPG_YR_TILE
-#define IPG_YR_TILE 5  // widths 4, 5, 6 measured 1.80, 1.77, 1.86 ms at 54,000 atoms (eight warps)
-#endif
-constexpr int YR_TILE = IPG_YR_TILE;
-
-__device__ __forceinline__ double yr_row(const SnapDev& S, const YConst& T, const YRowDev& row,
-                                         const double2* __restrict__ usl, const double* __restrict__ yc,
-                                         const double2* __restrict__ cas, int64_t n, int64_t atom, bool valid,
-                                         double2* __restrict__ yout) {
-  const int nma = row.mid ? row.mb + 1 : row.j + 1;
-  const int ntile = (nma + YR_TILE - 1) / YR_TILE;
-  double e = 0.0;
-  int ma0 = 0;
-  for (int k = 0; k < ntile; k++) {
-    const int w = (nma - ma0 + (ntile - k) - 1) / (ntile - k);  // remaining entries over remaining tiles
-    switch (w) {
-#define IPG_NT(NT) \
-  case NT:         \
-    if constexpr (NT <= YR_TILE) e += yr_tile<NT>(S, T, row, ma0, nma, usl, yc, cas, n, atom, valid, yout); \
-    break;
-      IPG_NT(1) IPG_NT(2) IPG_NT(3) IPG_NT(4) IPG_NT(5) IPG_NT(6)
-#undef IPG_NT
-      default:
-        break;
-    }
-    ma0 += w;
-  }
-  return e;
-}
-
-// Z output variant (k_snap_yrows<YM_Z>): every item's Z tile goes to zout[jjz][atom]
-// (entries of the half plane; the middle row of an even level up to ma = mb), nothing is
-// summed across items.  Z carries the 1/(j+1) of bnorm_flag (compute_z.jl:49-56).
-template <int NT>
-__device__ __forceinline__ void yr_tile_z(const SnapDev& S, const YConst& T, const YRowDev& row, int ma0, int nma,
-                                          const double2* __restrict__ usl, const double2* __restrict__ cas, int64_t n,
-                                          int64_t atom, bool valid, double2* __restrict__ zout) {
-  const int j = row.j, rs = j + 1;
-  const double bn = S.bnorm_flag ? 1.0 / (j + 1) : 1.0;
-  for (int t = row.t0; t < row.t1; t++) {
-    const YItemDev it = T.items[t];
-    double2 acc[NT];
-#pragma unroll
-    for (int i = 0; i < NT; i++) acc[i] = make_double2(0.0, 0.0);
-    const double2* __restrict__ cp = cas + it.ca / 2;
-    const int j1 = it.j1, j2 = it.j2, d = it.d;
-    for (int ib = 0; ib < it.nb; ib++) {
-      const int mb1 = it.mb1min + ib, mb2 = it.mb2max - ib;
-      const double cb = bn * T.cb[it.cg + ib];
-      if (2 * mb1 > j1)
-        yr_pair<NT, true>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, acc);
-      else
-        yr_pair<NT, false>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, acc);
-    }
-    if (valid) {
-      const int64_t z0 = it.jjz + row.mb * (j + 1) + ma0;
-#pragma unroll
-      for (int i = 0; i < NT; i++)
-        if (ma0 + i < nma) zout[(size_t)(z0 + i) * n + atom] = acc[i];
-    }
-  }
-}
-
-__device__ __forceinline__ void yr_row_z(const SnapDev& S, const YConst& T, const YRowDev& row,
-                                         const double2* __restrict__ usl, const double2* __restrict__ cas, int64_t n,
-                                         int64_t atom, bool valid, double2* __restrict__ zout) {
-  const int nma = row.mid ? row.mb + 1 : row.j + 1;
-  const int ntile = (nma + YR_TILE - 1) / YR_TILE;
-  int ma0 = 0;
-  for (int k = 0; k < ntile; k++) {
-    const int w = (nma - ma0 + (ntile - k) - 1) / (ntile - k);
-    switch (w) {
-#define IPG_NT(NT) \
-  case NT:         \
-    if constexpr (NT <= YR_TILE) yr_tile_z<NT>(S, T, row, ma0, nma, usl, cas, n, atom, valid, zout); \
-    break;
-      IPG_NT(1) IPG_NT(2) IPG_NT(3) IPG_NT(4) IPG_NT(5) IPG_NT(6)
-#undef IPG_NT
-      default:
-        break;
-    }
-    ma0 += w;
-  }
-}
-
-// Y and Z at once (k_snap_yrows<YM_YZ>): each item's Z tile is formed with unit coefficients,
-// written to zout[jjz][atom] as by yr_tile_z, and added into the row's Y with the item's
-// coefficient, so a later beta pullback of the same positions reads Z instead of recomputing
-// it.  Y' and the energy are as from yr_tile.
-template <int NT>
-__device__ __forceinline__ double yr_tile_yz(const SnapDev& S, const YConst& T, const YRowDev& row, int ma0, int nma,
-                                             const double2* __restrict__ usl, const double* __restrict__ yc,
-                                             const double2* __restrict__ cas, int64_t n, int64_t atom, bool valid,
-                                             double2* __restrict__ yout, double2* __restrict__ zout) {
-  double2 acc[NT];
-#pragma unroll
-  for (int i = 0; i < NT; i++) acc[i] = make_double2(0.0, 0.0);
-  const int j = row.j, rs = j + 1;
-  const double bn = S.bnorm_flag ? 1.0 / (j + 1) : 1.0;
-  for (int t = row.t0; t < row.t1; t++) {
-    const YItemDev it = T.items[t];
-    const double c = yc[it.trip];
-    const double2* __restrict__ cp = cas + it.ca / 2;
-    const int j1 = it.j1, j2 = it.j2, d = it.d;
-    double2 z[NT];
-#pragma unroll
-    for (int i = 0; i < NT; i++) z[i] = make_double2(0.0, 0.0);
-    for (int ib = 0; ib < it.nb; ib++) {
-      const int mb1 = it.mb1min + ib, mb2 = it.mb2max - ib;
-      const double cb = bn * T.cb[it.cg + ib];
-      if (2 * mb1 > j1)
-        yr_pair<NT, true>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, z);
-      else
-        yr_pair<NT, false>(usl, S.half_block, cp, rs, ma0, j1, j2, d, mb1, mb2, cb, z);
-    }
-    const int64_t z0 = it.jjz + row.mb * (j + 1) + ma0;
-#pragma unroll
-    for (int i = 0; i < NT; i++) {
-      if (valid && ma0 + i < nma) zout[(size_t)(z0 + i) * n + atom] = z[i];
-      acc[i].x = fma(c, z[i].x, acc[i].x);
-      acc[i].y = fma(c, z[i].y, acc[i].y);
-    }
-  }
-  double e = 0.0;
-#pragma unroll
-  for (int i = 0; i < NT; i++) {
-    const int ma = ma0 + i;
-    if (ma >= nma) break;
-    const double w = (row.mid && ma == nma - 1) ? 0.5 : 1.0;
-    const double2 y = make_double2(w * acc[i].x, w * acc[i].y);
-    const int h = row.h0 + ma;
-    if (valid) yout[(size_t)h * n + atom] = y;
-    const double2 u = usl[(size_t)h * YS_ATOMS];
-    e += u.x * y.x + u.y * y.y;
-  }
-  return e;
-}
-
-__device__ __forceinline__ double yr_row_yz(const SnapDev& S, const YConst& T, const YRowDev& row,
-                                            const double2* __restrict__ usl, const double* __restrict__ yc,
-                                            const double2* __restrict__ cas, int64_t n, int64_t atom, bool valid,
-                                            double2* __restrict__ yout, double2* __restrict__ zout) {
-  const int nma = row.mid ? row.mb + 1 : row.j + 1;
-  const int ntile = (nma + YR_TILE - 1) / YR_TILE;
-  double e = 0.0;
-  int ma0 = 0;
-  for (int k = 0; k < ntile; k++) {
-    const int w = (nma - ma0 + (ntile - k) - 1) / (ntile - k);
-    switch (w) {
-#define IPG_NT(NT) \
-  case NT:         \
-    if constexpr (NT <= YR_TILE) e += yr_tile_yz<NT>(S, T, row, ma0, nma, usl, yc, cas, n, atom, valid, yout, zout); \
-    break;
-      IPG_NT(1) IPG_NT(2) IPG_NT(3) IPG_NT(4) IPG_NT(5) IPG_NT(6)
-#undef IPG_NT
-      default:
-        break;
-    }
-    ma0 += w;
-  }
-  return e;
-}
-
-// YM: YM_Y writes Y' (yout [u_half][n]) and E_i; YM_Z writes Z (yout [idxz_max][n], nothing
-// summed across items); YM_YZ writes both (Z to zout).
-// NW: warps per block (the Utot tile of 32 atoms is shared by all of them; two blocks per SM).
-constexpr int YM_Y = 0, YM_Z = 1, YM_YZ = 2;
-template <int YM, int NW = YS_WARPS>
-__global__ void __launch_bounds__(NW * 32, 2) k_snap_yrows(const __grid_constant__ SnapDev S, const __grid_constant__ YConst T, int64_t n,
-                                                                 const int32_t* __restrict__ species,
-                                                                 const double2* __restrict__ utot,
-                                                                 double2* __restrict__ yout, double* __restrict__ Ei,
-                                                                 double2* __restrict__ zout) {
-  constexpr bool ZOUT = YM == YM_Z;
-  extern __shared__ __align__(16) unsigned char ysh[];  // layout: yr_smem
-  __shared__ int next_row;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int U = S.idxu_max, UH = S.u_half;
-  const YrSmem M = yr_smem(S.J, S.nsp, S.n_ytrip, S.n_yca, UH, S.n_yrows);
-  double* ycs = reinterpret_cast<double*>(ysh);  // [nsp][ntp] Y coefficient of each triple
-  double* cad = ycs + S.nsp * M.ntp;             // CG factors of every triple
-  const double2* cas = reinterpret_cast<const double2*>(cad);
-  double2* us = reinterpret_cast<double2*>(ysh + M.front);
-  double* erow = reinterpret_cast<double*>(ysh + M.front + M.u);  // [rows][32]
-  for (int idx = threadIdx.x; idx < S.nsp * M.ntp; idx += blockDim.x) {
-    const int sp = idx / M.ntp, t = idx - sp * M.ntp;
-    ycs[idx] = t < S.n_ytrip ? S.ycoef[(size_t)sp * S.idxz_max + S.ytrip_jjz[t]] : 0.0;
-  }
-  for (int idx = threadIdx.x; idx < S.n_yca; idx += blockDim.x) cad[idx] = S.yca[idx];
-  {
-    double* gap = cad + S.n_yca;
-    const int ngap = (M.front - 8 * (S.nsp * M.ntp + S.n_yca)) / 8;
-    for (int idx = threadIdx.x; idx < ngap; idx += blockDim.x) gap[idx] = 0.0;
-    for (int idx = threadIdx.x; idx < M.back / 8; idx += blockDim.x) erow[idx] = 0.0;
-  }
-  for (int64_t a0 = (int64_t)blockIdx.x * YS_ATOMS; a0 < n; a0 += (int64_t)gridDim.x * YS_ATOMS) {
-    const int na_blk = (int)((n - a0) < YS_ATOMS ? (n - a0) : YS_ATOMS);
-    for (int idx = threadIdx.x; idx < UH * YS_ATOMS; idx += blockDim.x) {
-      const int q = idx / YS_ATOMS, l = idx - q * YS_ATOMS;
-      us[idx] = l < na_blk ? utot[(size_t)(a0 + l) * U + S.u_of_h[q]] : make_double2(0.0, 0.0);
-    }
-    if (threadIdx.x == 0) next_row = 0;
-    __syncthreads();
-    const int64_t atom = a0 + lane;
-    const bool valid = lane < na_blk;
-    const int si = valid ? clamp_sp(species[atom], S.nsp) : 0;
-    const double* yc = ycs + si * M.ntp;
-    const double2* usl = us + lane;
-    // rows are handed out longest first to whichever warp is free; a row's result does
-    // not depend on the warp that computes it, and the energy is summed in row order
-    for (;;) {
-      int r = 0;
-      if (lane == 0) r = atomicAdd(&next_row, 1);
-      r = __shfl_sync(0xffffffffu, r, 0);
-      if (r >= T.nrows) break;
-      const YRowDev row = T.rows[r];
-      if (ZOUT)
-        yr_row_z(S, T, row, usl, cas, n, atom, valid, yout);  // yout: Z [idxz_max][n]
-      else if (YM == YM_YZ)
-        erow[r * YS_ATOMS + lane] = yr_row_yz(S, T, row, usl, yc, cas, n, atom, valid, yout, zout);
-      else
-        erow[r * YS_ATOMS + lane] = yr_row(S, T, row, usl, yc, cas, n, atom, valid, yout);
-    }
-    __syncthreads();
-    if (!ZOUT && warp == 0 && valid) {
-      double t = 0.0;
-      for (int r = 0; r < T.nrows; r++) t += erow[r * YS_ATOMS + lane];
-      Ei[atom] = (2.0 / 3.0) * t + S.ebias[si];
-    }
-    __syncthreads();
-  }
-}
-
 // ---- beta pullback from the register chains (twojmax <= YR_MAX_J) -------------------------
 // The cotangent g of the forces pulls back to
 //   gbeta[s][b] = sum over atoms i of species s of
@@ -1971,7 +1569,7 @@ __global__ void __launch_bounds__(NW * 32, 2) k_snap_yrows(const __grid_constant
 //   V_i = sum over neighbors j of (g_i - g_j) . dU_ij/dr_ij      (half plane of every level),
 // the terms t, levels and factors of each component being those of dB/dr (compute_b.jl:
 // 207-400).  V comes from k_snap_vsum (every chain of a neighbor per lane), Z from
-// k_snap_yrows<YM_Z>, and k_snap_gbeta contracts them with the atoms in lanes.
+// k_snap_ystream<YM_Z>, and k_snap_gbeta contracts them with the atoms in lanes.
 
 // V of atoms a0 .. a0+nc-1 as V[h][nc]: one warp per atom, lanes over neighbors (32 at a
 // time), v_h = A u_h + sum_k B_k du_k,h with A = dsfac gv.uhat, B_k = sfac gv_k, gv = g_i - g_j;
@@ -2209,7 +1807,7 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_gbeta(const __grid_const
   for (int q = threadIdx.x; q < nsp * K; q += blockDim.x) gpart[(size_t)blockIdx.x * nsp * K + q] = gacc[q];
 }
 
-// Bispectrum components from Z (k_snap_yrows<YM_Z>) and Utot for atoms a0 .. a0+nc-1
+// Bispectrum components from Z (k_snap_ystream<YM_Z>) and Utot for atoms a0 .. a0+nc-1
 // (compute_b.jl:17-94): B_b = 2 sum_half w Re(conj(U_j) Z(j1,j2,j)) - bzero_j, 32 atoms per
 // tile in lanes, the warps over components; Ei = beta[s_i] . B_i (the bzero shift inside B).
 // B [n][K] (optional) and Ei [n] are indexed by the global atom.
@@ -3509,7 +3107,6 @@ struct ipg_snap {
   bool generic_plain = false;  // plain path: the per-atom block kernel (IPG_GENERIC_PLAIN=1)
   bool generic_hvp = false;    // position pullback: the per-atom forward-mode kernel (IPG_GENERIC_HVP=1)
   int walk_warps = 4;       // atoms (warps) per block of the neighbor walk
-  int yr_warps = 12;        // warps per block of the adjoint Y kernel (8, 10, 12 or 16)
   std::vector<double> beta_host;  // last uploaded beta
   // last evaluation's pair count, cell grids and chunk table (host), for graph capture
   int64_t last_np = 0;
@@ -3574,10 +3171,8 @@ int upload_tables(ipg_snap* s) {
   size_t o_uoh = o_ysw + pad(h.ysched_w.size() * 8);
   size_t o_hinfo = o_uoh + pad(h.u_of_h.size() * 4);
   size_t o_hsgen = o_hinfo + pad(h.h_info.size() * 4);
-  size_t o_yrows = o_hsgen + pad(h.h_sgen.size() * 8);
-  size_t o_yit = o_yrows + pad(h.yrows.size() * sizeof(YRowDev));
-  size_t o_yca = o_yit + pad(h.yitems.size() * sizeof(YItemDev));
-  size_t o_ytj = o_yca + pad(h.yca.size() * 8);
+  size_t o_yks = o_hsgen + pad(h.h_sgen.size() * 8);
+  size_t o_ytj = o_yks + pad(h.ykstream.size() * 8);
   size_t total = o_ytj + pad(h.ytrip_jjz.size() * 4);
   CUDA_RET(ctx, cudaMalloc(&s->d_tables, total));
   char* b = static_cast<char*>(s->d_tables);
@@ -3597,9 +3192,7 @@ int upload_tables(ipg_snap* s) {
   memcpy(hostbuf.data() + o_uoh, h.u_of_h.data(), h.u_of_h.size() * 4);
   memcpy(hostbuf.data() + o_hinfo, h.h_info.data(), h.h_info.size() * 4);
   memcpy(hostbuf.data() + o_hsgen, h.h_sgen.data(), h.h_sgen.size() * 8);
-  memcpy(hostbuf.data() + o_yrows, h.yrows.data(), h.yrows.size() * sizeof(YRowDev));
-  memcpy(hostbuf.data() + o_yit, h.yitems.data(), h.yitems.size() * sizeof(YItemDev));
-  memcpy(hostbuf.data() + o_yca, h.yca.data(), h.yca.size() * 8);
+  memcpy(hostbuf.data() + o_yks, h.ykstream.data(), h.ykstream.size() * 8);
   memcpy(hostbuf.data() + o_ytj, h.ytrip_jjz.data(), h.ytrip_jjz.size() * 4);
   CUDA_RET(ctx, cudaMemcpy(b, hostbuf.data(), total, cudaMemcpyHostToDevice));
   SnapDev& d = s->dev;
@@ -3647,13 +3240,9 @@ int upload_tables(ipg_snap* s) {
   d.u_of_h = reinterpret_cast<const int32_t*>(b + o_uoh);
   d.h_info = reinterpret_cast<const int32_t*>(b + o_hinfo);
   d.h_sgen = reinterpret_cast<const double2*>(b + o_hsgen);
-  d.n_yrows = (int)h.yrows.size();
-  d.yrows = reinterpret_cast<const YRowDev*>(b + o_yrows);
-  d.yitems = reinterpret_cast<const YItemDev*>(b + o_yit);
-  d.yca = reinterpret_cast<const double*>(b + o_yca);
+  d.ykstream = reinterpret_cast<const double2*>(b + o_yks);
   d.ytrip_jjz = reinterpret_cast<const int32_t*>(b + o_ytj);
   d.n_ytrip = (int)h.ytrip_jjz.size();
-  d.n_yca = (int)h.yca.size();
   s->d_ymult = reinterpret_cast<double*>(b + o_ym);
   s->d_yjjb = reinterpret_cast<int32_t*>(b + o_yjjb);
   return IPG_OK;
@@ -3791,7 +3380,7 @@ struct EvalOut {
   PairList* pl_out = nullptr;          // receives the pair list (stays valid until the next build)
   const double2** utot_out = nullptr;  // receives Utot [n][idxu_max] when the chain kernel made it
   const double2** yw_out = nullptr;    // adjoint mode: receives the weighted Y [u_half][n] of the chain path
-  double2* zall = nullptr;  // adjoint mode: also write Z [idxz_max][n] here (row-blocked Y kernel only)
+  double2* zall = nullptr;  // adjoint mode: also write Z [idxz_max][n] here (streamed kernel only)
   bool* zall_done = nullptr;  // set when zall was written
 };
 
@@ -3803,16 +3392,7 @@ int64_t zrows_chunk(const ipg_snap* s, const SnapDev& dev, int64_t n) {
   return std::max<int64_t>(1, std::min(C, n));
 }
 
-// Shared memory and blocks per SM of k_snap_yrows<YM_Z>.
-int zrows_config(ipg_ctx* ctx, const SnapDev& dev, int* ysm, int* per_sm) {
-  *ysm = yr_smem(dev.J, dev.nsp, dev.n_ytrip, dev.n_yca, dev.u_half, dev.n_yrows).total();
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_yrows<YM_Z>, cudaFuncAttributeMaxDynamicSharedMemorySize, *ysm));
-  *per_sm = 1;
-  CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_snap_yrows<YM_Z>, YS_WARPS * 32, *ysm));
-  return IPG_OK;
-}
-
-// Plain dB/dr path on the register chains: per chunk of atoms, Z (row-blocked kernel), B and
+// Plain dB/dr path on the register chains: per chunk of atoms, Z (streamed kernel), B and
 // E_i (k_snap_bdesc), then dbl of the pairs those atoms own (k_snap_dbfused).
 int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl, const int32_t* d_species,
                  const double2* utot, double* B, double* Ei, double* dbl) {
@@ -3820,8 +3400,6 @@ int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
   const int64_t C = zrows_chunk(s, dev, n);
   double2* Z;
   IPG_RET(scratch(ctx, "snap_Z", (size_t)C * dev.idxz_max + 1, &Z));
-  int ysm, yper;
-  IPG_RET(zrows_config(ctx, dev, &ysm, &yper));
   const int bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)dev.K * YS_ATOMS * 8);
   CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
   int bper = 1;
@@ -3829,9 +3407,8 @@ int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
   for (int64_t a0 = 0; a0 < n; a0 += C) {
     const int64_t nc = std::min(C, n - a0);
     const int64_t tiles = (nc + YS_ATOMS - 1) / YS_ATOMS;
-    const int64_t yg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, yper));
-    IPG_TIMED_LAUNCH(ctx, "snap_zrows", k_snap_yrows<YM_Z>, (unsigned)yg, YS_WARPS * 32, ysm, dev, s->h.yconst, nc,
-                     d_species + a0, utot + (size_t)a0 * dev.idxu_max, Z, (double*)nullptr, (double2*)nullptr);
+    IPG_RET(launch_ystream(ctx, dev, s->h.yktab, YM_Z, "snap_zrows", nc, d_species + a0, utot + (size_t)a0 * dev.idxu_max, nullptr,
+                           nullptr, Z));
     const int64_t bg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, bper));
     IPG_TIMED_LAUNCH(ctx, "snap_bdesc", k_snap_bdesc, (unsigned)bg, GB_WARPS * 32, bsm, dev, a0, nc, d_species, Z,
                      utot, B, Ei);
@@ -3848,43 +3425,18 @@ int launch_y(ipg_snap* s, const SnapDev& dev, const char* tname, int64_t n, cons
              const double2* utot, double2* yout, double* Ei, double2* zall, bool* zall_done, bool* done) {
   ipg_ctx* ctx = s->ctx;
   *done = false;
-  size_t ysm = (size_t)dev.u_half * YS_ATOMS * sizeof(double2);
+  const size_t ysm = (size_t)dev.u_half * YS_ATOMS * sizeof(double2);
   if (n == 0 || ysm > 200 * 1024) return IPG_OK;  // atoms-in-lanes: the Utot of 32 atoms in shared memory
-  const bool rows = dev.J <= YR_MAX_J && !s->y_entries && s->h.yconst_ok;
-  const bool withz = rows && zall;
-  // warps per block of the Y-only kernel (IPG_YR_WARPS: 8, 10, 12 or 16)
-  const int yw = rows && !withz ? s->yr_warps : YS_WARPS;
-  const int ythreads = yw * 32;
-  const void* kfn = !rows       ? (const void*)k_snap_yatoms
-                    : withz     ? (const void*)k_snap_yrows<YM_YZ>
-                    : yw == 10  ? (const void*)k_snap_yrows<YM_Y, 10>
-                    : yw == 12  ? (const void*)k_snap_yrows<YM_Y, 12>
-                    : yw == 16  ? (const void*)k_snap_yrows<YM_Y, 16>
-                                : (const void*)k_snap_yrows<YM_Y>;
-  if (rows) ysm = yr_smem(dev.J, dev.nsp, dev.n_ytrip, dev.n_yca, dev.u_half, dev.n_yrows).total();
-  CUDA_RET(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ysm));
-  int per_sm = 1;
-  CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, ythreads, ysm));
-  const int64_t groups = (n + YS_ATOMS - 1) / YS_ATOMS;
-  const int64_t grid = std::min<int64_t>(groups, (int64_t)ctx->num_sms * std::max(1, per_sm));
-  if (withz) {
-    IPG_TIMED_LAUNCH(ctx, tname, k_snap_yrows<YM_YZ>, (unsigned)grid, ythreads, ysm, dev, s->h.yconst, n, d_species,
-                     utot, yout, Ei, zall);
-    if (zall_done) *zall_done = true;
-  } else if (rows && yw == 10) {
-    IPG_TIMED_LAUNCH(ctx, tname, (k_snap_yrows<YM_Y, 10>), (unsigned)grid, ythreads, ysm, dev, s->h.yconst, n,
-                     d_species, utot, yout, Ei, (double2*)nullptr);
-  } else if (rows && yw == 12) {
-    IPG_TIMED_LAUNCH(ctx, tname, (k_snap_yrows<YM_Y, 12>), (unsigned)grid, ythreads, ysm, dev, s->h.yconst, n,
-                     d_species, utot, yout, Ei, (double2*)nullptr);
-  } else if (rows && yw == 16) {
-    IPG_TIMED_LAUNCH(ctx, tname, (k_snap_yrows<YM_Y, 16>), (unsigned)grid, ythreads, ysm, dev, s->h.yconst, n,
-                     d_species, utot, yout, Ei, (double2*)nullptr);
-  } else if (rows) {
-    IPG_TIMED_LAUNCH(ctx, tname, k_snap_yrows<YM_Y>, (unsigned)grid, ythreads, ysm, dev, s->h.yconst, n, d_species,
-                     utot, yout, Ei, (double2*)nullptr);
+  if (dev.J <= YR_MAX_J && !s->y_entries) {
+    IPG_RET(launch_ystream(ctx, dev, s->h.yktab, zall ? YM_YZ : YM_Y, tname, n, d_species, utot, yout, Ei, zall));
+    if (zall && zall_done) *zall_done = true;
   } else {
-    IPG_TIMED_LAUNCH(ctx, tname, k_snap_yatoms, (unsigned)grid, ythreads, ysm, dev, n, d_species, utot, yout, Ei);
+    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_yatoms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ysm));
+    int per_sm = 1;
+    CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_yatoms, YS_WARPS * 32, ysm));
+    const int64_t groups = (n + YS_ATOMS - 1) / YS_ATOMS;
+    const int64_t grid = std::min<int64_t>(groups, (int64_t)ctx->num_sms * std::max(1, per_sm));
+    IPG_TIMED_LAUNCH(ctx, tname, k_snap_yatoms, (unsigned)grid, YS_WARPS * 32, ysm, dev, n, d_species, utot, yout, Ei);
   }
   *done = true;
   return IPG_OK;
@@ -4003,7 +3555,7 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
   } else if (need_plain) {
     IPG_RET(scratch(ctx, "snap_dbl", (size_t)np * K * 3 + 3, &dbl));
     io.dbl = dbl;
-    if (n && chains && dev.J <= YR_MAX_J && s->h.yconst_ok && cap == 0 && !s->generic_plain)
+    if (n && chains && dev.J <= YR_MAX_J && cap == 0 && !s->generic_plain)
       IPG_RET(plain_chains(s, dev, n, pl, d_species, io.utot_in, out.B, Ei, dbl));
     else if (n)
       IPG_RET(launch_atoms<MODE_PLAIN>(s, dev, io, n, nullptr));
@@ -4012,13 +3564,11 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
       if (n) IPG_TIMED_LAUNCH(ctx, "snap_contract", k_snap_contract, nblk(32 * n, 256), 256, 0, n, pl.d_off, d_species, nsp, dbl, dev.beta, K,
                                (int64_t)0, (int64_t)K, fvec);
     }
-  } else if (chains && n && dev.J <= YR_MAX_J && s->h.yconst_ok && cap == 0) {
-    // Z from the row-blocked kernel per chunk of atoms, then B (and E_i) per atom tile
+  } else if (chains && n && dev.J <= YR_MAX_J && cap == 0) {
+    // Z from the streamed kernel per chunk of atoms, then B (and E_i) per atom tile
     const int64_t C = zrows_chunk(s, dev, n);
     double2* Z;
     IPG_RET(scratch(ctx, "snap_Z", (size_t)C * dev.idxz_max + 1, &Z));
-    int ysm, yper;
-    IPG_RET(zrows_config(ctx, dev, &ysm, &yper));
     const int bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)K * YS_ATOMS * 8);
     CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
     int bper = 1;
@@ -4026,9 +3576,8 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     for (int64_t a0 = 0; a0 < n; a0 += C) {
       const int64_t nc = std::min(C, n - a0);
       const int64_t tiles = (nc + YS_ATOMS - 1) / YS_ATOMS;
-      const int64_t yg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, yper));
-      IPG_TIMED_LAUNCH(ctx, "snap_zrows", k_snap_yrows<YM_Z>, (unsigned)yg, YS_WARPS * 32, ysm, dev, s->h.yconst, nc,
-                       d_species + a0, io.utot_in + (size_t)a0 * dev.idxu_max, Z, (double*)nullptr, (double2*)nullptr);
+      IPG_RET(launch_ystream(ctx, dev, s->h.yktab, YM_Z, "snap_zrows", nc, d_species + a0, io.utot_in + (size_t)a0 * dev.idxu_max, nullptr,
+                           nullptr, Z));
       const int64_t bg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, bper));
       IPG_TIMED_LAUNCH(ctx, "snap_bdesc", k_snap_bdesc, (unsigned)bg, GB_WARPS * 32, bsm, dev, a0, nc, d_species, Z,
                        io.utot_in, out.B, Ei);
@@ -4139,7 +3688,7 @@ int snap_train_step(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
   double2* Z = nullptr;
   bool zdone = false;
   const bool chains = dev.J <= PAIR_CHAIN_MAX_J && !s->generic_adjoint && !dev.chem && !dev.quadratic;
-  if (chains && dev.J <= YR_MAX_J && s->h.yconst_ok && !s->y_entries && n &&
+  if (chains && dev.J <= YR_MAX_J && !s->y_entries && n &&
       (size_t)n * dev.idxz_max * sizeof(double2) <= TRAIN_Z_MAX) {
     IPG_RET(scratch(ctx, "train_Z", (size_t)n * dev.idxz_max + 1, &Z));
     oo.zall = Z;
@@ -4424,10 +3973,6 @@ int ipg_snap_create(ipg_ctx* ctx, const ipg_snap_params* params, ipg_snap** out)
   if (const char* g = getenv("IPG_VJP_CHUNK")) s->vjp_chunk = std::max<int64_t>(0, atoll(g));
   if (const char* g = getenv("IPG_GENERIC_PLAIN")) s->generic_plain = g[0] == '1';
   if (const char* g = getenv("IPG_GENERIC_HVP")) s->generic_hvp = g[0] == '1';
-  if (const char* g = getenv("IPG_YR_WARPS")) {
-    const int w = atoi(g);
-    s->yr_warps = (w == 8 || w == 10 || w == 16) ? w : 12;
-  }
   // cutoffs, utl.jl:41-56
   const int ns = p.nspecies;
   s->cutsq.assign(ns * ns, 0.0);
@@ -4610,7 +4155,7 @@ namespace {
 // resident.  g = cotangent of forces [3n] (device), gE scalar.
 // reuse_pl / reuse_utot: the pair list and Utot of an evaluation of the same positions just
 // before (snap_eval's pl_out / utot_out), or null to build them here.
-// reuse_Z: Z [idxz_max][n] of the same positions (k_snap_yrows<YM_YZ>), or null to form it here.
+// reuse_Z: Z [idxz_max][n] of the same positions (k_snap_ystream<YM_YZ>), or null to form it here.
 // v_out (optional): receives V [u_half][n] (V = sum_j (g_i - g_j) . d(sfac U_ij)/dr_ij) when the
 // chain path formed it in one chunk, else null.
 int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_species, int nconf,
@@ -4665,8 +4210,8 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
     IPG_RET(launch_utot(ctx, dev, n, pl.d_off, pl.d_j, pl.d_r, d_species, utot, s->utot_warps, !s->utot_split));
     io.utot_in = utot;
   }
-  if (io.utot_in && dev.J <= YR_MAX_J && s->h.yconst_ok) {
-    // register-chain path: Z (row-blocked kernel) and V per chunk of atoms, then the
+  if (io.utot_in && dev.J <= YR_MAX_J) {
+    // register-chain path: Z (streamed kernel) and V per chunk of atoms, then the
     // contraction
     const bool zgiven = reuse_Z && reuse_pl && reuse_utot;
     const int64_t C = zgiven ? n : zrows_chunk(s, dev, n);
@@ -4677,8 +4222,7 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
     else
       IPG_RET(scratch(ctx, "snap_Z", (size_t)C * dev.idxz_max + 1, &Z));
     IPG_RET(scratch(ctx, "snap_vjp_V", (size_t)C * dev.u_half + 1, &V));
-    int ysm, yper, gper = 1;
-    IPG_RET(zrows_config(ctx, dev, &ysm, &yper));
+    int gper = 1;
     const bool withB = gE != 0.0;
     const int gsm = (int)((withB ? 2 : 1) * (size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)nsp * K * 8);
     CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_gbeta, cudaFuncAttributeMaxDynamicSharedMemorySize, gsm));
@@ -4690,11 +4234,9 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
     for (int64_t c = 0; c < nchunk; c++) {
       const int64_t a0 = c * C, nc = std::min(C, n - a0);
       const int64_t tiles = (nc + YS_ATOMS - 1) / YS_ATOMS;
-      const int64_t yg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, yper));
       if (!zgiven)
-        IPG_TIMED_LAUNCH(ctx, "snap_zrows", k_snap_yrows<YM_Z>, (unsigned)yg, YS_WARPS * 32, ysm, dev, s->h.yconst,
-                         nc, d_species + a0, io.utot_in + (size_t)a0 * dev.idxu_max, Z, (double*)nullptr,
-                         (double2*)nullptr);
+        IPG_RET(launch_ystream(ctx, dev, s->h.yktab, YM_Z, "snap_zrows", nc, d_species + a0, io.utot_in + (size_t)a0 * dev.idxu_max, nullptr,
+                           nullptr, Z));
       IPG_RET(launch_vsum(ctx, dev, a0, nc, pl.d_off, pl.d_j, pl.d_r, d_species, d_g, V, s->pair_tangent));
       const int64_t gg = std::min(tiles, gmax);
       IPG_TIMED_LAUNCH(ctx, "snap_gbeta", k_snap_gbeta, (unsigned)gg, GB_WARPS * 32, gsm, dev, a0, nc, d_species, Z,
@@ -4764,7 +4306,7 @@ int ipg_snap_vjp(ipg_snap* s, int64_t n, const double* pos, const int32_t* speci
   // both pullbacks from one evaluation: its list, Utot and Z (Y kernel in its Y+Z mode) serve
   // the beta pullback, whose V (gF contracted with dU/dr) is the Utot tangent of H gF
   const bool fused = gbeta && gpos && gF && n > 0 && !d0.chem && !d0.quadratic && d0.J <= YR_MAX_J &&
-                     !s->generic_adjoint && !s->y_entries && s->h.yconst_ok && !s->generic_hvp;
+                     !s->generic_adjoint && !s->y_entries && !s->generic_hvp;
   if (gbeta && !fused) IPG_RET(ipg_snap_vjp_beta(s, n, pos, species, L, gE, gF, gbeta, nullptr));
   if (gbeta0) *gbeta0 = gE;
   if (!gpos || n == 0) return IPG_OK;
@@ -4936,7 +4478,7 @@ int ipg_snap_autotune(ipg_snap* s, int64_t n, const double* pos, const int32_t* 
     };
     int st = measure(best, &best.ms);
     // coordinate descent: each knob in turn, the others at their best so far
-    const bool rows_ok = s->dev.J <= YR_MAX_J && s->h.yconst_ok, chains_ok = s->dev.J <= PAIR_CHAIN_MAX_J && !s->generic_adjoint;
+    const bool rows_ok = s->dev.J <= YR_MAX_J, chains_ok = s->dev.J <= PAIR_CHAIN_MAX_J && !s->generic_adjoint;
     for (int knob = 0; knob < 5 && st == IPG_OK; knob++) {
       std::vector<int> vals;
       if (knob == 0 && rows_ok) vals = {0, 1};

@@ -27,39 +27,43 @@ struct DBDev {
 constexpr int SNAP_MAX_J = 12;
 constexpr int YS_WARPS = 8;     // warps of the atoms-in-lanes Y kernels
 constexpr int YS_ATOMS = 32;    // atoms per block of those kernels (one per lane)
-constexpr int YR_MAX_J = 8;     // largest twojmax of the row-blocked Y kernel
-constexpr int yr_rows(int J) { return J < 0 ? 0 : yr_rows(J - 1) + J / 2 + 1; }  // target rows (j, mb <= j/2)
+constexpr int YR_MAX_J = 8;     // largest twojmax of the streamed Y / Z kernel
 
-// Row-blocked Y kernel: a target row (j, mb) of the half plane of Y and the (j1, j2)
-// triples whose Z entries feed it.
-struct YRowDev {
-  int8_t j, mb, mid, pad;  // mid: middle row of an even level (weights vanish beyond ma = mb)
-  int32_t h0;              // half-plane index of (j, mb, ma = 0)
-  int32_t t0, t1;          // its triples: yitems[t0 .. t1)
+// Streamed Y / Z contraction (ipg_snap_y.cu): an item is the entries (k = -(2 mb - j), YT adjacent
+// columns c = 2 ma - j) of every level j, jmin <= j <= J of its parity.  Its weights [row pair]
+// [step][level][YT] follow one another in a stream of 16-byte units; a record is a run of row
+// pairs of one (j1, j2), as many as fit YREC units.  Items, records and row pairs travel as a
+// kernel parameter (constant bank), so that everything but the products runs on uniform registers.
+constexpr int YT = 2;                  // columns per item
+constexpr int YNJ = YR_MAX_J / 2 + 1;  // levels per item, at most
+constexpr int YGUARD = 2;              // a row walk reads at most two entries past either end of a row
+constexpr int YREC = 48;               // 16-byte units per record, at most
+// record: row pairs (4 bits) | steps of each << 4 | levels << 8 | first of them << 11 | first, last
+// record of its (j1, j2) << 14, 15 | size in units << 16 | first triple << 24
+constexpr int YF_STEPS = 4, YF_N = 8, YF_LO = 11, YF_SIZE = 16, YF_TRIP = 24;
+constexpr uint32_t YF_FIRST = 1u << 14, YF_LAST = 1u << 15;
+// row pair: byte offsets, in the block's half plane, of the first element of row 1 and of the
+// element of row 2 for column t = 0 (signed: it may lie before the row); bit 0: that row lies
+// beyond the half plane
+struct YkItem {
+  int32_t unit;            // first unit of its weights
+  int16_t rec, nrec, pair; // first record, records, first row pair
+  int16_t k, c0, nt, jmin; // nt: columns in use
+  int16_t pad;
 };
-struct YItemDev {
-  int8_t j1, j2, d, nb, mb1min, mb2max, pad0, pad1;  // d = (j1 + j2 - j) / 2
-  int32_t ca;   // offset in yca of the triple's CG factors, [m0/2][ma][2] (zero where out of range)
-  int32_t cg;   // idxcg_block[j1][j2][j]: the row factors cg[mb1 (j2+1) + mb2]
-  int32_t jjz;  // first Z entry of the triple (its Y coefficient)
-  int32_t trip; // index of the triple (its coefficient slot in the kernel's shared table)
+constexpr int YK_ITEMS = 40, YK_RECS = 1200, YK_PAIRS = 2400;
+struct YkTab {
+  YkItem item[YK_ITEMS];  // longest first
+  uint32_t rec[YK_RECS + 4];  // zero past the last: the walk looks two records ahead
+  int2 pair[YK_PAIRS];
+  int32_t nitem, pad;
 };
-static_assert(sizeof(YItemDev) == 24, "YItemDev layout");
-
-// The row-blocked Y kernel's warp-uniform tables, passed by value as a kernel parameter
-// (constant bank: uniform reads through the constant cache, private to each launch).
-constexpr int YC_ROWS = 28, YC_ITEMS = 400, YC_RP = 1536;
-struct YConst {
-  YRowDev rows[YC_ROWS];    // target rows, longest first
-  YItemDev items[YC_ITEMS]; // their triples (field cg: offset of the first row factor in cb)
-  double cb[YC_RP];         // cg[mb1][mb2] of every row pair of every item
-  int nrows, nitems, nrp, pad;
-};
+constexpr int YM_Y = 0, YM_Z = 1, YM_YZ = 2;  // what launch_ystream writes
 
 struct SnapDev {
   int J, nsp, K, idxu_max, idxz_max, u_half, ext_max, idxcg_max;
-  int switch_flag, bzero_flag, bnorm_flag, n_yrows;
-  int n_ytrip, n_yca;  // row-blocked Y kernel: triples, doubles in yca
+  int switch_flag, bzero_flag, bnorm_flag;
+  int n_ytrip;  // streamed Y / Z: triples
   double rcutfac, rmin0, rfac0, wself;
   double radii[IPG_MAX_SNAP_SPECIES], weight[IPG_MAX_SNAP_SPECIES];
   int idxu_block[SNAP_MAX_J + 2];
@@ -82,10 +86,7 @@ struct SnapDev {
   const int32_t* u_of_h;      // [u_half] index of half-plane entry h in the full Utot
   const int32_t* h_info;      // [u_half] m | j << 8 | (m within the row's weighted entries) << 16, m = column ma
   const double2* h_sgen;      // [u_half] the generator factors (s_m, s_{m-1}), s_m = sqrt((m+1)(j-m)), 0 off the row
-  // row-blocked Y kernel (twojmax <= YR_MAX_J): n_yrows target rows, longest first
-  const YRowDev* yrows;
-  const YItemDev* yitems;
-  const double* yca;
+  const double2* ykstream;    // streamed Y / Z (twojmax <= YR_MAX_J): the weights
   const int32_t* ytrip_jjz;  // [n_ytrip] first Z entry of each triple
   // explicit multi-element SNAP (chem_flag) and quadratic SNAP: K is then the number of
   // components per species block, klin of them linear (idxb_max per element triple), the rest
@@ -111,12 +112,14 @@ struct SnapHost {
   std::vector<int32_t> ysched_off, ysched_h, u_of_h, h_info;
   std::vector<double> h_sgen;  // 2 per half-plane entry
   std::vector<double> ysched_w;
-  std::vector<YRowDev> yrows;
-  std::vector<YItemDev> yitems;
-  std::vector<double> yca;
+  YkTab yktab;
+  std::vector<double> ykstream;  // 2 per 16-byte unit
   std::vector<int32_t> ytrip_jjz;
-  bool yconst_ok = false;  // the tables fit YConst
-  YConst yconst;
 };
 
 int snap_build_tables(const ipg_snap_params& p, SnapHost& h);
+
+struct ipg_ctx;
+// Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu).
+int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n, const int32_t* species,
+                   const double2* utot, double2* yout, double* Ei, double2* zout);

@@ -255,106 +255,101 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
   std::vector<int32_t> fill(h.y_off.begin(), h.y_off.end() - 1);
   for (int z = 0; z < h.idxz_max; z++) h.y_jjz[fill[h.zjju_half[z]]++] = z;
 
-  // Row-blocked Y schedule.  Target row (j, mb) of the half plane collects, for every
-  // triple (j1 >= j2, j), the Z entries (j1, j2, j, ma, mb) of all ma at once: the nb row
-  // pairs (mb1, mb2) are the same for every ma, and for one row pair
-  //   Z(ma) += cg[mb1][mb2] sum_ma2 cg[ma + d - ma2][ma2] U(j1, mb1, ma + d - ma2) U(j2, mb2, ma2)
-  // with d = (j1 + j2 - j)/2.  The CG factors ca[ma][ma2] of a triple are stored by column
-  // pair as [m0/2][ma][2] (yca; 16-byte pairs), zero where ma2 > j2 or ma1 = ma + d - ma2
-  // falls outside 0..j1.  Rows are listed longest first (the kernel hands them out in
-  // that order to whichever warp is free).
-  h.yrows.clear();
-  h.yitems.clear();
-  h.yca.clear();
+  // Streamed Y / Z contraction (layout: ipg_snap.cuh).  Items (k, YT adjacent columns c) in the
+  // doubled indices k = -(2 mb - j) >= 0, c = 2 ma - j; the centre row k = 0 needs c <= 0 only.
+  memset(&h.yktab, 0, sizeof(h.yktab));
+  h.ykstream.clear();
   h.ytrip_jjz.clear();
   if (J <= YR_MAX_J) {
-    std::vector<int32_t> ca_of(jd * jd * jd, -1), trip_of(jd * jd * jd, -1);
+    std::vector<int32_t> trip_of(jd * jd * jd, -1);
     for (int j1 = 0; j1 <= J; j1++)
       for (int j2 = 0; j2 <= j1; j2++)
-        for (int j = j1 - j2; j <= std::min(J, j1 + j2); j += 2) {
-          const int d = (j1 + j2 - j) / 2, cg0 = h.idxcg_block[blk(j1, j2, j)];
-          ca_of[blk(j1, j2, j)] = (int32_t)h.yca.size();
+        for (int j = j1 - j2; j <= std::min(J, j1 + j2); j += 2) {  // the levels of a pair are adjacent
           trip_of[blk(j1, j2, j)] = (int32_t)h.ytrip_jjz.size();
           h.ytrip_jjz.push_back(h.idxz_block[blk(j1, j2, j)]);
-          for (int m0 = 0; m0 <= j2; m0 += 2)  // column pairs (m0, m0 + 1), as [m0/2][ma][2]
-            for (int ma = 0; ma <= j; ma++)
-              for (int q = 0; q < 2; q++) {
-                const int ma2 = m0 + q, ma1 = ma + d - ma2;
-                const bool ok = ma2 <= j2 && ma1 >= 0 && ma1 <= j1;
-                h.yca.push_back(ok ? h.cglist[cg0 + ma1 * (j2 + 1) + ma2] : 0.0);
-              }
         }
-    struct Row {
-      YRowDev r;
-      std::vector<YItemDev> items;
-      double cost;
+    struct Item {
+      YkItem it;
+      std::vector<uint32_t> recs;
+      std::vector<int2> pairs;
+      std::vector<double> w;
+      double cost = 0.0;
     };
-    std::vector<Row> rows;
-    for (int j = 0; j <= J; j++)
-      for (int mb = 0; 2 * mb <= j; mb++) {
-        Row row;
-        row.r.j = (int8_t)j;
-        row.r.mb = (int8_t)mb;
-        row.r.mid = (int8_t)(2 * mb == j);
-        row.r.pad = 0;
-        row.r.h0 = h.half_block[j] + mb * (j + 1);
-        row.cost = 0.0;
-        const int nma = row.r.mid ? mb + 1 : j + 1;
+    std::vector<Item> items;
+    for (int k = 0; k <= J; k++) {
+      const int cmax = k == 0 ? 0 : J - ((J - k) & 1);
+      for (int c0 = -(J - ((J - k) & 1)); c0 <= cmax; c0 += 2 * YT) {
+        Item I;
+        memset(&I.it, 0, sizeof(I.it));
+        int nt = 0, jmin = J + 1;
+        for (int t = 0; t < YT && c0 + 2 * t <= cmax; t++) {
+          nt++;
+          jmin = std::min(jmin, std::max(k, std::abs(c0 + 2 * t)));
+        }
+        I.it.k = (int16_t)k;
+        I.it.c0 = (int16_t)c0;
+        I.it.nt = (int16_t)nt;
+        I.it.jmin = (int16_t)jmin;
         for (int j1 = 0; j1 <= J; j1++)
           for (int j2 = 0; j2 <= j1; j2++) {
-            if (j < j1 - j2 || j > std::min(J, j1 + j2) || ((j1 + j2 + j) & 1)) continue;
-            const int mb1min = std::max(0, (2 * mb - j - j2 + j1) / 2);
-            const int mb2max = (2 * mb - j - (2 * mb1min - j1) + j2) / 2;
-            const int nb = std::min(j1, (2 * mb - j + j2 + j1) / 2) - mb1min + 1;
-            if (nb <= 0) continue;
-            YItemDev it;
-            it.j1 = (int8_t)j1;
-            it.j2 = (int8_t)j2;
-            it.d = (int8_t)((j1 + j2 - j) / 2);
-            it.nb = (int8_t)nb;
-            it.mb1min = (int8_t)mb1min;
-            it.mb2max = (int8_t)mb2max;
-            it.pad0 = it.pad1 = 0;
-            it.ca = ca_of[blk(j1, j2, j)];
-            it.cg = h.idxcg_block[blk(j1, j2, j)];
-            it.jjz = h.idxz_block[blk(j1, j2, j)];
-            it.trip = trip_of[blk(j1, j2, j)];
-            row.items.push_back(it);
-            row.cost += nb * (6.0 * nma * (j2 + 1) + (nma + 2 * j2 + 8));
+            const int jlo = std::max(jmin, j1 - j2), jhi = std::min(J, j1 + j2);
+            if (((j1 + j2 - k) & 1) || jlo > jhi) continue;
+            const int N = (jhi - jlo) / 2 + 1;
+            const int E = (c0 + j1 + j2) / 2;  // ma1 + ma2 of column t is E + t
+            const int lo1 = std::max(0, E - j2), hi1 = std::min(j1, E + nt - 1);
+            if (lo1 > hi1) continue;
+            const size_t first = I.recs.size();
+            for (int mb1 = 0; mb1 <= j1; mb1++) {
+              const int mb2 = (j1 + j2 - k) / 2 - mb1;
+              if (mb2 < 0 || mb2 > j2) continue;
+              const bool mir1 = 2 * mb1 > j1, mir2 = 2 * mb2 > j2;  // at most one of them: k >= 0
+              const int e1 = h.half_block[j1] + (mir1 ? (j1 - mb1) * (j1 + 1) + j1 - lo1 : mb1 * (j1 + 1) + lo1);
+              const int ma2 = E - lo1;  // column t = 0 of the first step
+              const int e2 = h.half_block[j2] + (mir2 ? (j2 - mb2) * (j2 + 1) + j2 - ma2 : mb2 * (j2 + 1) + ma2);
+              const int steps = hi1 - lo1 + 1, units = steps * N * YT / 2;
+              if (I.recs.size() == first || (int)((I.recs.back() >> YF_SIZE) & 0xff) + units > YREC)
+                I.recs.push_back((uint32_t)steps << YF_STEPS | (uint32_t)N << YF_N | (uint32_t)((jlo - jmin) / 2) << YF_LO |
+                                 (uint32_t)trip_of[blk(j1, j2, jlo)] << YF_TRIP);
+              I.recs.back() += 1u | (uint32_t)units << YF_SIZE;
+              I.pairs.push_back(make_int2(e1 * YS_ATOMS * 16 | (int)mir1, e2 * YS_ATOMS * 16 | (int)mir2));
+              for (int ma1 = lo1; ma1 <= hi1; ma1++)
+                for (int j = jlo; j <= jhi; j += 2) {
+                  const int cg0 = h.idxcg_block[blk(j1, j2, j)];
+                  const double cb = h.cglist[cg0 + mb1 * (j2 + 1) + mb2] * (p.bnorm_flag ? 1.0 / (j + 1) : 1.0);
+                  for (int t = 0; t < YT; t++) {
+                    const int m2 = E + t - ma1, c = c0 + 2 * t;
+                    const bool ok = t < nt && m2 >= 0 && m2 <= j2 && std::abs(c) <= j;
+                    const int sg = mir1 ? ma1 + mb1 : (mir2 ? m2 + mb2 : 0);  // sign of the mirrored element
+                    I.w.push_back(ok ? ((sg & 1) ? -cb : cb) * h.cglist[cg0 + ma1 * (j2 + 1) + m2] : 0.0);
+                  }
+                }
+              I.cost += steps * YT * (4.0 + 2.0 * N) + 20.0;
+            }
+            if (I.recs.size() > first) {
+              I.recs[first] |= YF_FIRST;
+              I.recs.back() |= YF_LAST;
+            }
           }
-        rows.push_back(row);
+        items.push_back(std::move(I));
       }
-    std::vector<int> order(rows.size());
-    for (size_t q = 0; q < rows.size(); q++) order[q] = (int)q;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rows[a].cost > rows[b].cost; });
-    for (int q : order) {
-      YRowDev r = rows[q].r;
-      r.t0 = (int32_t)h.yitems.size();
-      h.yitems.insert(h.yitems.end(), rows[q].items.begin(), rows[q].items.end());
-      r.t1 = (int32_t)h.yitems.size();
-      h.yrows.push_back(r);
     }
-    // the constant-bank copy: item.cg becomes the offset of its first row factor in cb
-    memset(&h.yconst, 0, sizeof(h.yconst));
-    int nrp = 0;
-    for (const YItemDev& it : h.yitems) nrp += it.nb;
-    h.yconst_ok = (int)h.yrows.size() <= YC_ROWS && (int)h.yitems.size() <= YC_ITEMS && nrp <= YC_RP;
-    if (h.yconst_ok) {
-      YConst& C = h.yconst;
-      C.nrows = (int)h.yrows.size();
-      C.nitems = (int)h.yitems.size();
-      for (int q = 0; q < C.nrows; q++) C.rows[q] = h.yrows[q];
-      int o = 0;
-      for (int t = 0; t < C.nitems; t++) {
-        YItemDev it = h.yitems[t];
-        const int cg0 = it.cg;
-        it.cg = o;
-        for (int ib = 0; ib < it.nb; ib++)
-          C.cb[o++] = h.cglist[cg0 + (it.mb1min + ib) * (it.j2 + 1) + (it.mb2max - ib)];
-        C.items[t] = it;
-      }
-      C.nrp = o;
+    std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
+    YkTab& T = h.yktab;
+    int nrec = 0, npair = 0;
+    if (items.size() > (size_t)YK_ITEMS) return IPG_ERR_UNSUPPORTED;  // sized for YR_MAX_J
+    for (Item& I : items) {
+      if (nrec + I.recs.size() > (size_t)YK_RECS || npair + I.pairs.size() > (size_t)YK_PAIRS)
+        return IPG_ERR_UNSUPPORTED;
+      I.it.unit = (int32_t)(h.ykstream.size() / 2);
+      I.it.rec = (int16_t)nrec;
+      I.it.nrec = (int16_t)I.recs.size();
+      I.it.pair = (int16_t)npair;
+      for (uint32_t r : I.recs) T.rec[nrec++] = r;
+      for (const int2& q : I.pairs) T.pair[npair++] = q;
+      h.ykstream.insert(h.ykstream.end(), I.w.begin(), I.w.end());
+      T.item[T.nitem++] = I.it;
     }
+    h.ykstream.resize(h.ykstream.size() + 2 * 2 * YREC, 0.0);  // the walk copies up to two records past an item
   }
   return IPG_OK;
 }
