@@ -2855,148 +2855,11 @@ __global__ void __launch_bounds__(CONF_T) k_conf_reduce(int nconf, const int64_t
   if (threadIdx.x < 6 && W6) W6[6 * c + threadIdx.x] = sm[1 + threadIdx.x][0];
 }
 
-// Per-atom force descriptors: dB_k[block s][b][c] = sum_{p in out(k), s_k = s} dbl_p -
-// sum_{q in in(k), s_owner(q) = s} dbl_q   (snap.jl:289-290).  One thread per (atom, b*3+c).
-__global__ void k_snap_dB_atoms(int64_t n, int K, int nsp, const int64_t* __restrict__ off,
-                                const int64_t* __restrict__ in_off, const int64_t* __restrict__ in_pair,
-                                const int32_t* __restrict__ owner, const int32_t* __restrict__ species,
-                                const double* __restrict__ dbl, double* __restrict__ dB, int rows) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int64_t k = t / (3 * K);
-  int bc = (int)(t - k * 3 * K);
-  if (k >= n) return;
-  double acc[IPG_MAX_SNAP_SPECIES];
-#pragma unroll
-  for (int s = 0; s < IPG_MAX_SNAP_SPECIES; s++) acc[s] = 0.0;
-  const int sk = species[k];
-  double own = 0.0;
-  for (int64_t p = off[k]; p < off[k + 1]; p++) own += dbl[(size_t)p * 3 * K + bc];
-#pragma unroll
-  for (int s = 0; s < IPG_MAX_SNAP_SPECIES; s++)
-    if (s == sk) acc[s] += own;
-  for (int64_t q = in_off[k]; q < in_off[k + 1]; q++) {
-    int64_t p = in_pair[q];
-    int so = species[owner[p]];
-    double v = dbl[(size_t)p * 3 * K + bc];
-#pragma unroll
-    for (int s = 0; s < IPG_MAX_SNAP_SPECIES; s++)
-      if (s == so) acc[s] -= v;
-  }
-  const int b = bc / 3, c = bc - 3 * b;
-  if (rows)  // fitting layout: row 3k + c, column s*K + b
-    for (int s = 0; s < nsp; s++) dB[((size_t)k * 3 + c) * K * nsp + (size_t)s * K + b] = acc[s];
-  else
-    for (int s = 0; s < nsp; s++) dB[((size_t)k * K * nsp + (size_t)s * K + b) * 3 + c] = acc[s];
-}
-
-// Fitting rows of each configuration (one block per configuration, threads over columns):
-// Ae[c][s*K + k] = sum of B_i[k] over the atoms i of c with species s, and
-// Aw[c][v][s*K + k] = W of the configuration's atoms (the k_snap_W_desc sum, snap.jl:267-281).
-__global__ void k_snap_fit_rows(int nconf, const int64_t* __restrict__ conf_off, int K, int nsp,
-                                const int32_t* __restrict__ species, const double* __restrict__ B,
-                                const int64_t* __restrict__ off, const int32_t* __restrict__ nbr,
-                                const double* __restrict__ pos, const double* __restrict__ dbl,
-                                double* __restrict__ Ae, double* __restrict__ Aw) {
-  const int c = blockIdx.x;
-  if (c >= nconf) return;
-  const int64_t a0 = conf_off[c], a1 = conf_off[c + 1];
-  const int KN = K * nsp;
-  for (int col = threadIdx.x; col < KN; col += blockDim.x) {
-    const int sp = col / K, b = col - sp * K;
-    if (Ae) {
-      double e = 0.0;
-      for (int64_t i = a0; i < a1; i++)
-        if (clamp_sp(species[i], nsp) == sp) e += B[(size_t)i * K + b];
-      Ae[(size_t)c * KN + col] = e;
-    }
-    if (Aw) {
-      double w[6] = {0, 0, 0, 0, 0, 0};
-      for (int64_t i = a0; i < a1; i++) {
-        if (clamp_sp(species[i], nsp) != sp) continue;
-        const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-        for (int64_t p = off[i]; p < off[i + 1]; p++) {
-          const double* d = dbl + ((size_t)p * K + b) * 3;
-          const int64_t jn = nbr[p];
-          const double dx = xi - pos[3 * jn], dy = yi - pos[3 * jn + 1], dz = zi - pos[3 * jn + 2];
-          w[0] += d[0] * dx;
-          w[1] += d[1] * dy;
-          w[2] += d[2] * dz;
-          w[3] += d[1] * dz;
-          w[4] += d[0] * dz;
-          w[5] += d[0] * dy;
-        }
-      }
-      for (int v = 0; v < 6; v++) Aw[((size_t)c * 6 + v) * KN + col] = w[v];
-    }
-  }
-}
-
 // owner[p] = the centre atom of pair p: one warp per atom, lanes over its pairs (coalesced).
 __global__ void k_pair_owner(int64_t n, const int64_t* __restrict__ off, int32_t* __restrict__ owner) {
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;
   for (int64_t p = off[i] + (threadIdx.x & 31); p < off[i + 1]; p += 32) owner[p] = (int32_t)i;
-}
-
-// Virial descriptors W[block s][b][6] = sum over pairs of dB_i/dr_ij (x) (x_i - x_j)
-// (snap.jl:292-306), per-block partials [grid][nsp*K*6].  Thread per component b,
-// atoms strided over blocks.
-__global__ void k_snap_W_desc(int64_t n, int K, int nsp, const int64_t* __restrict__ off,
-                              const int32_t* __restrict__ nbr, const int32_t* __restrict__ species,
-                              const double* __restrict__ pos, const double* __restrict__ dbl,
-                              double* __restrict__ part) {
-  extern __shared__ double wsm[];  // [nsp][K][6]
-  for (int q = threadIdx.x; q < nsp * K * 6; q += blockDim.x) wsm[q] = 0.0;
-  __syncthreads();
-  for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
-    const int s = clamp_sp(species[i], nsp);
-    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-    for (int b = threadIdx.x; b < K; b += blockDim.x) {
-      double w[6] = {0, 0, 0, 0, 0, 0};
-      for (int64_t p = off[i]; p < off[i + 1]; p++) {
-        const double* d = dbl + ((size_t)p * K + b) * 3;
-        int64_t jn = nbr[p];
-        double dx = xi - pos[3 * jn], dy = yi - pos[3 * jn + 1], dz = zi - pos[3 * jn + 2];
-        w[0] += d[0] * dx;
-        w[1] += d[1] * dy;
-        w[2] += d[2] * dz;
-        w[3] += d[1] * dz;
-        w[4] += d[0] * dz;
-        w[5] += d[0] * dy;
-      }
-      for (int c = 0; c < 6; c++) wsm[((size_t)s * K + b) * 6 + c] += w[c];
-    }
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < nsp * K * 6; q += blockDim.x) part[(size_t)blockIdx.x * nsp * K * 6 + q] = wsm[q];
-}
-
-// The W descriptors when their [nsp][K][6] sums do not fit shared memory (quadratic SNAP):
-// one thread per component b sums every atom and pair in order, straight into W.
-__global__ void k_snap_W_cols(int64_t n, int K, int nsp, const int64_t* __restrict__ off,
-                              const int32_t* __restrict__ nbr, const int32_t* __restrict__ species,
-                              const double* __restrict__ pos, const double* __restrict__ dbl, double* __restrict__ W) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= K) return;
-  for (int s = 0; s < nsp; s++)
-    for (int c = 0; c < 6; c++) W[((size_t)s * K + b) * 6 + c] = 0.0;
-  for (int64_t i = 0; i < n; i++) {
-    const int s = clamp_sp(species[i], nsp);
-    const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-    double w[6] = {0, 0, 0, 0, 0, 0};
-    for (int64_t p = off[i]; p < off[i + 1]; p++) {
-      const double* d = dbl + ((size_t)p * K + b) * 3;
-      const int64_t jn = nbr[p];
-      const double dx = xi - pos[3 * jn], dy = yi - pos[3 * jn + 1], dz = zi - pos[3 * jn + 2];
-      w[0] += d[0] * dx;
-      w[1] += d[1] * dy;
-      w[2] += d[2] * dz;
-      w[3] += d[1] * dz;
-      w[4] += d[0] * dz;
-      w[5] += d[0] * dy;
-    }
-    for (int c = 0; c < 6; c++) W[((size_t)s * K + b) * 6 + c] += w[c];
-  }
 }
 
 __global__ void k_sum_partials(int64_t nblocks, int width, const double* __restrict__ part, double* __restrict__ out,
@@ -3468,6 +3331,7 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
   io.B = out.B;
   io.status = ctx->d_status;
   const bool need_plain = (mode == MODE_PLAIN) || out.dB || out.Wd || out.Aw;
+  const bool want_desc = out.dB || out.Wd || out.Aw || out.Ae;
   const bool chemq = dev.chem || dev.quadratic;  // element-resolved / quadratic SNAP kernel
   const bool chains = dev.J <= PAIR_CHAIN_MAX_J && !s->generic_adjoint && !chemq;
   if (chains && n) {  // Utot from the register-chain kernel
@@ -3620,33 +3484,14 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     if (nconf > 0)
       IPG_LAUNCH(ctx, k_conf_reduce, (unsigned)nconf, CONF_T, 0, nconf, d_cc, part, dev.beta0, out.E, out.W6);
   }
-  if (out.dB && n) {
-    int32_t* owner;
-    IPG_RET(scratch(ctx, "snap_owner", (size_t)np + 1, &owner));
-    IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
-    IPG_LAUNCH(ctx, k_snap_dB_atoms, nblk(n * 3 * K, 128), 128, 0, n, K, nsp, pl.d_off, pl.d_in_off, pl.d_in_pair,
-               owner, d_species, dbl, out.dB, out.dB_rows ? 1 : 0);
-  }
-  if ((out.Ae || out.Aw) && n) {
-    int64_t* d_coff;
-    IPG_RET(scratch(ctx, "snap_fit_off", (size_t)nconf + 1, &d_coff));
-    CUDA_RET(ctx, cudaMemcpyAsync(d_coff, h_atom_off, sizeof(int64_t) * (nconf + 1), cudaMemcpyHostToDevice,
-                                  ctx->stream));
-    IPG_LAUNCH(ctx, k_snap_fit_rows, (unsigned)nconf, 128, 0, nconf, d_coff, K, nsp, d_species, out.B, pl.d_off,
-               pl.d_j, d_pos, dbl, out.Ae, out.Aw);
-  }
-  if (out.Wd && (size_t)nsp * K * 6 * 8 > 200 * 1024) {
-    IPG_LAUNCH(ctx, k_snap_W_cols, nblk(K, 128), 128, 0, n, K, nsp, pl.d_off, pl.d_j, d_species, d_pos, dbl, out.Wd);
-  } else if (out.Wd) {
-    const int width = nsp * K * 6;
-    int64_t grid = std::min<int64_t>(std::max<int64_t>(n, 1), 2 * ctx->num_sms);
-    double* part;
-    IPG_RET(scratch(ctx, "snap_wpart", (size_t)grid * width, &part));
-    size_t sm = (size_t)width * 8;
-    if (sm > 48 * 1024)
-      CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_W_desc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    IPG_LAUNCH(ctx, k_snap_W_desc, (unsigned)grid, 64, sm, n, K, nsp, pl.d_off, pl.d_j, d_species, d_pos, dbl, part);
-    IPG_LAUNCH(ctx, k_sum_partials, nblk(width, 128), 128, 0, grid, width, part, out.Wd, 0.0);
+  if (want_desc && n) {
+    int32_t* owner = nullptr;
+    if (out.dB) {
+      IPG_RET(scratch(ctx, "snap_owner", (size_t)np + 1, &owner));
+      IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
+    }
+    IPG_RET(launch_descriptors(ctx, K, nsp, nconf, h_atom_off, pl, owner, d_species, d_pos, dbl, out.B, out.dB,
+                               out.dB_rows, out.Wd, out.Aw, out.Ae));
   }
   if (out.pl_out) *out.pl_out = pl;
   if (out.utot_out) *out.utot_out = io.utot_in;

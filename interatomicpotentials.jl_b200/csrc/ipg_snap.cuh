@@ -123,3 +123,10 @@ struct ipg_ctx;
 // Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu).
 int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n, const int32_t* species,
                    const double2* utot, double2* yout, double* Ei, double2* zout);
+// Descriptor outputs from dbl [pair][K][3], the dB/dr of every pair (ipg_snap_desc.cu): dB
+// [n][K nsp][3], or [3 n][K nsp] with rows; Wd [K nsp][6] of one configuration; the fitting rows
+// Aw [nconf][6][K nsp] and Ae [nconf][K nsp] (from B [n][K]).  Any output may be null; owner (of
+// each pair) and the list transpose are read for dB only.
+int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h_off, const PairList& pl,
+                       const int32_t* owner, const int32_t* species, const double* pos, const double* dbl,
+                       const double* B, double* dB, bool rows, double* Wd, double* Aw, double* Ae);
