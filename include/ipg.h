@@ -230,6 +230,12 @@ IPG_API int ipg_snap_ncoeff(const ipg_snap* snap, int32_t* K);
 IPG_API int ipg_snap_descriptors(ipg_snap* snap, int64_t n, const double* pos, const int32_t* species, const double L[3],
                          double* B, double* dB, double* W, uint32_t what);
 
+/* The same descriptors, each in the row layout of the fitting matrices, for callers that keep
+ * row-major arrays (the transposes are formed on the device):
+ *   dB [n][3][K*nspecies], W [6][K*nspecies]; B and `what` as above.                       */
+IPG_API int ipg_snap_descriptors_rows(ipg_snap* snap, int64_t n, const double* pos, const int32_t* species,
+                                      const double L[3], double* B, double* dB, double* W, uint32_t what);
+
 /* potential_energy / force / energy_and_force / virial_stress of LBasisPotential over
  * SNAP (src/BasisPotentials/basis_potentials.jl:14-57, linear_potential.jl:20-49):
  *   E = beta0 + sum_i beta[s_i] . B_i,  F_k = sum_blocks dB_k[:, block] . beta[block],

@@ -3854,8 +3854,11 @@ int ipg_snap_ncoeff(const ipg_snap* s, int32_t* K) {
   return IPG_OK;
 }
 
-int ipg_snap_descriptors(ipg_snap* s, int64_t n, const double* pos, const int32_t* species, const double L[3],
-                         double* B, double* dB, double* W, uint32_t what) {
+}  // extern "C"
+
+namespace {
+int snap_descriptors(ipg_snap* s, int64_t n, const double* pos, const int32_t* species, const double L[3], double* B,
+                     double* dB, double* W, uint32_t what, bool rows) {
   IPG_RET(check_common(s, n, pos, species, L));
   ipg_ctx* ctx = s->ctx;
   if (((what & IPG_DESC_B) && !B) || ((what & IPG_DESC_DB) && !dB && n) || ((what & IPG_DESC_W) && !W))
@@ -3874,7 +3877,8 @@ int ipg_snap_descriptors(ipg_snap* s, int64_t n, const double* pos, const int32_
   if (what & IPG_DESC_W) IPG_RET(scratch(ctx, "snap_out_W", (size_t)K * nsp * 6 + 1, &W_d));
   o.B = B_d;
   o.dB = dB_d;
-  o.Wd = W_d;
+  o.dB_rows = rows;
+  (rows ? o.Aw : o.Wd) = W_d;
   int64_t aoff[2] = {0, n};
   IPG_RET(snap_eval(s, n, d_pos, d_sp, 1, aoff, L, nullptr, 0.0, MODE_DESC, o));
   if (B_d && n) IPG_RET(ipg_copy_d2h(ctx, B, B_d, sizeof(double) * n * K));
@@ -3884,6 +3888,19 @@ int ipg_snap_descriptors(ipg_snap* s, int64_t n, const double* pos, const int32_
     else memset(W, 0, sizeof(double) * K * nsp * 6);
   }
   return ipg_status_check(ctx, "ipg_snap_descriptors");
+}
+}  // namespace
+
+extern "C" {
+
+int ipg_snap_descriptors(ipg_snap* s, int64_t n, const double* pos, const int32_t* species, const double L[3],
+                         double* B, double* dB, double* W, uint32_t what) {
+  return snap_descriptors(s, n, pos, species, L, B, dB, W, what, false);
+}
+
+int ipg_snap_descriptors_rows(ipg_snap* s, int64_t n, const double* pos, const int32_t* species, const double L[3],
+                              double* B, double* dB, double* W, uint32_t what) {
+  return snap_descriptors(s, n, pos, species, L, B, dB, W, what, true);
 }
 
 int ipg_snap_set_skin(ipg_snap* s, double skin) {

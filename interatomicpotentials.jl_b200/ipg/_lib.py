@@ -32,7 +32,7 @@ API_SYMBOLS = (
     "ipg_create", "ipg_destroy", "ipg_last_error", "ipg_set_stream", "ipg_version",
     "ipg_launch_count", "ipg_timing_enable", "ipg_timing_read", "ipg_neighbor_build", "ipg_neighbor_count", "ipg_nlist_size", "ipg_nlist_export", "ipg_nlist_free",
     "ipg_pair_eval", "ipg_pair_eval_dev", "ipg_pair_eval_noalloc", "ipg_snap_create", "ipg_snap_destroy", "ipg_snap_ncoeff",
-    "ipg_snap_descriptors", "ipg_snap_energy_forces", "ipg_snap_energy_forces_dev", "ipg_snap_vjp_beta",
+    "ipg_snap_descriptors", "ipg_snap_descriptors_rows", "ipg_snap_energy_forces", "ipg_snap_energy_forces_dev", "ipg_snap_vjp_beta",
     "ipg_snap_vjp", "ipg_snap_autotune", "ipg_snap_batch_descriptors", "ipg_snap_set_skin", "ipg_snap_skin_stats",
     "ipg_snap_batch_energy_forces", "ipg_snap_batch_energy_forces_dev", "ipg_snap_batch_loss_grad",
     "ipg_snap_batch_loss_grad_dev",
@@ -91,6 +91,7 @@ def lib():
         "ipg_snap_destroy": (C.c_int, [vp]),
         "ipg_snap_ncoeff": (C.c_int, [vp, C.POINTER(i32)]),
         "ipg_snap_descriptors": (C.c_int, [vp, i64, vp, vp, vp, vp, vp, vp, u32]),
+        "ipg_snap_descriptors_rows": (C.c_int, [vp, i64, vp, vp, vp, vp, vp, vp, u32]),
         "ipg_snap_energy_forces": (C.c_int, [vp, i64, vp, vp, vp, vp, d, i32, vp, vp, vp]),
         "ipg_snap_energy_forces_dev": (C.c_int, [vp, i64, vp, vp, vp, vp, d, i32, vp, vp, vp]),
         "ipg_snap_vjp_beta": (C.c_int, [vp, i64, vp, vp, vp, d, vp, vp, vp]),

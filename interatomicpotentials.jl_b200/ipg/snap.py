@@ -123,13 +123,12 @@ class SNAP:
         n = len(system)
         nsp = len(self.species)
         sp = self.species_ids(system)
-        B = np.zeros((n, self.K)) if what & DESC_B else None
-        dB = np.zeros((n, self.K * nsp, 3)) if what & DESC_DB else None
-        W = np.zeros((self.K * nsp, 6)) if what & DESC_W else None
-        self.ctx.check(lib().ipg_snap_descriptors(self._h, n, _vp(system.positions), _vp(sp), _vp(system.L), _vp(B),
-                                                  _vp(dB), _vp(W), what))
-        return B, (None if dB is None else np.ascontiguousarray(dB.transpose(0, 2, 1))), \
-            (None if W is None else np.ascontiguousarray(W.T))
+        B = np.empty((n, self.K)) if what & DESC_B else None
+        dB = np.empty((n, 3, self.K * nsp)) if what & DESC_DB else None
+        W = np.empty((6, self.K * nsp)) if what & DESC_W else None
+        self.ctx.check(lib().ipg_snap_descriptors_rows(self._h, n, _vp(system.positions), _vp(sp), _vp(system.L),
+                                                       _vp(B), _vp(dB), _vp(W), what))
+        return B, dB, W
 
     def energy_forces(self, system, beta, beta0=0.0, mode="adjoint"):
         """E, F (n, 3), W6 for E = beta0 + sum_i beta[s_i] . B_i; beta is (K,) or (nsp, K)."""
