@@ -24,6 +24,7 @@
 
 #include "ipg_snap.cuh"
 #include "ipg_snap_chain.cuh"
+#include "ipg_snap_geom.cuh"
 
 namespace {
 
@@ -58,71 +59,13 @@ __host__ __device__ inline bool needs_levels(int mode, bool has_utot, bool has_y
   return !(has_utot && (mode == MODE_DESC || mode == MODE_ADJY || (mode == MODE_ADJ && has_yout)));
 }
 
-// Species ids are validated by the neighbor build (status word); clamping here keeps a
-// bad id from indexing the per-species tables.
-__device__ __forceinline__ int clamp_sp(int s, int nsp) { return s < 0 ? 0 : (s >= nsp ? nsp - 1 : s); }
-
 __device__ __forceinline__ double2 cmul_conj(double2 a, double2 v) {  // conj(a) * v
   return make_double2(a.x * v.x + a.y * v.y, a.x * v.y - a.y * v.x);
-}
-
-__device__ __forceinline__ double sfac_of(const SnapDev& S, double r, double rcut) {  // compute_ui.jl:350-364
-  if (!S.switch_flag) return 1.0;
-  if (r <= S.rmin0) return 1.0;
-  if (r > rcut) return 0.0;
-  return 0.5 * (cos((r - S.rmin0) * (M_PI / (rcut - S.rmin0))) + 1.0);
-}
-__device__ __forceinline__ double dsfac_of(const SnapDev& S, double r, double rcut) {  // compute_ui.jl:366-380
-  if (!S.switch_flag) return 0.0;
-  if (r <= S.rmin0) return 0.0;
-  double rcutfac = M_PI / (rcut - S.rmin0);
-  return -0.5 * (sin((r - S.rmin0) * rcutfac) * rcutfac);
 }
 
 // Number of weight-1 half-plane entries of level l (rows 2mb < l, plus ma < l/2 of the
 // middle row for even l); the middle element of an even level has weight 1/2.
 __device__ __forceinline__ int nfull_of(int l) { return ((l + 1) / 2) * (l + 1) + ((l & 1) ? 0 : l / 2); }
-
-// Per-pair geometry for the derivative recursion (compute_duidrj, compute_ui.jl:328-347
-// and the prologue of compute_duarray, :191-216).
-struct PairGeom {
-  double2 a, b;
-  double2 da[3], db[3];
-  double u[3];
-  double sfac, dsfac;
-};
-
-__device__ __forceinline__ void geom_du(const SnapDev& S, double x, double y, double z, double rcut, double wj,
-                                        PairGeom& G) {
-  double rsq = x * x + y * y + z * z;
-  double r = sqrt(rsq);
-  double rscale0 = S.rfac0 * M_PI / (rcut - S.rmin0);
-  double theta0 = (r - S.rmin0) * rscale0;
-  double sn, cs;
-  sincos(theta0, &sn, &cs);
-  double z0 = r * cs / sn;
-  double dz0dr = z0 / r - (r * rscale0) * (rsq + z0 * z0) / rsq;
-  double rinv = 1.0 / r;
-  G.u[0] = x * rinv;
-  G.u[1] = y * rinv;
-  G.u[2] = z * rinv;
-  double r0inv = 1.0 / sqrt(r * r + z0 * z0);
-  G.a = make_double2(z0 * r0inv, -z * r0inv);
-  G.b = make_double2(y * r0inv, -x * r0inv);
-  double dr0invdr = -r0inv * r0inv * r0inv * (r + z0 * dz0dr);
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    double dr0 = dr0invdr * G.u[k];
-    double dz0 = dz0dr * G.u[k];
-    G.da[k] = make_double2(dz0 * r0inv + z0 * dr0, -z * dr0);
-    G.db[k] = make_double2(y * dr0, -x * dr0);
-  }
-  G.da[2].y += -r0inv;
-  G.db[0].y += -r0inv;
-  G.db[1].x += r0inv;
-  G.sfac = sfac_of(S, r, rcut) * wj;
-  G.dsfac = dsfac_of(S, r, rcut) * wj;
-}
 
 // One level of the Wigner recursion (compute_ui.jl:66-101, derivative :224-267) for
 // `ncomp` components (1: U only; 4: U and dU/dx, dU/dy, dU/dz), lanes over
@@ -1852,310 +1795,6 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_bdesc(const __grid_const
   }
 }
 
-// ---- plain dB/dr path from the register chains (twojmax <= YR_MAX_J) ----------------------
-// dB_i/dr_ij [b][k] = 2 sum_t fac_t sum_half w Re(conj(dU_ij,k) Z_i(t)) (compute_dbidrj.jl;
-// compute_b.jl:207-400).  Every Z triple z belongs to one component jjb(z) with one
-// multiplier m(z) (its coincidence count and, unnormalised, (j1+1)/(j+1)), the same pair the
-// Y coefficients use, so dB[b][k] = 2 sum_{z: jjb(z) = b} m(z) sum_half w Re(conj(dU_k) Z_z).
-// k_snap_dbfused computes each pair's dU row by row on the register chains and contracts the
-// rows with the owner's Z, the Z triples of a level unrolled at compile time (their tables
-// below are constexpr restatements of the host's idxz / idxb / y_jjb / y_mult loops).
-namespace plaintab {
-constexpr int zrow_count(int j) { return (j / 2 + 1) * (j + 1); }
-constexpr int imin(int a, int b) { return a < b ? a : b; }
-constexpr int idxb_of(int J, int a, int b, int c) {
-  int k = 0;
-  for (int j1 = 0; j1 <= J; j1++)
-    for (int j2 = 0; j2 <= j1; j2++)
-      for (int j = j1 - j2; j <= imin(J, j1 + j2); j += 2)
-        if (j >= j1) {
-          if (j1 == a && j2 == b && j == c) return k;
-          k++;
-        }
-  return -1;
-}
-constexpr int nb_of(int J) {
-  int k = 0;
-  for (int j1 = 0; j1 <= J; j1++)
-    for (int j2 = 0; j2 <= j1; j2++)
-      for (int j = j1 - j2; j <= imin(J, j1 + j2); j += 2)
-        if (j >= j1) k++;
-  return k;
-}
-constexpr int LMAX = 64;
-struct Level {  // the Z triples (j1, j2, L) of level L
-  int n = 0;
-  int z0[LMAX] = {};   // first Z entry
-  int jjb[LMAX] = {};  // component
-  double m[LMAX] = {}, mn[LMAX] = {};  // multiplier without / with bnorm_flag
-};
-// Group g of G: the triples whose component b has b % G == g, with jjb = b / G.
-constexpr Level level_of(int J, int L, int G = 1, int g = 0) {
-  Level T;
-  int z = 0;
-  for (int j1 = 0; j1 <= J; j1++)
-    for (int j2 = 0; j2 <= j1; j2++)
-      for (int j = j1 - j2; j <= imin(J, j1 + j2); j += 2) {
-        if (j == L && T.n < LMAX) {
-          int jjb = 0;
-          double mult = 1.0;
-          if (j >= j1) {
-            jjb = idxb_of(J, j1, j2, j);
-            mult = (j1 == j) ? ((j2 == j) ? 3.0 : 2.0) : 1.0;
-          } else if (j >= j2) {
-            jjb = idxb_of(J, j, j2, j1);
-            mult = (j2 == j) ? 2.0 : 1.0;
-          } else {
-            jjb = idxb_of(J, j2, j, j1);
-          }
-          if (jjb % G != g) {
-            z += zrow_count(j);
-            continue;
-          }
-          T.z0[T.n] = z;
-          T.jjb[T.n] = jjb / G;
-          T.mn[T.n] = mult;
-          T.m[T.n] = (j1 > j) ? mult * (j1 + 1.0) / (j + 1.0) : mult;
-          T.n++;
-        }
-        z += zrow_count(j);
-      }
-  return T;
-}
-}  // namespace plaintab
-
-// Plain dB/dr, one block per owner atom, warp-specialised: warp 0 (the producer) runs every
-// chain of up to 32 of the owner's pairs, one pair per lane, and hands each half-plane row of
-// dU/dr to warps 1..3 (the consumers, one per component k) through three row buffers in
-// shared memory; each consumer lane contracts the rows of its pair with the owner's
-// Z (staged in shared memory) into the 55 accumulators of dB[b][k].  dU never leaves the SM.
-// Hand-off by named barriers (ids 1..3: row buffer b full; 4..6: row buffer b free), DBF_T
-// threads each: the producer arrives on "full" and waits on "free", the consumers the
-// reverse; both sides walk the same row sequence, so every barrier generation completes.
-constexpr int DBF_T = 128;
-
-template <int ID>
-__device__ __forceinline__ void nbar_sync() {
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(DBF_T) : "memory");
-}
-template <int ID>
-__device__ __forceinline__ void nbar_arrive() {
-  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(DBF_T) : "memory");
-}
-// DBF_NBUF row buffers; buffer b: "full" is barrier 1 + b, "free" is barrier 4 + b (immediate ids)
-constexpr int DBF_NBUF = 3;
-__device__ __forceinline__ void row_full_arrive(int b) {
-  b == 0 ? nbar_arrive<1>() : (b == 1 ? nbar_arrive<2>() : nbar_arrive<3>());
-}
-__device__ __forceinline__ void row_full_wait(int b) { b == 0 ? nbar_sync<1>() : (b == 1 ? nbar_sync<2>() : nbar_sync<3>()); }
-__device__ __forceinline__ void row_free_arrive(int b) {
-  b == 0 ? nbar_arrive<4>() : (b == 1 ? nbar_arrive<5>() : nbar_arrive<6>());
-}
-__device__ __forceinline__ void row_free_wait(int b) { b == 0 ? nbar_sync<4>() : (b == 1 ? nbar_sync<5>() : nbar_sync<6>()); }
-
-template <int J>
-struct DbRowEmit {  // producer side: dU_k[ma] of this lane's pair into row buffer r % DBF_NBUF
-  const snapchain::Geom& G;
-  double2* rows;  // [2][3][J+1][32]
-  int lane, r;
-  template <int j>
-  __device__ __forceinline__ void row(const snapchain::Chain<J>& s, int mb) {
-    const int b = r % DBF_NBUF;
-    row_free_wait(b);  // the consumers are done with row r - DBF_NBUF
-    double2* rb = rows + b * 3 * (J + 1) * 32 + lane;
-    const int last = (2 * mb == j) ? mb : j;
-#pragma unroll
-    for (int ma = 0; ma <= j; ma++) {
-      if (ma > last) break;
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        rb[(k * (J + 1) + ma) * 32] = make_double2(fma(G.dsu[k], s.u[ma].x, G.sfac * s.d[k][ma].x),
-                                                   fma(G.dsu[k], s.u[ma].y, G.sfac * s.d[k][ma].y));
-    }
-    row_full_arrive(b);
-    r++;
-  }
-};
-
-// consumer side: row mb of level L.  The row's entries ma run in a loop; the level's Z triples
-// are unrolled inside it (one Z load and two FMAs each), so the code per level stays small.
-template <int J, int L, int Q, int NQ>
-__device__ __forceinline__ void dbf_dot(double (&c)[NQ], double2 d, const double2* __restrict__ zr) {
-  if constexpr (Q < NQ) {
-    constexpr int z0 = plaintab::level_of(J, L).z0[Q];
-    const double2 z = zr[z0];
-    c[Q] = fma(d.x, z.x, fma(d.y, z.y, c[Q]));
-    dbf_dot<J, L, Q + 1, NQ>(c, d, zr);
-  }
-}
-
-template <int J, int L, int Q, int NQ, int NB>
-__device__ __forceinline__ void dbf_add(double (&acc)[NB], const double (&c)[NQ], bool bnorm) {
-  if constexpr (Q < NQ) {
-    constexpr plaintab::Level T = plaintab::level_of(J, L);
-    constexpr int b = T.jjb[Q];
-    constexpr double m = T.m[Q], mn = T.mn[Q];
-    acc[b] = fma(bnorm ? mn : m, c[Q], acc[b]);
-    dbf_add<J, L, Q + 1, NQ, NB>(acc, c, bnorm);
-  }
-}
-
-template <int J, int L, int NB>
-__device__ __forceinline__ void dbf_row(double (&acc)[NB], int mb, const double2* __restrict__ rb,
-                                        const double2* __restrict__ zo, bool bnorm) {
-  if constexpr (L <= J) {
-    constexpr int NQ = plaintab::level_of(J, L).n;
-    const int last = (2 * mb == L) ? mb : L;
-    const double2* zr = zo + mb * (L + 1);
-    double c[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) c[q] = 0.0;
-#pragma unroll 1
-    for (int ma = 0; ma <= last; ma++) {
-      double2 d = rb[ma * 32];
-      if (2 * mb == L && ma == mb) {  // the middle element of an even level: weight 1/2
-        d.x *= 0.5;
-        d.y *= 0.5;
-      }
-      dbf_dot<J, L, 0, NQ>(c, d, zr + ma);
-    }
-    dbf_add<J, L, 0, NQ, NB>(acc, c, bnorm);
-  }
-}
-
-template <int J, int NB>
-__device__ __forceinline__ void dbf_consume(double (&acc)[NB], int j, int mb, const double2* __restrict__ rb,
-                                            const double2* __restrict__ zo, bool bnorm) {
-  switch (j) {
-#define IPG_L(LL) \
-  case LL:        \
-    dbf_row<J, LL, NB>(acc, mb, rb, zo, bnorm); \
-    break;
-    IPG_L(0) IPG_L(1) IPG_L(2) IPG_L(3) IPG_L(4) IPG_L(5) IPG_L(6) IPG_L(7) IPG_L(8)
-#undef IPG_L
-    default:
-      break;
-  }
-}
-
-// dbl[p][b][k] for the pairs of owners b0 .. b1-1; their Z in the chunk of atoms a0.. (stride zs)
-template <int J>
-__global__ void __launch_bounds__(DBF_T, 2) k_snap_dbfused(const __grid_constant__ SnapDev S, int64_t b0,
-                                                           const int64_t* __restrict__ off,
-                                                           const int32_t* __restrict__ nbr,
-                                                           const double* __restrict__ rij,
-                                                           const int32_t* __restrict__ species, int64_t a0,
-                                                           int64_t zs, const double2* __restrict__ Z,
-                                                           double* __restrict__ dbl) {
-  static_assert(J <= YR_MAX_J, "fused plain kernel covers twojmax <= 8");
-  constexpr int NB = plaintab::nb_of(J);
-  extern __shared__ __align__(16) unsigned char fsm[];
-  double2* zo = reinterpret_cast<double2*>(fsm);                 // [idxz_max] the owner's Z
-  double2* rows = zo + ((S.idxz_max + 1) & ~1);                  // [DBF_NBUF][3][J+1][32]
-  double2* save = rows + DBF_NBUF * 3 * (J + 1) * 32;            // [4 (J+1)][32] producer start rows
-  const int64_t o = b0 + blockIdx.x;
-  for (int z = threadIdx.x; z < S.idxz_max; z += DBF_T) zo[z] = Z[(size_t)z * zs + (o - a0)];
-  __syncthreads();
-  const int64_t pb = off[o], pe = off[o + 1];
-  const int npass = (int)((pe - pb + 31) / 32);  // block-uniform
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (npass == 0) return;
-  if (warp == 0) {
-    const int si = clamp_sp(species[o], S.nsp);
-    int r = 0;  // rows handed over so far
-    for (int pass = 0; pass < npass; pass++) {
-      const int64_t p = pb + pass * 32 + lane;
-      snapchain::Geom G;  // idle lanes: the identity rotation with zero weights
-      G.a = make_double2(1.0, 0.0);
-      G.b = make_double2(0.0, 0.0);
-      G.sfac = 0.0;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        G.da[k] = make_double2(0.0, 0.0);
-        G.db[k] = make_double2(0.0, 0.0);
-        G.dsu[k] = 0.0;
-      }
-      if (p < pe) {
-        const int sj = clamp_sp(species[nbr[p]], S.nsp);
-        const double rcut = (S.radii[si] + S.radii[sj]) * S.rcutfac;
-        PairGeom PG;
-        geom_du(S, rij[3 * p], rij[3 * p + 1], rij[3 * p + 2], rcut, S.weight[sj], PG);
-        G.a = PG.a;
-        G.b = PG.b;
-        G.sfac = PG.sfac;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          G.da[k] = PG.da[k];
-          G.db[k] = PG.db[k];
-          G.dsu[k] = PG.dsfac * PG.u[k];
-        }
-      }
-      DbRowEmit<J> e{G, rows, lane, r};
-      snapchain::all_chains_rows<J>(G, e, save, 32, lane);
-      r = e.r;
-    }
-#pragma unroll
-    for (int t = 0; t < DBF_NBUF; t++) row_free_wait((r + t) % DBF_NBUF);  // the consumers' last arrivals
-  } else {
-    const int k = warp - 1;
-    const bool bnorm = S.bnorm_flag != 0;
-#pragma unroll
-    for (int b = 0; b < DBF_NBUF; b++) row_free_arrive(b);  // every row buffer starts free
-    int r = 0;
-    for (int pass = 0; pass < npass; pass++) {
-      double acc[NB];
-#pragma unroll
-      for (int b = 0; b < NB; b++) acc[b] = 0.0;
-      for (int mb = -1; mb <= J / 2; mb++) {  // mb = -1: the row (0, 0)
-        const int j0 = mb < 0 ? 0 : (mb == 0 ? 1 : 2 * mb), j1 = mb < 0 ? 0 : J;
-        for (int j = j0; j <= j1; j++, r++) {
-          const int bsel = r % DBF_NBUF;
-          row_full_wait(bsel);
-          dbf_consume<J, NB>(acc, j, mb < 0 ? 0 : mb, rows + (bsel * 3 + k) * (J + 1) * 32 + lane, zo, bnorm);
-          row_free_arrive(bsel);
-        }
-      }
-      const int64_t p = pb + pass * 32 + lane;
-      if (p < pe) {
-        double* out = dbl + (size_t)p * NB * 3 + k;
-#pragma unroll
-        for (int b = 0; b < NB; b++) out[3 * b] = 2.0 * acc[b];
-      }
-    }
-  }
-}
-
-template <int J>
-int plain_fused_j(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const int64_t* off, const int32_t* nbr,
-                  const double* rij, const int32_t* species, int64_t a0, int64_t zs, const double2* Z, double* dbl) {
-  if constexpr (J > YR_MAX_J) {
-    return IPG_ERR_UNSUPPORTED;
-  } else {
-    if (plaintab::nb_of(J) != S.K) return ipg_fail(ctx, IPG_ERR_UNSUPPORTED, "plain chain tables disagree");
-    const size_t sm =
-        ((size_t)((S.idxz_max + 1) & ~1) + DBF_NBUF * 3 * (J + 1) * 32 + 4 * (J + 1) * 32) * sizeof(double2);
-    if (sm > 48 * 1024)
-      CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_dbfused<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    IPG_TIMED_LAUNCH(ctx, "snap_dbfused", k_snap_dbfused<J>, (unsigned)(b1 - b0), DBF_T, sm, S, b0, off, nbr, rij,
-                     species, a0, zs, Z, dbl);
-    return IPG_OK;
-  }
-}
-
-int plain_fused(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const int64_t* off, const int32_t* nbr,
-                const double* rij, const int32_t* species, int64_t a0, int64_t zs, const double2* Z, double* dbl) {
-  if (b1 <= b0) return IPG_OK;
-  switch (S.J) {
-#define IPG_J(JJ) \
-  case JJ:        \
-    return plain_fused_j<JJ>(ctx, S, b0, b1, off, nbr, rij, species, a0, zs, Z, dbl);
-    IPG_J(0) IPG_J(1) IPG_J(2) IPG_J(3) IPG_J(4) IPG_J(5) IPG_J(6) IPG_J(7) IPG_J(8)
-#undef IPG_J
-    default:
-      return IPG_ERR_UNSUPPORTED;
-  }
-}
-
 // Adjoint per-neighbor kernel: one thread per (directed pair, chain MB); see
 // ipg_snap_chain.cuh.  Yw is the weighted Y as [h][natoms]; part[p][MB][3] = chain MB's
 // share of dE_i/dr_ij.
@@ -3035,7 +2674,8 @@ int upload_tables(ipg_snap* s) {
   size_t o_hinfo = o_uoh + pad(h.u_of_h.size() * 4);
   size_t o_hsgen = o_hinfo + pad(h.h_info.size() * 4);
   size_t o_yks = o_hsgen + pad(h.h_sgen.size() * 8);
-  size_t o_ytj = o_yks + pad(h.ykstream.size() * 8);
+  size_t o_zfac = o_yks + pad(h.ykstream.size() * 8);
+  size_t o_ytj = o_zfac + pad(h.zfac.size() * 8);
   size_t total = o_ytj + pad(h.ytrip_jjz.size() * 4);
   CUDA_RET(ctx, cudaMalloc(&s->d_tables, total));
   char* b = static_cast<char*>(s->d_tables);
@@ -3056,6 +2696,7 @@ int upload_tables(ipg_snap* s) {
   memcpy(hostbuf.data() + o_hinfo, h.h_info.data(), h.h_info.size() * 4);
   memcpy(hostbuf.data() + o_hsgen, h.h_sgen.data(), h.h_sgen.size() * 8);
   memcpy(hostbuf.data() + o_yks, h.ykstream.data(), h.ykstream.size() * 8);
+  memcpy(hostbuf.data() + o_zfac, h.zfac.data(), h.zfac.size() * 8);
   memcpy(hostbuf.data() + o_ytj, h.ytrip_jjz.data(), h.ytrip_jjz.size() * 4);
   CUDA_RET(ctx, cudaMemcpy(b, hostbuf.data(), total, cudaMemcpyHostToDevice));
   SnapDev& d = s->dev;
@@ -3104,6 +2745,7 @@ int upload_tables(ipg_snap* s) {
   d.h_info = reinterpret_cast<const int32_t*>(b + o_hinfo);
   d.h_sgen = reinterpret_cast<const double2*>(b + o_hsgen);
   d.ykstream = reinterpret_cast<const double2*>(b + o_yks);
+  d.zfac = reinterpret_cast<const double*>(b + o_zfac);
   d.ytrip_jjz = reinterpret_cast<const int32_t*>(b + o_ytj);
   d.n_ytrip = (int)h.ytrip_jjz.size();
   s->d_ymult = reinterpret_cast<double*>(b + o_ym);
@@ -3256,9 +2898,10 @@ int64_t zrows_chunk(const ipg_snap* s, const SnapDev& dev, int64_t n) {
 }
 
 // Plain dB/dr path on the register chains: per chunk of atoms, Z (streamed kernel), B and
-// E_i (k_snap_bdesc), then dbl of the pairs those atoms own (k_snap_dbfused).
+// E_i (k_snap_bdesc), then dbl of the pairs those atoms own (k_snap_db), with
+// fvec also its contraction with beta.
 int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl, const int32_t* d_species,
-                 const double2* utot, double* B, double* Ei, double* dbl) {
+                 const double2* utot, double* B, double* Ei, double* dbl, double* fvec) {
   ipg_ctx* ctx = s->ctx;
   const int64_t C = zrows_chunk(s, dev, n);
   double2* Z;
@@ -3275,7 +2918,7 @@ int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
     const int64_t bg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, bper));
     IPG_TIMED_LAUNCH(ctx, "snap_bdesc", k_snap_bdesc, (unsigned)bg, GB_WARPS * 32, bsm, dev, a0, nc, d_species, Z,
                      utot, B, Ei);
-    IPG_RET(plain_fused(ctx, dev, a0, a0 + nc, pl.d_off, pl.d_j, pl.d_r, d_species, a0, nc, Z, dbl));
+    IPG_RET(launch_db(ctx, dev, a0, a0 + nc, pl, d_species, a0, nc, Z, dbl, fvec));
   }
   return IPG_OK;
 }
@@ -3419,14 +3062,15 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
   } else if (need_plain) {
     IPG_RET(scratch(ctx, "snap_dbl", (size_t)np * K * 3 + 3, &dbl));
     io.dbl = dbl;
-    if (n && chains && dev.J <= YR_MAX_J && cap == 0 && !s->generic_plain)
-      IPG_RET(plain_chains(s, dev, n, pl, d_species, io.utot_in, out.B, Ei, dbl));
-    else if (n)
+    const bool forces = out.F || out.W6;
+    if (forces) IPG_RET(scratch(ctx, "snap_fvec", 3 * (size_t)np + 3, &fvec));
+    if (n && chains && dev.J <= YR_MAX_J && cap == 0 && !s->generic_plain) {
+      IPG_RET(plain_chains(s, dev, n, pl, d_species, io.utot_in, out.B, Ei, dbl, fvec));
+    } else if (n) {
       IPG_RET(launch_atoms<MODE_PLAIN>(s, dev, io, n, nullptr));
-    if (out.F || out.W6) {
-      IPG_RET(scratch(ctx, "snap_fvec", 3 * (size_t)np + 3, &fvec));
-      if (n) IPG_TIMED_LAUNCH(ctx, "snap_contract", k_snap_contract, nblk(32 * n, 256), 256, 0, n, pl.d_off, d_species, nsp, dbl, dev.beta, K,
-                               (int64_t)0, (int64_t)K, fvec);
+      if (forces)
+        IPG_TIMED_LAUNCH(ctx, "snap_contract", k_snap_contract, nblk(32 * n, 256), 256, 0, n, pl.d_off, d_species,
+                         nsp, dbl, dev.beta, K, (int64_t)0, (int64_t)K, fvec);
     }
   } else if (chains && n && dev.J <= YR_MAX_J && cap == 0) {
     // Z from the streamed kernel per chunk of atoms, then B (and E_i) per atom tile
@@ -3791,19 +3435,9 @@ int ipg_snap_create(ipg_ctx* ctx, const ipg_snap_params* params, ipg_snap** out)
     delete s;
     return st;
   }
-  {  // rootpq table of the register-chain kernel (independent of twojmax)
-    constexpr int R = snapchain::RPQ_STRIDE;
-    double t[R * R] = {};
-    for (int a = 1; a < R; a++)
-      for (int b = 1; b < R; b++) t[a * R + b] = std::sqrt((double)a / (double)b);
-    cudaError_t e = cudaMemcpyToSymbol(snapchain::c_rpq, t, sizeof(t));
-    // generator factors sqrt((m + 1)(j - m)) of the derivative identity
-    constexpr int NR = snapchain::SGEN_ROWS;
-    double t2[R * NR * R] = {};
-    for (int j = 1; j < R; j++)
-      for (int mb = 0; mb < NR; mb++)
-        for (int m = 0; m < j; m++) t2[(j * NR + mb) * R + m] = std::sqrt((double)((m + 1) * (j - m)));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(snapchain::c_sgen, t2, sizeof(t2));
+  {  // tables of the register-chain kernels (independent of twojmax)
+    cudaError_t e = snapchain::upload_constants();
+    if (e == cudaSuccess) e = snapdb_upload_constants();
     if (e != cudaSuccess) {
       cudaFree(s->d_tables);
       delete s;

@@ -87,6 +87,7 @@ struct SnapDev {
   const int32_t* h_info;      // [u_half] m | j << 8 | (m within the row's weighted entries) << 16, m = column ma
   const double2* h_sgen;      // [u_half] the generator factors (s_m, s_{m-1}), s_m = sqrt((m+1)(j-m)), 0 off the row
   const double2* ykstream;    // streamed Y / Z (twojmax <= YR_MAX_J): the weights
+  const double* zfac;         // [idxz_max] 2 m(z) w of the dB/dr contraction
   const int32_t* ytrip_jjz;  // [n_ytrip] first Z entry of each triple
   // explicit multi-element SNAP (chem_flag) and quadratic SNAP: K is then the number of
   // components per species block, klin of them linear (idxb_max per element triple), the rest
@@ -107,6 +108,7 @@ struct SnapHost {
   std::vector<double> cglist, rootpq, bzero;
   std::vector<int32_t> y_off, y_jjz;
   std::vector<int32_t> y_jjb;     // component whose beta scales each Z entry in Y
+  std::vector<double> zfac;       // 2 y_mult, halved on the middle element of an even level
   std::vector<double> y_mult;     // multiplicity * (j1+1)/(j+1) factor of each Z entry
   std::vector<int32_t> zperm;     // Z entries sorted by (nb, na): equal trip counts per warp
   std::vector<int32_t> ysched_off, ysched_h, u_of_h, h_info;
@@ -130,3 +132,8 @@ int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, c
 int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h_off, const PairList& pl,
                        const int32_t* owner, const int32_t* species, const double* pos, const double* dbl,
                        const double* B, double* dB, bool rows, double* Wd, double* Aw, double* Ae);
+// dB/dr of the pairs of owners b0 .. b1-1 (dbl [pair][K][3]) from their Z (atoms a0.., stride zs),
+// and, with fvec, its contraction with the owner's beta (ipg_snap_db.cu).
+int launch_db(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const PairList& pl, const int32_t* species,
+              int64_t a0, int64_t zs, const double2* Z, double* dbl, double* fvec);
+cudaError_t snapdb_upload_constants();

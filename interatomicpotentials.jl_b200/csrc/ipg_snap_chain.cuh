@@ -27,7 +27,7 @@ namespace snapchain {
 
 constexpr int RPQ_STRIDE = SNAP_MAX_J + 2;
 // rootpq[p][q] = sqrt(p/q) (prebuilt_arrays.jl:314-321), one table for every twojmax.
-__constant__ double c_rpq[RPQ_STRIDE * RPQ_STRIDE];
+static __constant__ double c_rpq[RPQ_STRIDE * RPQ_STRIDE];  // one copy per source file: upload_constants
 
 constexpr int half_block(int j) { return j <= 0 ? 0 : half_block(j - 1) + ((j - 1) / 2 + 1) * j; }
 
@@ -802,7 +802,22 @@ __device__ __forceinline__ void all_chains_v(const Geom& G, double A, const doub
 // runtime row so that the compiler loads the factors where they are used instead of hoisting
 // all of them into registers for the whole neighbor loop (which spilled)
 constexpr int SGEN_ROWS = SNAP_MAX_J / 2 + 1;
-__constant__ double c_sgen[RPQ_STRIDE * SGEN_ROWS * RPQ_STRIDE];
+static __constant__ double c_sgen[RPQ_STRIDE * SGEN_ROWS * RPQ_STRIDE];
+
+// Fills this source file's copy of the tables (independent of twojmax).
+static inline cudaError_t upload_constants() {
+  constexpr int R = RPQ_STRIDE, NR = SGEN_ROWS;
+  double t[R * R] = {};
+  for (int a = 1; a < R; a++)
+    for (int b = 1; b < R; b++) t[a * R + b] = std::sqrt((double)a / (double)b);
+  const cudaError_t e = cudaMemcpyToSymbol(c_rpq, t, sizeof(t));
+  if (e != cudaSuccess) return e;
+  double t2[R * NR * R] = {};
+  for (int j = 1; j < R; j++)
+    for (int mb = 0; mb < NR; mb++)
+      for (int m = 0; m < j; m++) t2[(j * NR + mb) * R + m] = std::sqrt((double)((m + 1) * (j - m)));
+  return cudaMemcpyToSymbol(c_sgen, t2, sizeof(t2));
+}
 
 template <int J, int j>
 __device__ __forceinline__ void stage_vlie(const ChainU<J>& s, double A, double g1, double g2, double g3, int mb,
@@ -1030,57 +1045,6 @@ __device__ __forceinline__ void all_chains_hvp_lie(double2 a, double2 at, double
 #define IPG_LEVEL(JJ) \
   case JJ:            \
     level_hvp_lie<J, JJ>(s, a, at, b, bt, mb, yw, yd, ys, acc, save, nt, tid);
-      IPG_LEVEL(1) IPG_LEVEL(2) IPG_LEVEL(3) IPG_LEVEL(4) IPG_LEVEL(5) IPG_LEVEL(6)
-      IPG_LEVEL(7) IPG_LEVEL(8) IPG_LEVEL(9) IPG_LEVEL(10) IPG_LEVEL(11) IPG_LEVEL(12)
-#undef IPG_LEVEL
-      default:
-        break;
-    }
-  }
-}
-
-}  // namespace snapchain
-
-
-namespace snapchain {
-
-// ---- every half-plane row of one neighbor handed to an emitter, in chain order ------------
-// emit.template row<j>(s, mb) runs after row mb of level j is in registers: row (0, 0) first,
-// then chain 0 over levels 1..J, chain mb over levels 2mb..J.  The rows of all lanes of a warp
-// come in the same order, so the emitter may synchronise the warp with other warps per row.
-template <int J, int j, class Emit>
-__device__ __forceinline__ void level_em(Chain<J>& s, const Geom& G, int mb, Emit& emit, double2* save, int nt,
-                                         int tid) {
-  if constexpr (j <= J) {
-    advance_rt<J, j>(s, G, mb);
-    emit.template row<j>(s, mb);
-    if constexpr (j % 2 == 1 && (j + 1) / 2 <= J / 2)
-      if (j == 2 * mb + 1) save_mirror<J, j>(s, save, nt, tid);
-  }
-}
-
-template <int J, class Emit>
-__device__ __forceinline__ void all_chains_rows(const Geom& G, Emit& emit, double2* save, int nt, int tid) {
-  static_assert(J <= 12, "level switch covers twojmax <= 12");
-  Chain<J> s;
-#pragma unroll
-  for (int c = 0; c <= J; c++) {
-    s.u[c] = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int k = 0; k < 3; k++) s.d[k][c] = make_double2(0.0, 0.0);
-  }
-  s.u[0] = make_double2(1.0, 0.0);
-  emit.template row<0>(s, 0);
-#pragma unroll 1
-  for (int mb = 0; mb <= J / 2; mb++) {
-    if (mb > 0) {
-      asm volatile("" ::: "memory");
-      load_row_rt<J>(s, save, nt, tid, 2 * mb);
-    }
-    switch (mb == 0 ? 1 : 2 * mb) {
-#define IPG_LEVEL(JJ) \
-  case JJ:            \
-    level_em<J, JJ>(s, G, mb, emit, save, nt, tid);
       IPG_LEVEL(1) IPG_LEVEL(2) IPG_LEVEL(3) IPG_LEVEL(4) IPG_LEVEL(5) IPG_LEVEL(6)
       IPG_LEVEL(7) IPG_LEVEL(8) IPG_LEVEL(9) IPG_LEVEL(10) IPG_LEVEL(11) IPG_LEVEL(12)
 #undef IPG_LEVEL

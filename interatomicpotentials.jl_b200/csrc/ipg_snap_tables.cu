@@ -202,6 +202,15 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
     h.y_jjb[z] = jjb;
     h.y_mult[z] = mult;
   }
+  h.zfac.assign(h.idxz_max, 0.0);
+  for (int j1 = 0; j1 <= J; j1++)
+    for (int j2 = 0; j2 <= j1; j2++)
+      for (int j = j1 - j2; j <= std::min(J, j1 + j2); j += 2)
+        for (int mb = 0; 2 * mb <= j; mb++)
+          for (int ma = 0; ma <= j; ma++) {
+            const int z = h.idxz_block[blk(j1, j2, j)] + mb * (j + 1) + ma;
+            h.zfac[z] = (2 * mb == j && ma == mb ? 1.0 : 2.0) * h.y_mult[z];
+          }
   h.y_off.assign(h.u_half + 1, 0);
   for (int z = 0; z < h.idxz_max; z++) h.y_off[h.zjju_half[z] + 1]++;
   for (int q = 0; q < h.u_half; q++) h.y_off[q + 1] += h.y_off[q];
