@@ -188,8 +188,10 @@ IPG_API int ipg_pair_eval_noalloc(void* stream, int64_t n, const double* d_pos, 
  * quadratic_flag (quadratic SNAP, the option of LAMMPS_SNAP/snap.jl:45-47): the K linear
  *   components are followed by 0.5 B_k^2 and B_k B_l (l > k), K + K(K+1)/2 in all; beta and
  *   the descriptors use that length.
- * With chem_flag or quadratic_flag the evaluation runs the per-atom element-resolved kernel
- *   (forces through dB/dr in either mode) and ipg_snap_vjp's position pullback returns
+ * With chem_flag or quadratic_flag the descriptors, the plain mode, both flags together,
+ *   literal_chem_z and twojmax above 8 run the per-atom element-resolved kernel (forces through
+ *   dB/dr); the adjoint mode otherwise runs on the Y of every element.  ipg_snap_vjp's position
+ *   pullback returns
  *   IPG_ERR_UNSUPPORTED.  wselfall_flag puts wself on every element's Utot.                */
 #define IPG_MAX_SNAP_SPECIES 8
 typedef struct ipg_snap_params {

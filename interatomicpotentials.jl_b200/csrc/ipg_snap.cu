@@ -1278,7 +1278,8 @@ __global__ void __launch_bounds__(128) k_snap_utot(const __grid_constant__ SnapD
 
 // Utot of every atom in one launch: one warp per atom, lanes over neighbors (32 at a time),
 // every chain of a neighbor in its lane (snapchain::all_chains_utot); the sums over lanes go
-// through a per-warp staging buffer in shared memory, in fixed order.
+// through a per-warp staging buffer in shared memory, in fixed order.  elem >= 0: the Utot of that
+// element (its neighbors, and wself on the centre's element or, with wselfall, on every one).
 constexpr int UTA_WARPS = 4;
 template <int J>
 __global__ void __launch_bounds__(UTA_WARPS * 32) k_snap_utot_all(const __grid_constant__ SnapDev S, int64_t n,
@@ -1286,7 +1287,7 @@ __global__ void __launch_bounds__(UTA_WARPS * 32) k_snap_utot_all(const __grid_c
                                                                   const int32_t* __restrict__ nbr,
                                                                   const double* __restrict__ rij,
                                                                   const int32_t* __restrict__ species,
-                                                                  double2* __restrict__ utot) {
+                                                                  double2* __restrict__ utot, int elem) {
   __shared__ double2 buf[UTA_WARPS][snapchain::UT_SLOTS * 33];
   __shared__ int dst[UTA_WARPS][snapchain::UT_SLOTS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1300,7 +1301,7 @@ __global__ void __launch_bounds__(UTA_WARPS * 32) k_snap_utot_all(const __grid_c
   st.ut = reinterpret_cast<double*>(utot + (size_t)i * S.idxu_max);
   st.lane = lane;
   st.nslot = 0;
-  st.wself = S.wself;
+  st.wself = elem < 0 || si == elem || S.wselfall ? S.wself : 0.0;
   for (int64_t p0 = beg; p0 < (end > beg ? end : beg + 1); p0 += 32) {
     const int64_t p = p0 + lane;
     double2 a = make_double2(1.0, 0.0), b = make_double2(0.0, 0.0);
@@ -1315,7 +1316,7 @@ __global__ void __launch_bounds__(UTA_WARPS * 32) k_snap_utot_all(const __grid_c
       const double r0inv = 1.0 / sqrt(r * r + z0 * z0);
       a = make_double2(r0inv * z0, -r0inv * z);
       b = make_double2(r0inv * y, -r0inv * x);
-      sw = sfac_of(S, r, rcut) * S.weight[sj];
+      sw = elem < 0 || sj == elem ? sfac_of(S, r, rcut) * S.weight[sj] : 0.0;
     }
     st.first = p0 == beg;
     snapchain::all_chains_utot<J>(a, b, sw, st);
@@ -1324,9 +1325,9 @@ __global__ void __launch_bounds__(UTA_WARPS * 32) k_snap_utot_all(const __grid_c
 
 template <int J>
 int launch_utot_all(ipg_ctx* ctx, const SnapDev& S, int64_t n, const int64_t* off, const int32_t* nbr,
-                    const double* rij, const int32_t* species, double2* utot) {
+                    const double* rij, const int32_t* species, double2* utot, int elem) {
   IPG_TIMED_LAUNCH(ctx, "snap_utot", k_snap_utot_all<J>, nblk(n, UTA_WARPS), UTA_WARPS * 32, 0, S, n, off, nbr, rij,
-                   species, utot);
+                   species, utot, elem);
   return IPG_OK;
 }
 
@@ -1342,16 +1343,17 @@ int launch_utot_chains(ipg_ctx* ctx, const SnapDev& S, int64_t n, const int64_t*
 }
 
 // warps: atoms (warps) per block, 1..4, of the per-chain kernels; all_chains: one launch of
-// k_snap_utot_all instead.
+// k_snap_utot_all instead; elem (all_chains only): the Utot of one element, -1 of all.
 int launch_utot(ipg_ctx* ctx, const SnapDev& S, int64_t n, const int64_t* off, const int32_t* nbr,
-                const double* rij, const int32_t* species, double2* utot, int warps = 4, bool all_chains = true) {
+                const double* rij, const int32_t* species, double2* utot, int warps = 4, bool all_chains = true,
+                int elem = -1) {
   if (n == 0) return IPG_OK;
   warps = std::max(1, std::min(4, warps));
   if (all_chains) {
     switch (S.J) {
 #define IPG_J(JJ) \
   case JJ:        \
-    return launch_utot_all<JJ>(ctx, S, n, off, nbr, rij, species, utot);
+    return launch_utot_all<JJ>(ctx, S, n, off, nbr, rij, species, utot, elem);
       IPG_J(0) IPG_J(1) IPG_J(2) IPG_J(3) IPG_J(4) IPG_J(5) IPG_J(6) IPG_J(7) IPG_J(8) IPG_J(9) IPG_J(10)
 #undef IPG_J
       default:
@@ -1932,15 +1934,17 @@ __global__ void __launch_bounds__(PAIR_LIE_T) k_snap_pair_lie(const __grid_const
                                                               const double* __restrict__ rij,
                                                               const int32_t* __restrict__ species,
                                                               const double2* __restrict__ Yw,
-                                                              double* __restrict__ part) {
+                                                              double* __restrict__ part, int ne) {
   extern __shared__ double2 ylie[];  // [3][u_half][PAIR_LIE_ATOMS]: Yw, Y2, Y3 of a group of owners
   const int64_t np = *d_np;          // the live count (capacity mode sizes the grid larger)
   const int64_t p0 = (int64_t)blockIdx.x * blockDim.x, p = p0 + threadIdx.x;
   if (p0 >= np) return;  // block-uniform
-  const int first = owner[p0];
-  const int lastat = owner[(p0 + blockDim.x < np ? p0 + blockDim.x : np) - 1];
+  // Y columns: one per owner, or with ne elements ne per owner (the neighbor's element picks)
+  const int first = owner[p0] * ne;
+  const int lastat = owner[(p0 + blockDim.x < np ? p0 + blockDim.x : np) - 1] * ne + ne - 1;
   const int UH = S.u_half;
   const int i = p < np ? owner[p] : -1;
+  int v = i;  // the pair's column
   // the first group's Y' goes to shared memory by asynchronous copies (zero-filled beyond each
   // row's weighted entries, which the Y kernel leaves unset) while the pair geometry is computed
   auto stage = [&](int g0, int nat) {
@@ -1959,6 +1963,7 @@ __global__ void __launch_bounds__(PAIR_LIE_T) k_snap_pair_lie(const __grid_const
   double c0[3] = {0.0, 0.0, 0.0}, cT[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
   if (p < np) {
     const int si = clamp_sp(species[i], S.nsp), sj = clamp_sp(species[nbr[p]], S.nsp);
+    if (ne > 1) v = i * ne + sj;
     const double rcut = (S.radii[si] + S.radii[sj]) * S.rcutfac;
     PairGeom PG;
     geom_du(S, rij[3 * p], rij[3 * p + 1], rij[3 * p + 2], rcut, S.weight[sj], PG);
@@ -1996,8 +2001,8 @@ __global__ void __launch_bounds__(PAIR_LIE_T) k_snap_pair_lie(const __grid_const
       ylie[(size_t)(2 * UH + h) * PAIR_LIE_ATOMS + a] = make_double2(A.y + B.y, -(A.x + B.x));
     }
     __syncthreads();
-    if (i >= g0 && i < g0 + nat)
-      snapchain::all_chains_lie<J>(a, b, ylie + (i - g0), PAIR_LIE_ATOMS, UH, S0, T);
+    if (v >= g0 && v < g0 + nat)
+      snapchain::all_chains_lie<J>(a, b, ylie + (v - g0), PAIR_LIE_ATOMS, UH, S0, T);
   }
   if (p >= np) return;
   double* out = part + (size_t)p * 3;
@@ -2008,22 +2013,22 @@ __global__ void __launch_bounds__(PAIR_LIE_T) k_snap_pair_lie(const __grid_const
 template <int J>
 int launch_pair_lie_t(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t* d_np, int64_t natoms,
                       const int32_t* owner, const int32_t* nbr, const double* rij, const int32_t* species,
-                      const double2* Yw, double* part) {
+                      const double2* Yw, double* part, int ne) {
   const size_t sm = pair_lie_smem(S.u_half);
   if (sm > 48 * 1024)
     CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_pair_lie<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  IPG_TIMED_LAUNCH(ctx, "snap_pair", k_snap_pair_lie<J>, nblk(np, PAIR_LIE_T), PAIR_LIE_T, sm, S, d_np, natoms, owner,
-                   nbr, rij, species, Yw, part);
+  IPG_TIMED_LAUNCH(ctx, "snap_pair", k_snap_pair_lie<J>, nblk(np, PAIR_LIE_T), PAIR_LIE_T, sm, S, d_np, natoms * ne,
+                   owner, nbr, rij, species, Yw, part, ne);
   return IPG_OK;
 }
 
 int launch_pair_lie(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t* d_np, int64_t natoms, const int32_t* owner,
-                    const int32_t* nbr, const double* rij, const int32_t* species, const double2* Yw, double* part) {
+                    const int32_t* nbr, const double* rij, const int32_t* species, const double2* Yw, double* part, int ne = 1) {
   if (np == 0) return IPG_OK;
   switch (S.J) {
 #define IPG_J(JJ) \
   case JJ:        \
-    return launch_pair_lie_t<JJ>(ctx, S, np, d_np, natoms, owner, nbr, rij, species, Yw, part);
+    return launch_pair_lie_t<JJ>(ctx, S, np, d_np, natoms, owner, nbr, rij, species, Yw, part, ne);
     IPG_J(0) IPG_J(1) IPG_J(2) IPG_J(3) IPG_J(4) IPG_J(5) IPG_J(6) IPG_J(7) IPG_J(8) IPG_J(9) IPG_J(10)
 #undef IPG_J
     default:
@@ -2676,7 +2681,10 @@ int upload_tables(ipg_snap* s) {
   size_t o_yks = o_hsgen + pad(h.h_sgen.size() * 8);
   size_t o_zfac = o_yks + pad(h.ykstream.size() * 8);
   size_t o_ytj = o_zfac + pad(h.zfac.size() * 8);
-  size_t total = o_ytj + pad(h.ytrip_jjz.size() * 4);
+  size_t o_ytb = o_ytj + pad(h.ytrip_jjz.size() * 4);
+  size_t o_ytf = o_ytb + pad(h.ytrip_b.size() * 4);
+  size_t o_ylev = o_ytf + pad(h.ytrip_fac.size() * 8);
+  size_t total = o_ylev + pad(h.ylev.size() * 4);
   CUDA_RET(ctx, cudaMalloc(&s->d_tables, total));
   char* b = static_cast<char*>(s->d_tables);
   std::vector<char> hostbuf(total, 0);
@@ -2697,6 +2705,9 @@ int upload_tables(ipg_snap* s) {
   memcpy(hostbuf.data() + o_hsgen, h.h_sgen.data(), h.h_sgen.size() * 8);
   memcpy(hostbuf.data() + o_yks, h.ykstream.data(), h.ykstream.size() * 8);
   memcpy(hostbuf.data() + o_zfac, h.zfac.data(), h.zfac.size() * 8);
+  memcpy(hostbuf.data() + o_ytb, h.ytrip_b.data(), h.ytrip_b.size() * 4);
+  memcpy(hostbuf.data() + o_ytf, h.ytrip_fac.data(), h.ytrip_fac.size() * 8);
+  memcpy(hostbuf.data() + o_ylev, h.ylev.data(), h.ylev.size() * 4);
   memcpy(hostbuf.data() + o_ytj, h.ytrip_jjz.data(), h.ytrip_jjz.size() * 4);
   CUDA_RET(ctx, cudaMemcpy(b, hostbuf.data(), total, cudaMemcpyHostToDevice));
   SnapDev& d = s->dev;
@@ -2746,6 +2757,9 @@ int upload_tables(ipg_snap* s) {
   d.h_sgen = reinterpret_cast<const double2*>(b + o_hsgen);
   d.ykstream = reinterpret_cast<const double2*>(b + o_yks);
   d.zfac = reinterpret_cast<const double*>(b + o_zfac);
+  d.ytrip_b = reinterpret_cast<const int32_t*>(b + o_ytb);
+  d.ytrip_fac = reinterpret_cast<const double*>(b + o_ytf);
+  d.ylev = reinterpret_cast<const int32_t*>(b + o_ylev);
   d.ytrip_jjz = reinterpret_cast<const int32_t*>(b + o_ytj);
   d.n_ytrip = (int)h.ytrip_jjz.size();
   s->d_ymult = reinterpret_cast<double*>(b + o_ym);
@@ -2948,6 +2962,57 @@ int launch_y(ipg_snap* s, const SnapDev& dev, const char* tname, int64_t n, cons
   return IPG_OK;
 }
 
+// Element-resolved or quadratic SNAP by the adjoint route: Utot of every element, Z of every
+// element pair per chunk of atoms, Y of every element from Z, E_i, and the pair forces fvec.
+int chem_adjoint(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl, const int32_t* d_species, double* Ei,
+                 double* fvec) {
+  ipg_ctx* ctx = s->ctx;
+  const int ne = dev.nelem, M = dev.idxz_max, U = dev.idxu_max;
+  double2 *utot, *Z, *yout;
+  double *coef, *B = nullptr;
+  int32_t* owner;
+  IPG_RET(scratch(ctx, "snap_utot", (size_t)ne * n * U + 1, &utot));
+  for (int e = 0; e < ne; e++)
+    IPG_RET(launch_utot(ctx, dev, n, pl.d_off, pl.d_j, pl.d_r, d_species, utot + (size_t)e * n * U, s->utot_warps, true,
+                        ne > 1 ? e : -1));
+  // Z of a chunk within about 4 GiB
+  const int64_t most = std::max<int64_t>(YS_ATOMS, (int64_t(4) << 30) / ((int64_t)ne * ne * M * 16) / YS_ATOMS * YS_ATOMS);
+  const int64_t C = std::min(n, most);
+  IPG_RET(scratch(ctx, "snap_Z", (size_t)C * ne * ne * M + 1, &Z));
+  IPG_RET(scratch(ctx, "chem_coef", (size_t)C * ne * ne * ne * dev.n_ytrip + 1, &coef));
+  IPG_RET(scratch(ctx, "snap_yout", (size_t)n * ne * dev.u_half + 1, &yout));
+  IPG_RET(scratch(ctx, "snap_owner", (size_t)pl.npairs + 1, &owner));
+  SnapDev lin = dev;  // the linear components alone
+  lin.K = dev.klin;
+  int bper = 1, bsm = 0;
+  if (dev.quadratic) {
+    IPG_RET(scratch(ctx, "chem_B", (size_t)n * dev.klin + 1, &B));
+    bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)dev.klin * YS_ATOMS * 8);
+    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
+    CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bper, k_snap_bdesc, GB_WARPS * 32, bsm));
+  }
+  for (int64_t a0 = 0; a0 < n; a0 += C) {
+    const int64_t nc = std::min(C, n - a0);
+    for (int p = 0; p < ne; p++)
+      for (int q = 0; q < ne; q++)
+        IPG_RET(launch_ystream(ctx, dev, s->h.yktab, YM_Z, "snap_zrows", nc, d_species + a0,
+                               utot + ((size_t)p * n + a0) * U, nullptr, nullptr, Z + (size_t)(p * ne + q) * M * nc,
+                               utot + ((size_t)q * n + a0) * U));
+    if (dev.quadratic) {
+      const int64_t tiles = (nc + YS_ATOMS - 1) / YS_ATOMS;
+      const int64_t bg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, bper));
+      IPG_TIMED_LAUNCH(ctx, "snap_bdesc", k_snap_bdesc, (unsigned)bg, GB_WARPS * 32, bsm, lin, a0, nc, d_species, Z,
+                       utot, B, Ei);
+      IPG_RET(launch_quad_coef(ctx, dev, a0, nc, d_species, B, Ei, coef));
+    } else {
+      IPG_RET(launch_chem_coef(ctx, dev, a0, nc, d_species, coef));
+    }
+    IPG_RET(launch_chem_y(ctx, dev, n, a0, nc, d_species, coef, Z, utot, yout, dev.quadratic ? nullptr : Ei));
+  }
+  IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
+  return launch_pair_lie(ctx, dev, pl.npairs, pl.d_np, n, owner, pl.d_j, pl.d_r, d_species, yout, fvec, ne);
+}
+
 // Energy / forces / descriptors for device inputs.  mode: MODE_DESC (B/E only), MODE_ADJ,
 // MODE_PLAIN.  Writes device outputs; does not synchronise.
 int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_species, int nconf,
@@ -2984,7 +3049,13 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     io.utot_in = utot;
   }
   int nch = 1;
-  if (chemq) {
+  // the adjoint route for chem_flag or quadratic_flag (not both, not the literal Z index)
+  const bool chem_adj = chemq && mode == MODE_ADJ && !want_desc && !out.B && dev.J <= YR_MAX_J &&
+                        !(dev.chem && dev.quadratic) && !dev.literal_chem_z && !s->generic_adjoint;
+  if (chem_adj) {
+    IPG_RET(scratch(ctx, "snap_fvec", 3 * (size_t)np + 3, &fvec));
+    if (n) IPG_RET(chem_adjoint(s, dev, n, pl, d_species, Ei, fvec));
+  } else if (chemq) {
     // chem_flag / quadratic_flag: B (and E_i), and dB_lin/dr of every pair when forces or
     // force descriptors are wanted; the forces contract dB/dr with beta (quadratic: with each
     // atom's effective linear coefficients), the descriptors read the extended dB/dr.

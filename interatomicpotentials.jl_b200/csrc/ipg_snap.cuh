@@ -89,6 +89,9 @@ struct SnapDev {
   const double2* ykstream;    // streamed Y / Z (twojmax <= YR_MAX_J): the weights
   const double* zfac;         // [idxz_max] 2 m(z) w of the dB/dr contraction
   const int32_t* ytrip_jjz;  // [n_ytrip] first Z entry of each triple
+  const int32_t* ytrip_b;    // [n_ytrip] its component | the derivative terms it serves (bits 0-2) << 16
+  const double* ytrip_fac;   // [n_ytrip] factor of each of those terms
+  const int32_t* ylev;       // [J+2] offsets, then the triples of every level in order
   // explicit multi-element SNAP (chem_flag) and quadratic SNAP: K is then the number of
   // components per species block, klin of them linear (idxb_max per element triple), the rest
   // the products B_k B_l (k <= l) of quadratic_flag
@@ -116,15 +119,18 @@ struct SnapHost {
   std::vector<double> ysched_w;
   YkTab yktab;
   std::vector<double> ykstream;  // 2 per 16-byte unit
-  std::vector<int32_t> ytrip_jjz;
+  std::vector<int32_t> ytrip_jjz, ytrip_b, ylev;
+  std::vector<double> ytrip_fac;
 };
 
 int snap_build_tables(const ipg_snap_params& p, SnapHost& h);
 
 struct ipg_ctx;
-// Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu).
-int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n, const int32_t* species,
-                   const double2* utot, double2* yout, double* Ei, double2* zout);
+// Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu); with
+// utot2 (YM_Z) the second factor of every product comes from it.
+int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n,
+                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout,
+                   const double2* utot2 = nullptr);
 // Descriptor outputs from dbl [pair][K][3], the dB/dr of every pair (ipg_snap_desc.cu): dB
 // [n][K nsp][3], or [3 n][K nsp] with rows; Wd [K nsp][6] of one configuration; the fitting rows
 // Aw [nconf][6][K nsp] and Ae [nconf][K nsp] (from B [n][K]).  Any output may be null; owner (of
@@ -137,3 +143,14 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
 int launch_db(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const PairList& pl, const int32_t* species,
               int64_t a0, int64_t zs, const double2* Z, double* dbl, double* fvec);
 cudaError_t snapdb_upload_constants();
+// Element-resolved and quadratic SNAP by the adjoint route (ipg_snap_chem.cu), twojmax <= YR_MAX_J.
+// All of atoms a0 .. a0+nc-1: coef [nelem][nelem^2][n_ytrip][nc] is the weight of every Z triple of
+// every element pair in the Y of every element.
+int launch_chem_coef(ipg_ctx* ctx, const SnapDev& S, int64_t a0, int64_t nc, const int32_t* species, double* coef);
+// Quadratic SNAP (one element): E_i and the coefficients from the linear B [n][klin].
+int launch_quad_coef(ipg_ctx* ctx, const SnapDev& S, int64_t a0, int64_t nc, const int32_t* species, const double* B,
+                     double* Ei, double* coef);
+// Weighted Y' [u_half][n nelem] (atom-major elements) from Z [nelem^2][idxz_max][nc], and with
+// Ei (element-resolved linear SNAP) the energies, from utot [nelem][n][idxu_max].
+int launch_chem_y(ipg_ctx* ctx, const SnapDev& S, int64_t n, int64_t a0, int64_t nc, const int32_t* species,
+                  const double* coef, const double2* Z, const double2* utot, double2* yout, double* Ei);

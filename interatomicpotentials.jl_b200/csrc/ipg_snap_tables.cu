@@ -269,6 +269,9 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
   memset(&h.yktab, 0, sizeof(h.yktab));
   h.ykstream.clear();
   h.ytrip_jjz.clear();
+  h.ytrip_b.clear();
+  h.ytrip_fac.clear();
+  h.ylev.clear();
   if (J <= YR_MAX_J) {
     std::vector<int32_t> trip_of(jd * jd * jd, -1);
     for (int j1 = 0; j1 <= J; j1++)
@@ -277,11 +280,33 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
           trip_of[blk(j1, j2, j)] = (int32_t)h.ytrip_jjz.size();
           h.ytrip_jjz.push_back(h.idxz_block[blk(j1, j2, j)]);
         }
+    // the component of each triple and the terms of its derivative (compute_b.jl:104-400) that read it
+    h.ytrip_b.assign(h.ytrip_jjz.size(), 0);
+    h.ytrip_fac.assign(h.ytrip_jjz.size(), 0.0);
+    for (int b = 0; b < h.idxb_max; b++)
+      for (int t = 0; t < 3; t++)
+        for (size_t q = 0; q < h.ytrip_jjz.size(); q++)
+          if (h.ytrip_jjz[q] == h.db[b].z0[t]) {
+            h.ytrip_b[q] = b | (((h.ytrip_b[q] >> 16) | (1 << t)) << 16);
+            h.ytrip_fac[q] = h.db[b].fac[t];
+          }
+    h.ylev.assign(J + 2, 0);
+    for (int j = 0; j <= J; j++) {
+      for (int j1 = 0; j1 <= J; j1++)
+        for (int j2 = 0; j2 <= j1; j2++)
+          if (j >= j1 - j2 && j <= std::min(J, j1 + j2) && !((j1 + j2 + j) & 1))
+            h.ylev.push_back(trip_of[blk(j1, j2, j)]);
+      h.ylev[j + 1] = (int32_t)h.ylev.size() - (J + 2);
+    }
+    struct YkRows {
+      int8_t j1, j2, mb1, mb2, lo1, hi1, jlo, N, E, mir;  // mir: the row beyond the half plane (0, 1, 2)
+    };
     struct Item {
       YkItem it;
       std::vector<uint32_t> recs;
       std::vector<int2> pairs;
-      std::vector<double> w;
+      std::vector<YkRows> rows;  // of every row pair, for its weights
+      size_t units = 0;
       double cost = 0.0;
     };
     std::vector<Item> items;
@@ -321,17 +346,9 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
                                  (uint32_t)trip_of[blk(j1, j2, jlo)] << YF_TRIP);
               I.recs.back() += 1u | (uint32_t)units << YF_SIZE;
               I.pairs.push_back(make_int2(e1 * YS_ATOMS * 16 | (int)mir1, e2 * YS_ATOMS * 16 | (int)mir2));
-              for (int ma1 = lo1; ma1 <= hi1; ma1++)
-                for (int j = jlo; j <= jhi; j += 2) {
-                  const int cg0 = h.idxcg_block[blk(j1, j2, j)];
-                  const double cb = h.cglist[cg0 + mb1 * (j2 + 1) + mb2] * (p.bnorm_flag ? 1.0 / (j + 1) : 1.0);
-                  for (int t = 0; t < YT; t++) {
-                    const int m2 = E + t - ma1, c = c0 + 2 * t;
-                    const bool ok = t < nt && m2 >= 0 && m2 <= j2 && std::abs(c) <= j;
-                    const int sg = mir1 ? ma1 + mb1 : (mir2 ? m2 + mb2 : 0);  // sign of the mirrored element
-                    I.w.push_back(ok ? ((sg & 1) ? -cb : cb) * h.cglist[cg0 + ma1 * (j2 + 1) + m2] : 0.0);
-                  }
-                }
+              I.rows.push_back({(int8_t)j1, (int8_t)j2, (int8_t)mb1, (int8_t)mb2, (int8_t)lo1, (int8_t)hi1, (int8_t)jlo,
+                                (int8_t)N, (int8_t)E, (int8_t)(mir1 ? 1 : (mir2 ? 2 : 0))});
+              I.units += units;
               I.cost += steps * YT * (4.0 + 2.0 * N) + 20.0;
             }
             if (I.recs.size() > first) {
@@ -345,20 +362,39 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
     YkTab& T = h.yktab;
     int nrec = 0, npair = 0;
+    size_t nu = 2 * YREC;  // the walk copies up to two records past an item
+    for (const Item& I : items) nu += I.units;
+    h.ykstream.assign(2 * nu, 0.0);
+    double* out = h.ykstream.data();
     if (items.size() > (size_t)YK_ITEMS) return IPG_ERR_UNSUPPORTED;  // sized for YR_MAX_J
     for (Item& I : items) {
       if (nrec + I.recs.size() > (size_t)YK_RECS || npair + I.pairs.size() > (size_t)YK_PAIRS)
         return IPG_ERR_UNSUPPORTED;
-      I.it.unit = (int32_t)(h.ykstream.size() / 2);
+      I.it.unit = (int32_t)((out - h.ykstream.data()) / 2);
       I.it.rec = (int16_t)nrec;
       I.it.nrec = (int16_t)I.recs.size();
       I.it.pair = (int16_t)npair;
       for (uint32_t r : I.recs) T.rec[nrec++] = r;
       for (const int2& q : I.pairs) T.pair[npair++] = q;
-      h.ykstream.insert(h.ykstream.end(), I.w.begin(), I.w.end());
       T.item[T.nitem++] = I.it;
+      for (const YkRows& R : I.rows) {  // its weights, [step][level][YT]
+        const double* cgj[YNJ];
+        double cb[YNJ];
+        for (int q = 0; q < R.N; q++) {
+          const int j = R.jlo + 2 * q;
+          cgj[q] = h.cglist.data() + h.idxcg_block[blk(R.j1, R.j2, j)];
+          cb[q] = cgj[q][R.mb1 * (R.j2 + 1) + R.mb2] * (p.bnorm_flag ? 1.0 / (j + 1) : 1.0);
+        }
+        for (int ma1 = R.lo1; ma1 <= R.hi1; ma1++)
+          for (int q = 0; q < R.N; q++)
+            for (int t = 0; t < YT; t++) {
+              const int m2 = R.E + t - ma1, c = I.it.c0 + 2 * t;
+              const bool ok = t < I.it.nt && m2 >= 0 && m2 <= R.j2 && std::abs(c) <= R.jlo + 2 * q;
+              const int sg = R.mir == 1 ? ma1 + R.mb1 : (R.mir == 2 ? m2 + R.mb2 : 0);  // sign of the mirrored element
+              *out++ = ok ? ((sg & 1) ? -cb[q] : cb[q]) * cgj[q][ma1 * (R.j2 + 1) + m2] : 0.0;
+            }
+      }
     }
-    h.ykstream.resize(h.ykstream.size() + 2 * 2 * YREC, 0.0);  // the walk copies up to two records past an item
   }
   return IPG_OK;
 }

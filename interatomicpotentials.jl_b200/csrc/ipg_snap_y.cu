@@ -43,12 +43,15 @@ constexpr int YK_SLOTS = 3;  // ring: the record in use and two in flight
 // the 32 atoms, [u_half][32] double2 | zero guard | energies [items][32] | record rings.
 // Window elements before the first or after the last column of a row meet weights of exactly
 // zero, so they only have to be finite: neighbors in the half plane (the same atom's), or guard.
+// With two sets of Utot (row 1 from one, row 2 from the other) a second half plane and guard follow.
 struct YkSmem {
-  int coef, guard, u, energy, ring;
-  __host__ __device__ int total() const { return coef + 2 * guard + u + energy + ring; }
+  int coef, guard, u, energy, ring, sets;
+  __host__ __device__ int planes() const { return guard + sets * (u + guard); }
+  __host__ __device__ int total() const { return coef + planes() + energy + ring; }
 };
-__host__ __device__ inline YkSmem yk_smem(int nsp, int ntrip, int uh, int nitems) {
+__host__ __device__ inline YkSmem yk_smem(int nsp, int ntrip, int uh, int nitems, bool two) {
   YkSmem m;
+  m.sets = two ? 2 : 1;
   m.coef = (8 * nsp * ntrip + 15) & ~15;
   m.guard = YGUARD * YS_ATOMS * 16;
   m.u = uh * YS_ATOMS * 16;
@@ -122,7 +125,8 @@ __device__ __forceinline__ void yk_pair(unsigned p1, unsigned p2, int d1, int d2
 // One record: its m row pairs (from pi on), n steps each, into Z[0 .. N-1] (the N levels of the
 // (j1, j2) pair that the item holds).
 template <int N>
-__device__ __forceinline__ void yk_record(const YkTab& T, unsigned us, int pi, int m, int n, bool first, unsigned wt,
+__device__ __forceinline__ void yk_record(const YkTab& T, unsigned us, unsigned us2, int pi, int m, int n, bool first,
+                                          unsigned wt,
                                           double2 (&Z)[YNJ][YT]) {
   if (first) {
 #pragma unroll
@@ -138,7 +142,7 @@ __device__ __forceinline__ void yk_record(const YkTab& T, unsigned us, int pi, i
     unsigned m1 = (unsigned)x.x << 31, m2 = (unsigned)x.y << 31;
     // kept in registers: the compiler would form them again in every step
     asm volatile("" : "+r"(d1), "+r"(d2), "+r"(m1), "+r"(m2));
-    yk_pair<N>(us + (unsigned)(x.x & ~1), us + (unsigned)(x.y & ~1), d1, d2, m1, m2, wt, n, Z);
+    yk_pair<N>(us + (unsigned)(x.x & ~1), us2 + (unsigned)(x.y & ~1), d1, d2, m1, m2, wt, n, Z);
     wt += wn;
   }
 }
@@ -202,37 +206,44 @@ __device__ __forceinline__ void yk_finish(const SnapDev& S, const YkItem& it, in
 // blockIdx.y, blockIdx.y + gridDim.y, ...; the items' energies then go to eitem [items][n] and
 // k_snap_yenergy adds them.  An item's result does not depend on the warp that computes it, and
 // energies are summed in item order, so neither split nor scheduling changes any bit.
-template <int YM>
+// TWO: row 2 from a second Utot (the element pairs of chem_flag; Z only).
+template <int YM, bool TWO>
 __global__ void __launch_bounds__(YK_T, 2) k_snap_ystream(const __grid_constant__ SnapDev S,
                                                           const __grid_constant__ YkTab T, int64_t n,
                                                           const int32_t* __restrict__ species,
                                                           const double2* __restrict__ utot,
+                                                          const double2* __restrict__ utot2,
                                                           double2* __restrict__ yout, double* __restrict__ Ei,
                                                           double2* __restrict__ zout, double* __restrict__ eitem) {
   extern __shared__ __align__(16) unsigned char ysh[];
   __shared__ int next_item;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int UH = S.u_half, NI = T.nitem;
-  const YkSmem M = yk_smem(S.nsp, S.n_ytrip, UH, NI);
+  const YkSmem M = yk_smem(S.nsp, S.n_ytrip, UH, NI, TWO);
   double* coefs = reinterpret_cast<double*>(ysh);  // [nsp][n_ytrip]
   double2* guard0 = reinterpret_cast<double2*>(ysh + M.coef);
   double2* us = reinterpret_cast<double2*>(ysh + M.coef + M.guard);
   double2* guard1 = reinterpret_cast<double2*>(ysh + M.coef + M.guard + M.u);
-  double* erow = reinterpret_cast<double*>(ysh + M.coef + 2 * M.guard + M.u);
-  double2* ring = reinterpret_cast<double2*>(ysh + M.coef + 2 * M.guard + M.u + M.energy) +
-                  warp * YK_SLOTS * YREC;
+  double2* us2 = TWO ? guard1 + YGUARD * YS_ATOMS : us;
+  double* erow = reinterpret_cast<double*>(ysh + M.coef + M.planes());
+  double2* ring = reinterpret_cast<double2*>(ysh + M.coef + M.planes() + M.energy) + warp * YK_SLOTS * YREC;
   if (YM != YM_Z)
     for (int q = threadIdx.x; q < S.nsp * S.n_ytrip; q += YK_T) {
       const int sp = q / S.n_ytrip, t = q - sp * S.n_ytrip;
       coefs[q] = S.ycoef[(size_t)sp * S.idxz_max + S.ytrip_jjz[t]];
     }
-  for (int q = threadIdx.x; q < YGUARD * YS_ATOMS; q += YK_T) guard0[q] = guard1[q] = make_double2(0.0, 0.0);
+  for (int q = threadIdx.x; q < YGUARD * YS_ATOMS; q += YK_T) {
+    guard0[q] = guard1[q] = make_double2(0.0, 0.0);
+    if (TWO) us2[UH * YS_ATOMS + q] = make_double2(0.0, 0.0);
+  }
   const bool split = gridDim.y > 1;
   for (int64_t a0 = (int64_t)blockIdx.x * YS_ATOMS; a0 < n; a0 += (int64_t)gridDim.x * YS_ATOMS) {
     const int na_blk = (int)((n - a0) < YS_ATOMS ? (n - a0) : YS_ATOMS);
     for (int idx = threadIdx.x; idx < UH * YS_ATOMS; idx += YK_T) {
       const int q = idx / YS_ATOMS, l = idx - q * YS_ATOMS;
-      us[idx] = l < na_blk ? utot[(size_t)(a0 + l) * S.idxu_max + S.u_of_h[q]] : make_double2(0.0, 0.0);
+      const size_t at = (size_t)(a0 + l) * S.idxu_max + S.u_of_h[q];
+      us[idx] = l < na_blk ? utot[at] : make_double2(0.0, 0.0);
+      if (TWO) us2[idx] = l < na_blk ? utot2[at] : make_double2(0.0, 0.0);
     }
     if (threadIdx.x == 0) next_item = blockIdx.y;
     __syncthreads();
@@ -243,6 +254,7 @@ __global__ void __launch_bounds__(YK_T, 2) k_snap_ystream(const __grid_constant_
     const double* coef = coefs + si * S.n_ytrip;
     const double2* usl = us + lane;
     const unsigned usa = (unsigned)__cvta_generic_to_shared(usl), ringa = (unsigned)__cvta_generic_to_shared(ring);
+    const unsigned usb = TWO ? (unsigned)__cvta_generic_to_shared(us2 + lane) : usa;
     // items are handed out longest first to whichever warp is free
     for (;;) {
       int r = 0;
@@ -287,7 +299,7 @@ __global__ void __launch_bounds__(YK_T, 2) k_snap_ystream(const __grid_constant_
         slot = slot == 2 ? 0 : slot + 1;
 #define YK_CASE(N)                                                                             \
   case N:                                                                                      \
-    yk_record<N>(T, usa, pi, m, n_steps, first, wt, Z);                                        \
+    yk_record<N>(T, usa, usb, pi, m, n_steps, first, wt, Z);                                   \
     if (last) yk_finish<YM, N>(S, it, lo, trip, coef, n, atom, valid, Z, Y, zout);             \
     break;
         switch ((f >> YF_N) & 7) {
@@ -350,13 +362,14 @@ __global__ void k_snap_yenergy(const __grid_constant__ SnapDev S, int nitem, int
   Ei[i] = (2.0 / 3.0) * t + S.ebias[si];
 }
 
-template <int YM>
-int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const char* tname, int64_t n, const int32_t* species,
-                     const double2* utot, double2* yout, double* Ei, double2* zout) {
-  const int smem = yk_smem(dev.nsp, dev.n_ytrip, dev.u_half, tab.nitem).total();
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_ystream<YM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+template <int YM, bool TWO = false>
+int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const char* tname, int64_t n,
+                     const int32_t* species, const double2* utot, const double2* utot2, double2* yout, double* Ei, double2* zout) {
+  const auto kernel = k_snap_ystream<YM, TWO>;
+  const int smem = yk_smem(dev.nsp, dev.n_ytrip, dev.u_half, tab.nitem, TWO).total();
+  CUDA_RET(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int per_sm = 1;
-  CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_ystream<YM>, YK_T, smem));
+  CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, YK_T, smem));
   const int64_t resident = (int64_t)ctx->num_sms * std::max(1, per_sm);
   const int64_t tiles = (n + YS_ATOMS - 1) / YS_ATOMS;
   // Fewer tiles than resident blocks: the items of a tile go to several blocks, at most one
@@ -366,17 +379,22 @@ int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const c
   const dim3 grid((unsigned)std::min(tiles, resident), (unsigned)nsplit);
   double* eitem = nullptr;
   if (YM != YM_Z && nsplit > 1) IPG_RET(scratch(ctx, "snap_yitem", (size_t)tab.nitem * n, &eitem));
-  IPG_TIMED_LAUNCH(ctx, tname, k_snap_ystream<YM>, grid, YK_T, smem, dev, tab, n, species, utot, yout, Ei, zout, eitem);
+  IPG_TIMED_LAUNCH(ctx, tname, kernel, grid, YK_T, smem, dev, tab, n, species, utot, utot2, yout, Ei, zout, eitem);
   if (eitem) IPG_LAUNCH(ctx, k_snap_yenergy, (unsigned)((n + 127) / 128), 128, 0, dev, tab.nitem, n, species, eitem, Ei);
   return IPG_OK;
 }
 
 }  // namespace
 
-int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n, const int32_t* species,
-                   const double2* utot, double2* yout, double* Ei, double2* zout) {
+int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n,
+                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout,
+                   const double2* utot2) {
   if (n <= 0) return IPG_OK;
-  if (ym == YM_Z) return launch_ystream_m<YM_Z>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
-  if (ym == YM_YZ) return launch_ystream_m<YM_YZ>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
-  return launch_ystream_m<YM_Y>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
+  if (utot2 && utot2 != utot) {
+    if (ym != YM_Z) return IPG_ERR_ARG;
+    return launch_ystream_m<YM_Z, true>(ctx, dev, tab, tname, n, species, utot, utot2, yout, Ei, zout);
+  }
+  if (ym == YM_Z) return launch_ystream_m<YM_Z>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
+  if (ym == YM_YZ) return launch_ystream_m<YM_YZ>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
+  return launch_ystream_m<YM_Y>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
 }
