@@ -96,82 +96,98 @@ struct PairBox {
 // Per-warp shared memory of the half-stencil walk.
 struct HalfWarp {
   double f[3][32];     // the forces of a batch
+  double col[3][32];   // column sums of the tile
   float4 home[32];     // the rows' cell-relative positions
-  unsigned rows[32];   // per row: the pairs of the batch that belong to it
-  unsigned cols[32];   // per column, likewise
+  int rows[32];        // per row: first pair of the batch that belongs to it | their count << 8
   uint16_t q[96];      // queued pairs, row | column << 8
 };
 
+// get_displacement (nnlist.jl:18-21) along an axis when |dx| < L (disp_axis_dev's result).
+__device__ __forceinline__ double disp_near(double L, double dx) {
+  if (isinf(L)) return dx;
+  const double d = dx < 0.0 ? __dadd_rn(dx, L) : (dx == 0.0 ? 0.0 : dx);
+  return __dmul_rn(2.0, d) < L ? d : __dsub_rn(d, L);
+}
+
 // Evaluates the first nh queued pairs (one per lane) and hands each pair's force to its row
-// owner (fa += f) and its column owner (ft -= f).  E and W accumulate lane-wise.
+// owner (fa += f) and its column's sum (-= f).  E and W accumulate lane-wise.
 //
-// The hand-off: forces go to shared memory, each owner gets the bit mask of its pairs (a row's
-// pairs are contiguous in the queue; a column's come from a match over the lanes) and adds them
-// in queue order: about three steps for the columns and seven for the rows of a batch, where
-// handing the columns over one row at a time took ten, each between two warp barriers.
-__device__ __forceinline__ void half_eval(const PairTerms& TT, const PairBox& B, int nh, int lane,
-                                          int row0, int col0, const int32_t* __restrict__ cell_atoms,
-                                          const double4* __restrict__ spos, HalfWarp& st, double* acc, double* fa,
-                                          double* ft) {
+// The hand-off, in queue order: a row's pairs are contiguous, so its owner lane adds a run of the
+// batch's forces; a column's pairs take turns by their rank among the pairs of that column (a match
+// over the lanes), each turn touching a column at most once.  About nine and four short steps a
+// batch, all with warp-uniform trip counts.
+__device__ __forceinline__ void half_eval(const PairTerms& TT, const PairBox& B, int nh, int lane, int row0, int col0,
+                                          const int32_t* __restrict__ cell_atoms, const double4* __restrict__ spos,
+                                          HalfWarp& st, double* acc, double* fa) {
   constexpr unsigned FULL = 0xffffffffu;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  int row = 64, col = 32 + lane;  // idle lanes: no row, a column of their own
   const bool act = lane < nh;
-  if (act) {
-    const int e = st.q[lane];
-    row = e & 0xff;
-    col = e >> 8;
-    const double4 xa = spos[row0 + row], xt = spos[col0 + col];
-    const int32_t ia = cell_atoms[row0 + row], it = cell_atoms[col0 + col];
-    const double d2 = sumsq3_dev(pe_axis_dev(B.L[0], xa.x, xt.x), pe_axis_dev(B.L[1], xa.y, xt.y),
-                                 pe_axis_dev(B.L[2], xa.z, xt.z));
-    // r = get_displacement(x_lo, x_hi) seen from the row atom
-    const bool lo = ia < it;
-    const double sg = lo ? 1.0 : -1.0;
-    const double r0 = sg * disp_axis_dev(B.L[0], lo ? xa.x : xt.x, lo ? xt.x : xa.x);
-    const double r1 = sg * disp_axis_dev(B.L[1], lo ? xa.y : xt.y, lo ? xt.y : xa.y);
-    const double r2 = sg * disp_axis_dev(B.L[2], lo ? xa.z : xt.z, lo ? xt.z : xa.z);
-    double V, g;
-    pair_terms_sum(TT, r0 * r0 + r1 * r1 + r2 * r2, d2, (int)xa.w, (int)xt.w, V, g);
-    fx = g * r0;
-    fy = g * r1;
-    fz = g * r2;
-    acc[0] += V;
-    // empirical_potential.jl:63-64: r * f' -> [xx, yy, zz, zy, zx, yx]
-    acc[1] += r0 * fx;
-    acc[2] += r1 * fy;
-    acc[3] += r2 * fz;
-    acc[4] += r2 * fy;
-    acc[5] += r2 * fx;
-    acc[6] += r1 * fx;
+  const int e = act ? st.q[lane] : 0;  // idle lanes: the first row and column, and no force
+  const int row = e & 0xff, col = e >> 8;
+  const double4 xa = spos[row0 + row], xt = spos[col0 + col];
+  // r = get_displacement(x_lo, x_hi) seen from the row atom
+  const bool lo = cell_atoms[row0 + row] < cell_atoms[col0 + col];
+  const double x0 = __dsub_rn(xa.x, xt.x), x1 = __dsub_rn(xa.y, xt.y), x2 = __dsub_rn(xa.z, xt.z);
+  double d2, r0, r1, r2;
+  if (__all_sync(FULL, fabs(x0) < B.L[0] && fabs(x1) < B.L[1] && fabs(x2) < B.L[2])) {
+    const double a0 = fabs(x0), a1 = fabs(x1), a2 = fabs(x2);  // PeriodicEuclidean (an open axis has L = inf)
+    d2 = sumsq3_dev(fmin(a0, __dsub_rn(B.L[0], a0)), fmin(a1, __dsub_rn(B.L[1], a1)), fmin(a2, __dsub_rn(B.L[2], a2)));
+    r0 = disp_near(B.L[0], lo ? x0 : -x0);
+    r1 = disp_near(B.L[1], lo ? x1 : -x1);
+    r2 = disp_near(B.L[2], lo ? x2 : -x2);
+  } else {  // a separation of a box length or more
+    d2 = sumsq3_dev(pe_axis_dev(B.L[0], xa.x, xt.x), pe_axis_dev(B.L[1], xa.y, xt.y), pe_axis_dev(B.L[2], xa.z, xt.z));
+    r0 = disp_axis_dev(B.L[0], lo ? xa.x : xt.x, lo ? xt.x : xa.x);
+    r1 = disp_axis_dev(B.L[1], lo ? xa.y : xt.y, lo ? xt.y : xa.y);
+    r2 = disp_axis_dev(B.L[2], lo ? xa.z : xt.z, lo ? xt.z : xa.z);
   }
+  double V, g;
+  pair_terms_sum_warp(TT, act, r0 * r0 + r1 * r1 + r2 * r2, d2, (int)xa.w, (int)xt.w, V, g);
+  if (!act) r0 = r1 = r2 = 0.0;
+  const double gs = lo ? g : -g;  // the row atom's force is along r for lo, against it otherwise
+  const double fx = gs * r0, fy = gs * r1, fz = gs * r2;
+  acc[0] += V;
+  // empirical_potential.jl:63-64: r * f' -> [xx, yy, zz, zy, zx, yx]
+  const double hx = g * r0, hy = g * r1, hz = g * r2;
+  acc[1] += r0 * hx;
+  acc[2] += r1 * hy;
+  acc[3] += r2 * hz;
+  acc[4] += r2 * hy;
+  acc[5] += r2 * hx;
+  acc[6] += r1 * hx;
   st.f[0][lane] = fx;
   st.f[1][lane] = fy;
   st.f[2][lane] = fz;
-  st.rows[lane] = 0u;
-  st.cols[lane] = 0u;
-  const int prev = __shfl_up_sync(FULL, row, 1);
-  const unsigned heads = __ballot_sync(FULL, lane == 0 || row != prev);  // first pair of each row, first idle lane
-  const unsigned same = __match_any_sync(FULL, col);
+  st.rows[lane] = 0;
+  const int key = act ? row : 64;
+  const int prev = __shfl_up_sync(FULL, key, 1);
+  const unsigned heads = __ballot_sync(FULL, lane == 0 || key != prev);  // first pair of each row, first idle lane
+  const unsigned same = __match_any_sync(FULL, act ? col : 32 + lane);
+  const int rank = __popc(same & ((1u << lane) - 1u));
   __syncwarp();
+  int len = 0;
   if (act && ((heads >> lane) & 1u)) {
     const unsigned above = heads & (0xfffffffeu << lane);  // later heads
-    const int end = above ? __ffs(above) - 1 : 32;         // idle lanes start a run of their own
-    st.rows[row] = (end == 32 ? FULL : (1u << end) - 1u) & (FULL << lane);
+    len = (above ? __ffs(above) - 1 : 32) - lane;          // idle lanes start a run of their own
+    st.rows[row] = lane | len << 8;
   }
-  if (act && (same & ((1u << lane) - 1u)) == 0u) st.cols[col] = same;
-  __syncwarp();
-  for (unsigned m = st.rows[lane]; m; m &= m - 1u) {
-    const int b = __ffs(m) - 1;
-    fa[0] += st.f[0][b];
-    fa[1] += st.f[1][b];
-    fa[2] += st.f[2][b];
+  const int turns = (int)__reduce_max_sync(FULL, (unsigned)rank) + 1;
+  const int longest = (int)__reduce_max_sync(FULL, (unsigned)len);
+  for (int k = 0; k < turns; k++) {
+    if (act && rank == k) {
+      st.col[0][col] -= fx;
+      st.col[1][col] -= fy;
+      st.col[2][col] -= fz;
+    }
+    __syncwarp();
   }
-  for (unsigned m = st.cols[lane]; m; m &= m - 1u) {
-    const int b = __ffs(m) - 1;
-    ft[0] -= st.f[0][b];
-    ft[1] -= st.f[1][b];
-    ft[2] -= st.f[2][b];
+  const int run = st.rows[lane], n = run >> 8;
+  const double* f = &st.f[0][run & 0xff];
+  for (int k = 0; k < longest; k++, f++) {
+    if (k < n) {
+      fa[0] += f[0];
+      fa[1] += f[32];
+      fa[2] += f[64];
+    }
   }
   __syncwarp();
 }
@@ -190,13 +206,15 @@ __device__ __forceinline__ void pbuf_put(double* __restrict__ P, int64_t n, int 
   }
 }
 
-// Bound by FP64 issue and latency of the term code.  Against full 64-bit tests of every candidate,
-// rows loaded one by one and the old hand-off: 4.1 M atoms, five terms 35.8 -> 17.7 ms a call;
-// 32,000 atoms 540 -> 309 us; 1,000 atoms, one term 92 -> 70 us.
+// Bound by FP64 issue and latency of the term code.  Full 64-bit tests of every candidate, rows
+// loaded one by one and a hand-off between two warp barriers a row took 35.8 ms a call at 4.1 M atoms
+// with five terms; 32-bit tests and masked hand-offs 17.7 ms; warp-uniform control flow in
+// half_eval (terms, cutoffs, distances, hand-off: lane-wise branches cost reconvergence around
+// each) 15.2 ms.  32,000 atoms: 540, 309, 273 us; 1,000 atoms, one term: 92, 70, 67 us.
 // PAIR_MINB: resident blocks per SM the register allocation is bounded for; 3, 4, 5, 6 (164, 128,
-// 96, 80 registers) took 21.2, 17.7, 17.9, 17.5 ms at 4.1 M atoms and 364, 309, 314, 322 us at
-// 32,000.
-constexpr int PAIR_MINB = 4;
+// 96, 80 registers) took 18.9, 15.7, 15.2, 15.2 ms at 4.1 M atoms, 323, 275, 273, 281 us at 32,000
+// and 66.8, 66.1, 67.1, 69.0 us at 1,000.
+constexpr int PAIR_MINB = 5;
 __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_constant__ PairTerms TT,
                                                                  const __grid_constant__ PairBox B, int64_t n,
                                                                  const ConfGrid* __restrict__ grid, int64_t ncells,
@@ -265,7 +283,7 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
         const float bx = b.x + sx, by = b.y + sy, bz = b.z + sz;
         // a cell with itself: the rows before the lane's own slot; another cell: every row
         const int lim = !tv ? 0 : (k == 0 && ts - rc < ra ? ts - rc : ra);
-        double ft[3] = {0.0, 0.0, 0.0};  // column sums of lane atom ts
+        st.col[0][lane] = st.col[1][lane] = st.col[2][lane] = 0.0;
         int nh = 0;
         __syncwarp();
         for (int q = 0; q < ra + 2; q += 2) {  // the last step evaluates what is left
@@ -284,7 +302,7 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
           // one call site of the term code: full batches, then the rest after the last row
           while (nh >= 32 || (q >= ra && nh > 0)) {
             const int m = nh < 32 ? nh : 32;
-            half_eval(TT, B, m, lane, rc, cc, cell_atoms, spos, st, acc, fa, ft);
+            half_eval(TT, B, m, lane, rc, cc, cell_atoms, spos, st, acc, fa);
             uint16_t e0 = 0, e1 = 0;  // the rest of the queue (fewer than 64 pairs) moves up
             if (lane < nh - m) e0 = st.q[m + lane];
             if (lane + 32 < nh - m) e1 = st.q[m + lane + 32];
@@ -295,7 +313,10 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
             __syncwarp();
           }
         }
-        if (tv) pbuf_put(P, n, tgt_kind, ts, ft, multi);
+        if (tv) {
+          const double ft[3] = {st.col[0][lane], st.col[1][lane], st.col[2][lane]};
+          pbuf_put(P, n, tgt_kind, ts, ft, multi);
+        }
         __syncwarp();
       }
       if (lane < ra) pbuf_put(P, n, home_kind, rc + lane, fa, multi);

@@ -24,6 +24,7 @@ struct PairTerms {
   int nterms;
   double rcut_max;
   double rmax2_hi;  // rcut_max^2 (1 + 1e-12): candidates beyond it are out for sure
+  int same_cut;     // every term has the cutoff rcut_max
   PairTermDev t[IPG_MAX_PAIR_TERMS];
 };
 
@@ -93,6 +94,8 @@ inline int pair_prepare_terms(const ipg_pair_term* terms, int nterms, PairTerms&
         return IPG_ERR_ARG;
     }
   }
+  pt.same_cut = 1;
+  for (int k = 0; k < nterms; k++) pt.same_cut &= pt.t[k].rcut == pt.rcut_max;
   pt.rmax2_hi = pt.rcut_max * pt.rcut_max * (1.0 + 1e-12);
   return IPG_OK;
 }
@@ -155,6 +158,11 @@ __device__ __forceinline__ void pair_term_eval(const PairTermDev& t, double R, d
   }
 }
 
+// sqrt(d2) within the term's cutoff, decided as by the square root.
+__device__ __forceinline__ bool pair_within(const PairTermDev& T, double d2) {
+  return !(d2 > T.rc2_hi) && !(d2 >= T.rc2_lo && sqrt(d2) > T.rcut);
+}
+
 // Sum of c_t V_t and c_t g_t over the terms that apply to a pair: d2 the squared distance of
 // the cutoffs (a term counts when sqrt(d2) <= rcut, decided as by the square root), r2 = |r|^2
 // of the formulas, species si and sj for the filters (src/types/empirical_potential.jl:26-43,
@@ -167,13 +175,35 @@ __device__ __forceinline__ void pair_terms_sum(const PairTerms& TT, double r2, d
   const double R = r2 > 0.0 ? r2 * ir : sqrt(r2);
   for (int t = 0; t < TT.nterms; t++) {
     const PairTermDev& T = TT.t[t];
-    if (d2 > T.rc2_hi) continue;
-    if (d2 >= T.rc2_lo && sqrt(d2) > T.rcut) continue;
+    if (!pair_within(T, d2)) continue;
     if (!((T.mask >> si) & 1ull) || !((T.mask >> sj) & 1ull)) continue;
     double v, gg;
     pair_term_eval(T, R, ir, ir2, v, gg);
     V += T.coeff * v;
     g += T.coeff * gg;
+  }
+}
+
+// The same for a whole warp, one pair per lane, act on the lanes that hold one: the control flow is
+// uniform (terms that no lane needs are skipped, the others are evaluated by every lane and
+// selected), which a lane-wise filter paid for with reconvergence around every term.
+__device__ __forceinline__ void pair_terms_sum_warp(const PairTerms& TT, bool act, double r2, double d2, int si,
+                                                    int sj, double& V, double& g) {
+  V = 0.0;
+  g = 0.0;
+  const double ir = rsqrt(r2), ir2 = ir * ir;
+  const double R = r2 > 0.0 ? r2 * ir : sqrt(r2);
+  const unsigned long long pm = (1ull << si) | (1ull << sj);  // both species in the term's set
+  if (TT.same_cut && TT.nterms) act = act && pair_within(TT.t[0], d2);
+  for (int t = 0; t < TT.nterms; t++) {
+    const PairTermDev& T = TT.t[t];
+    bool on = act && (~T.mask & pm) == 0ull;
+    if (!TT.same_cut) on = on && pair_within(T, d2);
+    if (!__any_sync(0xffffffffu, on)) continue;
+    double v, gg;
+    pair_term_eval(T, R, ir, ir2, v, gg);
+    V += on ? T.coeff * v : 0.0;
+    g += on ? T.coeff * gg : 0.0;
   }
 }
 

@@ -61,3 +61,28 @@ def test_half_tiles_edges(case):
     scale = np.max(np.abs(fo)) if case != "at_cutoff" else 1e-2  # a perfect lattice's forces cancel
     assert np.max(np.abs(f - fo)) <= TOL * scale
     assert rel_err(w, wo) <= TOL
+
+
+# terms of one cutoff with species filters, and of several cutoffs: a warp's lanes then differ in the terms they need
+TERMS = {
+    "one_cutoff": [("Ar", "Ne"), ("Ar",), ("Ne",), ("Kr", "Ar")],
+    "cutoffs": [("Ar", "Ne", "Kr"), ("Ar",), ("Ne", "Kr"), ("Kr",)],
+}
+
+
+@pytest.mark.parametrize("case", sorted(TERMS))
+@pytest.mark.parametrize("n", [1, 2, 33, 700])
+def test_half_tiles_mixed_terms(case, n):
+    rng = np.random.default_rng(n)
+    L = max(6.5, (n / 0.25) ** (1 / 3))
+    s = ipg.System(rng.uniform(0, L, (n, 3)), list(rng.choice(["Ar", "Ne", "Kr"], n)), [L] * 3)
+    p = None
+    for t, names in enumerate(TERMS[case]):
+        rc = 3.0 if case == "one_cutoff" else 3.0 - 0.4 * t
+        q = (0.5 + 0.25 * t) * ipg.Morse(0.1 + 0.1 * t, 0.5, 1.5, rc, list(names))
+        p = q if p is None else p + q
+    e, f, w = ipg.empirical.pair_eval(s, ipg.empirical.empirical_terms(p), ctx=ipg.Context(0))
+    eo, fo, wo = oracle_eval(s, p)
+    assert abs(e - eo) <= TOL * max(abs(eo), 1e-300)
+    assert np.max(np.abs(f - fo), initial=0.0) <= TOL * max(np.max(np.abs(fo)), 1e-300)
+    assert rel_err(w, wo) <= TOL
