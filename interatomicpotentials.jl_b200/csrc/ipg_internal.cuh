@@ -234,8 +234,7 @@ struct CellList {
   int32_t* d_cell_atoms = nullptr; // [n] atom ids in cell order (ascending inside a cell)
   int32_t* d_slot_of = nullptr;    // [n] slot of each atom
   double4* d_spos = nullptr;       // [n] positions in slot order (w = species as double)
-  bool want_rel = false;           // in: also build d_srel
-  float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell
+  float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell, w = atom id's bits
 };
 
 // Builds the cell list for `radius` (prefix selects the scratch buffers used).
@@ -276,6 +275,18 @@ int ipg_max_disp2(ipg_ctx* ctx, const CellList& cl, const double* d_pos, const d
 int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const int32_t* d_species, int nsp,
                     const double* h_cut, int mode, bool want_transpose, PairList& pl, bool sorted = true,
                     int64_t cap = 0, int walk_warps = 4, bool count_only = false);
+
+// Squared threshold of a 32-bit distance test on cell-relative positions (CellList::d_srel): no pair
+// within rcut fails it.  Each coordinate of each
+// atom is at most about one cell edge (cs) and rounded to 32 bits, as are the shift between the
+// cells (at most cs) and the difference (at most 2 cs): at most 6 * 2^-24 cs per axis, less than
+// 7e-7 cs in distance; the squares and their sum add a relative 3 * 2^-24.
+__host__ __device__ inline float prefilter_threshold(const ConfGrid& g, double rcut) {
+  const double cs = fmax(g.cs[0], fmax(g.cs[1], g.cs[2]));
+  const double r = rcut + 2e-6 * cs;
+  const double t = r * r * (1.0 + 1e-6);
+  return t < 1e30 ? (float)t : 1e30f;
+}
 
 // Device helper: the distinct neighbor-cell coordinates along one axis (<= 3).
 __device__ __forceinline__ int stencil_axis(int c, int nc, bool per, int* out) {

@@ -84,8 +84,8 @@ __device__ __forceinline__ int64_t cell_of_atom(int64_t i, const double* __restr
   return g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
 }
 
-// Atom i of cell c (of grid g) into slot s of the cell order; srel (optional) receives its
-// position relative to the cell's lower corner.
+// Atom i of cell c (of grid g) into slot s of the cell order; srel receives its position
+// relative to the cell's lower corner, and its id in w.
 __device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid& g, int64_t c,
                                            const double* __restrict__ pos, const int32_t* __restrict__ species,
                                            int nsp, int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
@@ -96,12 +96,10 @@ __device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid&
   sp = sp < 0 ? 0 : (sp > nsp - 1 ? nsp - 1 : sp);  // bad ids were reported with the cell
   const double x = pos[3 * (int64_t)i], y = pos[3 * (int64_t)i + 1], z = pos[3 * (int64_t)i + 2];
   spos[s] = make_double4(x, y, z, (double)sp);
-  if (srel) {
-    const int k = (int)(c - g.cell_off), nxy = g.nc[0] * g.nc[1];
-    const int cz = k / nxy, cy = (k - cz * nxy) / g.nc[0], cx = k - cz * nxy - cy * g.nc[0];
-    srel[s] = make_float4((float)(cell_wrap(g, 0, x) - cx * g.cs[0]), (float)(cell_wrap(g, 1, y) - cy * g.cs[1]),
-                          (float)(cell_wrap(g, 2, z) - cz * g.cs[2]), 0.0f);
-  }
+  const int k = (int)(c - g.cell_off), nxy = g.nc[0] * g.nc[1];
+  const int cz = k / nxy, cy = (k - cz * nxy) / g.nc[0], cx = k - cz * nxy - cy * g.nc[0];
+  srel[s] = make_float4((float)(cell_wrap(g, 0, x) - cx * g.cs[0]), (float)(cell_wrap(g, 1, y) - cy * g.cs[1]),
+                        (float)(cell_wrap(g, 2, z) - cz * g.cs[2]), __int_as_float(i));
 }
 
 __global__ void k_cell_count(int64_t n, const double* __restrict__ pos, const int32_t* __restrict__ species, int nsp,
@@ -408,17 +406,32 @@ __global__ void k_clamp_offsets(int64_t n, int64_t* __restrict__ off, int64_t ca
   }
 }
 
-// The same walk with one warp per cell: every atom of a cell has the same stencil, so each
-// chunk of 32 candidates is loaded once and tested against every atom of a group of up to 32
-// atoms of the cell, in two phases.  Phase 1 applies only the first test of pair_ok (the
-// periodic distance against the candidate radius, with the same arithmetic, so the same
-// decision; a separation of a box length or more is left to the full test), WALK_ILP atoms at
-// a time so that their independent FP64 chains overlap, and queues the (atom, candidate) pairs
-// that pass in (atom, lane) order in a per-warp ring.  Phase 2 runs the full pair_ok on 32
-// queued pairs at a time, one per lane, and emits the members after each atom's running count
-// (shared memory).  One test in eight passes: with the member path inside the chunk loop, the
-// few members of a chunk made every lane run it.  Each atom's hits come out in candidate order,
-// as from k_pair_walk.
+// The same walk by cells: every atom of a cell has the same stencil, so a warp takes a group of
+// 32 >> split atoms of a cell, loads each chunk of 32 candidates once and tests it against every
+// atom of the group, in two phases.  Phase 1 applies a test that is false only when pair_ok is,
+// WALK_ILP atoms at a time so that their chains overlap, and queues the (atom, candidate) pairs
+// that pass in (atom, lane) order in a per-warp ring.  Phase 2 runs the full pair_ok on 32 queued
+// pairs at a time, one per lane, and emits the members after each atom's running count (shared
+// memory).  One test in eight passes: with the member path inside the chunk loop, the few members
+// of a chunk made every lane run it.  Each atom's hits come out in candidate order, as from
+// k_pair_walk: lane k of the warp holds the k-th cell of the stencil in that order, and the chunks
+// run through the cells' atoms end to end (walk_chunk), the next one loading while the present
+// one is tested.
+//
+// Phase 1 tests in 32 bits on cell-relative positions where the grid allows it (REL: the walk's
+// radius within the cells', at least 3 cells on every periodic axis, so that a pair within the
+// radius is at the image that its two cells define; the threshold covers the rounding,
+// prefilter_threshold), and otherwise as pair_ok does: the periodic distance against the radius,
+// with the same arithmetic; a separation of a box length or more is left to the full test.
+//
+// Bound by latency (a cell is a serial chain of chunks) and, in the 64-bit test, FP64 issue.  Against
+// one warp a cell, ranges listed serially, no loads ahead and the 64-bit test only: 345 -> 315 us a
+// call at 8,192 atoms in 14s, 2,580 -> 2,525 at 54,000 in 31s, 519 -> 477 at 1,999, 206 -> 182 at 249
+// (the whole energy and forces; REL alone 18, 60, 5 and 4 us of these).
+// The split: a cell's atoms go to 8 warps where there are no more cells than SMs (249 atoms in 8
+// cells: 182 against 193 us; 1,999 in 64: 477 against 488).  Beyond that every warp's start (the
+// stencil's cells, the first chunk) costs more than the shorter chains give: 512 cells 3,146
+// against 3,125 us a pullback, 1,728 cells 2,607 against 2,525.
 constexpr int WALKC_WARPS = 4;
 constexpr int WALK_ILP = 4;    // atoms per phase-1 step
 constexpr int WALK_RING = 256;  // queue entries per warp (a step adds at most 32 * WALK_ILP to fewer than 32)
@@ -429,6 +442,17 @@ struct WalkAtom {
 };
 struct WalkQ {
   int32_t slot, ii;  // candidate slot, group atom
+};
+struct WalkShared {
+  WalkAtom a[32];
+  float4 rel[32];  // the atoms' cell-relative positions, w = id
+  WalkQ q[WALK_RING];
+};
+// Lane k: the k-th non-empty cell of the stencil.
+struct WalkStencil {
+  int start, base;  // its first candidate's place in the walk (INT_MAX: no cell), slot minus place
+  float sx, sy, sz;  // its corner relative to the home cell's at the image of the stencil
+  int total;         // candidates
 };
 
 // The first test of pair_ok: false only when pair_ok is false.  Branch-free: every term is
@@ -444,136 +468,244 @@ __device__ __forceinline__ bool walk_prefilter(const PairTest& t, const double* 
   return other & (far | (sumsq3_dev(m0, m1, m2) <= t.rcut2_hi));
 }
 
+// Stencil of cell cc, in stencil_ranges' order (z, y in the order of stencil_axis, x ascending).
+__device__ __forceinline__ void walk_stencil(const ConfGrid& g, const int* cc, const int64_t* __restrict__ cell_start,
+                                             int lane, WalkShared& sh, WalkStencil& st) {
+  constexpr unsigned FULL = 0xffffffffu;
+  int ax[3][3], na[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) na[a] = stencil_axis(cc[a], g.nc[a], !isinf(g.L[a]), ax[a]);
+  int beg = 0, len = 0;
+  float s[3] = {0.0f, 0.0f, 0.0f};
+  if (lane < na[0] * na[1] * na[2]) {
+    const int k[3] = {lane % na[0], lane / na[0] % na[1], lane / (na[0] * na[1])};
+    int c[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (a == 0) {  // the k-th smallest of the distinct cells
+        c[0] = 0;
+        for (int q = 0; q < na[0]; q++) {
+          int below = 0;
+          for (int u = 0; u < na[0]; u++) below += ax[0][u] < ax[0][q];
+          if (below == k[0]) c[0] = ax[0][q];
+        }
+      } else {
+        c[a] = ax[a][k[a]];
+      }
+      int d = c[a] - cc[a];  // in -1..1 but for the wrap
+      d = d > 1 ? d - g.nc[a] : (d < -1 ? d + g.nc[a] : d);
+      s[a] = (float)(d * g.cs[a]);
+    }
+    const int64_t cell = g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
+    beg = (int)cell_start[cell];
+    len = (int)cell_start[cell + 1] - beg;
+  }
+  int incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += v;
+  }
+  st.total = __shfl_sync(FULL, incl, 31);
+  // the empty cells drop out (through the warp's shared memory)
+  const unsigned some = __ballot_sync(FULL, len > 0);
+  if (len > 0) {
+    const int at = __popc(some & ((1u << lane) - 1u));
+    sh.q[at] = WalkQ{incl - len, beg - (incl - len)};
+    sh.rel[at] = make_float4(s[0], s[1], s[2], 0.0f);
+  }
+  __syncwarp();
+  const bool have = lane < __popc(some);
+  st.start = have ? sh.q[lane].slot : INT_MAX;
+  st.base = have ? sh.q[lane].ii : 0;
+  st.sx = have ? sh.rel[lane].x : 0.0f;
+  st.sy = have ? sh.rel[lane].y : 0.0f;
+  st.sz = have ? sh.rel[lane].z : 0.0f;
+  __syncwarp();
+}
+
+// A chunk of candidates: lane l holds the one at place P + l.
+struct WalkChunk {
+  int slot;  // -1: past the last candidate
+  int32_t j;
+  float4 r;   // REL: relative to the home cell's corner
+  double4 x;  // otherwise
+};
+template <bool REL>
+__device__ __forceinline__ void walk_chunk(const WalkStencil& st, int P, int lane,
+                                           const int32_t* __restrict__ cell_atoms, const double4* __restrict__ spos,
+                                           const float4* __restrict__ srel, WalkChunk& ch) {
+  constexpr unsigned FULL = 0xffffffffu;
+  // the cell of place P + l is the last that starts at or before it
+  const int d = st.start - P;
+  const int before = __popc(__ballot_sync(FULL, d <= 0));
+  const unsigned marks = __reduce_or_sync(FULL, d > 0 && d < 32 ? 1u << d : 0u);
+  const int k = before - 1 + __popc(marks & ((2u << lane) - 1u));
+  const int base = __shfl_sync(FULL, st.base, k);
+  const bool in = P + lane < st.total;
+  ch.slot = in ? base + P + lane : -1;
+  if (REL) {
+    const float sx = __shfl_sync(FULL, st.sx, k), sy = __shfl_sync(FULL, st.sy, k), sz = __shfl_sync(FULL, st.sz, k);
+    if (in) {
+      ch.r = srel[ch.slot];
+      ch.r.x += sx;
+      ch.r.y += sy;
+      ch.r.z += sz;
+      ch.j = __float_as_int(ch.r.w);
+    }
+  } else if (in) {
+    ch.j = cell_atoms[ch.slot];
+    ch.x = spos[ch.slot];
+  }
+}
+
+// The group of G atoms in sh against every candidate (WM as for k_pair_walk_cells).
+template <int WM, bool REL>
+__device__ __forceinline__ void walk_group(const PairTest& t, const ConfGrid& g, const WalkStencil& st, int G,
+                                           int lane, float thr, const int32_t* __restrict__ cell_atoms,
+                                           const double4* __restrict__ spos, const float4* __restrict__ srel,
+                                           WalkShared& sh, int32_t* __restrict__ outj, double* __restrict__ outr) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned lt = (1u << lane) - 1u;
+  WalkAtom* A = sh.a;
+  const bool half = t.mode == IPG_NLIST_HALF;
+  int P = 0, ii = 0;
+  unsigned head = 0, tail = 0;  // ring positions (mod WALK_RING) of the first and next entries
+  WalkChunk cur, nxt;
+  walk_chunk<REL>(st, 0, lane, cell_atoms, spos, srel, nxt);
+  // the (chunk, atoms) sequence flattened, so that phase 2 has one call site: each pass takes one
+  // step of phase 1, then drains full batches, and the remainder after the last step
+  for (;;) {
+    const bool more = P < st.total;  // warp-uniform
+    if (more) {
+      if (ii == 0) {
+        cur = nxt;
+        if (P + 32 < st.total) walk_chunk<REL>(st, P + 32, lane, cell_atoms, spos, srel, nxt);
+      }
+      bool cand[WALK_ILP];
+#pragma unroll
+      for (int k = 0; k < WALK_ILP; k++) {
+        const int a = ii + k < G ? ii + k : ii;
+        const bool in = (cur.slot >= 0) & (ii + k < G);
+        if (REL) {
+          const float4 h = sh.rel[a];
+          const int32_t i = __float_as_int(h.w);
+          const float x = h.x - cur.r.x, y = h.y - cur.r.y, z = h.z - cur.r.z;
+          cand[k] = in & (half ? cur.j > i : cur.j != i) & (fmaf(x, x, fmaf(y, y, z * z)) <= thr);
+        } else {
+          cand[k] = in & walk_prefilter(t, g.L, A[a].i, A[a].x, cur.j, cur.x);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < WALK_ILP; k++) {
+        const unsigned bal = __ballot_sync(FULL, cand[k]);
+        if (cand[k]) sh.q[(tail + __popc(bal & lt)) % WALK_RING] = WalkQ{cur.slot, ii + k};
+        tail += __popc(bal);
+      }
+      ii += WALK_ILP;
+      if (ii >= G) {
+        ii = 0;
+        P += 32;
+      }
+    }
+    while (tail - head >= 32u || (!more && tail != head)) {  // phase 2 on the next m queued pairs
+      __syncwarp();
+      const int m = tail - head < 32u ? (int)(tail - head) : 32;
+      bool ok = false;
+      int e_ii = 0;
+      int32_t e_j = 0;
+      double rr[3];
+      if (lane < m) {
+        const WalkQ e = sh.q[(head + lane) % WALK_RING];
+        e_ii = e.ii;
+        e_j = cell_atoms[e.slot];
+        ok = pair_ok(t, g.L, A[e_ii].i, A[e_ii].x, e_j, spos[e.slot], rr);
+      }
+      const unsigned bal = __ballot_sync(FULL, ok);
+      // lanes of the same atom: its members rank after the atom's running count
+      const unsigned grp = __match_any_sync(FULL, lane < m ? e_ii : 32 + lane);
+      if (WM != 0 && ok) {
+        const int64_t o = A[e_ii].base + A[e_ii].cnt + __popc(bal & grp & lt);
+        if (o < A[e_ii].end) {  // a list cut at the capacity (capacity mode) drops its tail
+          outj[o] = e_j;
+          outr[3 * o] = rr[0];
+          outr[3 * o + 1] = rr[1];
+          outr[3 * o + 2] = rr[2];
+        }
+      }
+      __syncwarp();
+      if (lane < m && (grp >> lane) == 1u) A[e_ii].cnt += __popc(bal & grp);  // the group's last lane
+      head += m;
+      __syncwarp();
+    }
+    if (!more) break;
+  }
+}
+
 // WM 0: count each atom's hits into cnt (and their maximum into *maxcnt); 1: emit them at
 // off[i]..off[i+1]; 2: both at once, emitting into kcap padded slots per atom (i * kcap ..),
 // hits beyond kcap dropped (the count and *maxcnt still see them).
 template <int WM>
 __global__ void __launch_bounds__(WALKC_WARPS * 32) k_pair_walk_cells(
-    int64_t ncells, PairTest t, const ConfGrid* __restrict__ grid, const int32_t* __restrict__ conf,
-    const int64_t* __restrict__ cell_start, const int32_t* __restrict__ cell_atoms, const double4* __restrict__ spos,
-    int64_t* __restrict__ cnt, const int64_t* __restrict__ off, int32_t* __restrict__ outj,
-    double* __restrict__ outr, int kcap, int* __restrict__ maxcnt) {
-  constexpr bool EMIT = WM != 0;
-  __shared__ WalkAtom sa[WALKC_WARPS][32];
-  __shared__ WalkQ sq[WALKC_WARPS][WALK_RING];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * WALKC_WARPS + w;
+    int64_t ncells, int split, bool rel_ok, PairTest t, const ConfGrid* __restrict__ grid,
+    const int32_t* __restrict__ conf, const int64_t* __restrict__ cell_start, const int32_t* __restrict__ cell_atoms,
+    const double4* __restrict__ spos, const float4* __restrict__ srel, int64_t* __restrict__ cnt,
+    const int64_t* __restrict__ off, int32_t* __restrict__ outj, double* __restrict__ outr, int kcap,
+    int* __restrict__ maxcnt) {
+  __shared__ WalkShared shw[WALKC_WARPS];
+  const int lane = threadIdx.x & 31;
+  WalkShared& sh = shw[threadIdx.x >> 5];
+  const int64_t u = (int64_t)blockIdx.x * WALKC_WARPS + (threadIdx.x >> 5);
+  const int64_t c = u >> split;
   if (c >= ncells) return;  // warp-uniform; the kernel synchronises only within a warp
-  const int64_t s0 = cell_start[c], s1 = cell_start[c + 1];
-  if (s0 == s1) return;
+  const int gw = 32 >> split;  // atoms of a group; a cell's groups go to its 2^split warps in turn
+  const int64_t s0 = cell_start[c] + gw * (u & ((1 << split) - 1)), s1 = cell_start[c + 1];
+  if (s0 >= s1) return;
   const ConfGrid g = grid[conf[cell_atoms[s0]]];
   int cc[3];
   {
-    const double4 x0 = spos[s0];
-    cell_coords(g, x0.x, x0.y, x0.z, cc);
+    const int64_t k = c - g.cell_off;
+    const int nxy = g.nc[0] * g.nc[1];
+    cc[2] = (int)(k / nxy);
+    const int rem = (int)(k - (int64_t)cc[2] * nxy);
+    cc[1] = rem / g.nc[0];
+    cc[0] = rem - cc[1] * g.nc[0];
   }
-  StencilRanges R;
-  stencil_ranges(g, cc, cell_start, R);
-  const unsigned lt = (1u << lane) - 1u;
-  WalkAtom* A = sa[w];
-  WalkQ* Q = sq[w];
+  WalkStencil st;
+  walk_stencil(g, cc, cell_start, lane, sh, st);
+  bool rel = rel_ok;
+#pragma unroll
+  for (int a = 0; a < 3; a++) rel &= isinf(g.L[a]) || g.nc[a] >= 3;
+  const float thr = prefilter_threshold(g, t.rcut);
   for (int64_t g0 = s0; g0 < s1; g0 += 32) {
-    const int G = (int)((s1 - g0) < 32 ? (s1 - g0) : 32);
+    const int G = (int)((s1 - g0) < gw ? (s1 - g0) : gw);
     __syncwarp();
     if (lane < G) {
       const int32_t i = cell_atoms[g0 + lane];
-      A[lane].i = i;
-      A[lane].cnt = 0;
-      A[lane].x = spos[g0 + lane];
+      sh.rel[lane] = srel[g0 + lane];
+      sh.a[lane].i = i;
+      sh.a[lane].cnt = 0;
+      sh.a[lane].x = spos[g0 + lane];
       if (WM == 1) {
-        A[lane].base = off[i];
-        A[lane].end = off[i + 1];
+        sh.a[lane].base = off[i];
+        sh.a[lane].end = off[i + 1];
       } else {
-        A[lane].base = (int64_t)i * kcap;
-        A[lane].end = (int64_t)i * kcap + kcap;
+        sh.a[lane].base = (int64_t)i * kcap;
+        sh.a[lane].end = (int64_t)i * kcap + kcap;
       }
     }
     __syncwarp();
-    // the (range, chunk, atoms) sequence flattened, so that phase 2 has one call site: each
-    // pass takes one step of phase 1, then drains full batches, and the remainder after the
-    // last step
-    int r = 0;
-    while (r < R.n && R.beg[r] >= R.end[r]) r++;
-    int64_t q0 = r < R.n ? R.beg[r] : 0, q = 0;
-    int ii = 0;
-    unsigned head = 0, tail = 0;  // ring positions (mod WALK_RING) of the first and next entries
-    bool inq = false;
-    int32_t j = 0;
-    double4 xj = make_double4(0.0, 0.0, 0.0, 0.0);
-    for (;;) {
-      const bool more = r < R.n;  // warp-uniform
-      if (more) {
-        if (ii == 0) {  // a new chunk of candidates
-          q = q0 + lane;
-          inq = q < R.end[r];
-          if (inq) {
-            j = cell_atoms[q];
-            xj = spos[q];
-          }
-        }
-        bool cand[WALK_ILP];
-#pragma unroll
-        for (int k = 0; k < WALK_ILP; k++) {
-          const int a = ii + k < G ? ii + k : ii;
-          cand[k] = inq & (ii + k < G) & walk_prefilter(t, g.L, A[a].i, A[a].x, j, xj);
-        }
-#pragma unroll
-        for (int k = 0; k < WALK_ILP; k++) {
-          const unsigned bal = __ballot_sync(0xffffffffu, cand[k]);
-          if (cand[k]) Q[(tail + __popc(bal & lt)) % WALK_RING] = WalkQ{(int32_t)q, ii + k};
-          tail += __popc(bal);
-        }
-        ii += WALK_ILP;
-        if (ii >= G) {
-          ii = 0;
-          q0 += 32;
-          if (q0 >= R.end[r]) {
-            do r++;
-            while (r < R.n && R.beg[r] >= R.end[r]);
-            if (r < R.n) q0 = R.beg[r];
-          }
-        }
-      }
-      while (tail - head >= 32u || (!more && tail != head)) {  // phase 2 on the next m queued pairs
-        __syncwarp();
-        const int m = tail - head < 32u ? (int)(tail - head) : 32;
-        bool ok = false;
-        int e_ii = 0;
-        int32_t e_j = 0;
-        double rr[3];
-        if (lane < m) {
-          const WalkQ e = Q[(head + lane) % WALK_RING];
-          e_ii = e.ii;
-          e_j = cell_atoms[e.slot];
-          ok = pair_ok(t, g.L, A[e_ii].i, A[e_ii].x, e_j, spos[e.slot], rr);
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, ok);
-        // lanes of the same atom: its members rank after the atom's running count
-        const unsigned grp = __match_any_sync(0xffffffffu, lane < m ? e_ii : 32 + lane);
-        if (EMIT && ok) {
-          const int64_t o = A[e_ii].base + A[e_ii].cnt + __popc(bal & grp & lt);
-          if (o < A[e_ii].end) {  // a list cut at the capacity (capacity mode) drops its tail
-            outj[o] = e_j;
-            outr[3 * o] = rr[0];
-            outr[3 * o + 1] = rr[1];
-            outr[3 * o + 2] = rr[2];
-          }
-        }
-        __syncwarp();
-        if (lane < m && (grp >> lane) == 1u) A[e_ii].cnt += __popc(bal & grp);  // the group's last lane
-        head += m;
-        __syncwarp();
-      }
-      if (!more) break;
-    }
+    if (rel)
+      walk_group<WM, true>(t, g, st, G, lane, thr, cell_atoms, spos, srel, sh, outj, outr);
+    else
+      walk_group<WM, false>(t, g, st, G, lane, thr, cell_atoms, spos, srel, sh, outj, outr);
     if (WM != 1) {
       int km = 0;
       if (lane < G) {
-        km = A[lane].cnt;
-        cnt[A[lane].i] = km;
+        km = sh.a[lane].cnt;
+        cnt[sh.a[lane].i] = km;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) km = max(km, __shfl_xor_sync(0xffffffffu, km, o));
+      km = __reduce_max_sync(0xffffffffu, km);
       if (lane == 0) atomicMax(maxcnt, km);
     }
   }
@@ -737,8 +869,7 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
   IPG_RET(scratch(ctx, (pre + "cell_atoms").c_str(), n, &cl.d_cell_atoms));
   IPG_RET(scratch(ctx, (pre + "slot_of").c_str(), n, &cl.d_slot_of));
   IPG_RET(scratch(ctx, (pre + "spos").c_str(), n, &cl.d_spos));
-  cl.d_srel = nullptr;
-  if (cl.want_rel) IPG_RET(scratch(ctx, (pre + "srel").c_str(), n, &cl.d_srel));
+  IPG_RET(scratch(ctx, (pre + "srel").c_str(), n, &cl.d_srel));
   count = cl.d_cell_start;
   if (n > 0 && n <= SMALL_ATOMS && cell_total <= SMALL_CELLS) {
     IPG_LAUNCH(ctx, k_cells_small, 1, SMALL_T, 0, (int)n, (int)cell_total, d_pos, d_species, nsp, cl.d_grid, nconf,
@@ -819,15 +950,17 @@ int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const 
     IPG_RET(scratch(ctx, (pre + "pad_j").c_str(), (size_t)n * kcap + 1, &pad_j));
     IPG_RET(scratch(ctx, (pre + "pad_r").c_str(), 3 * (size_t)n * kcap + 3, &pad_r));
   }
+  const int split = cl.ncells <= ctx->num_sms ? 3 : 0;
+  const bool rel_ok = t.rcut <= cl.radius;
   if (n > 0) {
     if (by_cell && kcap > 0)
-      IPG_LAUNCH(ctx, k_pair_walk_cells<2>, nblk(cl.ncells, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, t,
-                 cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cnt, nullptr, pad_j, pad_r, kcap,
-                 maxcnt);
+      IPG_LAUNCH(ctx, k_pair_walk_cells<2>, nblk(cl.ncells << split, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, split,
+                 rel_ok, t, cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cl.d_srel, cnt, nullptr, pad_j,
+                 pad_r, kcap, maxcnt);
     else if (by_cell)
-      IPG_LAUNCH(ctx, k_pair_walk_cells<0>, nblk(cl.ncells, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, t,
-                 cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cnt, nullptr, nullptr, nullptr, 0,
-                 maxcnt);
+      IPG_LAUNCH(ctx, k_pair_walk_cells<0>, nblk(cl.ncells << split, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, split,
+                 rel_ok, t, cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cl.d_srel, cnt, nullptr, nullptr,
+                 nullptr, 0, maxcnt);
     else
       IPG_LAUNCH(ctx, k_pair_walk<false>, nblk(32 * n, wt), wt, 0, n, t, cl.d_grid, cl.d_conf, cl.d_cell_start,
                  cl.d_cell_atoms, cl.d_spos, cnt, nullptr, nullptr, nullptr);
@@ -853,9 +986,9 @@ int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const 
     if (by_cell && kcap > 0 && (cap > 0 || hmax <= kcap))
       IPG_LAUNCH(ctx, k_pad_compact, nblk(n * kcap, 256), 256, 0, n, kcap, pl.d_off, pad_j, pad_r, pl.d_j, pl.d_r);
     else if (by_cell)
-      IPG_LAUNCH(ctx, k_pair_walk_cells<1>, nblk(cl.ncells, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, t,
-                 cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, nullptr, pl.d_off, pl.d_j,
-                 pl.d_r, 0, nullptr);
+      IPG_LAUNCH(ctx, k_pair_walk_cells<1>, nblk(cl.ncells << split, WALKC_WARPS), WALKC_WARPS * 32, 0, cl.ncells, split,
+                 rel_ok, t, cl.d_grid, cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cl.d_srel, nullptr, pl.d_off,
+                 pl.d_j, pl.d_r, 0, nullptr);
     else
       IPG_LAUNCH(ctx, k_pair_walk<true>, nblk(32 * n, wt), wt, 0, n, t, cl.d_grid, cl.d_conf, cl.d_cell_start,
                  cl.d_cell_atoms, cl.d_spos, nullptr, pl.d_off, pl.d_j, pl.d_r);

@@ -22,7 +22,7 @@
 // Only one candidate in eight is within the cutoff, so the row walk tests them in 32 bits on
 // cell-relative positions: with at least 3 cells on every periodic axis a pair within the cutoff
 // is at the image that its two cells define, so no minimum image is needed, and the test's
-// threshold covers the rounding of the 32-bit coordinates (pair_prefilter_threshold).  It only
+// threshold covers the rounding of the 32-bit coordinates (prefilter_threshold).  It only
 // proposes; the reference's own test and all arithmetic of the pairs it proposes are 64-bit.
 //
 // The half stencil visits each pair of neighboring cells once only when every periodic axis
@@ -336,17 +336,6 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
   }
 }
 
-// Squared threshold of the 32-bit test: no pair within rcut fails it.  Each coordinate of each
-// atom is at most about one cell edge (cs) and rounded to 32 bits, as are the shift between the
-// cells (at most cs) and the difference (at most 2 cs): at most 6 * 2^-24 cs per axis, less than
-// 7e-7 cs in distance; the squares and their sum add a relative 3 * 2^-24.
-float pair_prefilter_threshold(const ConfGrid& g, double rcut) {
-  const double cs = std::max(g.cs[0], std::max(g.cs[1], g.cs[2]));
-  const double r = rcut + 2e-6 * cs;
-  const double t = r * r * (1.0 + 1e-6);
-  return t < 1e30 ? (float)t : 1e30f;
-}
-
 // E and W6 from the per-block partials of nblocks blocks in a fixed order (one block of
 // FINISH_T threads); component 0 goes to E, 1..6 to W6 (either may be null).
 constexpr int FINISH_T = 256;
@@ -437,7 +426,6 @@ int pair_eval_device(ipg_ctx* ctx, int64_t n, const double* d_pos, const int32_t
   IPG_RET(ipg_status_reset(ctx));
   int64_t aoff[2] = {0, n};
   CellList cl;
-  cl.want_rel = true;
   IPG_RET(ipg_build_cells(ctx, "pair_", n, d_pos, d_species, 64, 1, aoff, L, pt.rcut_max, cl));
   if (grid_out) *grid_out = cl.h_grid;
   const ConfGrid& g = cl.h_grid[0];
@@ -459,7 +447,7 @@ int pair_eval_device(ipg_ctx* ctx, int64_t n, const double* d_pos, const int32_t
     IPG_RET(scratch(ctx, "pair_partial", (size_t)nb * 7, &partial));
     IPG_RET(scratch(ctx, "pair_pbuf", (size_t)PBUF_SLOTS * 3 * n, &P));
     IPG_LAUNCH(ctx, k_pair_half, (unsigned)nb, PAIR_T, 0, pt, box, n, cl.d_grid, cl.ncells, cl.d_cell_start,
-               cl.d_cell_atoms, cl.d_spos, cl.d_srel, pair_prefilter_threshold(g, pt.rcut_max), P, partial);
+               cl.d_cell_atoms, cl.d_spos, cl.d_srel, prefilter_threshold(g, pt.rcut_max), P, partial);
     if (want_f)
       IPG_LAUNCH(ctx, k_pair_finish, (unsigned)((n + FINISH_T - 1) / FINISH_T + 1), FINISH_T, 0, n, cl.d_grid,
                  cl.d_cell_atoms, cl.d_spos, P, d_F, nb, partial, Eo, Wo);
