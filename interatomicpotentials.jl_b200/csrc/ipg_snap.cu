@@ -1669,46 +1669,69 @@ int launch_vsum(ipg_ctx* ctx, const SnapDev& S, int64_t a0, int64_t nc, const in
   }
 }
 
-// sum over the half plane of level l, entries z0.. of Z: w Re(conj(X) Z), w = 1 below the
-// middle element of an even level, 1/2 on it (the weights of compute_b.jl:207-400)
-__device__ __forceinline__ double half_dot(const double2* __restrict__ xs, int l, int hb,
-                                           const double2* __restrict__ Z, int64_t z0, int64_t zs) {
-  const int nf = nfull_of(l);
+// sums over the half plane of level l, entries z0.. of Z: w Re(conj(X) Z) and, with TWO, the same of
+// Y (at X's layout), w = 1 below the middle element of an even level, 1/2 on it (the weights of
+// compute_b.jl:207-400).  Z is read ILP entries at a time, the last ones of a level too: the loads'
+// latency is what the contractions wait for.
+template <bool TWO, int ILP>
+__device__ __forceinline__ void half_dot(const double2* __restrict__ xs, const double2* __restrict__ ys, int l, int hb,
+                                         const double2* __restrict__ Z, int64_t z0, int64_t zs, double& sx,
+                                         double& sy) {
+  const int nf = nfull_of(l), nt = nf + !(l & 1);
   const double2* __restrict__ x = xs + (size_t)hb * YS_ATOMS;
+  const double2* __restrict__ y = ys + (size_t)hb * YS_ATOMS;
   const double2* __restrict__ z = Z + z0 * zs;
-  double s0 = 0.0, s1 = 0.0;
-  for (int e = 0; e < nf; e++) {
-    const double2 a = x[(size_t)e * YS_ATOMS], c = z[e * zs];
-    s0 = fma(a.x, c.x, s0);
-    s1 = fma(a.y, c.y, s1);
+  double s0 = 0.0, s1 = 0.0, t0 = 0.0, t1 = 0.0;
+#pragma unroll 1
+  for (int e = 0; e < nt; e += ILP, x += ILP * YS_ATOMS, y += ILP * YS_ATOMS, z += ILP * zs) {
+    double2 c[ILP];
+#pragma unroll
+    for (int k = 0; k < ILP; k++)
+      if (e + k < nt) c[k] = z[k * zs];
+#pragma unroll
+    for (int k = 0; k < ILP; k++)
+      if (e + k < nt) {
+        if (e + k == nf) {
+          c[k].x *= 0.5;
+          c[k].y *= 0.5;
+        }
+        const double2 a = x[k * YS_ATOMS];
+        s0 = fma(a.x, c[k].x, s0);
+        s1 = fma(a.y, c[k].y, s1);
+        if (TWO) {
+          const double2 b = y[k * YS_ATOMS];
+          t0 = fma(b.x, c[k].x, t0);
+          t1 = fma(b.y, c[k].y, t1);
+        }
+      }
   }
-  double s = s0 + s1;
-  if (!(l & 1)) {
-    const int e = (l / 2) * (l + 1) + l / 2;
-    const double2 a = x[(size_t)e * YS_ATOMS], c = z[e * zs];
-    s += 0.5 * (a.x * c.x + a.y * c.y);
-  }
-  return s;
+  sx = s0 + s1;
+  sy = t0 + t1;
 }
 
 // Contraction of V (and, with gE != 0, Utot for B) with Z for atoms a0 .. a0+nc-1: 32 atoms
 // per tile in lanes, V (Utot) of the tile staged in shared memory as [u_half][32], the warps
 // of a block taking components b = warp, warp + GB_WARPS, ...; per species, the lane values
-// are warp sums added in tile order to the block's partial gpart[block][nsp][K].
+// are warp sums added in tile order to the block's partial gpart[block][nsp][K].  Bound by the
+// latency of the reads of Z.  With WITHB shared memory holds one block an SM, whose registers then
+// allow eight reads in flight a warp, and V and Utot share one read of their common term: 251 -> 197 us
+// at 16,000 atoms, J = 8.  Without, two blocks an SM and six reads (64 registers): a training step of
+// 512 configurations 35.81 -> 35.70 ms; three or four reads 36.1, 35.9, eight reads and one block 37.1.
 constexpr int GB_WARPS = 16;
-__global__ void __launch_bounds__(GB_WARPS * 32) k_snap_gbeta(const __grid_constant__ SnapDev S, int64_t a0,
+template <bool WITHB>
+__global__ void __launch_bounds__(GB_WARPS * 32, WITHB ? 1 : 2) k_snap_gbeta(const __grid_constant__ SnapDev S, int64_t a0,
                                                               int64_t nc, const int32_t* __restrict__ species,
                                                               const double2* __restrict__ Z,
                                                               const double2* __restrict__ V,
                                                               const double2* __restrict__ utot, double gE,
                                                               double* __restrict__ gpart) {
+  constexpr int ILP = WITHB ? 8 : 6;
   extern __shared__ __align__(16) unsigned char gsh[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int UH = S.u_half, K = S.K, nsp = S.nsp;
-  const bool withB = gE != 0.0;
   double2* vs = reinterpret_cast<double2*>(gsh);  // [UH][32]
-  double2* us = vs + (size_t)UH * YS_ATOMS;       // [UH][32] when withB
-  double* gacc = reinterpret_cast<double*>(us + (withB ? (size_t)UH * YS_ATOMS : 0));  // [nsp][K]
+  double2* us = vs + (size_t)UH * YS_ATOMS;       // [UH][32] when WITHB
+  double* gacc = reinterpret_cast<double*>(us + (WITHB ? (size_t)UH * YS_ATOMS : 0));  // [nsp][K]
   for (int q = threadIdx.x; q < nsp * K; q += blockDim.x) gacc[q] = 0.0;
   const int64_t ntile = (nc + YS_ATOMS - 1) / YS_ATOMS;
   for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x) {
@@ -1718,7 +1741,7 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_gbeta(const __grid_const
     for (int idx = threadIdx.x; idx < UH * YS_ATOMS; idx += blockDim.x) {
       const int q = idx / YS_ATOMS, l = idx - q * YS_ATOMS;
       vs[idx] = l < na ? V[(size_t)q * nc + l0 + l] : make_double2(0.0, 0.0);
-      if (withB)
+      if (WITHB)
         us[idx] = l < na ? utot[(size_t)(a0 + l0 + l) * S.idxu_max + S.u_of_h[q]] : make_double2(0.0, 0.0);
     }
     __syncthreads();
@@ -1730,18 +1753,19 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_gbeta(const __grid_const
     const double2* Zl = Z + la;
     for (int b = warp; b < K; b += GB_WARPS) {
       const DBDev d = S.db[b];
-      double tot = 0.0;
+      double tot = 0.0, B = 0.0;
 #pragma unroll
       for (int term = 0; term < 3; term++) {
         const int l = d.l[term];
-        tot += d.fac[term] * half_dot(vl, l, S.half_block[l], Zl, d.z0[term], nc);
+        double s, u;
+        if (WITHB && term == 0)
+          half_dot<true, ILP>(vl, ul, l, S.half_block[l], Zl, d.z0[0], nc, s, B);
+        else
+          half_dot<false, ILP>(vl, vl, l, S.half_block[l], Zl, d.z0[term], nc, s, u);
+        tot += d.fac[term] * s;
       }
       double val = 2.0 * tot;
-      if (withB) {
-        const int l = d.l[0];
-        const double B = 2.0 * half_dot(ul, l, S.half_block[l], Zl, d.z0[0], nc) - (S.bzero_flag ? S.bzero[l] : 0.0);
-        val += gE * B;
-      }
+      if (WITHB) val += gE * (2.0 * B - (S.bzero_flag ? S.bzero[d.l[0]] : 0.0));
       for (int sp = 0; sp < nsp; sp++) {
         const double x = warp_sum(si == sp ? val : 0.0);
         if (lane == 0) gacc[sp * K + b] += x;
@@ -1756,7 +1780,7 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_gbeta(const __grid_const
 // (compute_b.jl:17-94): B_b = 2 sum_half w Re(conj(U_j) Z(j1,j2,j)) - bzero_j, 32 atoms per
 // tile in lanes, the warps over components; Ei = beta[s_i] . B_i (the bzero shift inside B).
 // B [n][K] (optional) and Ei [n] are indexed by the global atom.
-__global__ void __launch_bounds__(GB_WARPS * 32) k_snap_bdesc(const __grid_constant__ SnapDev S, int64_t a0,
+__global__ void __launch_bounds__(GB_WARPS * 32, 2) k_snap_bdesc(const __grid_constant__ SnapDev S, int64_t a0,
                                                               int64_t nc, const int32_t* __restrict__ species,
                                                               const double2* __restrict__ Z,
                                                               const double2* __restrict__ utot, double* __restrict__ B,
@@ -1781,8 +1805,9 @@ __global__ void __launch_bounds__(GB_WARPS * 32) k_snap_bdesc(const __grid_const
     for (int b = warp; b < K; b += GB_WARPS) {
       const DBDev d = S.db[b];
       const int l = d.l[0];
-      const double v = 2.0 * half_dot(us + lane, l, S.half_block[l], Z + la, d.z0[0], nc) -
-                       (S.bzero_flag ? S.bzero[l] : 0.0);
+      double h, u;
+      half_dot<false, 4>(us + lane, us + lane, l, S.half_block[l], Z + la, d.z0[0], nc, h, u);
+      const double v = 2.0 * h - (S.bzero_flag ? S.bzero[l] : 0.0);
       bs[b * YS_ATOMS + lane] = v;
       if (B && valid) B[(size_t)(a0 + la) * K + b] = v;
     }
@@ -3792,8 +3817,9 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
     int gper = 1;
     const bool withB = gE != 0.0;
     const int gsm = (int)((withB ? 2 : 1) * (size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)nsp * K * 8);
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_gbeta, cudaFuncAttributeMaxDynamicSharedMemorySize, gsm));
-    CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gper, k_snap_gbeta, GB_WARPS * 32, gsm));
+    const auto gbeta = withB ? k_snap_gbeta<true> : k_snap_gbeta<false>;
+    CUDA_RET(ctx, cudaFuncSetAttribute(gbeta, cudaFuncAttributeMaxDynamicSharedMemorySize, gsm));
+    CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gper, gbeta, GB_WARPS * 32, gsm));
     const int64_t gmax = (int64_t)ctx->num_sms * std::max(1, gper);
     double* gpart;
     IPG_RET(scratch(ctx, "snap_gpart", (size_t)(nchunk * gmax) * nsp * K + 1, &gpart));
@@ -3806,7 +3832,7 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
                            nullptr, Z));
       IPG_RET(launch_vsum(ctx, dev, a0, nc, pl.d_off, pl.d_j, pl.d_r, d_species, d_g, V, s->pair_tangent));
       const int64_t gg = std::min(tiles, gmax);
-      IPG_TIMED_LAUNCH(ctx, "snap_gbeta", k_snap_gbeta, (unsigned)gg, GB_WARPS * 32, gsm, dev, a0, nc, d_species, Z,
+      IPG_TIMED_LAUNCH(ctx, "snap_gbeta", gbeta, (unsigned)gg, GB_WARPS * 32, gsm, dev, a0, nc, d_species, Z,
                        V, io.utot_in, gE, gpart + (size_t)rows * nsp * K);
       rows += gg;
     }
