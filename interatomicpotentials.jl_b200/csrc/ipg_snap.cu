@@ -3018,11 +3018,7 @@ int chem_adjoint(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
   }
   for (int64_t a0 = 0; a0 < n; a0 += C) {
     const int64_t nc = std::min(C, n - a0);
-    for (int p = 0; p < ne; p++)
-      for (int q = 0; q < ne; q++)
-        IPG_RET(launch_ystream(ctx, dev, s->h.yktab, YM_Z, "snap_zrows", nc, d_species + a0,
-                               utot + ((size_t)p * n + a0) * U, nullptr, nullptr, Z + (size_t)(p * ne + q) * M * nc,
-                               utot + ((size_t)q * n + a0) * U));
+    IPG_RET(launch_zpairs(ctx, dev, s->h.yktab, nc, d_species + a0, ne, utot + (size_t)a0 * U, n * U, Z, M * nc));
     if (dev.quadratic) {
       const int64_t tiles = (nc + YS_ATOMS - 1) / YS_ATOMS;
       const int64_t bg = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * std::max(1, bper));

@@ -126,11 +126,13 @@ struct SnapHost {
 int snap_build_tables(const ipg_snap_params& p, SnapHost& h);
 
 struct ipg_ctx;
-// Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu); with
-// utot2 (YM_Z) the second factor of every product comes from it.
+// Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu).
 int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n,
-                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout,
-                   const double2* utot2 = nullptr);
+                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout);
+// Z of every ordered pair (p, q) of ne elements, zstride apart: the first factor of every product from
+// element p's Utot, the second from q's (ustride apart).
+int launch_zpairs(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int64_t n, const int32_t* species, int ne,
+                  const double2* utot, int64_t ustride, double2* zout, int64_t zstride);
 // Descriptor outputs from dbl [pair][K][3], the dB/dr of every pair (ipg_snap_desc.cu): dB
 // [n][K nsp][3], or [3 n][K nsp] with rows; Wd [K nsp][6] of one configuration; the fitting rows
 // Aw [nconf][6][K nsp] and Ae [nconf][K nsp] (from B [n][K]).  Any output may be null; owner (of

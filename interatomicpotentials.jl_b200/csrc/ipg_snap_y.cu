@@ -206,15 +206,17 @@ __device__ __forceinline__ void yk_finish(const SnapDev& S, const YkItem& it, in
 // blockIdx.y, blockIdx.y + gridDim.y, ...; the items' energies then go to eitem [items][n] and
 // k_snap_yenergy adds them.  An item's result does not depend on the warp that computes it, and
 // energies are summed in item order, so neither split nor scheduling changes any bit.
-// TWO: row 2 from a second Utot (the element pairs of chem_flag; Z only).
+// TWO: row 2 from a second Utot (chem_flag; Z only), for blockIdx.z = p ne + q that of element q against
+// element p's (ustride apart; zstride between the pairs' Z).
 template <int YM, bool TWO>
 __global__ void __launch_bounds__(YK_T, 2) k_snap_ystream(const __grid_constant__ SnapDev S,
                                                           const __grid_constant__ YkTab T, int64_t n,
                                                           const int32_t* __restrict__ species,
-                                                          const double2* __restrict__ utot,
-                                                          const double2* __restrict__ utot2,
+                                                          const double2* __restrict__ utot0,
+                                                          const double2* __restrict__ utot20,
                                                           double2* __restrict__ yout, double* __restrict__ Ei,
-                                                          double2* __restrict__ zout, double* __restrict__ eitem) {
+                                                          double2* __restrict__ zout0, double* __restrict__ eitem,
+                                                          int ne, int64_t ustride, int64_t zstride) {
   extern __shared__ __align__(16) unsigned char ysh[];
   __shared__ int next_item;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -236,6 +238,9 @@ __global__ void __launch_bounds__(YK_T, 2) k_snap_ystream(const __grid_constant_
     guard0[q] = guard1[q] = make_double2(0.0, 0.0);
     if (TWO) us2[UH * YS_ATOMS + q] = make_double2(0.0, 0.0);
   }
+  const double2* __restrict__ utot = TWO ? utot0 + (blockIdx.z / ne) * ustride : utot0;
+  const double2* __restrict__ utot2 = TWO ? utot20 + (blockIdx.z % ne) * ustride : utot0;
+  double2* __restrict__ zout = TWO ? zout0 + blockIdx.z * zstride : zout0;
   const bool split = gridDim.y > 1;
   for (int64_t a0 = (int64_t)blockIdx.x * YS_ATOMS; a0 < n; a0 += (int64_t)gridDim.x * YS_ATOMS) {
     const int na_blk = (int)((n - a0) < YS_ATOMS ? (n - a0) : YS_ATOMS);
@@ -364,22 +369,27 @@ __global__ void k_snap_yenergy(const __grid_constant__ SnapDev S, int nitem, int
 
 template <int YM, bool TWO = false>
 int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const char* tname, int64_t n,
-                     const int32_t* species, const double2* utot, const double2* utot2, double2* yout, double* Ei, double2* zout) {
+                     const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout,
+                     const double2* utot2 = nullptr, int ne = 1, int64_t ustride = 0, int64_t zstride = 0) {
   const auto kernel = k_snap_ystream<YM, TWO>;
   const int smem = yk_smem(dev.nsp, dev.n_ytrip, dev.u_half, tab.nitem, TWO).total();
   CUDA_RET(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int per_sm = 1;
   CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, YK_T, smem));
   const int64_t resident = (int64_t)ctx->num_sms * std::max(1, per_sm);
-  const int64_t tiles = (n + YS_ATOMS - 1) / YS_ATOMS;
+  const int64_t tiles = (n + YS_ATOMS - 1) / YS_ATOMS, pairs = TWO ? (int64_t)ne * ne : 1;
   // Fewer tiles than resident blocks: the items of a tile go to several blocks, at most one
   // block per YK_WARPS items (249 atoms, twojmax 8: 167 us with one block per tile, 74 us split).
+  // The tiles of a last, partly filled wave stay whole: split so that the wave ends earlier they
+  // took longer (each block stages its tile's Utot again): 3,160 against 3,060 us a pullback of 16,000
+  // atoms, 2,544 against 2,520 at 54,000.
   const int64_t most = (tab.nitem + YK_WARPS - 1) / YK_WARPS;
-  const int64_t nsplit = std::max<int64_t>(1, std::min(most, resident / std::max<int64_t>(1, tiles)));
-  const dim3 grid((unsigned)std::min(tiles, resident), (unsigned)nsplit);
+  const int64_t nsplit = std::max<int64_t>(1, std::min(most, resident / std::max<int64_t>(1, tiles * pairs)));
+  const dim3 grid((unsigned)std::min(tiles, resident), (unsigned)nsplit, (unsigned)pairs);
   double* eitem = nullptr;
   if (YM != YM_Z && nsplit > 1) IPG_RET(scratch(ctx, "snap_yitem", (size_t)tab.nitem * n, &eitem));
-  IPG_TIMED_LAUNCH(ctx, tname, kernel, grid, YK_T, smem, dev, tab, n, species, utot, utot2, yout, Ei, zout, eitem);
+  IPG_TIMED_LAUNCH(ctx, tname, kernel, grid, YK_T, smem, dev, tab, n, species, utot, utot2, yout, Ei, zout, eitem, ne,
+                   ustride, zstride);
   if (eitem) IPG_LAUNCH(ctx, k_snap_yenergy, (unsigned)((n + 127) / 128), 128, 0, dev, tab.nitem, n, species, eitem, Ei);
   return IPG_OK;
 }
@@ -387,14 +397,28 @@ int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const c
 }  // namespace
 
 int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n,
-                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout,
-                   const double2* utot2) {
+                   const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout) {
   if (n <= 0) return IPG_OK;
-  if (utot2 && utot2 != utot) {
-    if (ym != YM_Z) return IPG_ERR_ARG;
-    return launch_ystream_m<YM_Z, true>(ctx, dev, tab, tname, n, species, utot, utot2, yout, Ei, zout);
-  }
-  if (ym == YM_Z) return launch_ystream_m<YM_Z>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
-  if (ym == YM_YZ) return launch_ystream_m<YM_YZ>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
-  return launch_ystream_m<YM_Y>(ctx, dev, tab, tname, n, species, utot, utot, yout, Ei, zout);
+  if (ym == YM_Z) return launch_ystream_m<YM_Z>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
+  if (ym == YM_YZ) return launch_ystream_m<YM_YZ>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
+  return launch_ystream_m<YM_Y>(ctx, dev, tab, tname, n, species, utot, yout, Ei, zout);
+}
+
+int launch_zpairs(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int64_t n, const int32_t* species, int ne,
+                  const double2* utot, int64_t ustride, double2* zout, int64_t zstride) {
+  if (n <= 0) return IPG_OK;
+  constexpr const char* tname = "snap_zrows";
+  // Few tiles: every pair in one launch, (p, p) from two copies of the same plane (1,999 atoms, two
+  // elements, twojmax 6: 488 -> 392 us a call).  Otherwise one plane for (p, p), which leaves room for more blocks.
+  if (ne > 1 && (n + YS_ATOMS - 1) / YS_ATOMS <= ctx->num_sms)
+    return launch_ystream_m<YM_Z, true>(ctx, dev, tab, tname, n, species, utot, nullptr, nullptr, zout, utot, ne, ustride,
+                                        zstride);
+  for (int p = 0; p < ne; p++)
+    for (int q = 0; q < ne; q++) {
+      const double2 *u = utot + p * ustride, *u2 = utot + q * ustride;
+      double2* z = zout + (p * ne + q) * zstride;
+      IPG_RET(p == q ? (launch_ystream_m<YM_Z>(ctx, dev, tab, tname, n, species, u, nullptr, nullptr, z))
+                     : (launch_ystream_m<YM_Z, true>(ctx, dev, tab, tname, n, species, u, nullptr, nullptr, z, u2)));
+    }
+  return IPG_OK;
 }
