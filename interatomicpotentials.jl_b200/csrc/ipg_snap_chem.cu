@@ -10,7 +10,7 @@
 // each atom's effective linear coefficients beta_k + sum_l a_kl B_l.
 //
 // Forces then cost one pass of the pair kernel on U instead of nelem^2 contractions of every
-// pair's dU with the owner's Z.  1,999 atoms, two species, twojmax 6: 3251 -> 511 us per call.
+// pair's dU with the owner's Z.  1,999 atoms, two species, twojmax 6: 3251 -> 364 us per call.
 #include <algorithm>
 
 #include "ipg_snap.cuh"
@@ -80,20 +80,24 @@ __global__ void __launch_bounds__(QC_WARPS * 32) k_quad_coef(const __grid_consta
   }
 }
 
-// Y' of one row (level j, row mb) of 32 atoms per warp, every element at once: per element pair
-// and triple of the level, a tile of CY_MA elements of Z against nelem coefficients.  Bound by the
-// reads of Z (each element once).  The rows' energies go to epart [rows][nc].
+// Y' of one tile (level j, row mb, CY_MA elements) of 32 atoms per warp, every element at once: per
+// element pair and triple of the level, the tile's Z against nelem coefficients.  Bound by the latency
+// of the reads of Z (each element once): with a warp a row 88 us at 1,999 atoms, two elements, twojmax 6,
+// with a warp a tile 52.
+// The tiles' energies go to epart [tiles][nc].
 constexpr int CY_MA = 3, CY_WARPS = 4;
+__host__ __device__ inline int cy_tiles(int j) { return (j + CY_MA) / CY_MA; }  // of a row of level j
 template <int NE>
 __global__ void __launch_bounds__(CY_WARPS * 32) k_chem_y(const __grid_constant__ SnapDev S, int64_t n, int64_t a0,
                                                           int64_t nc, const double* __restrict__ coef,
                                                           const double2* __restrict__ Z,
                                                           const double2* __restrict__ utot, double2* __restrict__ yout,
-                                                          double* __restrict__ epart, int nrow, int e0) {
+                                                          double* __restrict__ epart, int ntile, int e0) {
   const int lane = threadIdx.x & 31, r = blockIdx.y * CY_WARPS + (threadIdx.x >> 5);
-  if (r >= nrow) return;
-  int j = 0, mb = r;  // rows in order: level 0, level 1, ...
-  while (mb > j / 2) mb -= j / 2 + 1, j++;
+  if (r >= ntile) return;
+  int j = S.J, x0 = r;  // the largest level first: its tiles take the longest
+  while (x0 >= (j / 2 + 1) * cy_tiles(j)) x0 -= (j / 2 + 1) * cy_tiles(j), j--;
+  const int mb = x0 / cy_tiles(j), m0 = x0 % cy_tiles(j) * CY_MA;
   const int64_t l = (int64_t)blockIdx.x * 32 + lane;
   const bool valid = l < nc;
   const int64_t la = valid ? l : nc - 1;
@@ -103,14 +107,14 @@ __global__ void __launch_bounds__(CY_WARPS * 32) k_chem_y(const __grid_constant_
   const int32_t* trips = lev + S.J + 2;
   const int nma = 2 * mb == j ? mb + 1 : j + 1, h0 = S.half_block[j] + mb * (j + 1);
   double en = 0.0;
-  for (int m0 = 0; m0 < nma; m0 += CY_MA) {
+  if (m0 < nma) {  // the row of a level's middle ends there
     double2 acc[NE][CY_MA];
 #pragma unroll
     for (int e = 0; e < NE; e++)
 #pragma unroll
       for (int m = 0; m < CY_MA; m++) acc[e][m] = make_double2(0.0, 0.0);
     for (int pq = 0; pq < ne * ne; pq++)
-#pragma unroll 2
+#pragma unroll 4
       for (int x = t0; x < t1; x++) {
         const int t = trips[x];
         const double2* z = Z + ((size_t)pq * M + S.ytrip_jjz[t] + mb * (j + 1) + m0) * nc + la;
@@ -147,15 +151,15 @@ __global__ void __launch_bounds__(CY_WARPS * 32) k_chem_y(const __grid_constant_
   if (epart && valid) epart[(size_t)r * nc + l] = (e0 ? epart[(size_t)r * nc + l] : 0.0) + en;
 }
 
-// E_i = (2/3) sum of the rows' energies, shifted by beta of the triples that carry bzero.
-__global__ void k_chem_energy(const __grid_constant__ SnapDev S, int64_t a0, int64_t nc, int nrow,
+// E_i = (2/3) sum of the tiles' energies, shifted by beta of the triples that carry bzero.
+__global__ void k_chem_energy(const __grid_constant__ SnapDev S, int64_t a0, int64_t nc, int ntile,
                               const int32_t* __restrict__ species, const double* __restrict__ epart,
                               double* __restrict__ Ei) {
   const int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= nc) return;
   double t = 0.0;
 #pragma unroll 5
-  for (int r = 0; r < nrow; r++) t += epart[(size_t)r * nc + l];
+  for (int r = 0; r < ntile; r++) t += epart[(size_t)r * nc + l];
   t *= 2.0 / 3.0;
   if (S.bzero_flag) {
     const int ne = S.nelem, KB = S.klin / (ne * ne * ne), si = sp_of(species, a0 + l, S.nsp);
@@ -189,24 +193,24 @@ int launch_quad_coef(ipg_ctx* ctx, const SnapDev& S, int64_t a0, int64_t nc, con
 int launch_chem_y(ipg_ctx* ctx, const SnapDev& S, int64_t n, int64_t a0, int64_t nc, const int32_t* species,
                   const double* coef, const double2* Z, const double2* utot, double2* yout, double* Ei) {
   if (nc <= 0) return IPG_OK;
-  int nrow = 0;
-  for (int j = 0; j <= S.J; j++) nrow += j / 2 + 1;
+  int ntile = 0;
+  for (int j = 0; j <= S.J; j++) ntile += (j / 2 + 1) * cy_tiles(j);
   double* epart = nullptr;
-  if (Ei) IPG_RET(scratch(ctx, "chem_epart", (size_t)nrow * nc, &epart));
-  const dim3 grid((unsigned)((nc + 31) / 32), (unsigned)((nrow + CY_WARPS - 1) / CY_WARPS));
+  if (Ei) IPG_RET(scratch(ctx, "chem_epart", (size_t)ntile * nc, &epart));
+  const dim3 grid((unsigned)((nc + 31) / 32), (unsigned)((ntile + CY_WARPS - 1) / CY_WARPS));
   for (int e0 = 0; e0 < S.nelem; e0 += 3) {  // three elements per pass over Z
     const int k = std::min(3, S.nelem - e0);
     if (k == 1)
       IPG_TIMED_LAUNCH(ctx, "snap_atom", k_chem_y<1>, grid, CY_WARPS * 32, 0, S, n, a0, nc, coef, Z, utot, yout,
-                       epart, nrow, e0);
+                       epart, ntile, e0);
     else if (k == 2)
       IPG_TIMED_LAUNCH(ctx, "snap_atom", k_chem_y<2>, grid, CY_WARPS * 32, 0, S, n, a0, nc, coef, Z, utot, yout,
-                       epart, nrow, e0);
+                       epart, ntile, e0);
     else
       IPG_TIMED_LAUNCH(ctx, "snap_atom", k_chem_y<3>, grid, CY_WARPS * 32, 0, S, n, a0, nc, coef, Z, utot, yout,
-                       epart, nrow, e0);
+                       epart, ntile, e0);
   }
   if (Ei)
-    IPG_LAUNCH(ctx, k_chem_energy, (unsigned)((nc + 127) / 128), 128, 0, S, a0, nc, nrow, species, epart, Ei);
+    IPG_LAUNCH(ctx, k_chem_energy, (unsigned)((nc + 127) / 128), 128, 0, S, a0, nc, ntile, species, epart, Ei);
   return IPG_OK;
 }
