@@ -250,12 +250,11 @@ struct PairList {
   int64_t* d_off = nullptr;  // [n+1]
   int32_t* d_j = nullptr;    // [npairs]
   double* d_r = nullptr;     // [npairs][3]
-  int64_t* d_in_off = nullptr;  // [n+1]   transpose: pairs whose neighbor is atom k
-  int64_t* d_in_pair = nullptr; // [npairs]
+  int64_t* d_rev = nullptr;  // [npairs]   transpose: the reverse of each pair (-1: none)
 };
 
 // mode: IPG_NLIST_HALF (cut[0] = rcut) or IPG_NLIST_FULL (cut = nsp*nsp cutsq), with
-// IPG_NLIST_LITERAL_SQRT optionally or-ed in.  want_transpose builds d_in_off/d_in_pair.
+// IPG_NLIST_LITERAL_SQRT optionally or-ed in.  want_transpose builds d_rev.
 // sorted: each atom's neighbors ascending (the reference's order); otherwise the
 // emission order (stencil cells in fixed order, ascending inside a cell), which is
 // equally deterministic.

@@ -396,9 +396,12 @@ __global__ void k_max_disp2(int64_t n, const ConfGrid* __restrict__ grid, const 
 // Capacity mode: a total above cap is an error (status), and every offset is cut at cap
 // so that all later kernels stay inside the buffers.
 // (Offsets are non-decreasing, so cutting each one at cap on its own is the same as
-// cutting the lists; no thread reads another's offset.)
-__global__ void k_clamp_offsets(int64_t n, int64_t* __restrict__ off, int64_t cap, int* __restrict__ status) {
+// cutting the lists; no thread reads another's offset.)  So is, in the padded walk (kcap > 0), an
+// atom with more hits than slots.
+__global__ void k_clamp_offsets(int64_t n, int64_t* __restrict__ off, int64_t cap, const int* __restrict__ maxcnt,
+                                int kcap, int* __restrict__ status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && kcap > 0 && *maxcnt > kcap) atomicExch(status, IPG_ERR_CAPACITY);
   if (i > n) return;
   if (off[i] > cap) {
     if (i == n) atomicExch(status, IPG_ERR_CAPACITY);
@@ -711,11 +714,6 @@ __global__ void __launch_bounds__(WALKC_WARPS * 32) k_pair_walk_cells(
   }
 }
 
-// Capacity mode of the padded walk: an atom with more hits than slots is a capacity error.
-__global__ void k_kcap_check(const int* __restrict__ maxcnt, int kcap, int* __restrict__ status) {
-  if (threadIdx.x == 0 && *maxcnt > kcap) atomicExch(status, IPG_ERR_CAPACITY);
-}
-
 // Padded emission (k_pair_walk_cells<2>) to the CSR list: slot t of atom i goes to off[i] + t.
 __global__ void k_pad_compact(int64_t n, int kcap, const int64_t* __restrict__ off, const int32_t* __restrict__ pj,
                               const double* __restrict__ pr, int32_t* __restrict__ j, double* __restrict__ r) {
@@ -754,22 +752,17 @@ __global__ void k_pair_sort(int64_t n, const int64_t* __restrict__ off, int32_t*
   }
 }
 
-// Transpose: for every atom k, the pairs p whose neighbor is k, in ascending p.  The lists it
-// serves (the full SNAP lists) are symmetric with one image per pair, so the pairs whose
-// neighbor is k are those owned by k's own neighbors i, and ascending p is ascending i: pair
-// (i -> k) takes slot #{q owned by k : j[q] < i} of k's in-list.  No atomics, no sort.  (A
-// list cut at a capacity is not symmetric; its slots stay in bounds and the capacity error
-// discards the result.)
-__global__ void k_in_count(const int64_t* __restrict__ d_np, const int32_t* __restrict__ j,
-                           int64_t* __restrict__ cnt) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= *d_np) return;
-  atomicAdd((unsigned long long*)&cnt[j[p]], 1ull);
-}
-// One warp per owner i, one lane per pair (i -> k) (32 at a time); each lane counts the
-// neighbors of k below i on its own, so the lanes' loads overlap.
-__global__ void k_in_rank(int64_t n, const int64_t* __restrict__ off, const int32_t* __restrict__ j,
-                          const int64_t* __restrict__ in_off, int64_t* __restrict__ in_pair) {
+// Transpose: rev[p] of pair p = (i -> k) is the pair (k -> i).  The lists it serves (the full SNAP
+// lists) are symmetric with one image per pair, so the pairs whose neighbor is i are the reverses of
+// those that i owns.  (No reverse, -1: a list cut at a capacity, whose result the capacity error
+// discards, or a pair at the cutoff to the last bit, which the rounding of the two minimum images can
+// put on one list only.)
+//
+// One warp per owner i, one lane per pair (32 at a time); each lane looks through the neighbors of k
+// on its own, so the lanes' loads overlap: 48 us at 54,000 atoms, 6 at 249.  Lists of their own for the
+// pairs that end at each atom took counts, their scan and a clear besides, 10 us at 249 atoms.
+__global__ void k_rev_pair(int64_t n, const int64_t* __restrict__ off, const int32_t* __restrict__ j,
+                           int64_t* __restrict__ rev) {
   const int lane = threadIdx.x & 31;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;  // warp-uniform
@@ -777,11 +770,11 @@ __global__ void k_in_rank(int64_t n, const int64_t* __restrict__ off, const int3
   for (int64_t p = off[i] + lane; p < p1; p += 32) {
     const int32_t k = j[p];
     const int64_t q0 = off[k], q1 = off[k + 1];
-    int64_t rank = 0;
+    int64_t r = -1;
 #pragma unroll 4
-    for (int64_t q = q0; q < q1; q++) rank += j[q] < i;
-    const int64_t slot = in_off[k] + rank;
-    if (slot < in_off[k + 1]) in_pair[slot] = p;
+    for (int64_t q = q0; q < q1; q++)
+      if (j[q] == i) r = q;
+    rev[p] = r;
   }
 }
 
@@ -889,15 +882,9 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
 }
 
 namespace {
-// The in-lists of a symmetric list (k_in_rank): in_off by counting, in_pair by rank.
 int build_transpose(ipg_ctx* ctx, const std::string& pre, int64_t n, PairList& pl) {
-  IPG_RET(scratch(ctx, (pre + "in_off").c_str(), n + 1, &pl.d_in_off));
-  IPG_RET(scratch(ctx, (pre + "in_pair").c_str(), pl.npairs + 1, &pl.d_in_pair));
-  CUDA_RET(ctx, cudaMemsetAsync(pl.d_in_off, 0, sizeof(int64_t) * (n + 1), ctx->stream));
-  if (pl.npairs > 0) IPG_LAUNCH(ctx, k_in_count, nblk(pl.npairs, 256), 256, 0, pl.d_np, pl.d_j, pl.d_in_off);
-  IPG_RET(ipg_scan_i64(ctx, pl.d_in_off, pl.d_in_off, n + 1));
-  if (pl.npairs > 0)
-    IPG_LAUNCH(ctx, k_in_rank, nblk(32 * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_in_off, pl.d_in_pair);
+  IPG_RET(scratch(ctx, (pre + "rev").c_str(), pl.npairs + 1, &pl.d_rev));
+  if (pl.npairs > 0) IPG_LAUNCH(ctx, k_rev_pair, nblk(32 * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev);
   return IPG_OK;
 }
 }  // namespace
@@ -970,8 +957,8 @@ int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const 
   int hmax = 0;
   if (cap > 0) {  // capacity mode: no read-back
     pl.npairs = cap;
-    IPG_LAUNCH(ctx, k_clamp_offsets, nblk(n + 1, 256), 256, 0, n, pl.d_off, cap, ctx->d_status);
-    if (kcap > 0 && n > 0) IPG_LAUNCH(ctx, k_kcap_check, 1, 32, 0, maxcnt, kcap, ctx->d_status);
+    IPG_LAUNCH(ctx, k_clamp_offsets, nblk(n + 1, 256), 256, 0, n, pl.d_off, cap, maxcnt, n > 0 ? kcap : 0,
+               ctx->d_status);
   } else {
     CUDA_RET(ctx, cudaMemcpyAsync(&pl.npairs, pl.d_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_RET(ctx, cudaMemcpyAsync(&hmax, maxcnt, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

@@ -2401,22 +2401,22 @@ __global__ void k_snap_contract(int64_t n, const int64_t* __restrict__ off, cons
   }
 }
 
-// F_k = sum_{p in out(k)} f_p - sum_{q in in(k)} f_q; per-atom virial contribution
-// w6[k] = sum_{p in out(k)} f_p (x) (x_k - x_j(p)) with absolute positions
+// F_k = sum over k's pairs p of f_p - f_rev(p), rev(p) the reverse pair; per-atom virial contribution
+// w6[k] = sum over p of f_p (x) (x_k - x_j(p)) with absolute positions
 // (snap.jl:292-306 contracted with beta): [xx, yy, zz, yz, xz, xy] as in the reference.
 //
-// Bound by the latency of dependent loads (in_pair -> fvec, nbr -> pos), so an atom's pairs are
-// spread over GATHER_LANES lanes (lane t takes pairs t, t + GATHER_LANES, ... of each list) and
-// the lanes are summed by a fixed tree.  Eight lanes: about 25 pairs per list leave three or
-// four loads per lane in flight, and four atoms still share a warp, so full systems stay
-// coalesced.  One thread per atom walked both lists serially: 42 us at 249 and 8,192 atoms, 55 us at
-// 54,000 (twojmax 8); now 13, 12 and 47 us.
+// Bound by the latency of dependent loads (rev -> fvec, nbr -> pos), so an atom's pairs are
+// spread over GATHER_LANES lanes (lane t takes pairs t, t + GATHER_LANES, ...) and the lanes are
+// summed by a fixed tree.  Eight lanes: about 25 pairs leave three or four loads of each kind per
+// lane in flight, and four atoms still share a warp, so full systems stay coalesced.  ONE: one
+// share per pair, whose loads then overlap.  One thread per atom over separate lists took 42 us at
+// 249 and 55 at 54,000 atoms (twojmax 8), eight lanes 13 and 47, eight lanes over the reverses 8 and 32.
 constexpr int GATHER_LANES = 8;
+template <bool ONE>
 __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* __restrict__ off,
                                                      const int32_t* __restrict__ nbr,
-                                                     const int64_t* __restrict__ in_off,
-                                                     const int64_t* __restrict__ in_pair,
-                                                     const double* __restrict__ fvec, int nch,
+                                                     const int64_t* __restrict__ rev,
+                                                     const double* __restrict__ fvec, int nchains,
                                                      const double* __restrict__ pos, double* __restrict__ F,
                                                      double* __restrict__ w6) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2424,23 +2424,30 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
   const int64_t k0 = t / GATHER_LANES;
   const bool valid = k0 < n;
   const int64_t k = valid ? k0 : 0;  // idle groups of the last warp stay for the shuffles
+  const int nch = ONE ? 1 : nchains;
   double f[3] = {0, 0, 0};
   double w[6] = {0, 0, 0, 0, 0, 0};
   const double xk = pos[3 * k], yk = pos[3 * k + 1], zk = pos[3 * k + 2];
-  const int64_t p1 = valid ? off[k + 1] : 0, q1 = valid ? in_off[k + 1] : 0;
+  const int64_t p1 = valid ? off[k + 1] : 0;
 #pragma unroll 4
   for (int64_t p = valid ? off[k] + g : 0; p < p1; p += GATHER_LANES) {
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int q = 0; q < nch; q++) {  // the chains' shares of this pair, in fixed order
-      const double* fv = fvec + ((size_t)p * nch + q) * 3;
+    const int64_t jn = nbr[p], q = rev[p];
+    double a = 0.0, b = 0.0, c = 0.0, ra = 0.0, rb = 0.0, rc = 0.0;
+    for (int r = 0; r < nch; r++) {  // the chains' shares of this pair, in fixed order
+      const double* fv = fvec + ((size_t)p * nch + r) * 3;
       a += fv[0];
       b += fv[1];
       c += fv[2];
+      if (q >= 0) {
+        const double* fr = fvec + ((size_t)q * nch + r) * 3;
+        ra += fr[0];
+        rb += fr[1];
+        rc += fr[2];
+      }
     }
-    f[0] += a;
-    f[1] += b;
-    f[2] += c;
-    const int64_t jn = nbr[p];
+    f[0] += a - ra;
+    f[1] += b - rb;
+    f[2] += c - rc;
     const double dx = xk - pos[3 * jn], dy = yk - pos[3 * jn + 1], dz = zk - pos[3 * jn + 2];
     w[0] += a * dx;
     w[1] += b * dy;
@@ -2448,20 +2455,6 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
     w[3] += b * dz;
     w[4] += a * dz;
     w[5] += a * dy;
-  }
-#pragma unroll 4
-  for (int64_t q = valid ? in_off[k] + g : 0; q < q1; q += GATHER_LANES) {
-    const int64_t p = in_pair[q];
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (int r = 0; r < nch; r++) {
-      const double* fv = fvec + ((size_t)p * nch + r) * 3;
-      a += fv[0];
-      b += fv[1];
-      c += fv[2];
-    }
-    f[0] -= a;
-    f[1] -= b;
-    f[2] -= c;
   }
 #pragma unroll
   for (int o = GATHER_LANES / 2; o > 0; o >>= 1) {
@@ -2486,6 +2479,7 @@ __global__ void k_chunk_reduce(const int64_t* __restrict__ chunks, const double*
   __shared__ double sm[7][128];
   const int64_t a0 = chunks[3 * blockIdx.x + 1], a1 = chunks[3 * blockIdx.x + 2];
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
   for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
     acc[0] += Ei ? Ei[i] : 0.0;
     if (w6)
@@ -3188,8 +3182,8 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
   if (out.W6) IPG_RET(scratch(ctx, "snap_w6", 6 * (size_t)n + 6, &w6));
   IPG_RET(ipg_side_join(ctx));  // the list transpose (side stream) is read from here on
   if ((out.F || out.W6) && fvec && n)
-    IPG_TIMED_LAUNCH(ctx, "snap_gather", k_snap_gather, nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_in_off,
-                     pl.d_in_pair, fvec, nch, d_pos, out.F, w6);
+    IPG_TIMED_LAUNCH(ctx, "snap_gather", (nch == 1 ? k_snap_gather<true> : k_snap_gather<false>),
+                     nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, fvec, nch, d_pos, out.F, w6);
   if (out.E || out.W6) {
     // chunk table: [config, first atom, end] per chunk, then each config's chunk range
     std::vector<int64_t>& ch = s->chunk_tab;
@@ -3226,7 +3220,7 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
       IPG_RET(scratch(ctx, "snap_owner", (size_t)np + 1, &owner));
       IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
     }
-    IPG_RET(launch_descriptors(ctx, K, nsp, nconf, h_atom_off, pl, owner, d_species, d_pos, dbl, out.B, out.dB,
+    IPG_RET(launch_descriptors(ctx, K, nsp, nconf, h_atom_off, pl, d_species, d_pos, dbl, out.B, out.dB,
                                out.dB_rows, out.Wd, out.Aw, out.Ae));
   }
   if (out.pl_out) *out.pl_out = pl;
@@ -3998,8 +3992,8 @@ int ipg_snap_vjp(ipg_snap* s, int64_t n, const double* pos, const int32_t* speci
       const int64_t grid = std::min<int64_t>(n, (int64_t)ctx->num_sms * std::max(1, per_sm));
       IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_snap_hvp, (unsigned)grid, nw * 32, HL.total, dev, io, d_v, fd);
     }
-    IPG_LAUNCH(ctx, k_snap_gather, nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_in_off, pl.d_in_pair, fd, 1,
-               d_pos, Fd, (double*)nullptr);
+    IPG_LAUNCH(ctx, k_snap_gather<true>, nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, fd, 1, d_pos,
+               Fd, (double*)nullptr);
   }
   IPG_LAUNCH(ctx, k_vjp_pos, nblk((int64_t)m, 256), 256, 0, (int64_t)m, F0, gE, Fd, gp);
   if (fused)

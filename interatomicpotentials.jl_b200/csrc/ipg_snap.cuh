@@ -135,11 +135,11 @@ int launch_zpairs(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int64_t n,
                   const double2* utot, int64_t ustride, double2* zout, int64_t zstride);
 // Descriptor outputs from dbl [pair][K][3], the dB/dr of every pair (ipg_snap_desc.cu): dB
 // [n][K nsp][3], or [3 n][K nsp] with rows; Wd [K nsp][6] of one configuration; the fitting rows
-// Aw [nconf][6][K nsp] and Ae [nconf][K nsp] (from B [n][K]).  Any output may be null; owner (of
-// each pair) and the list transpose are read for dB only.
+// Aw [nconf][6][K nsp] and Ae [nconf][K nsp] (from B [n][K]).  Any output may be null; the list
+// transpose is read for dB only.
 int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h_off, const PairList& pl,
-                       const int32_t* owner, const int32_t* species, const double* pos, const double* dbl,
-                       const double* B, double* dB, bool rows, double* Wd, double* Aw, double* Ae);
+                       const int32_t* species, const double* pos, const double* dbl, const double* B,
+                       double* dB, bool rows, double* Wd, double* Aw, double* Ae);
 // dB/dr of the pairs of owners b0 .. b1-1 (dbl [pair][K][3]) from their Z (atoms a0.., stride zs),
 // and, with fvec, its contraction with the owner's beta (ipg_snap_db.cu).
 int launch_db(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const PairList& pl, const int32_t* species,

@@ -13,7 +13,7 @@ constexpr int DG_V = 7;       // partial sums per (species, component): W (6) an
 
 // One block takes a chunk of atoms of one configuration (blockIdx.x) and DG_T columns
 // t = 3 b + c (blockIdx.y) of dB/dr, dbl [pair][K][3]:
-//   dB_k[block s][b][c] = sum over out(k), s_k = s, of dbl_p - sum over in(k), s_owner = s, of
+//   dB_k[block s][b][c] = sum over k's pairs, s_k = s, of dbl_p - sum over their reverses, s_owner = s, of
 //     dbl_q (snap.jl:289-290), if dB is wanted;
 //   W of the chunk: dB_i/dr_ij (x) (x_i - x_j), absolute positions (snap.jl:292-306), and the sums
 //     of B, both per species, into part [chunk][nsp][K][7] (dbl null: the sums of B alone).
@@ -27,9 +27,7 @@ template <int NSP>
 __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict__ chunks, int K, int nsp,
                                                       const int64_t* __restrict__ off,
                                                       const int32_t* __restrict__ nbr,
-                                                      const int64_t* __restrict__ in_off,
-                                                      const int64_t* __restrict__ in_pair,
-                                                      const int32_t* __restrict__ owner,
+                                                      const int64_t* __restrict__ rev,
                                                       const int32_t* __restrict__ species,
                                                       const double* __restrict__ pos, const double* __restrict__ dbl,
                                                       const double* __restrict__ B, double* __restrict__ dB, int rows,
@@ -89,20 +87,19 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
         w[s][3] += bi;
       }
     if (!dB) continue;
-    for (int64_t q0 = in_off[i], q1 = in_off[i + 1]; q0 < q1; q0 += DG_PAIRS) {
+    for (int64_t q0 = off[i], q1 = off[i + 1]; q0 < q1; q0 += DG_PAIRS) {
       const int m = (int)(q1 - q0 < DG_PAIRS ? q1 - q0 : DG_PAIRS);
       __syncthreads();
       for (int t = threadIdx.x; t < m; t += DG_T) {
-        const int64_t p = in_pair[q0 + t];
-        const int so = species[owner[p]];
-        sp[t] = p;
+        const int so = species[nbr[q0 + t]];  // the reverse pair's owner
+        sp[t] = rev[q0 + t];
         ss[t] = so < 0 ? 0 : (so >= nsp ? nsp - 1 : so);
       }
       __syncthreads();
       if (act) {
 #pragma unroll 8
         for (int t = 0; t < m; t++) {
-          const double v = dbl[(size_t)sp[t] * C + col];
+          const double v = sp[t] >= 0 ? dbl[(size_t)sp[t] * C + col] : 0.0;
 #pragma unroll
           for (int s = 0; s < NSP; s++) acc[s] -= NSP == 1 || ss[t] == s ? v : 0.0;
         }
@@ -164,17 +161,17 @@ __global__ void __launch_bounds__(256) k_desc_reduce(const int64_t* __restrict__
 
 template <int NSP>
 int launch_gather(ipg_ctx* ctx, dim3 grid, const int64_t* chunks, int K, int nsp, const PairList& pl,
-                  const int32_t* owner, const int32_t* species, const double* pos, const double* dbl, const double* B,
+                  const int32_t* species, const double* pos, const double* dbl, const double* B,
                   double* dB, bool rows, double* part, bool want_w) {
-  IPG_LAUNCH(ctx, k_desc_gather<NSP>, grid, DG_T, 0, chunks, K, nsp, pl.d_off, pl.d_j, pl.d_in_off, pl.d_in_pair,
-             owner, species, pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
+  IPG_LAUNCH(ctx, k_desc_gather<NSP>, grid, DG_T, 0, chunks, K, nsp, pl.d_off, pl.d_j, pl.d_rev, species,
+              pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
   return IPG_OK;
 }
 
 }  // namespace
 
 int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h_off, const PairList& pl,
-                       const int32_t* owner, const int32_t* species, const double* pos, const double* dbl,
+                       const int32_t* species, const double* pos, const double* dbl,
                        const double* B, double* dB, bool rows, double* Wd, double* Aw, double* Ae) {
   const int64_t n = h_off[nconf];
   const bool sums = Wd || Aw || Ae;
@@ -207,13 +204,13 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
   const double* Bs = Ae ? B : nullptr;
   const bool want_w = Wd || Aw;
   if (nsp == 1)
-    IPG_RET(launch_gather<1>(ctx, grid, d_tab, K, nsp, pl, owner, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<1>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else if (nsp == 2)
-    IPG_RET(launch_gather<2>(ctx, grid, d_tab, K, nsp, pl, owner, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<2>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else if (nsp <= 4)
-    IPG_RET(launch_gather<4>(ctx, grid, d_tab, K, nsp, pl, owner, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<4>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else
-    IPG_RET(launch_gather<8>(ctx, grid, d_tab, K, nsp, pl, owner, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<8>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   if (sums)
     IPG_LAUNCH(ctx, k_desc_reduce, dim3((unsigned)((width + 31) / 32), (unsigned)nconf), 256, 0,
                d_tab + tab.size(), KN, part, Wd, Aw, Ae);

@@ -360,7 +360,7 @@ __global__ void k_snap_yenergy(const __grid_constant__ SnapDev S, int nitem, int
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double t = 0.0;
-#pragma unroll 8
+#pragma unroll 32
   for (int r = 0; r < nitem; r++) t += eitem[(size_t)r * n + i];
   int si = species[i];
   si = si < 0 ? 0 : (si >= S.nsp ? S.nsp - 1 : si);
