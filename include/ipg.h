@@ -80,7 +80,7 @@ IPG_API int ipg_launch_count(const ipg_ctx* ctx, int64_t* out);
  * "snap_pair" (per-neighbor adjoint forces), "snap_gather" (force gather), "snap_zrows" (Z),
  * "snap_bdesc" (B), "snap_dbfused" (plain dB/dr), "snap_contract" (plain-path contraction),
  * "snap_vsum" and "snap_gbeta" (beta pullback; "snap_vsum" also carries the Utot tangent of
- * the position pullback), "snap_hvp_y" (its two polarized Y evaluations), "snap_hvp" (the
+ * the position pullback), "snap_hvp_y" (its tangent of Y), "snap_hvp" (the
  * rest of the exact Hessian-vector product: the pair part, or the per-atom forward-mode
  * kernel).  Unknown names read as zero. */
 IPG_API int ipg_timing_enable(ipg_ctx* ctx, int on);
@@ -267,9 +267,9 @@ IPG_API int ipg_snap_vjp_beta(ipg_snap* snap, int64_t n, const double* pos, cons
  *   gpos [3n] = d(gE E + gF . F)/dpos = -gE F - H gF    (H: Hessian of E).
  * Both terms are exact: F from one adjoint evaluation, H gF as the directional derivative of
  * the adjoint force computation along gF (the second-order extension of compute_dij.jl:5-74):
- * the tangent of Utot (the beta pullback's V kernel), the tangent of Y by polarization of the
- * quadratic form Y(Utot) (two Y evaluations at Utot +/- s Utot_dot, s a power of two; no
- * truncation term), and forward-mode tangents through the Wigner recursion and dE/dr per pair.
+ * the tangent of Utot (the beta pullback's V kernel), the tangent of Y as the polar form of
+ * the quadratic form Y(Utot) (one pass over Utot and its tangent), and forward-mode tangents
+ * through the Wigner recursion and dE/dr per pair.
  * Environment IPG_GENERIC_HVP=1 at ipg_snap_create selects the per-atom kernel that carries
  * every phase in forward mode instead (same results to rounding).  Any of gbeta, gbeta0, gpos
  * may be NULL; beta [nspecies][K] is needed for gpos.  twojmax above 8 returns
@@ -281,7 +281,7 @@ IPG_API int ipg_snap_vjp(ipg_snap* snap, int64_t n, const double* pos, const int
 
 /* Autotuner: times the adjoint evaluation of this configuration under each candidate kernel
  * configuration and keeps the fastest for the handle.  Coordinate descent over the Y kernel
- * (row-blocked or one Z entry at a time: the twojmax-dependent shared-memory layout), the
+ * (streamed or one Z entry at a time), the
  * per-neighbor kernel (all chains of a pair per thread, or one chain per thread), the Utot
  * kernel (all chains in one launch, or one launch per chain with 1, 2 or 4 atoms per block)
  * and the atoms (warps) per block of the neighbor walk (1, 2, 4).  cache_path

@@ -129,6 +129,9 @@ struct ipg_ctx;
 // Y' and E_i (YM_Y), Z (YM_Z) or both (YM_YZ) of n atoms from their Utot (ipg_snap_y.cu).
 int launch_ystream(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int ym, const char* tname, int64_t n,
                    const int32_t* species, const double2* utot, double2* yout, double* Ei, double2* zout);
+// Tangent of Y' along Udot = -V (V [u_half][n] as written by k_snap_vlie): ydot [u_half][n].
+int launch_ytangent(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int64_t n, const int32_t* species,
+                    const double2* utot, const double2* V, double2* ydot);
 // Z of every ordered pair (p, q) of ne elements, zstride apart: the first factor of every product from
 // element p's Utot, the second from q's (ustride apart).
 int launch_zpairs(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, int64_t n, const int32_t* species, int ne,
