@@ -2066,72 +2066,9 @@ int launch_pair_lie(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t* d
 // atoms.  dE_i/dr_ij = 2 sum_h w Re(conj(D_k,h) Y_h), D_k = dsfac uhat_k U + sfac dU/dr_k,
 // depends on the pair geometry and on the centre atom's Y.  Its tangent along rdot = v_j - v_i
 // has a pair-local part (U, dU and the geometry along rdot: the second-order chain of
-// snapchain::all_chains_hvp) and a Y part (Ydot).  Y is a quadratic form in Utot, so
-// Ydot = [Y(U + s Udot) - Y(U - s Udot)] / (2s) exactly in exact arithmetic (the terms in s^2
-// cancel identically; no truncation term), with s a power of two per atom that gives U and
-// s Udot the same magnitude; Udot comes from k_snap_vsum (V with g = v is -Udot).
-
-// Per atom (one warp): s = 2^k with s max|Udot| ~ max|U| over the half plane, and the half
-// plane of U -/+ s V into Up / Um (full Utot layout; the Y kernel reads only these entries).
-// V holds the half plane up to the middle element of an even level; the entries beyond it are
-// the inversion-symmetric mirrors of entries of the same row (compute_ui.jl:105-125).
-__global__ void k_hvp_split(const __grid_constant__ SnapDev S, int64_t n, const double2* __restrict__ utot,
-                            const double2* __restrict__ V, double2* __restrict__ Up, double2* __restrict__ Um,
-                            double* __restrict__ scale) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;  // warp-uniform
-  const int U = S.idxu_max, UH = S.u_half;
-  auto vdot = [&](int h) -> double2 {  // Udot = -V, mirrored where V is not stored
-    int j = 0;
-    while (j < S.J && S.half_block[j + 1] <= h) j++;
-    const int e = h - S.half_block[j], mb = e / (j + 1), ma = e - mb * (j + 1);
-    if (2 * mb == j && ma > mb) {
-      const double2 m = V[(size_t)(S.half_block[j] + mb * (j + 1) + (j - ma)) * n + i];
-      const double sg = ((ma + mb) & 1) ? -1.0 : 1.0;
-      return make_double2(-sg * m.x, sg * m.y);  // -( (-1)^(ma+mb) conj(m) )
-    }
-    const double2 v = V[(size_t)h * n + i];
-    return make_double2(-v.x, -v.y);
-  };
-  double mu = 0.0, mv = 0.0;
-  for (int h = lane; h < UH; h += 32) {
-    const double2 u = utot[(size_t)i * U + S.u_of_h[h]], d = vdot(h);
-    mu = fmax(mu, fmax(fabs(u.x), fabs(u.y)));
-    mv = fmax(mv, fmax(fabs(d.x), fabs(d.y)));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mu = fmax(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-    mv = fmax(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-  }
-  int ex = 0;
-  if (mv > 0.0 && mu > 0.0) {  // s = 2^round(log2(mu / mv)), exact to multiply and divide by
-    int eu, ev;
-    frexp(mu, &eu);
-    frexp(mv, &ev);
-    ex = eu - ev;
-  }
-  const double s = ldexp(1.0, ex);
-  if (lane == 0) scale[i] = s;
-  for (int h = lane; h < UH; h += 32) {
-    const size_t e = (size_t)i * U + S.u_of_h[h];
-    const double2 u = utot[e], d = vdot(h);
-    Up[e] = make_double2(fma(s, d.x, u.x), fma(s, d.y, u.y));
-    Um[e] = make_double2(fma(-s, d.x, u.x), fma(-s, d.y, u.y));
-  }
-}
-
-// Ydot[h][i] = (Yp - Ym) / (2 s_i)
-__global__ void k_hvp_ydot(int64_t n, int uh, const double2* __restrict__ Yp, const double2* __restrict__ Ym,
-                           const double* __restrict__ scale, double2* __restrict__ Yd) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)uh * n) return;
-  const int64_t i = t % n;
-  const double f = 0.5 / scale[i];
-  const double2 a = Yp[t], b = Ym[t];
-  Yd[t] = make_double2((a.x - b.x) * f, (a.y - b.y) * f);
-}
+// snapchain::all_chains_hvp) and a Y part (Ydot).  Y is a quadratic form in Utot, so Ydot is its
+// polar form, U Udot + Udot U in place of every product (launch_ytangent); Udot comes from
+// k_snap_vsum (V with g = v is -Udot).
 
 // fdot[p][k] = the tangent of dE_i/dr_ij[k] along v (one (pair, k) per thread, k = blockIdx.y):
 //   2 (cudot T0 + cu T2 + sfacdot T1 + sfac T3 + cu T4 + sfac T5),  cu = dsfac uhat_k,
@@ -3940,31 +3877,18 @@ int ipg_snap_vjp(ipg_snap* s, int64_t n, const double* pos, const int32_t* speci
       IPG_RET(set_beta(s, beta, 0.0, dev));
     }
     if (utot && yw && dev.J <= YR_MAX_J && !s->generic_hvp) {
-      // register chains: Udot (k_snap_vsum), Ydot by polarization (two Y launches), the
-      // second-order pair chains (k_snap_pair_hvp)
-      const int U = dev.idxu_max, UH = dev.u_half;
-      double2 *V, *Up, *Um, *Yp, *Ym, *Yd;
-      double *sc, *ebuf;
+      // register chains: Udot (k_snap_vsum), Ydot, the second-order pair chains (k_snap_pair_hvp)
+      const int UH = dev.u_half;
+      double2 *V, *Yd;
       int32_t* owner;
       IPG_RET(scratch(ctx, "hvp_V", (size_t)UH * n + 1, &V));
-      IPG_RET(scratch(ctx, "hvp_Up", (size_t)U * n + 1, &Up));
-      IPG_RET(scratch(ctx, "hvp_Um", (size_t)U * n + 1, &Um));
-      IPG_RET(scratch(ctx, "hvp_Yp", (size_t)UH * n + 1, &Yp));
-      IPG_RET(scratch(ctx, "hvp_Ym", (size_t)UH * n + 1, &Ym));
       IPG_RET(scratch(ctx, "hvp_Yd", (size_t)UH * n + 1, &Yd));
-      IPG_RET(scratch(ctx, "hvp_scale", (size_t)n, &sc));
-      IPG_RET(scratch(ctx, "hvp_E", (size_t)n, &ebuf));
       IPG_RET(scratch(ctx, "snap_owner", (size_t)pl.npairs + 1, &owner));
       if (Vg)
         V = const_cast<double2*>(Vg);
       else
         IPG_RET(launch_vsum(ctx, dev, 0, n, pl.d_off, pl.d_j, pl.d_r, d_sp, d_v, V, s->pair_tangent));
-      IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_hvp_split, nblk(32 * n, 256), 256, 0, dev, n, utot, V, Up, Um, sc);
-      bool d1 = false, d2 = false;
-      IPG_RET(launch_y(s, dev, "snap_hvp_y", n, d_sp, Up, Yp, ebuf, nullptr, nullptr, &d1));
-      IPG_RET(launch_y(s, dev, "snap_hvp_y", n, d_sp, Um, Ym, ebuf, nullptr, nullptr, &d2));
-      if (!d1 || !d2) return ipg_fail(ctx, IPG_ERR_UNSUPPORTED, "position pullback: no atoms-in-lanes Y kernel");
-      IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_hvp_ydot, nblk((int64_t)UH * n, 256), 256, 0, n, UH, Yp, Ym, sc, Yd);
+      IPG_RET(launch_ytangent(ctx, dev, s->h.yktab, n, d_sp, utot, V, Yd));
       IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
       IPG_RET(launch_pair_hvp(ctx, dev, pl.npairs, pl.d_np, n, owner, pl.d_j, pl.d_r, d_sp, d_v, yw, Yd, fd,
                               s->pair_tangent));
