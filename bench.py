@@ -46,12 +46,12 @@ WORKLOAD = ("snap_j8: SNAP twojmax=8 (55 components), 2 species (weights 1.0/0.5
 
 # timing name -> kernel
 PAIR_KERNEL = "tangent" if os.environ.get("IPG_PAIR_TANGENT", "0") == "1" else "lie"
-KERNEL_NAMES = {"snap_atom": "k_snap_yrows", "snap_utot": "k_snap_utot_all<8>",
+KERNEL_NAMES = {"snap_atom": "k_snap_ystream", "snap_utot": "k_snap_utot_all<8>",
                 "snap_pair": "k_snap_pair_adj_all<8>" if PAIR_KERNEL == "tangent" else "k_snap_pair_lie<8>"}
 # DRAM bytes (read + write) per atom of one launch, from the ncu --set full captures on the
-# 16,000-atom case summarised in profiles/k_snap_{yrows,pair_lie,pair_adj_all,utot_all}_snap_j8.md;
+# 16,000-atom case summarised in profiles/k_snap_{ystream,pair_lie,pair_adj_all,utot_all}_snap_j8.md;
 # scaled by atoms (pairs per atom are the same).
-NCU_DRAM_BYTES_PER_ATOM = {"snap_atom": (51.886336e6 + 2.899200e6) / 16000,
+NCU_DRAM_BYTES_PER_ATOM = {"snap_atom": (52.707584e6 + 2.899200e6) / 16000,
                            "snap_pair": ((52.742144e6 + 0.953088e6) if PAIR_KERNEL == "tangent"
                                          else (50.157056e6 + 0.847360e6)) / 16000,
                            "snap_utot": (11.558912e6 + 16.316928e6) / 16000}
@@ -538,10 +538,10 @@ def main():
                 pair[name]["hbm"] = {"algorithmic_bytes": nbytes, "kernel_ms": k_ms, "achieved_GBps": gbps,
                                      "peak_GBps": HBM_PEAK, "frac": gbps / HBM_PEAK if gbps else None,
                                      "peak_source": "MEASURED_PEAKS.json hbm_gbs"}
-                # what bounds it instead: the ncu counters of k_pair_half<3> on the 1 M-atom
+                # what bounds it instead: the ncu counters of k_pair_half on the 32,000-atom
                 # case of the same lattice (profiles/k_pair_half_lc_1m.md)
-                pair[name]["ncu_pipes"] = {"kernel": "k_pair_half<3>", "fp64_pipe_pct": 19.7, "issue_active_pct": 40.2,
-                                           "dram_pct_of_peak": 1.05, "bound": "FP64 latency (wait stalls)",
+                pair[name]["ncu_pipes"] = {"kernel": "k_pair_half", "fp64_pipe_pct": 13.3, "issue_active_pct": 42.9,
+                                           "dram_pct_of_peak": 0.1, "bound": "FP64 latency (wait stalls)",
                                            "source": "profiles/k_pair_half_lc_1m.md"}
         line["lj_pairs_per_s"] = pair
 
