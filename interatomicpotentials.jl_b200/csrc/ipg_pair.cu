@@ -439,9 +439,12 @@ int pair_eval_device(ipg_ctx* ctx, int64_t n, const double* d_pos, const int32_t
   IPG_RET(ipg_timing_mark(ctx, "pair_eval", true));
   if (half) {
     const int64_t items = cl.ncells * HALF_OFFSETS;
-    // grid-stride: a fixed grid of a few waves of resident blocks
-    nb = std::max<int64_t>(1, std::min<int64_t>((items + PAIR_WARPS - 1) / PAIR_WARPS,
-                                                (int64_t)ctx->num_sms * PAIR_MINB * 4));
+    // Grid-stride over the items: a block costs its start, its reduction and the wait for its slowest
+    // warp, so it takes several items a warp, but no fewer blocks than fill the GPU once; large systems
+    // take up to 16 waves, which even out the cells.  Against four waves at most: 32,000 atoms (18,000
+    // items) 274 -> 241 us with six items a warp, 261 with three; 4.1 M atoms 15.2 -> 14.8 ms.
+    const int64_t one = (items + PAIR_WARPS - 1) / PAIR_WARPS, wave = (int64_t)ctx->num_sms * PAIR_MINB;
+    nb = std::max<int64_t>(1, std::min(one, std::max(wave, std::min(one / 6, 16 * wave))));
     const PairBox box = {{g.L[0], g.L[1], g.L[2]}};
     double* P;
     IPG_RET(scratch(ctx, "pair_partial", (size_t)nb * 7, &partial));
