@@ -250,11 +250,22 @@ struct PairList {
   int64_t* d_off = nullptr;  // [n+1]
   int32_t* d_j = nullptr;    // [npairs]
   double* d_r = nullptr;     // [npairs][3]
-  int64_t* d_rev = nullptr;  // [npairs]   transpose: the reverse of each pair (-1: none)
+  int64_t* d_rev = nullptr;  // [npairs]   transpose: the reverse of each pair; none: -2 - the next of its chain
+  int64_t* d_one = nullptr;  // [n]        1 + the head of the chain of the pairs that end at an atom and have no
+                             //            reverse (0: none); behind d_off, which a build clears with it
 };
 
+// The pair that follows `after` in ascending order among the pairs that end at an atom and have no
+// reverse (-1: no more), from `one` of the atom.  The chain's own order is that of arrival.
+__device__ __forceinline__ int64_t next_one_sided(int64_t one, const int64_t* __restrict__ rev, int64_t after) {
+  int64_t best = -1;
+  for (int64_t q = one - 1; q >= 0; q = -2 - rev[q])
+    if (q > after && (best < 0 || q < best)) best = q;
+  return best;
+}
+
 // mode: IPG_NLIST_HALF (cut[0] = rcut) or IPG_NLIST_FULL (cut = nsp*nsp cutsq), with
-// IPG_NLIST_LITERAL_SQRT optionally or-ed in.  want_transpose builds d_rev.
+// IPG_NLIST_LITERAL_SQRT optionally or-ed in.  want_transpose builds d_rev and d_one.
 // sorted: each atom's neighbors ascending (the reference's order); otherwise the
 // emission order (stencil cells in fixed order, ascending inside a cell), which is
 // equally deterministic.

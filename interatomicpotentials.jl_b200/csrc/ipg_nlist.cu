@@ -753,16 +753,16 @@ __global__ void k_pair_sort(int64_t n, const int64_t* __restrict__ off, int32_t*
 }
 
 // Transpose: rev[p] of pair p = (i -> k) is the pair (k -> i).  The lists it serves (the full SNAP
-// lists) are symmetric with one image per pair, so the pairs whose neighbor is i are the reverses of
-// those that i owns.  (No reverse, -1: a list cut at a capacity, whose result the capacity error
-// discards, or a pair at the cutoff to the last bit, which the rounding of the two minimum images can
-// put on one list only.)
+// lists) have one image per pair and are symmetric but for pairs at the cutoff to the last bit, which
+// the rounding of the two minimum images can put on one list only (and lists cut at a capacity, whose
+// result the capacity error discards).  So the pairs that end at i are the reverses of those that i
+// owns, and the chain of the pairs without a reverse: one[i] - 1, then rev[p] = -2 - the next (-1: none).
 //
 // One warp per owner i, one lane per pair (32 at a time); each lane looks through the neighbors of k
 // on its own, so the lanes' loads overlap: 48 us at 54,000 atoms, 6 at 249.  Lists of their own for the
 // pairs that end at each atom took counts, their scan and a clear besides, 10 us at 249 atoms.
 __global__ void k_rev_pair(int64_t n, const int64_t* __restrict__ off, const int32_t* __restrict__ j,
-                           int64_t* __restrict__ rev) {
+                           int64_t* __restrict__ rev, int64_t* __restrict__ one) {
   const int lane = threadIdx.x & 31;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= n) return;  // warp-uniform
@@ -774,6 +774,7 @@ __global__ void k_rev_pair(int64_t n, const int64_t* __restrict__ off, const int
 #pragma unroll 4
     for (int64_t q = q0; q < q1; q++)
       if (j[q] == i) r = q;
+    if (r < 0) r = -1 - (int64_t)atomicExch((unsigned long long*)&one[k], (unsigned long long)(p + 1));
     rev[p] = r;
   }
 }
@@ -884,7 +885,8 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
 namespace {
 int build_transpose(ipg_ctx* ctx, const std::string& pre, int64_t n, PairList& pl) {
   IPG_RET(scratch(ctx, (pre + "rev").c_str(), pl.npairs + 1, &pl.d_rev));
-  if (pl.npairs > 0) IPG_LAUNCH(ctx, k_rev_pair, nblk(32 * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev);
+  if (pl.npairs > 0)
+    IPG_LAUNCH(ctx, k_rev_pair, nblk(32 * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, pl.d_one);
   return IPG_OK;
 }
 }  // namespace
@@ -918,9 +920,10 @@ int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const 
   int64_t n = cl.n;
   pl.n = n;
   int64_t* cnt;
-  IPG_RET(scratch(ctx, (pre + "off").c_str(), n + 1, &pl.d_off));
+  IPG_RET(scratch(ctx, (pre + "off").c_str(), 2 * n + 1, &pl.d_off));
+  pl.d_one = pl.d_off + n + 1;
   cnt = pl.d_off;
-  CUDA_RET(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (n + 1), ctx->stream));
+  CUDA_RET(ctx, cudaMemsetAsync(cnt, 0, sizeof(int64_t) * (want_transpose ? 2 * n + 1 : n + 1), ctx->stream));
   const bool by_cell = ctx->walk_by_cell;
   // One walk instead of two when a previous build of this list gave the per-atom maximum:
   // emit into padded slots while counting, then compact (or, if an atom overflowed its
@@ -1032,8 +1035,9 @@ int ipg_filter_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const
   t.rcut2_hi = t.rcut * t.rcut * (1.0 + 1e-12);
   const int64_t n = cl.n;
   pl.n = n;
-  IPG_RET(scratch(ctx, (pre + "off").c_str(), n + 1, &pl.d_off));
-  CUDA_RET(ctx, cudaMemsetAsync(pl.d_off, 0, sizeof(int64_t) * (n + 1), ctx->stream));
+  IPG_RET(scratch(ctx, (pre + "off").c_str(), 2 * n + 1, &pl.d_off));
+  pl.d_one = pl.d_off + n + 1;
+  CUDA_RET(ctx, cudaMemsetAsync(pl.d_off, 0, sizeof(int64_t) * (2 * n + 1), ctx->stream));
   if (n > 0)
     IPG_LAUNCH(ctx, k_filter_walk<false>, nblk(32 * n, 128), 128, 0, n, t, cl.d_grid, cl.d_conf, cached.d_off,
                cached.d_j, d_pos, d_species, nsp, pl.d_off, nullptr, nullptr, nullptr, ctx->d_status);

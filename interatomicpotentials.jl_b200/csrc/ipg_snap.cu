@@ -2338,7 +2338,8 @@ __global__ void k_snap_contract(int64_t n, const int64_t* __restrict__ off, cons
   }
 }
 
-// F_k = sum over k's pairs p of f_p - f_rev(p), rev(p) the reverse pair; per-atom virial contribution
+// F_k = sum over k's pairs p of f_p - f_rev(p), rev(p) the reverse pair, minus f of the pairs that end at
+// k and have no reverse (k_rev_pair); per-atom virial contribution
 // w6[k] = sum over p of f_p (x) (x_k - x_j(p)) with absolute positions
 // (snap.jl:292-306 contracted with beta): [xx, yy, zz, yz, xz, xy] as in the reference.
 //
@@ -2353,6 +2354,7 @@ template <bool ONE>
 __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* __restrict__ off,
                                                      const int32_t* __restrict__ nbr,
                                                      const int64_t* __restrict__ rev,
+                                                     const int64_t* __restrict__ one,
                                                      const double* __restrict__ fvec, int nchains,
                                                      const double* __restrict__ pos, double* __restrict__ F,
                                                      double* __restrict__ w6) {
@@ -2366,6 +2368,7 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
   double w[6] = {0, 0, 0, 0, 0, 0};
   const double xk = pos[3 * k], yk = pos[3 * k + 1], zk = pos[3 * k + 2];
   const int64_t p1 = valid ? off[k + 1] : 0;
+  const int64_t first = valid && g == 0 ? one[k] : 0;
 #pragma unroll 4
   for (int64_t p = valid ? off[k] + g : 0; p < p1; p += GATHER_LANES) {
     const int64_t jn = nbr[p], q = rev[p];
@@ -2393,6 +2396,10 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
     w[4] += a * dz;
     w[5] += a * dy;
   }
+  for (int64_t q = next_one_sided(first, rev, -1); q >= 0; q = next_one_sided(first, rev, q))
+    for (int r = 0; r < nch; r++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) f[c] -= fvec[((size_t)q * nch + r) * 3 + c];
 #pragma unroll
   for (int o = GATHER_LANES / 2; o > 0; o >>= 1) {
 #pragma unroll
@@ -3126,7 +3133,8 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
   IPG_RET(ipg_side_join(ctx));  // the list transpose (side stream) is read from here on
   if ((out.F || out.W6) && fvec && n)
     IPG_TIMED_LAUNCH(ctx, "snap_gather", (nch == 1 ? k_snap_gather<true> : k_snap_gather<false>),
-                     nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, fvec, nch, d_pos, out.F, w6);
+                     nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, pl.d_one, fvec, nch, d_pos, out.F,
+                     w6);
   if (out.E || out.W6) {
     // chunk table: [config, first atom, end] per chunk, then each config's chunk range
     std::vector<int64_t>& ch = s->chunk_tab;
@@ -3922,8 +3930,8 @@ int ipg_snap_vjp(ipg_snap* s, int64_t n, const double* pos, const int32_t* speci
       const int64_t grid = std::min<int64_t>(n, (int64_t)ctx->num_sms * std::max(1, per_sm));
       IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_snap_hvp, (unsigned)grid, nw * 32, HL.total, dev, io, d_v, fd);
     }
-    IPG_LAUNCH(ctx, k_snap_gather<true>, nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, fd, 1, d_pos,
-               Fd, (double*)nullptr);
+    IPG_LAUNCH(ctx, k_snap_gather<true>, nblk(GATHER_LANES * n, 128), 128, 0, n, pl.d_off, pl.d_j, pl.d_rev, pl.d_one, fd, 1,
+               d_pos, Fd, (double*)nullptr);
   }
   IPG_LAUNCH(ctx, k_vjp_pos, nblk((int64_t)m, 256), 256, 0, (int64_t)m, F0, gE, Fd, gp);
   if (fused)

@@ -13,8 +13,8 @@ constexpr int DG_V = 7;       // partial sums per (species, component): W (6) an
 
 // One block takes a chunk of atoms of one configuration (blockIdx.x) and DG_T columns
 // t = 3 b + c (blockIdx.y) of dB/dr, dbl [pair][K][3]:
-//   dB_k[block s][b][c] = sum over k's pairs, s_k = s, of dbl_p - sum over their reverses, s_owner = s, of
-//     dbl_q (snap.jl:289-290), if dB is wanted;
+//   dB_k[block s][b][c] = sum over k's pairs, s_k = s, of dbl_p - sum over their reverses and the pairs
+//     that end at k without one (k_rev_pair), s_owner = s, of dbl_q (snap.jl:289-290), if dB is wanted;
 //   W of the chunk: dB_i/dr_ij (x) (x_i - x_j), absolute positions (snap.jl:292-306), and the sums
 //     of B, both per species, into part [chunk][nsp][K][7] (dbl null: the sums of B alone).
 // Bound by the reads of dbl: each pair's K x 3 numbers twice (once for its owner, once for its
@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
                                                       const int64_t* __restrict__ off,
                                                       const int32_t* __restrict__ nbr,
                                                       const int64_t* __restrict__ rev,
+                                                      const int64_t* __restrict__ one, int64_t n,
                                                       const int32_t* __restrict__ species,
                                                       const double* __restrict__ pos, const double* __restrict__ dbl,
                                                       const double* __restrict__ B, double* __restrict__ dB, int rows,
@@ -105,6 +106,20 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
         }
       }
     }
+    const int64_t first = one[i];
+    for (int64_t q = next_one_sided(first, rev, -1); q >= 0; q = next_one_sided(first, rev, q)) {  // rare
+      int64_t lo = 0, hi = n - 1;  // the owner: the last atom whose pairs start at or before q
+      while (lo < hi) {
+        const int64_t mid = (lo + hi + 1) / 2;
+        if (off[mid] <= q) lo = mid;
+        else hi = mid - 1;
+      }
+      int so = species[lo];
+      so = so < 0 ? 0 : (so >= nsp ? nsp - 1 : so);
+      const double v = act ? dbl[(size_t)q * C + col] : 0.0;
+#pragma unroll
+      for (int s = 0; s < NSP; s++) acc[s] -= NSP == 1 || so == s ? v : 0.0;
+    }
     if (act) {
 #pragma unroll
       for (int s = 0; s < NSP; s++)
@@ -160,11 +175,11 @@ __global__ void __launch_bounds__(256) k_desc_reduce(const int64_t* __restrict__
 }
 
 template <int NSP>
-int launch_gather(ipg_ctx* ctx, dim3 grid, const int64_t* chunks, int K, int nsp, const PairList& pl,
+int launch_gather(ipg_ctx* ctx, dim3 grid, const int64_t* chunks, int64_t n, int K, int nsp, const PairList& pl,
                   const int32_t* species, const double* pos, const double* dbl, const double* B,
                   double* dB, bool rows, double* part, bool want_w) {
-  IPG_LAUNCH(ctx, k_desc_gather<NSP>, grid, DG_T, 0, chunks, K, nsp, pl.d_off, pl.d_j, pl.d_rev, species,
-              pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
+  IPG_LAUNCH(ctx, k_desc_gather<NSP>, grid, DG_T, 0, chunks, K, nsp, pl.d_off, pl.d_j, pl.d_rev, pl.d_one, n,
+             species, pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
   return IPG_OK;
 }
 
@@ -204,13 +219,13 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
   const double* Bs = Ae ? B : nullptr;
   const bool want_w = Wd || Aw;
   if (nsp == 1)
-    IPG_RET(launch_gather<1>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<1>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else if (nsp == 2)
-    IPG_RET(launch_gather<2>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<2>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else if (nsp <= 4)
-    IPG_RET(launch_gather<4>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<4>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   else
-    IPG_RET(launch_gather<8>(ctx, grid, d_tab, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
+    IPG_RET(launch_gather<8>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
   if (sums)
     IPG_LAUNCH(ctx, k_desc_reduce, dim3((unsigned)((width + 31) / 32), (unsigned)nconf), 256, 0,
                d_tab + tab.size(), KN, part, Wd, Aw, Ae);
