@@ -217,6 +217,7 @@ struct ConfGrid {
   double cs[3];  // cell edge (>= search radius on every axis with more than one cell)
   int nc[3];     // cells per axis
   int pad;
+  double rel;    // unit of CellList::d_srel: the power of two that takes the longest cell edge into [1, 2)
   int64_t cell_off;  // first global cell id of this configuration
   int64_t atom_off;
   int64_t natoms;
@@ -234,7 +235,8 @@ struct CellList {
   int32_t* d_cell_atoms = nullptr; // [n] atom ids in cell order (ascending inside a cell)
   int32_t* d_slot_of = nullptr;    // [n] slot of each atom
   double4* d_spos = nullptr;       // [n] positions in slot order (w = species as double)
-  float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell, w = atom id's bits
+  float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell, times
+                                   //     ConfGrid::rel; w = atom id's bits
 };
 
 // Builds the cell list for `radius` (prefix selects the scratch buffers used).
@@ -287,15 +289,16 @@ int ipg_build_pairs(ipg_ctx* ctx, const char* prefix, const CellList& cl, const 
                     int64_t cap = 0, int walk_warps = 4, bool count_only = false);
 
 // Squared threshold of a 32-bit distance test on cell-relative positions (CellList::d_srel): no pair
-// within rcut fails it.  Each coordinate of each
+// within rcut fails it.  They are in units of about a cell edge, so that their squares are far from the
+// ends of the 32-bit range whatever the unit of length.  Each coordinate of each
 // atom is at most about one cell edge (cs) and rounded to 32 bits, as are the shift between the
 // cells (at most cs) and the difference (at most 2 cs): at most 6 * 2^-24 cs per axis, less than
 // 7e-7 cs in distance; the squares and their sum add a relative 3 * 2^-24.
 __host__ __device__ inline float prefilter_threshold(const ConfGrid& g, double rcut) {
   const double cs = fmax(g.cs[0], fmax(g.cs[1], g.cs[2]));
-  const double r = rcut + 2e-6 * cs;
+  const double r = (rcut + 2e-6 * cs) * g.rel;
   const double t = r * r * (1.0 + 1e-6);
-  return t < 1e30 ? (float)t : 1e30f;
+  return t < 1e30 ? (float)t : 1e30f;  // squared distances of stencil neighbors are below 100
 }
 
 // Device helper: the distinct neighbor-cell coordinates along one axis (<= 3).

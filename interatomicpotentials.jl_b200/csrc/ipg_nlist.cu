@@ -85,7 +85,7 @@ __device__ __forceinline__ int64_t cell_of_atom(int64_t i, const double* __restr
 }
 
 // Atom i of cell c (of grid g) into slot s of the cell order; srel receives its position
-// relative to the cell's lower corner, and its id in w.
+// relative to the cell's lower corner (in units of g.rel), and its id in w.
 __device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid& g, int64_t c,
                                            const double* __restrict__ pos, const int32_t* __restrict__ species,
                                            int nsp, int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
@@ -98,8 +98,9 @@ __device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid&
   spos[s] = make_double4(x, y, z, (double)sp);
   const int k = (int)(c - g.cell_off), nxy = g.nc[0] * g.nc[1];
   const int cz = k / nxy, cy = (k - cz * nxy) / g.nc[0], cx = k - cz * nxy - cy * g.nc[0];
-  srel[s] = make_float4((float)(cell_wrap(g, 0, x) - cx * g.cs[0]), (float)(cell_wrap(g, 1, y) - cy * g.cs[1]),
-                        (float)(cell_wrap(g, 2, z) - cz * g.cs[2]), __int_as_float(i));
+  srel[s] = make_float4((float)((cell_wrap(g, 0, x) - cx * g.cs[0]) * g.rel),
+                        (float)((cell_wrap(g, 1, y) - cy * g.cs[1]) * g.rel),
+                        (float)((cell_wrap(g, 2, z) - cz * g.cs[2]) * g.rel), __int_as_float(i));
 }
 
 __global__ void k_cell_count(int64_t n, const double* __restrict__ pos, const int32_t* __restrict__ species, int nsp,
@@ -497,7 +498,7 @@ __device__ __forceinline__ void walk_stencil(const ConfGrid& g, const int* cc, c
       }
       int d = c[a] - cc[a];  // in -1..1 but for the wrap
       d = d > 1 ? d - g.nc[a] : (d < -1 ? d + g.nc[a] : d);
-      s[a] = (float)(d * g.cs[a]);
+      s[a] = (float)(d * g.cs[a] * g.rel);
     }
     const int64_t cell = g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
     beg = (int)cell_start[cell];
@@ -845,6 +846,8 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
       tot *= g.nc[a];
     }
     for (int a = 0; a < 3; a++) g.cs[a] = e3[a] > 0.0 ? e3[a] / g.nc[a] : 1.0;
+    const int e2 = std::ilogb(std::max(g.cs[0], std::max(g.cs[1], g.cs[2])));
+    g.rel = std::ldexp(1.0, -std::max(-1000, std::min(1000, e2)));
     g.cell_off = cell_total;
     cell_total += tot;
   }

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
     const int a0 = (int)cell_start[A], a1 = (int)cell_start[A + 1], t0 = (int)cell_start[T],
               t1 = (int)cell_start[T + 1];
     // the target cell's corner relative to the home cell's, at the image these two cells define
-    const float sx = (float)(dx * g.cs[0]), sy = (float)(dy * g.cs[1]), sz = (float)(dz * g.cs[2]);
+    const float sx = (float)(dx * g.cs[0] * g.rel), sy = (float)(dy * g.cs[1] * g.rel), sz = (float)(dz * g.cs[2] * g.rel);
     const int home_kind = k, tgt_kind = k == 0 ? 0 : HALF_OFFSETS - 1 + k;
     // cells of at most 32 atoms are one tile and its sums are stored; larger cells take
     // several tiles, whose sums accumulate into zeroed slots, as do the row and column sums
