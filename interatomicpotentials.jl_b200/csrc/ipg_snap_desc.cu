@@ -11,8 +11,8 @@ constexpr int DG_T = 192;     // threads over the columns (component, direction)
 constexpr int DG_PAIRS = 64;  // pairs staged at a time
 constexpr int DG_V = 7;       // partial sums per (species, component): W (6) and B
 
-// One block takes a chunk of atoms of one configuration (blockIdx.x) and DG_T columns
-// t = 3 b + c (blockIdx.y) of dB/dr, dbl [pair][K][3]:
+// One block takes one of nchunk chunks of atoms, each of one configuration, and DG_T columns t = 3 b + c
+// of dB/dr, dbl [pair][K][3] (chunk + nchunk x tile of columns in blockIdx.x: neither has a limit of its own):
 //   dB_k[block s][b][c] = sum over k's pairs, s_k = s, of dbl_p - sum over their reverses and the pairs
 //     that end at k without one (k_rev_pair), s_owner = s, of dbl_q (snap.jl:289-290), if dB is wanted;
 //   W of the chunk: dB_i/dr_ij (x) (x_i - x_j), absolute positions (snap.jl:292-306), and the sums
@@ -24,7 +24,7 @@ constexpr int DG_V = 7;       // partial sums per (species, component): W (6) an
 // configurations of at most 250 atoms, twojmax 6: 127 (plus 5) against 2,096 us, nearly all of it
 // in a kernel that walked each configuration serially.
 template <int NSP>
-__global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict__ chunks, int K, int nsp,
+__global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict__ chunks, int nchunk, int K, int nsp,
                                                       const int64_t* __restrict__ off,
                                                       const int32_t* __restrict__ nbr,
                                                       const int64_t* __restrict__ rev,
@@ -36,8 +36,9 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
   __shared__ double sd[DG_PAIRS][3];
   __shared__ int64_t sp[DG_PAIRS];
   __shared__ int ss[DG_PAIRS];
-  const int64_t a0 = chunks[2 * blockIdx.x], a1 = chunks[2 * blockIdx.x + 1];
-  const int col = blockIdx.y * DG_T + threadIdx.x, C = 3 * K;
+  const int chunk = blockIdx.x % nchunk;
+  const int64_t a0 = chunks[2 * chunk], a1 = chunks[2 * chunk + 1];
+  const int col = blockIdx.x / nchunk * DG_T + threadIdx.x, C = 3 * K;
   const bool act = col < C;
   const int b = col / 3, c = col - 3 * b;
   double w[NSP][4];  // per species: the three virial sums of this direction, and B (c = 0)
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
 #pragma unroll
   for (int s = 0; s < NSP; s++) {
     if (s >= nsp) break;
-    double* o = part + (((size_t)blockIdx.x * nsp + s) * K + b) * DG_V;
+    double* o = part + (((size_t)chunk * nsp + s) * K + b) * DG_V;
     o[c] = w[s][0];
     if (c == 0) {
       o[4] = w[s][1];
@@ -148,18 +149,20 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
   }
 }
 
-// Sums of a configuration's chunks in a fixed order: eight rows of chunks, then the rows.
+// Sums of a configuration's chunks in a fixed order: eight rows of chunks, then the rows (one block a
+// configuration and 32 columns, configurations first).
 //   Wd [K nsp][6] (one configuration), Aw [nconf][6][K nsp], Ae [nconf][K nsp]; any may be null.
-__global__ void __launch_bounds__(256) k_desc_reduce(const int64_t* __restrict__ conf_chunk, int KN,
+__global__ void __launch_bounds__(256) k_desc_reduce(const int64_t* __restrict__ conf_chunk, int nconf, int KN,
                                                      const double* __restrict__ part, double* __restrict__ Wd,
                                                      double* __restrict__ Aw, double* __restrict__ Ae) {
   __shared__ double sm[8][32];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, conf = blockIdx.y;
-  const int t = blockIdx.x * 32 + x, width = KN * DG_V;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, conf = blockIdx.x % nconf;
+  const int t = blockIdx.x / nconf * 32 + x, width = KN * DG_V;
   double v = 0.0;
   if (t < width) {
 #pragma unroll 4
-    for (int64_t q = conf_chunk[conf] + y; q < conf_chunk[conf + 1]; q += 8) v += part[(size_t)q * width + t];
+    for (int64_t q = conf_chunk[conf] - conf_chunk[0] + y; q < conf_chunk[conf + 1] - conf_chunk[0]; q += 8)
+      v += part[(size_t)q * width + t];
   }
   sm[y][x] = v;
   __syncthreads();
@@ -175,11 +178,12 @@ __global__ void __launch_bounds__(256) k_desc_reduce(const int64_t* __restrict__
 }
 
 template <int NSP>
-int launch_gather(ipg_ctx* ctx, dim3 grid, const int64_t* chunks, int64_t n, int K, int nsp, const PairList& pl,
+int launch_gather(ipg_ctx* ctx, int nchunk, const int64_t* chunks, int64_t n, int K, int nsp, const PairList& pl,
                   const int32_t* species, const double* pos, const double* dbl, const double* B,
                   double* dB, bool rows, double* part, bool want_w) {
-  IPG_LAUNCH(ctx, k_desc_gather<NSP>, grid, DG_T, 0, chunks, K, nsp, pl.d_off, pl.d_j, pl.d_rev, pl.d_one, n,
-             species, pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
+  const int ytiles = (3 * K + DG_T - 1) / DG_T;
+  IPG_LAUNCH(ctx, k_desc_gather<NSP>, (unsigned)nchunk * ytiles, DG_T, 0, chunks, nchunk, K, nsp, pl.d_off, pl.d_j,
+             pl.d_rev, pl.d_one, n, species, pos, dbl, B, dB, rows ? 1 : 0, part, want_w ? 1 : 0);
   return IPG_OK;
 }
 
@@ -192,9 +196,11 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
   const bool sums = Wd || Aw || Ae;
   if (n <= 0 || (!dB && !sums)) return IPG_OK;
   const int ytiles = (3 * K + DG_T - 1) / DG_T, KN = K * nsp;
-  // Atoms per chunk: about eight blocks per SM, and the chunks' sums within 128 MB.
-  const int64_t width = (int64_t)KN * DG_V;
-  const int64_t most = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 8 / ytiles, (int64_t(16) << 20) / width));
+  // Atoms per chunk: about eight blocks per SM.  The chunks' sums take at most 128 MB (or one
+  // configuration's, if that is more: a configuration is at least one chunk), so configurations whose
+  // chunks would take more follow in another pair of launches.
+  const int64_t width = (int64_t)KN * DG_V, room = std::max<int64_t>(1, (int64_t(16) << 20) / width);
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->num_sms * 8 / ytiles, room));
   const int64_t per = std::max<int64_t>(1, (n + most - 1) / most);
   std::vector<int64_t> tab;
   std::vector<int64_t> cc(nconf + 1, 0);
@@ -205,7 +211,6 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
     }
     cc[c + 1] = (int64_t)tab.size() / 2;
   }
-  const int64_t nchunk = cc[nconf];
   int64_t* hb = host_scratch<int64_t>(ctx, "desc_chunks_h", tab.size() + cc.size());
   memcpy(hb, tab.data(), sizeof(int64_t) * tab.size());
   memcpy(hb + tab.size(), cc.data(), sizeof(int64_t) * cc.size());
@@ -213,21 +218,28 @@ int launch_descriptors(ipg_ctx* ctx, int K, int nsp, int nconf, const int64_t* h
   IPG_RET(scratch(ctx, "desc_chunks", tab.size() + cc.size(), &d_tab));
   CUDA_RET(ctx, cudaMemcpyAsync(d_tab, hb, sizeof(int64_t) * (tab.size() + cc.size()), cudaMemcpyHostToDevice,
                                 ctx->stream));
+  std::vector<int> group = {0};  // first configurations of the launches
+  int64_t largest = 0;           // chunks of a group
+  for (int c = 0; c < nconf; c++) {
+    if (c > group.back() && (cc[c + 1] - cc[group.back()] > room || c - group.back() >= room)) group.push_back(c);
+    largest = std::max(largest, cc[c + 1] - cc[group.back()]);
+  }
+  group.push_back(nconf);
   double* part = nullptr;
-  if (sums) IPG_RET(scratch(ctx, "desc_part", (size_t)nchunk * width, &part));
-  const dim3 grid((unsigned)nchunk, (unsigned)ytiles);
+  if (sums) IPG_RET(scratch(ctx, "desc_part", (size_t)largest * width, &part));
   const double* Bs = Ae ? B : nullptr;
   const bool want_w = Wd || Aw;
-  if (nsp == 1)
-    IPG_RET(launch_gather<1>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
-  else if (nsp == 2)
-    IPG_RET(launch_gather<2>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
-  else if (nsp <= 4)
-    IPG_RET(launch_gather<4>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
-  else
-    IPG_RET(launch_gather<8>(ctx, grid, d_tab, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
-  if (sums)
-    IPG_LAUNCH(ctx, k_desc_reduce, dim3((unsigned)((width + 31) / 32), (unsigned)nconf), 256, 0,
-               d_tab + tab.size(), KN, part, Wd, Aw, Ae);
+  for (size_t q = 0; q + 1 < group.size(); q++) {
+    const int c0 = group[q], nc = group[q + 1] - c0;
+    const int nchunk = (int)(cc[group[q + 1]] - cc[c0]);
+    const int64_t* chunks = d_tab + 2 * cc[c0];
+    const auto gather = nsp == 1 ? launch_gather<1> : nsp == 2 ? launch_gather<2>
+                                  : nsp <= 4 ? launch_gather<4> : launch_gather<8>;
+    if (nchunk)
+      IPG_RET(gather(ctx, nchunk, chunks, n, K, nsp, pl, species, pos, dbl, Bs, dB, rows, part, want_w));
+    if (sums)
+      IPG_LAUNCH(ctx, k_desc_reduce, (unsigned)nc * (unsigned)((width + 31) / 32), 256, 0, d_tab + tab.size() + c0, nc,
+                 KN, part, Wd, Aw ? Aw + (size_t)c0 * 6 * KN : nullptr, Ae ? Ae + (size_t)c0 * KN : nullptr);
+  }
   return IPG_OK;
 }
