@@ -257,13 +257,25 @@ struct PairList {
                              //            reverse (0: none); behind d_off, which a build clears with it
 };
 
-// The pair that follows `after` in ascending order among the pairs that end at an atom and have no
-// reverse (-1: no more), from `one` of the atom.  The chain's own order is that of arrival.
-__device__ __forceinline__ int64_t next_one_sided(int64_t one, const int64_t* __restrict__ rev, int64_t after) {
-  int64_t best = -1;
-  for (int64_t q = one - 1; q >= 0; q = -2 - rev[q])
-    if (q > after && (best < 0 || q < best)) best = q;
-  return best;
+// f(p) of the pairs that end at an atom and have no reverse, from `one` of the atom, in ascending order
+// (the chain's own order is that of arrival).  An atom has at most a shell of them; more are in a list cut at
+// a capacity, whose result is thrown away: they come as they are, in time linear in their number.
+template <class F>
+__device__ __forceinline__ void for_one_sided(int64_t one, const int64_t* __restrict__ rev, F f) {
+  constexpr int MOST = 256;
+  int m = 0;
+  for (int64_t q = one - 1; q >= 0 && m <= MOST; q = -2 - rev[q]) m++;
+  if (m > MOST) {
+    for (int64_t q = one - 1; q >= 0; q = -2 - rev[q]) f(q);
+    return;
+  }
+  for (int64_t last = -1; m > 0; m--) {
+    int64_t best = INT64_MAX;
+    for (int64_t q = one - 1; q >= 0; q = -2 - rev[q])
+      if (q > last && q < best) best = q;
+    f(best);
+    last = best;
+  }
 }
 
 // mode: IPG_NLIST_HALF (cut[0] = rcut) or IPG_NLIST_FULL (cut = nsp*nsp cutsq), with

@@ -2338,6 +2338,21 @@ __global__ void k_snap_contract(int64_t n, const int64_t* __restrict__ off, cons
   }
 }
 
+// Sum of f over the pairs that end at an atom and have no reverse (out of line: the gather's registers).
+__device__ __noinline__ double3 one_sided_sum(int64_t one, const int64_t* __restrict__ rev,
+                                              const double* __restrict__ fvec, int nch) {
+  double3 s = make_double3(0.0, 0.0, 0.0);
+  for_one_sided(one, rev, [&](int64_t q) {
+    for (int r = 0; r < nch; r++) {
+      const double* v = fvec + ((size_t)q * nch + r) * 3;
+      s.x += v[0];
+      s.y += v[1];
+      s.z += v[2];
+    }
+  });
+  return s;
+}
+
 // F_k = sum over k's pairs p of f_p - f_rev(p), rev(p) the reverse pair, minus f of the pairs that end at
 // k and have no reverse (k_rev_pair); per-atom virial contribution
 // w6[k] = sum over p of f_p (x) (x_k - x_j(p)) with absolute positions
@@ -2368,7 +2383,7 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
   double w[6] = {0, 0, 0, 0, 0, 0};
   const double xk = pos[3 * k], yk = pos[3 * k + 1], zk = pos[3 * k + 2];
   const int64_t p1 = valid ? off[k + 1] : 0;
-  const int64_t first = valid && g == 0 ? one[k] : 0;
+  const int64_t first = one[k];
 #pragma unroll 4
   for (int64_t p = valid ? off[k] + g : 0; p < p1; p += GATHER_LANES) {
     const int64_t jn = nbr[p], q = rev[p];
@@ -2396,10 +2411,12 @@ __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* _
     w[4] += a * dz;
     w[5] += a * dy;
   }
-  for (int64_t q = next_one_sided(first, rev, -1); q >= 0; q = next_one_sided(first, rev, q))
-    for (int r = 0; r < nch; r++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) f[c] -= fvec[((size_t)q * nch + r) * 3 + c];
+  if (first && valid && g == 0) {  // rare
+    const double3 s = one_sided_sum(first, rev, fvec, nch);
+    f[0] -= s.x;
+    f[1] -= s.y;
+    f[2] -= s.z;
+  }
 #pragma unroll
   for (int o = GATHER_LANES / 2; o > 0; o >>= 1) {
 #pragma unroll

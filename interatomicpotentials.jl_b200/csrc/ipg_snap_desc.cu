@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
       }
     }
     const int64_t first = one[i];
-    for (int64_t q = next_one_sided(first, rev, -1); q >= 0; q = next_one_sided(first, rev, q)) {  // rare
+    for_one_sided(first, rev, [&](int64_t q) {
       int64_t lo = 0, hi = n - 1;  // the owner: the last atom whose pairs start at or before q
       while (lo < hi) {
         const int64_t mid = (lo + hi + 1) / 2;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
       const double v = act ? dbl[(size_t)q * C + col] : 0.0;
 #pragma unroll
       for (int s = 0; s < NSP; s++) acc[s] -= NSP == 1 || so == s ? v : 0.0;
-    }
+    });
     if (act) {
 #pragma unroll
       for (int s = 0; s < NSP; s++)
