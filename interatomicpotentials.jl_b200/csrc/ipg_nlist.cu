@@ -715,18 +715,23 @@ __global__ void __launch_bounds__(WALKC_WARPS * 32) k_pair_walk_cells(
   }
 }
 
-// Padded emission (k_pair_walk_cells<2>) to the CSR list: slot t of atom i goes to off[i] + t.
+// Padded emission (k_pair_walk_cells<2>) to the CSR list: slot t of atom i goes to off[i] + t.  In
+// capacity mode an atom may have more hits than its kcap slots: the list is then thrown away
+// (k_clamp_offsets reports it), but the kernels that follow still read it, so the entries without a slot
+// become pairs of the atom with itself (at the last slot's distance).  They held what the buffer had: the
+// atoms of another, possibly larger system, or nothing yet.
 __global__ void k_pad_compact(int64_t n, int kcap, const int64_t* __restrict__ off, const int32_t* __restrict__ pj,
                               const double* __restrict__ pr, int32_t* __restrict__ j, double* __restrict__ r) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n * kcap) return;
-  const int64_t i = s / kcap;
-  const int64_t o = off[i] + (s - i * kcap);
-  if (o >= off[i + 1]) return;
-  j[o] = pj[s];
-  r[3 * o] = pr[3 * s];
-  r[3 * o + 1] = pr[3 * s + 1];
-  r[3 * o + 2] = pr[3 * s + 2];
+  const int64_t i = s / kcap, t = s - i * kcap, e = off[i + 1];
+  for (int64_t b = off[i] + t, o = b; o < e; o++) {
+    j[o] = o == b ? pj[s] : (int32_t)i;
+    r[3 * o] = pr[3 * s];
+    r[3 * o + 1] = pr[3 * s + 1];
+    r[3 * o + 2] = pr[3 * s + 2];
+    if (t + 1 < kcap) break;
+  }
 }
 
 // Sorts each atom's list by neighbor index (insertion sort; lists are short).
