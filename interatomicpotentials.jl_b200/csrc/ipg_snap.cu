@@ -3182,15 +3182,9 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     if (nconf > 0)
       IPG_LAUNCH(ctx, k_conf_reduce, (unsigned)nconf, CONF_T, 0, nconf, d_cc, part, dev.beta0, out.E, out.W6);
   }
-  if (want_desc && n) {
-    int32_t* owner = nullptr;
-    if (out.dB) {
-      IPG_RET(scratch(ctx, "snap_owner", (size_t)np + 1, &owner));
-      IPG_LAUNCH(ctx, k_pair_owner, nblk(32 * n, 256), 256, 0, n, pl.d_off, owner);
-    }
+  if (want_desc && n)
     IPG_RET(launch_descriptors(ctx, K, nsp, nconf, h_atom_off, pl, d_species, d_pos, dbl, out.B, out.dB,
                                out.dB_rows, out.Wd, out.Aw, out.Ae));
-  }
   if (out.pl_out) *out.pl_out = pl;
   if (out.utot_out) *out.utot_out = io.utot_in;
   return ipg_side_join(ctx);

@@ -36,3 +36,19 @@ def test_fitting_rows(twojmax, quadratic, nconf):
         assert (rows == rows[:1]).all()
         close = lambda a, b: np.max(np.abs(a - b), initial=0.0) <= TOL * max(1.0, np.max(np.abs(b), initial=0.0))  # noqa: E731
         assert close(Ae[q], B.sum(0)) and close(rows[0], dB.transpose(0, 2, 1)) and close(Aw[q], W.T)
+
+
+def test_no_launch_without_a_reader():
+    """Force descriptors come out of the pass that forms the virial ones: no launch more."""
+    from ipg._lib import DESC_DB, DESC_W
+    rng = np.random.default_rng(4)
+    s = ipg.System(rng.uniform(0, 9, (60, 3)), ["A"] * 60, [9.0] * 3)
+    snap = ipg.SNAP(60, 4, ["A"], 3.0, 0.0, 0.99363, [0.5], [1.0], switch_flag=True, ctx=ipg.Context(0))
+
+    def launches(what):
+        snap._descriptors(s, what)
+        k = snap.ctx.launch_count()
+        snap._descriptors(s, what)
+        return snap.ctx.launch_count() - k
+
+    assert launches(DESC_DB | DESC_W) == launches(DESC_W)
