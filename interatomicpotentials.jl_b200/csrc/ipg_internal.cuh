@@ -233,7 +233,6 @@ struct CellList {
   int32_t* d_conf = nullptr;       // [n] configuration of each atom
   int64_t* d_cell_start = nullptr; // [ncells+1]
   int32_t* d_cell_atoms = nullptr; // [n] atom ids in cell order (ascending inside a cell)
-  int32_t* d_slot_of = nullptr;    // [n] slot of each atom
   double4* d_spos = nullptr;       // [n] positions in slot order (w = species as double)
   float4* d_srel = nullptr;        // [n] positions relative to the lower corner of the atom's cell, times
                                    //     ConfGrid::rel; w = atom id's bits

@@ -7,7 +7,7 @@
 //   scan           cell_start
 //   k_cell_fill    atom ids into their cells, in arrival order
 //   k_cell_place   each atom's rank among its cell's ids (deterministic slot order): cell_atoms,
-//                  slot_of, spos
+//                  spos
 //   k_cells_small  all of these in one block, for few atoms and cells
 // and, for a materialised list:
 //   k_pair_count / scan / k_pair_emit / k_pair_sort, optionally the transpose.
@@ -88,10 +88,9 @@ __device__ __forceinline__ int64_t cell_of_atom(int64_t i, const double* __restr
 // relative to the cell's lower corner (in units of g.rel), and its id in w.
 __device__ __forceinline__ void place_atom(int32_t i, int64_t s, const ConfGrid& g, int64_t c,
                                            const double* __restrict__ pos, const int32_t* __restrict__ species,
-                                           int nsp, int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
+                                           int nsp, int32_t* __restrict__ cell_atoms,
                                            double4* __restrict__ spos, float4* __restrict__ srel) {
   cell_atoms[s] = i;
-  slot_of[i] = (int32_t)s;
   int sp = species ? species[i] : 0;
   sp = sp < 0 ? 0 : (sp > nsp - 1 ? nsp - 1 : sp);  // bad ids were reported with the cell
   const double x = pos[3 * (int64_t)i], y = pos[3 * (int64_t)i + 1], z = pos[3 * (int64_t)i + 2];
@@ -134,7 +133,7 @@ __global__ void __launch_bounds__(128) k_cell_place(int64_t n, const int32_t* __
                                                     const int32_t* __restrict__ conf,
                                                     const double* __restrict__ pos,
                                                     const int32_t* __restrict__ species, int nsp,
-                                                    int32_t* __restrict__ cell_atoms, int32_t* __restrict__ slot_of,
+                                                    int32_t* __restrict__ cell_atoms,
                                                     double4* __restrict__ spos, float4* __restrict__ srel) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(128) k_cell_place(int64_t n, const int32_t* __
   int64_t rank = 0;
 #pragma unroll 8
   for (int64_t q = s0; q < s1; q++) rank += unsorted[q] < i;
-  place_atom(i, s0 + rank, grid[conf[i]], c, pos, species, nsp, cell_atoms, slot_of, spos, srel);
+  place_atom(i, s0 + rank, grid[conf[i]], c, pos, species, nsp, cell_atoms, spos, srel);
 }
 
 // The whole cell list in one block (count, scan, fill, rank, place through shared memory), for
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(SMALL_T) k_cells_small(int n, int ncells, cons
                                                          const ConfGrid* __restrict__ grid, int nconf,
                                                          int32_t* conf, int64_t* __restrict__ cell_start,
                                                          int32_t* __restrict__ cell_atoms,
-                                                         int32_t* __restrict__ slot_of, double4* __restrict__ spos,
+                                                         double4* __restrict__ spos,
                                                          float4* __restrict__ srel, int* status) {
   __shared__ int start[SMALL_CELLS + 1];
   __shared__ int32_t unsorted[SMALL_ATOMS];
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(SMALL_T) k_cells_small(int n, int ncells, cons
     const int s0 = start[cell[q]], s1 = start[cell[q] + 1];
     int rank = 0;
     for (int k = s0; k < s1; k++) rank += unsorted[k] < i;
-    place_atom(i, s0 + rank, grid[conf[i]], cell[q], pos, species, nsp, cell_atoms, slot_of, spos, srel);
+    place_atom(i, s0 + rank, grid[conf[i]], cell[q], pos, species, nsp, cell_atoms, spos, srel);
   }
 }
 
@@ -869,13 +868,12 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
   IPG_RET(scratch(ctx, (pre + "cell_arrival").c_str(), n, &arrival));
   IPG_RET(scratch(ctx, (pre + "cell_unsorted").c_str(), n, &unsorted));
   IPG_RET(scratch(ctx, (pre + "cell_atoms").c_str(), n, &cl.d_cell_atoms));
-  IPG_RET(scratch(ctx, (pre + "slot_of").c_str(), n, &cl.d_slot_of));
   IPG_RET(scratch(ctx, (pre + "spos").c_str(), n, &cl.d_spos));
   IPG_RET(scratch(ctx, (pre + "srel").c_str(), n, &cl.d_srel));
   count = cl.d_cell_start;
   if (n > 0 && n <= SMALL_ATOMS && cell_total <= SMALL_CELLS) {
     IPG_LAUNCH(ctx, k_cells_small, 1, SMALL_T, 0, (int)n, (int)cell_total, d_pos, d_species, nsp, cl.d_grid, nconf,
-               cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_slot_of, cl.d_spos, cl.d_srel,
+               cl.d_conf, cl.d_cell_start, cl.d_cell_atoms, cl.d_spos, cl.d_srel,
                ctx->d_status);
     return IPG_OK;
   }
@@ -886,7 +884,7 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
   IPG_RET(ipg_scan_i64(ctx, count, cl.d_cell_start, cell_total + 1));
   IPG_LAUNCH(ctx, k_cell_fill, nblk(n, 256), 256, 0, n, cell_of, arrival, cl.d_cell_start, unsorted);
   IPG_LAUNCH(ctx, k_cell_place, nblk(n, 128), 128, 0, n, unsorted, cell_of, cl.d_cell_start, cl.d_grid,
-             cl.d_conf, d_pos, d_species, nsp, cl.d_cell_atoms, cl.d_slot_of, cl.d_spos, cl.d_srel);
+             cl.d_conf, d_pos, d_species, nsp, cl.d_cell_atoms, cl.d_spos, cl.d_srel);
   return IPG_OK;
 }
 
