@@ -48,6 +48,7 @@ struct ipg_ctx {
   bool capturing = false;
   uint64_t scratch_gen = 0;
   bool walk_by_cell = true;  // neighbor walk: one warp per cell (false: one warp per atom)
+  bool chain_constants = false;  // the constant tables of the SNAP register chains are uploaded
   bool pair_full_stencil = false;  // pair potentials: full-stencil walk even where the half stencil applies
   // single-pass neighbor walk: per list prefix, the per-atom slot count of the padded
   // emission (from the largest count of the previous build; 0 = walk twice)

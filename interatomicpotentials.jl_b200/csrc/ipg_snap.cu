@@ -2664,16 +2664,16 @@ int upload_tables(ipg_snap* s) {
   size_t o_uoh = o_ysw + pad(h.ysched_w.size() * 8);
   size_t o_hinfo = o_uoh + pad(h.u_of_h.size() * 4);
   size_t o_hsgen = o_hinfo + pad(h.h_info.size() * 4);
-  size_t o_yks = o_hsgen + pad(h.h_sgen.size() * 8);
-  size_t o_zfac = o_yks + pad(h.ykstream.size() * 8);
+  size_t o_zfac = o_hsgen + pad(h.h_sgen.size() * 8);
   size_t o_ytj = o_zfac + pad(h.zfac.size() * 8);
   size_t o_ytb = o_ytj + pad(h.ytrip_jjz.size() * 4);
   size_t o_ytf = o_ytb + pad(h.ytrip_b.size() * 4);
   size_t o_ylev = o_ytf + pad(h.ytrip_fac.size() * 8);
-  size_t total = o_ylev + pad(h.ylev.size() * 4);
+  size_t o_yks = o_ylev + pad(h.ylev.size() * 4);  // last and by far the largest: copied from where it is
+  size_t total = o_yks + pad(h.ykstream.size() * 8);
   CUDA_RET(ctx, cudaMalloc(&s->d_tables, total));
   char* b = static_cast<char*>(s->d_tables);
-  std::vector<char> hostbuf(total, 0);
+  std::vector<char> hostbuf(o_yks, 0);
   memcpy(hostbuf.data() + o_rpq, h.rootpq.data(), h.rootpq.size() * 8);
   memcpy(hostbuf.data() + o_cg, h.cglist.data(), h.cglist.size() * 8);
   memcpy(hostbuf.data() + o_ym, h.y_mult.data(), h.y_mult.size() * 8);
@@ -2689,13 +2689,14 @@ int upload_tables(ipg_snap* s) {
   memcpy(hostbuf.data() + o_uoh, h.u_of_h.data(), h.u_of_h.size() * 4);
   memcpy(hostbuf.data() + o_hinfo, h.h_info.data(), h.h_info.size() * 4);
   memcpy(hostbuf.data() + o_hsgen, h.h_sgen.data(), h.h_sgen.size() * 8);
-  memcpy(hostbuf.data() + o_yks, h.ykstream.data(), h.ykstream.size() * 8);
   memcpy(hostbuf.data() + o_zfac, h.zfac.data(), h.zfac.size() * 8);
   memcpy(hostbuf.data() + o_ytb, h.ytrip_b.data(), h.ytrip_b.size() * 4);
   memcpy(hostbuf.data() + o_ytf, h.ytrip_fac.data(), h.ytrip_fac.size() * 8);
   memcpy(hostbuf.data() + o_ylev, h.ylev.data(), h.ylev.size() * 4);
   memcpy(hostbuf.data() + o_ytj, h.ytrip_jjz.data(), h.ytrip_jjz.size() * 4);
-  CUDA_RET(ctx, cudaMemcpy(b, hostbuf.data(), total, cudaMemcpyHostToDevice));
+  CUDA_RET(ctx, cudaMemcpy(b, hostbuf.data(), o_yks, cudaMemcpyHostToDevice));
+  if (!h.ykstream.empty())
+    CUDA_RET(ctx, cudaMemcpy(b + o_yks, h.ykstream.data(), h.ykstream.size() * 8, cudaMemcpyHostToDevice));
   SnapDev& d = s->dev;
   memset(&d, 0, sizeof(d));
   d.J = h.J;
@@ -3483,14 +3484,19 @@ int ipg_snap_create(ipg_ctx* ctx, const ipg_snap_params* params, ipg_snap** out)
     delete s;
     return st;
   }
-  {  // tables of the register-chain kernels (independent of twojmax)
-    cudaError_t e = snapchain::upload_constants();
-    if (e == cudaSuccess) e = snapdb_upload_constants();
+  {  // tables of the register-chain kernels (independent of twojmax): once per context
+    cudaError_t e = cudaSuccess;
+    if (!ctx->chain_constants) {
+      e = snapchain::upload_constants();
+      if (e == cudaSuccess) e = snapdb_upload_constants();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the copies from pageable memory are done
     if (e != cudaSuccess) {
       cudaFree(s->d_tables);
       delete s;
-      return ipg_cuda_check(ctx, e, "rootpq upload");
+      return ipg_cuda_check(ctx, e, "table upload");
     }
+    ctx->chain_constants = true;
   }
   if (const char* g = getenv("IPG_GENERIC_ADJOINT")) s->generic_adjoint = g[0] == '1';
   if (const char* g = getenv("IPG_PAIR_SPLIT")) s->pair_split = g[0] == '1';

@@ -14,16 +14,19 @@
 
 namespace {
 
-// Factorials as long double (64-bit mantissa): exact wherever the reference's Int64
-// products are exact (twojmax <= 8), and free of Int64 overflow beyond that.
-long double fact(int n) {
-  long double f = 1.0L;
-  for (int k = 2; k <= n; k++) f *= k;
-  return f;
-}
+// Factorials, up to the largest of delta_cg, as long double (64-bit mantissa): exact wherever the
+// reference's Int64 products are exact (twojmax <= 8), and free of Int64 overflow beyond that.
+struct Factorials {
+  long double f[3 * SNAP_MAX_J / 2 + 2];
+  Factorials() {
+    f[0] = f[1] = 1.0L;
+    for (int k = 2; k < 3 * SNAP_MAX_J / 2 + 2; k++) f[k] = f[k - 1] * k;
+  }
+  long double operator()(int n) const { return f[n]; }
+};
 
 // prebuilt_arrays.jl:250-257
-double delta_cg(int j1, int j2, int j) {
+double delta_cg(const Factorials& fact, int j1, int j2, int j) {
   long double den = fact((j1 + j2 + j) / 2 + 1);
   long double num = fact((j1 + j2 - j) / 2) * fact((j1 - j2 + j) / 2) * fact((-j1 + j2 + j) / 2);
   return std::sqrt((double)num / (double)den);
@@ -133,10 +136,12 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
     for (int b = 1; b <= J; b++) h.rootpq[a * (J + 2) + b] = std::sqrt((double)a / (double)b);
 
   h.cglist.assign(h.idxcg_max, 0.0);
+  const Factorials fact;
   int idx = 0;
   for (int j1 = 0; j1 <= J; j1++)
     for (int j2 = 0; j2 <= j1; j2++)
-      for (int j = j1 - j2; j <= std::min(J, j1 + j2); j += 2)
+      for (int j = j1 - j2; j <= std::min(J, j1 + j2); j += 2) {
+        const double delta = delta_cg(fact, j1, j2, j);
         for (int m1 = 0; m1 <= j1; m1++) {
           int aa2 = 2 * m1 - j1;
           for (int m2 = 0; m2 <= j2; m2++, idx++) {
@@ -154,9 +159,10 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
             int cc2 = 2 * m - j;
             long double sf = fact((j1 + aa2) / 2) * fact((j1 - aa2) / 2) * fact((j2 + bb2) / 2) * fact((j2 - bb2) / 2) *
                          fact((j + cc2) / 2) * fact((j - cc2) / 2) * (long double)(j + 1);
-            h.cglist[idx] = sum * delta_cg(j1, j2, j) * std::sqrt((double)sf);
+            h.cglist[idx] = sum * delta * std::sqrt((double)sf);
           }
         }
+      }
 
   // bzero (prebuilt_arrays.jl:52-63); wself = 1
   h.bzero.assign(jd, 0.0);
@@ -216,12 +222,14 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
   for (int q = 0; q < h.u_half; q++) h.y_off[q + 1] += h.y_off[q];
   // Z entries in order of their loop shape, so that the threads of a warp that take
   // consecutive entries run identical (nb, na) trip counts
-  h.zperm.resize(h.idxz_max);
-  for (int z = 0; z < h.idxz_max; z++) h.zperm[z] = z;
-  std::stable_sort(h.zperm.begin(), h.zperm.end(), [&](int a, int b) {
-    const ZDev &p = h.idxz[a], &q = h.idxz[b];
-    return p.nb != q.nb ? p.nb < q.nb : p.na < q.na;
-  });
+  {  // counted into the places of each (nb, na), both at most J + 1
+    std::vector<int> place((jd + 1) * (jd + 1) + 1, 0);
+    auto shape = [&](int z) { return h.idxz[z].nb * (jd + 1) + h.idxz[z].na; };
+    for (int z = 0; z < h.idxz_max; z++) place[shape(z) + 1]++;
+    for (size_t q = 1; q < place.size(); q++) place[q] += place[q - 1];
+    h.zperm.resize(h.idxz_max);
+    for (int z = 0; z < h.idxz_max; z++) h.zperm[place[shape(z)]++] = z;
+  }
   // Y schedule: every half-plane entry with nonzero weight goes to one of YS_WARPS warps,
   // longest first to the least loaded warp (cost = inner terms of its Z entries)
   {
@@ -283,13 +291,14 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
     // the component of each triple and the terms of its derivative (compute_b.jl:104-400) that read it
     h.ytrip_b.assign(h.ytrip_jjz.size(), 0);
     h.ytrip_fac.assign(h.ytrip_jjz.size(), 0.0);
+    std::vector<int32_t> trip_at(h.idxz_max, -1);  // by first Z entry
+    for (size_t q = 0; q < h.ytrip_jjz.size(); q++) trip_at[h.ytrip_jjz[q]] = (int32_t)q;
     for (int b = 0; b < h.idxb_max; b++)
-      for (int t = 0; t < 3; t++)
-        for (size_t q = 0; q < h.ytrip_jjz.size(); q++)
-          if (h.ytrip_jjz[q] == h.db[b].z0[t]) {
-            h.ytrip_b[q] = b | (((h.ytrip_b[q] >> 16) | (1 << t)) << 16);
-            h.ytrip_fac[q] = h.db[b].fac[t];
-          }
+      for (int t = 0; t < 3; t++) {
+        const int q = trip_at[h.db[b].z0[t]];
+        h.ytrip_b[q] = b | (((h.ytrip_b[q] >> 16) | (1 << t)) << 16);
+        h.ytrip_fac[q] = h.db[b].fac[t];
+      }
     h.ylev.assign(J + 2, 0);
     for (int j = 0; j <= J; j++) {
       for (int j1 = 0; j1 <= J; j1++)
@@ -310,11 +319,16 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
       double cost = 0.0;
     };
     std::vector<Item> items;
+    items.reserve(YK_ITEMS);
     for (int k = 0; k <= J; k++) {
       const int cmax = k == 0 ? 0 : J - ((J - k) & 1);
       for (int c0 = -(J - ((J - k) & 1)); c0 <= cmax; c0 += 2 * YT) {
-        Item I;
+        items.emplace_back();
+        Item& I = items.back();
         memset(&I.it, 0, sizeof(I.it));
+        I.recs.reserve(64);
+        I.pairs.reserve(128);
+        I.rows.reserve(128);
         int nt = 0, jmin = J + 1;
         for (int t = 0; t < YT && c0 + 2 * t <= cmax; t++) {
           nt++;
@@ -356,7 +370,6 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
               I.recs.back() |= YF_LAST;
             }
           }
-        items.push_back(std::move(I));
       }
     }
     std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
@@ -385,14 +398,14 @@ int snap_build_tables(const ipg_snap_params& p, SnapHost& h) {
           cgj[q] = h.cglist.data() + h.idxcg_block[blk(R.j1, R.j2, j)];
           cb[q] = cgj[q][R.mb1 * (R.j2 + 1) + R.mb2] * (p.bnorm_flag ? 1.0 / (j + 1) : 1.0);
         }
-        for (int ma1 = R.lo1; ma1 <= R.hi1; ma1++)
-          for (int q = 0; q < R.N; q++)
-            for (int t = 0; t < YT; t++) {
-              const int m2 = R.E + t - ma1, c = I.it.c0 + 2 * t;
-              const bool ok = t < I.it.nt && m2 >= 0 && m2 <= R.j2 && std::abs(c) <= R.jlo + 2 * q;
-              const int sg = R.mir == 1 ? ma1 + R.mb1 : (R.mir == 2 ? m2 + R.mb2 : 0);  // sign of the mirrored element
-              *out++ = ok ? ((sg & 1) ? -cb[q] : cb[q]) * cgj[q][ma1 * (R.j2 + 1) + m2] : 0.0;
-            }
+        for (int ma1 = R.lo1; ma1 <= R.hi1; ma1++, out += R.N * YT)  // zero where an index is out of range
+          for (int t = 0; t < I.it.nt; t++) {
+            const int m2 = R.E + t - ma1, c = std::abs(I.it.c0 + 2 * t);
+            if (m2 < 0 || m2 > R.j2) continue;
+            const int sg = R.mir == 1 ? ma1 + R.mb1 : (R.mir == 2 ? m2 + R.mb2 : 0);  // sign of the mirrored element
+            for (int q = c > R.jlo ? (c - R.jlo) / 2 : 0; q < R.N; q++)
+              out[q * YT + t] = ((sg & 1) ? -cb[q] : cb[q]) * cgj[q][ma1 * (R.j2 + 1) + m2];
+          }
       }
     }
   }
