@@ -382,6 +382,17 @@ static int scan_level(ipg_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, 
   return IPG_OK;
 }
 
+int ipg_raise_smem_limit(ipg_ctx* ctx, const void* kernel, size_t bytes) {
+  static std::mutex m;
+  static std::map<std::pair<int, const void*>, size_t> limit;  // by device and kernel
+  std::lock_guard<std::mutex> lock(m);
+  size_t& now = limit[{ctx->device, kernel}];
+  if (bytes <= now) return IPG_OK;
+  CUDA_RET(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  now = bytes;
+  return IPG_OK;
+}
+
 int ipg_scan_i64(ipg_ctx* ctx, const int64_t* in, int64_t* out, int64_t n_plus_1) {
   if (n_plus_1 <= 0) return IPG_OK;
   return scan_level(ctx, in, out, n_plus_1, 0);

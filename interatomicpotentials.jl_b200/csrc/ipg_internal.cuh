@@ -169,6 +169,15 @@ void ipg_copy_team_free(ipg_ctx* ctx);
     IPG_RET(ipg_timing_mark((ctx), (name), false));                \
   } while (0)
 
+// Raises the dynamic shared memory that a kernel may be launched with to `bytes`.  The limit belongs to
+// the process, not to a context, and is never lowered: another thread may be about to launch the same
+// kernel with more.
+int ipg_raise_smem_limit(ipg_ctx* ctx, const void* kernel, size_t bytes);
+template <class F>
+int ipg_smem_limit(ipg_ctx* ctx, F* kernel, size_t bytes) {
+  return ipg_raise_smem_limit(ctx, reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // Resets the device status word (async) and reads it back after a sync.
 int ipg_status_reset(ipg_ctx* ctx);
 int ipg_status_check(ipg_ctx* ctx, const char* what);

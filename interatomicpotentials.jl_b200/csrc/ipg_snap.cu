@@ -1641,14 +1641,14 @@ int launch_vsum_j(ipg_ctx* ctx, const SnapDev& S, int64_t a0, int64_t nc, const 
   if (!tangent) {
     const size_t sl = (size_t)VS_WARPS * snapchain::UT_SLOTS * 33 * sizeof(double2);
     if (sl > 48 * 1024)
-      CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_vlie<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
+      IPG_RET(ipg_smem_limit(ctx, k_snap_vlie<J>, sl));
     IPG_TIMED_LAUNCH(ctx, "snap_vsum", k_snap_vlie<J>, nblk(nc, VS_WARPS), VS_WARPS * 32, sl, S, a0, nc, off, nbr,
                      rij, species, g, V);
     return IPG_OK;
   }
   const size_t sm = ((size_t)4 * (J + 1) * VS_WARPS * 32 + (size_t)VS_WARPS * snapchain::UT_SLOTS * 33) * sizeof(double2);
   if (sm > 48 * 1024)
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_vsum<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_vsum<J>, sm));
   IPG_TIMED_LAUNCH(ctx, "snap_vsum", k_snap_vsum<J>, nblk(nc, VS_WARPS), VS_WARPS * 32, sm, S, a0, nc, off, nbr, rij,
                    species, g, V);
   return IPG_OK;
@@ -1921,7 +1921,7 @@ int launch_pair_all(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t* d
   const int ystage = with_y <= 113 * 1024 ? PAIR_Y_ATOMS : 0;
   const size_t sm = ystage ? with_y : base;
   if (sm > 48 * 1024)
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_pair_adj_all<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_pair_adj_all<J>, sm));
   IPG_TIMED_LAUNCH(ctx, "snap_pair", k_snap_pair_adj_all<J>, nblk(np, PAIR_ALL_T), PAIR_ALL_T, sm, S, d_np, natoms,
                    owner, nbr, rij, species, Yw, part, ystage);
   return IPG_OK;
@@ -2041,7 +2041,7 @@ int launch_pair_lie_t(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t*
                       const double2* Yw, double* part, int ne) {
   const size_t sm = pair_lie_smem(S.u_half);
   if (sm > 48 * 1024)
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_pair_lie<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_pair_lie<J>, sm));
   IPG_TIMED_LAUNCH(ctx, "snap_pair", k_snap_pair_lie<J>, nblk(np, PAIR_LIE_T), PAIR_LIE_T, sm, S, d_np, natoms * ne,
                    owner, nbr, rij, species, Yw, part, ne);
   return IPG_OK;
@@ -2239,7 +2239,7 @@ int launch_pair_hvp_lie_j(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int6
                           const double* v, const double2* Yw, const double2* Yd, double* fdot) {
   const size_t sm = hvp_lie_smem(J, S.u_half);
   if (sm > 48 * 1024)
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_pair_hvp_lie<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_pair_hvp_lie<J>, sm));
   IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_snap_pair_hvp_lie<J>, nblk(np, HVP_LIE_T), HVP_LIE_T, sm, S, d_np, natoms, owner,
                    nbr, rij, species, v, Yw, Yd, fdot);
   return IPG_OK;
@@ -2254,7 +2254,7 @@ int launch_pair_hvp_j(ipg_ctx* ctx, const SnapDev& S, int64_t np, const int64_t*
   const int ystage = with_y <= 113 * 1024 ? HVP_Y_ATOMS : 0;  // two blocks per SM still fit
   const size_t sm = ystage ? with_y : base;
   if (sm > 48 * 1024)
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_pair_hvp<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_pair_hvp<J>, sm));
   const dim3 grid((unsigned)nblk(np, HVP_T), 3);
   IPG_TIMED_LAUNCH(ctx, "snap_hvp", k_snap_pair_hvp<J>, grid, HVP_T, sm, S, d_np, natoms, owner, nbr, rij, species,
                    v, Yw, Yd, fdot, ystage);
@@ -2763,7 +2763,7 @@ int launch_atoms(ipg_snap* s, const SnapDev& dev, const SnapIO& io, int64_t nato
   size_t smem = L.total;
   if (smem > 227 * 1024)
     return ipg_fail(ctx, IPG_ERR_UNSUPPORTED, "twojmax %d needs %zu bytes of shared memory per block", dev.J, smem);
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_atom<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  IPG_RET(ipg_smem_limit(ctx, k_snap_atom<MODE>, smem));
   int per_sm = s->blocks_per_sm;
   if (per_sm <= 0) {
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_atom<MODE>, threads, smem));
@@ -2908,7 +2908,7 @@ int plain_chains(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
   double2* Z;
   IPG_RET(scratch(ctx, "snap_Z", (size_t)C * dev.idxz_max + 1, &Z));
   const int bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)dev.K * YS_ATOMS * 8);
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
+  IPG_RET(ipg_smem_limit(ctx, k_snap_bdesc, bsm));
   int bper = 1;
   CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bper, k_snap_bdesc, GB_WARPS * 32, bsm));
   for (int64_t a0 = 0; a0 < n; a0 += C) {
@@ -2938,7 +2938,7 @@ int launch_y(ipg_snap* s, const SnapDev& dev, const char* tname, int64_t n, cons
     IPG_RET(launch_ystream(ctx, dev, s->h.yktab, zall ? YM_YZ : YM_Y, tname, n, d_species, utot, yout, Ei, zall));
     if (zall && zall_done) *zall_done = true;
   } else {
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_yatoms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ysm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_yatoms, ysm));
     int per_sm = 1;
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_yatoms, YS_WARPS * 32, ysm));
     const int64_t groups = (n + YS_ATOMS - 1) / YS_ATOMS;
@@ -2975,7 +2975,7 @@ int chem_adjoint(ipg_snap* s, const SnapDev& dev, int64_t n, const PairList& pl,
   if (dev.quadratic) {
     IPG_RET(scratch(ctx, "chem_B", (size_t)n * dev.klin + 1, &B));
     bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)dev.klin * YS_ATOMS * 8);
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_bdesc, bsm));
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bper, k_snap_bdesc, GB_WARPS * 32, bsm));
   }
   for (int64_t a0 = 0; a0 < n; a0 += C) {
@@ -3057,7 +3057,7 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     if (CL.total > 227 * 1024)
       return ipg_fail(ctx, IPG_ERR_UNSUPPORTED, "chem/quadratic SNAP needs %zu bytes of shared memory", CL.total);
     const void* kfn = plain ? (const void*)k_snap_chem<true> : (const void*)k_snap_chem<false>;
-    CUDA_RET(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CL.total));
+    IPG_RET(ipg_smem_limit(ctx, kfn, CL.total));
     int per_sm = 1;
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, 128, CL.total));
     const int64_t grid = std::min<int64_t>(std::max<int64_t>(n, 1), (int64_t)ctx->num_sms * std::max(1, per_sm));
@@ -3132,7 +3132,7 @@ int snap_eval(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_spec
     double2* Z;
     IPG_RET(scratch(ctx, "snap_Z", (size_t)C * dev.idxz_max + 1, &Z));
     const int bsm = (int)((size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)K * YS_ATOMS * 8);
-    CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_bdesc, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
+    IPG_RET(ipg_smem_limit(ctx, k_snap_bdesc, bsm));
     int bper = 1;
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bper, k_snap_bdesc, GB_WARPS * 32, bsm));
     for (int64_t a0 = 0; a0 < n; a0 += C) {
@@ -3776,7 +3776,7 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
     const bool withB = gE != 0.0;
     const int gsm = (int)((withB ? 2 : 1) * (size_t)dev.u_half * YS_ATOMS * sizeof(double2) + (size_t)nsp * K * 8);
     const auto gbeta = withB ? k_snap_gbeta<true> : k_snap_gbeta<false>;
-    CUDA_RET(ctx, cudaFuncSetAttribute(gbeta, cudaFuncAttributeMaxDynamicSharedMemorySize, gsm));
+    IPG_RET(ipg_smem_limit(ctx, gbeta, gsm));
     CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gper, gbeta, GB_WARPS * 32, gsm));
     const int64_t gmax = (int64_t)ctx->num_sms * std::max(1, gper);
     double* gpart;
@@ -3801,7 +3801,7 @@ int snap_vjp_device(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* 
   int threads = s->threads;
   SmemLayout L = smem_layout(dev, threads / 32, MODE_VJP, true);
   int per_sm = 1;
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_atom<MODE_VJP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total));
+  IPG_RET(ipg_smem_limit(ctx, k_snap_atom<MODE_VJP>, L.total));
   CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_atom<MODE_VJP>, threads, L.total));
   int64_t grid = std::min<int64_t>(std::max<int64_t>(n, 1), (int64_t)ctx->num_sms * std::max(1, per_sm));
   double* gpart;
@@ -3941,7 +3941,7 @@ int ipg_snap_vjp(ipg_snap* s, int64_t n, const double* pos, const int32_t* speci
       io.species = d_sp;
       io.fvec = fv;
       io.status = ctx->d_status;
-      CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_hvp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HL.total));
+      IPG_RET(ipg_smem_limit(ctx, k_snap_hvp, HL.total));
       int per_sm = 1;
       CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_snap_hvp, nw * 32, HL.total));
       const int64_t grid = std::min<int64_t>(n, (int64_t)ctx->num_sms * std::max(1, per_sm));

@@ -299,7 +299,7 @@ int launch_db_j(ipg_ctx* ctx, const SnapDev& S, int64_t b0, int64_t b1, const Pa
                 int64_t a0, int64_t zs, const double2* Z, double* dbl, double* fvec) {
   if (plaintab::nb_of(J) != S.K) return ipg_fail(ctx, IPG_ERR_UNSUPPORTED, "plain chain tables disagree");
   const int sm = (int)((2 * (J + 1) * DB_ROW + (size_t)S.idxz_max) * sizeof(double2));
-  CUDA_RET(ctx, cudaFuncSetAttribute(k_snap_db<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  IPG_RET(ipg_smem_limit(ctx, k_snap_db<J>, sm));
   IPG_TIMED_LAUNCH(ctx, "snap_dbfused", k_snap_db<J>, (unsigned)(b1 - b0), DB_T, sm, S, b0, pl.d_off, pl.d_j, pl.d_r,
                    species, a0, zs, Z, dbl, fvec);
   return IPG_OK;

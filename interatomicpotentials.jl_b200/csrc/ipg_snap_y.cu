@@ -413,7 +413,7 @@ int launch_ystream_m(ipg_ctx* ctx, const SnapDev& dev, const YkTab& tab, const c
   constexpr int warps = yk_warps(PL), YK_T = warps * 32;
   const auto kernel = k_snap_ystream<YM, PL>;
   const int smem = yk_smem(dev.nsp, dev.n_ytrip, dev.u_half, tab.nitem, PL).total();
-  CUDA_RET(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  IPG_RET(ipg_smem_limit(ctx, kernel, smem));
   int per_sm = 1;
   CUDA_RET(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, YK_T, smem));
   const int64_t resident = (int64_t)ctx->num_sms * std::max(1, per_sm);
