@@ -57,6 +57,14 @@ int ipg_scratch(ipg_ctx* ctx, const char* name, size_t bytes, void** out) {
   return IPG_OK;
 }
 
+void ipg_scratch_free(ipg_ctx* ctx, const std::string& prefix) {
+  for (auto it = ctx->bufs.lower_bound(prefix); it != ctx->bufs.end() && it->first.compare(0, prefix.size(), prefix) == 0;) {
+    if (it->second.p) cudaFree(it->second.p);
+    it = ctx->bufs.erase(it);
+  }
+  ctx->walk_kcap.erase(prefix);
+}
+
 int ipg_status_reset(ipg_ctx* ctx) {
   CUDA_RET(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
   return IPG_OK;

@@ -47,6 +47,7 @@ struct ipg_ctx {
   // differs refers to freed buffers and is discarded.
   bool capturing = false;
   uint64_t scratch_gen = 0;
+  uint64_t handles = 0;  // SNAP handles created so far
   bool walk_by_cell = true;  // neighbor walk: one warp per cell (false: one warp per atom)
   bool chain_constants = false;  // the constant tables of the SNAP register chains are uploaded
   bool pair_full_stencil = false;  // pair potentials: full-stencil walk even where the half stencil applies
@@ -127,6 +128,8 @@ int ipg_cuda_check(ipg_ctx* ctx, cudaError_t e, const char* what);
 
 // Named device scratch: grows (never shrinks) to at least `bytes`.
 int ipg_scratch(ipg_ctx* ctx, const char* name, size_t bytes, void** out);
+// Frees the device scratch whose name starts with `prefix` (nothing may be using it).
+void ipg_scratch_free(ipg_ctx* ctx, const std::string& prefix);
 template <class T>
 int scratch(ipg_ctx* ctx, const char* name, size_t count, T** out) {
   void* p = nullptr;

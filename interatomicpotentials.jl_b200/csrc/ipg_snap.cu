@@ -2579,6 +2579,7 @@ __global__ void k_loss_grad(int64_t n, const double* __restrict__ F, const doubl
 // ---------------------------------------------------------------------------------
 struct ipg_snap {
   ipg_ctx* ctx = nullptr;
+  uint64_t id = 0;  // of the handles of its context
   ipg_snap_params p;
   SnapHost h;
   SnapDev dev;
@@ -2634,7 +2635,7 @@ struct ipg_snap {
     int nconf = 0;
     std::vector<int64_t> off;
     std::vector<double> L;
-    CellList cl;      // buffers under the "skin_" prefix
+    CellList cl;      // buffers under skin_prefix, this handle's own
     PairList pairs;   // the list with enlarged cutoffs
     double* ref = nullptr;     // positions at the build
     int32_t* ref_sp = nullptr;  // species at the build (a change rebuilds the list)
@@ -2809,6 +2810,9 @@ int set_beta(ipg_snap* s, const double* beta, double beta0, SnapDev& dev) {
 int snap_neighbors_inner(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_species, int nconf,
                          const int64_t* h_atom_off, const double* h_L, PairList& pl, int64_t cap);
 
+// Scratch of a list that outlives the call: other handles of the context have theirs.
+std::string skin_prefix(const ipg_snap* s) { return "skin" + std::to_string(s->id) + "_"; }
+
 // Neighbor build for a set of configurations (device positions); cap > 0: capacity mode.
 int snap_neighbors(ipg_snap* s, int64_t n, const double* d_pos, const int32_t* d_species, int nconf,
                    const int64_t* h_atom_off, const double* h_L, PairList& pl, int64_t cap = 0) {
@@ -2840,12 +2844,14 @@ int snap_neighbors_inner(ipg_snap* s, int64_t n, const double* d_pos, const int3
         const double r = std::sqrt(s->cutsq[q]) + s->skin;
         cut2[q] = r * r;
       }
-      IPG_RET(ipg_build_cells(s->ctx, "skin_", n, d_pos, d_species, nsp, nconf, h_atom_off, h_L,
+      C.valid = false;  // the build overwrites its buffers
+      const std::string pre = skin_prefix(s);
+      IPG_RET(ipg_build_cells(s->ctx, pre.c_str(), n, d_pos, d_species, nsp, nconf, h_atom_off, h_L,
                               s->radius + s->skin, C.cl));
-      IPG_RET(ipg_build_pairs(s->ctx, "skin_", C.cl, d_species, nsp, cut2.data(), IPG_NLIST_FULL, false, C.pairs,
+      IPG_RET(ipg_build_pairs(s->ctx, pre.c_str(), C.cl, d_species, nsp, cut2.data(), IPG_NLIST_FULL, false, C.pairs,
                               false, 0, s->walk_warps));
-      IPG_RET(scratch(s->ctx, "skin_ref", 3 * (size_t)n, &C.ref));
-      IPG_RET(scratch(s->ctx, "skin_ref_sp", (size_t)n, &C.ref_sp));
+      IPG_RET(scratch(s->ctx, (pre + "ref").c_str(), 3 * (size_t)n, &C.ref));
+      IPG_RET(scratch(s->ctx, (pre + "ref_sp").c_str(), (size_t)n, &C.ref_sp));
       CUDA_RET(s->ctx, cudaMemcpyAsync(C.ref, d_pos, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
                                        s->ctx->stream));
       CUDA_RET(s->ctx, cudaMemcpyAsync(C.ref_sp, d_species, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice,
@@ -3474,6 +3480,7 @@ int ipg_snap_create(ipg_ctx* ctx, const ipg_snap_params* params, ipg_snap** out)
   CUDA_RET(ctx, cudaSetDevice(ctx->device));
   ipg_snap* s = new ipg_snap();
   s->ctx = ctx;
+  s->id = ctx->handles++;
   s->p = p;
   if (snap_build_tables(p, s->h) != IPG_OK) {
     delete s;
@@ -3532,6 +3539,7 @@ int ipg_snap_destroy(ipg_snap* s) {
   for (auto& g : s->graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
   if (s->d_tables) cudaFree(s->d_tables);
+  ipg_scratch_free(s->ctx, skin_prefix(s));
   delete s;
   return IPG_OK;
 }
