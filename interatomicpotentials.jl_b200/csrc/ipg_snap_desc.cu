@@ -11,6 +11,27 @@ constexpr int DG_T = 192;     // threads over the columns (component, direction)
 constexpr int DG_PAIRS = 64;  // pairs staged at a time
 constexpr int DG_V = 7;       // partial sums per (species, component): W (6) and B
 
+// Sum of dbl over the pairs that end at an atom, have no reverse and an owner of species s (out of line: the
+// gather's registers).
+__device__ __noinline__ double one_sided_db(int64_t one, const int64_t* __restrict__ rev,
+                                            const int64_t* __restrict__ off, int64_t n,
+                                            const int32_t* __restrict__ species, int nsp, int s,
+                                            const double* __restrict__ dbl, int C) {
+  double sum = 0.0;
+  for_one_sided(one, rev, [&](int64_t q) {
+    int64_t lo = 0, hi = n - 1;  // the owner: the last atom whose pairs start at or before q
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) / 2;
+      if (off[mid] <= q) lo = mid;
+      else hi = mid - 1;
+    }
+    int so = species[lo];
+    so = so < 0 ? 0 : (so >= nsp ? nsp - 1 : so);
+    if (so == s) sum += dbl[(size_t)q * C];
+  });
+  return sum;
+}
+
 // One block takes one of nchunk chunks of atoms, each of one configuration, and DG_T columns t = 3 b + c
 // of dB/dr, dbl [pair][K][3] (chunk + nchunk x tile of columns in blockIdx.x: neither has a limit of its own):
 //   dB_k[block s][b][c] = sum over k's pairs, s_k = s, of dbl_p - sum over their reverses and the pairs
@@ -51,6 +72,7 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
 #pragma unroll
     for (int s = 0; s < NSP; s++) acc[s] = 0.0;
     const double bi = B && act && c == 0 ? B[(size_t)i * K + b] : 0.0;
+    const int64_t first = dB ? one[i] : 0;
     double own = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
     for (int64_t p0 = off[i], p1 = dbl ? off[i + 1] : p0; p0 < p1; p0 += DG_PAIRS) {
       const int m = (int)(p1 - p0 < DG_PAIRS ? p1 - p0 : DG_PAIRS);
@@ -107,20 +129,10 @@ __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict_
         }
       }
     }
-    const int64_t first = one[i];
-    for_one_sided(first, rev, [&](int64_t q) {
-      int64_t lo = 0, hi = n - 1;  // the owner: the last atom whose pairs start at or before q
-      while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) / 2;
-        if (off[mid] <= q) lo = mid;
-        else hi = mid - 1;
-      }
-      int so = species[lo];
-      so = so < 0 ? 0 : (so >= nsp ? nsp - 1 : so);
-      const double v = act ? dbl[(size_t)q * C + col] : 0.0;
+    if (first && act) {  // rare
 #pragma unroll
-      for (int s = 0; s < NSP; s++) acc[s] -= NSP == 1 || so == s ? v : 0.0;
-    });
+      for (int s = 0; s < NSP; s++) acc[s] -= one_sided_db(first, rev, off, n, species, nsp, s, dbl + col, C);
+    }
     if (act) {
 #pragma unroll
       for (int s = 0; s < NSP; s++)
