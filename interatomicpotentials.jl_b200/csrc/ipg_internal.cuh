@@ -229,8 +229,8 @@ struct ConfGrid {
   double lo[3];  // grid origin
   double cs[3];  // cell edge (>= search radius on every axis with more than one cell)
   int nc[3];     // cells per axis
-  int pad;
-  double rel;    // unit of CellList::d_srel: the power of two that takes the longest cell edge into [1, 2)
+  float edge[3]; // the cell edge in units of CellList::d_srel
+  double rel;    // the power of two that takes the longest cell edge into [1, 2): unit of CellList::d_srel
   int64_t cell_off;  // first global cell id of this configuration
   int64_t atom_off;
   int64_t natoms;

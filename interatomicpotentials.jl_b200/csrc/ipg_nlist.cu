@@ -497,7 +497,7 @@ __device__ __forceinline__ void walk_stencil(const ConfGrid& g, const int* cc, c
       }
       int d = c[a] - cc[a];  // in -1..1 but for the wrap
       d = d > 1 ? d - g.nc[a] : (d < -1 ? d + g.nc[a] : d);
-      s[a] = (float)(d * g.cs[a] * g.rel);
+      s[a] = d * g.edge[a];
     }
     const int64_t cell = g.cell_off + ((int64_t)c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0];
     beg = (int)cell_start[cell];
@@ -852,6 +852,7 @@ int ipg_build_cells(ipg_ctx* ctx, const char* prefix, int64_t n, const double* d
     for (int a = 0; a < 3; a++) g.cs[a] = e3[a] > 0.0 ? e3[a] / g.nc[a] : 1.0;
     const int e2 = std::ilogb(std::max(g.cs[0], std::max(g.cs[1], g.cs[2])));
     g.rel = std::ldexp(1.0, -std::max(-1000, std::min(1000, e2)));
+    for (int a = 0; a < 3; a++) g.edge[a] = (float)(g.cs[a] * g.rel);
     g.cell_off = cell_total;
     cell_total += tot;
   }

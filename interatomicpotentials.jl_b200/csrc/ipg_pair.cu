@@ -206,7 +206,9 @@ __device__ __forceinline__ void pbuf_put(double* __restrict__ P, int64_t n, int 
   }
 }
 
-// Bound by FP64 issue and latency of the term code.  Full 64-bit tests of every candidate, rows
+// Bound by issue slots (61% at a million atoms, the FP64 pipe 25%, DRAM 2%) and the latency of dependent
+// instructions (2.9 cycles an issue waiting); at 32,000 atoms also by the wait for the last warps (issue 50%
+// of the active cycles).  Full 64-bit tests of every candidate, rows
 // loaded one by one and a hand-off between two warp barriers a row took 35.8 ms a call at 4.1 M atoms
 // with five terms; 32-bit tests and masked hand-offs 17.7 ms; warp-uniform control flow in
 // half_eval (terms, cutoffs, distances, hand-off: lane-wise branches cost reconvergence around
@@ -251,7 +253,7 @@ __global__ void __launch_bounds__(PAIR_T, PAIR_MINB) k_pair_half(const __grid_co
     const int a0 = (int)cell_start[A], a1 = (int)cell_start[A + 1], t0 = (int)cell_start[T],
               t1 = (int)cell_start[T + 1];
     // the target cell's corner relative to the home cell's, at the image these two cells define
-    const float sx = (float)(dx * g.cs[0] * g.rel), sy = (float)(dy * g.cs[1] * g.rel), sz = (float)(dz * g.cs[2] * g.rel);
+    const float sx = dx * g.edge[0], sy = dy * g.edge[1], sz = dz * g.edge[2];
     const int home_kind = k, tgt_kind = k == 0 ? 0 : HALF_OFFSETS - 1 + k;
     // cells of at most 32 atoms are one tile and its sums are stored; larger cells take
     // several tiles, whose sums accumulate into zeroed slots, as do the row and column sums
