@@ -51,10 +51,14 @@ KERNEL_NAMES = {"snap_atom": "k_snap_ystream", "snap_utot": "k_snap_utot_all<8>"
 # DRAM bytes (read + write) per atom of one launch, from the ncu --set full captures on the
 # 16,000-atom case summarised in profiles/k_snap_{ystream,pair_lie,pair_adj_all,utot_all}_snap_j8.md;
 # scaled by atoms (pairs per atom are the same).
-NCU_DRAM_BYTES_PER_ATOM = {"snap_atom": (52.707584e6 + 2.899200e6) / 16000,
+NCU_DRAM_BYTES_PER_ATOM = {"snap_atom": (52.268544e6 + 2.836736e6) / 16000,
                            "snap_pair": ((52.742144e6 + 0.953088e6) if PAIR_KERNEL == "tangent"
                                          else (50.157056e6 + 0.847360e6)) / 16000,
                            "snap_utot": (11.558912e6 + 16.316928e6) / 16000}
+# what the roofline's operations count where it is not what the kernel executes
+FLOPS_SOURCE = {"snap_atom": "the reference's loops, entry by entry; the kernel forms each product once for every "
+                             "level, and its FP64 pipe is active 42% of the cycles (ncu, 16,000 atoms: "
+                             "profiles/k_snap_ystream_snap_j8.md)"}
 
 
 def _hbm_peak():
@@ -355,6 +359,7 @@ def main():
                 "peak": fp64_peak, "unit": "TFLOP/s", "frac": per_kernel[dom]["frac"] if dom else None,
                 "traffic": traffic, "kernel": KERNEL_NAMES.get(dom), "flops_per_launch": kflops.get(dom),
                 "avg_launch_ms": per_kernel[dom]["avg_launch_ms"] if dom else None,
+                "flops_source": FLOPS_SOURCE.get(dom, "along the kernel's own loops"),
                 "peak_source": "measured DFMA probe (libipg_probe.so) in this run; the HBM peak of "
                                "MEASURED_PEAKS.json does not bound these FP64-pipe kernels",
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on the "
@@ -538,10 +543,11 @@ def main():
                 pair[name]["hbm"] = {"algorithmic_bytes": nbytes, "kernel_ms": k_ms, "achieved_GBps": gbps,
                                      "peak_GBps": HBM_PEAK, "frac": gbps / HBM_PEAK if gbps else None,
                                      "peak_source": "MEASURED_PEAKS.json hbm_gbs"}
-                # what bounds it instead: the ncu counters of k_pair_half on the 32,000-atom
-                # case of the same lattice (profiles/k_pair_half_lc_1m.md)
-                pair[name]["ncu_pipes"] = {"kernel": "k_pair_half", "fp64_pipe_pct": 13.3, "issue_active_pct": 42.9,
-                                           "dram_pct_of_peak": 0.1, "bound": "FP64 latency (wait stalls)",
+                # what bounds it instead: the ncu counters of k_pair_half on 1,048,576 atoms of the
+                # same lattice (profiles/k_pair_half_lc_1m.md)
+                pair[name]["ncu_pipes"] = {"kernel": "k_pair_half", "n_atoms": 1048576, "fp64_pipe_pct": 24.6,
+                                           "issue_active_pct": 60.9, "dram_pct_of_peak": 2.4,
+                                           "bound": "issue slots and the latency of dependent instructions",
                                            "source": "profiles/k_pair_half_lc_1m.md"}
         line["lj_pairs_per_s"] = pair
 

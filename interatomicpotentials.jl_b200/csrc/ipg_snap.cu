@@ -2363,7 +2363,8 @@ __device__ __noinline__ double3 one_sided_sum(int64_t one, const int64_t* __rest
 // summed by a fixed tree.  Eight lanes: about 25 pairs leave three or four loads of each kind per
 // lane in flight, and four atoms still share a warp, so full systems stay coalesced.  ONE: one
 // share per pair, whose loads then overlap.  One thread per atom over separate lists took 42 us at
-// 249 and 55 at 54,000 atoms (twojmax 8), eight lanes 13 and 47, eight lanes over the reverses 8 and 32.
+// 249 and 55 at 54,000 atoms (twojmax 8), eight lanes 13 and 47, eight lanes over the reverses 8 and 32,
+// with the pairs that have none 9 and 34.
 constexpr int GATHER_LANES = 8;
 template <bool ONE>
 __global__ void __launch_bounds__(128) k_snap_gather(int64_t n, const int64_t* __restrict__ off,

@@ -41,8 +41,8 @@ __device__ __noinline__ double one_sided_db(int64_t one, const int64_t* __restri
 // Bound by the reads of dbl: each pair's K x 3 numbers twice (once for its owner, once for its
 // neighbor), in rows of 3 K consecutive doubles; W rides on the owner's read.  An atom's pairs are
 // staged in shared memory, so the column threads read nothing else.  8,192 atoms, twojmax 8, two
-// species: 181 us (plus 25 us of k_desc_reduce) for what a kernel per output did in 570 us; 48
-// configurations of at most 250 atoms, twojmax 6: 127 (plus 5) against 2,096 us, nearly all of it
+// species: 155 us (plus 26 us of k_desc_reduce) for what a kernel per output did in 570 us; 48
+// configurations of at most 250 atoms, twojmax 6: 108 (plus 5) against 2,096 us, nearly all of it
 // in a kernel that walked each configuration serially.
 template <int NSP>
 __global__ void __launch_bounds__(DG_T) k_desc_gather(const int64_t* __restrict__ chunks, int nchunk, int K, int nsp,

@@ -22,13 +22,13 @@
 // are walked backwards, the conjugate taken by an integer flip of the sign bit and the signs kept
 // in the weights, so that one step loop per number of levels serves them all: the code of a
 // variant per mirror case and four steps at a time no longer fitted the instruction cache (the
-// warps of a block run different items) and took 2.5 ms where this takes 1.43 ms; four columns
+// warps of a block run different items) and took 2.5 ms where this takes 1.36 ms; four columns
 // per item, half the warps, 3.9 ms.
 //
-// Bound: issue slots (59%; 40% of them FP64, the shared-memory pipe 67% busy) and the latency of
-// shared-memory loads at 16 warps per SM.  Against the kernel that formed one row of entries at a
-// time, twojmax 8: Y 1.73 -> 1.43 ms at 54,000 atoms; Y 0.60 -> 0.47 ms, Y and Z 0.69 -> 0.58 ms
-// at 16,000.
+// Bound: issue slots (57% of the active cycles, the FP64 pipe 42%, shared-memory wavefronts 58% of
+// their peak; Y at 16,000 atoms) and the latency of shared-memory loads at 16 warps per SM.  Against
+// the kernel that formed one row of entries at a time, twojmax 8: Y 1.73 -> 1.36 ms at 54,000 atoms;
+// Y 0.60 -> 0.47 ms, Y and Z 0.69 -> 0.58 ms at 16,000.
 #include <algorithm>
 
 #include "ipg_snap.cuh"
